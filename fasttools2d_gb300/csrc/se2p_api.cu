@@ -54,6 +54,8 @@ enum Slot {
     S_PROBE,                                    // the atomic-rate probe's array
     S_MGRID, S_MGMAX, S_MUK, S_MZM,             // k space of several right-hand sides
     S_GORDER, S_GPCNT, S_GPSTART,               // patch-major target order of the gather
+    // tensor-core k space: factor records, tiles and items of the points spread
+    S_TCFAC, S_TCTILE, S_TCCNT, S_TCSTART, S_TCLIST, S_TCLTMP, S_TCITEMS,
     S_COUNT_SLOTS
 };
 
@@ -96,6 +98,8 @@ struct se2p_plan_st {
     int tw_len[2] = {0, 0};
     const void *tw_dev[2] = {nullptr, nullptr};
     std::vector<float4> tw_host[2];
+    // set by a tensor-core kernel whose wait ran out (mapped host memory)
+    int *tc_err = nullptr, *tc_err_dev = nullptr;
     // pending (start, end) event pairs per stage, resolved by se2p_plan_stage_times
     std::vector<std::pair<cudaEvent_t, cudaEvent_t>> pending[T_NUM_STAGES];
     double stage_ms[T_NUM_STAGES] = {0};
@@ -586,10 +590,106 @@ static int gather_fixed_bits(const SpreadArgs &sa)
     return std::min(62, 64 - e);
 }
 
+// A tensor-core kernel of an earlier call gave up waiting: its results are void.
+static int tc_check(se2p_plan pl)
+{
+    volatile int *e = pl->tc_err;
+    if (!*e) return SE2P_OK;
+    *e = 0;
+    return fail(pl, SE2P_ERR_CUDA, "a tensor-core kernel ran out of time waiting for its operands");
+}
+
+// Points in tiles for the tensor-core spread.
+struct TcSet {
+    TcPointArgs pa{};
+    int *list = nullptr, *nitems = nullptr;
+    int4 *items = nullptr;
+    unsigned long long s = 0;            // exp(-2 alpha) 2^64
+};
+
+// Whether the tensor-core spread runs.  It can for w = h P/2, where both axes'
+// factors are at most 1 (its weights are formed for that), grids of at least a
+// patch and stencils that leave a tile.  It costs about 24 ns per item and pair of
+// grids, an item holding at most a tile's sources; k_spread_fix about 0.1 ms and
+// 1.1 ns per source and grid: with few sources per tile the latter wins (2^16
+// sources, SLP: 0.59 against 0.25 ms on 2688^2 nodes, 0.20 against 0.23 ms on
+// 1344^2, 0.12 against 0.23 ms on 512^2; 1000 sources: 0.06 against 0.16 ms).
+static bool tc_ok(const SpreadArgs &sa, int nc)
+{
+    if (sa.P < 4 || sa.P > kTcMaxP || sa.Mx < kTcX || sa.My < kTcY ||
+        !(std::fabs(sa.w - sa.h * sa.P / 2) <= 1e-14 * sa.w))
+        return false;
+    const double ntile = std::ceil((double)sa.Mx / (kTcX - sa.P)) * std::ceil((double)sa.My / (kTcY - sa.P));
+    return 24.0 * ((nc + 1) / 2) * std::min(ntile, (double)sa.ns) <= 1e5 + 1.1 * nc * (double)sa.ns;
+}
+
+static int tc_sources(se2p_plan pl, const SpreadArgs &sa, cudaStream_t ks, TcSet &t)
+{
+    TcPointArgs &pa = t.pa;
+    pa.p = sa.sp;
+    pa.n = sa.ns;
+    pa.Lhx = sa.Lhx;
+    pa.Lhy = sa.Lhy;
+    pa.h = sa.h;
+    pa.inv_h = 1.0 / sa.h;
+    const double alpha = -sa.a * sa.h * sa.h;
+    pa.al2 = (unsigned long long)std::llround(std::ldexp(alpha * 1.4426950408889634074, 59));
+    t.s = (unsigned long long)std::llround(std::ldexp(std::exp(-2.0 * alpha), 62)) << 2;
+    pa.Mx = sa.Mx;
+    pa.My = sa.My;
+    pa.P = sa.P;
+    pa.Tx = kTcX - sa.P;
+    pa.Ty = kTcY - sa.P;
+    pa.ntx = (sa.Mx + pa.Tx - 1) / pa.Tx;
+    pa.nty = (sa.My + pa.Ty - 1) / pa.Ty;
+    const int ntile = pa.ntx * pa.nty;
+    const size_t n = (size_t)(sa.ns > 0 ? sa.ns : 1);
+    // small sets: smaller items, so that every SM has one
+    const int kmax = std::min(kTcK, std::max(32, (int)((sa.ns + 2 * sm_count() - 1) / (2 * sm_count()) + 15) / 16 * 16));
+    char *fac = nullptr;
+    int *start = nullptr, *ltmp = nullptr;
+    CKS(ensure_t(pl, S_TCFAC, n * kTcPointBytes, &fac));
+    CKS(ensure_t(pl, S_TCTILE, n, &pa.tile));
+    CKS(ensure_t(pl, S_TCCNT, (size_t)ntile, &pa.count));
+    CKS(ensure_t(pl, S_TCSTART, 2 * (size_t)ntile + 2, &start));
+    CKS(ensure_t(pl, S_TCLIST, n, &t.list));
+    CKS(ensure_t(pl, S_TCLTMP, 2 * n, &ltmp));
+    CKS(ensure_t(pl, S_TCITEMS, std::min(n, (size_t)ntile) + n / kmax + 1, &t.items));
+    pa.fac = fac;
+    int *istart = start + ntile + 1;
+    t.nitems = istart + ntile;
+    CK(launch_tc_points(pa, kmax, sa.perm, start, istart, t.list, ltmp, t.items, t.nitems, sa.bound, ks,
+                        pl->launches));
+    return SE2P_OK;
+}
+
+static int tc_spread(se2p_plan pl, const SpreadArgs &sa, const TcSet &t, int nc, cudaStream_t ks)
+{
+    TcSpreadArgs ta{};
+    ta.fac = t.pa.fac;
+    ta.list = t.list;
+    ta.items = t.items;
+    ta.nitems = t.nitems;
+    ta.coef = sa.coef;
+    ta.grid = reinterpret_cast<long long *>(sa.grid);
+    ta.Mx = sa.Mx;
+    ta.My = sa.My;
+    ta.P = sa.P;
+    ta.Tx = t.pa.Tx;
+    ta.Ty = t.pa.Ty;
+    ta.nty = t.pa.nty;
+    ta.s = t.s;
+    ta.bound = sa.bound;
+    ta.err = pl->tc_err_dev;
+    CK(launch_spread_tc(ta, nc, ks, pl->launches));
+    return SE2P_OK;
+}
+
 // Runs the spread of nc components of sa.coef into sa.grid.  With *fixb set
-// on return, the grid holds k_spread_fix's integers or (when the bound slot
-// *fixb is all ones: crowded sources) the FP64 spread's doubles, and the pack
-// of fft_fwd_1d reads which; with *fixb null it holds doubles.
+// on return, the grid holds the integers of the tensor-core spread or of
+// k_spread_fix, or (when the bound slot *fixb is all ones: crowded sources)
+// the FP64 spread's doubles, and the pack of fft_fwd_1d reads which; with
+// *fixb null it holds doubles.
 static int spread(se2p_plan pl, SpreadArgs &sa, int nc, bool allow_fixed, cudaStream_t ks,
                   const unsigned long long **fixb)
 {
@@ -603,7 +703,13 @@ static int spread(se2p_plan pl, SpreadArgs &sa, int nc, bool allow_fixed, cudaSt
         sa.bound = reinterpret_cast<const unsigned long long *>(
             ws + spread_bound_slot(sa.Mx, sa.My, sa.P));
         CK(launch_spread_bound(sa, nc, kfac, mult, ws, ks, pl->launches));
-        CK(launch_spread_fix(sa, nc, kY, ks, pl->launches));
+        if (tc_ok(sa, nc)) {
+            TcSet t;
+            CKS(tc_sources(pl, sa, ks, t));
+            CKS(tc_spread(pl, sa, t, nc, ks));
+        } else {
+            CK(launch_spread_fix(sa, nc, kY, ks, pl->launches));
+        }
         *fixb = sa.bound;
     }
     CK(launch_spread(sa, nc, ks, pl->launches));
@@ -728,6 +834,7 @@ static int fft_inv_1d(se2p_plan pl, cudaStream_t ks, int Mx, int My, cufftDouble
 int run(se2p_plan pl, const Job &J, const Io &io)
 {
     DeviceGuard guard(pl->device);
+    CKS(tc_check(pl));
     cudaStream_t st = pl->stream;
     bool host_io = false;
     const int64_t ns = io.ns, nt = io.nt;
@@ -1015,6 +1122,7 @@ int run(se2p_plan pl, const Job &J, const Io &io)
         sa.w = J.w;
         sa.a = -2 * J.xi * J.xi / J.eta;
         sa.e1 = e1;
+        sa.perm = sperm;
         const unsigned long long *fixb = nullptr;
         {
             StageTimer tm(pl, T_SPREAD, ks);
@@ -1146,8 +1254,12 @@ int run(se2p_plan pl, const Job &J, const Io &io)
     CKS(finish_out(pl, o_uks));
     CKS(finish_out(pl, o_ukd));
     delete t_out;
-    if (host_io) CK(cudaStreamSynchronize(st));
-    else CK(cudaGetLastError());
+    if (host_io) {
+        CK(cudaStreamSynchronize(st));
+        CKS(tc_check(pl));
+    } else {
+        CK(cudaGetLastError());
+    }
     return SE2P_OK;
 }
 
@@ -1165,6 +1277,7 @@ struct AdjIo {
 int run_adjoint(se2p_plan pl, const Job &J, const AdjIo &io)
 {
     DeviceGuard guard(pl->device);
+    CKS(tc_check(pl));
     cudaStream_t st = pl->stream;
     bool host_io = false;
     const int64_t ns = io.ns, nt = io.nt;
@@ -1321,6 +1434,7 @@ int run_adjoint(se2p_plan pl, const Job &J, const AdjIo &io)
     sa.w = J.w;
     sa.a = -2 * J.xi * J.xi / J.eta;
     sa.e1 = e1;
+    sa.perm = tperm;
     const unsigned long long *fixb = nullptr;
     {
         StageTimer tm(pl, T_SPREAD, ks);
@@ -1409,8 +1523,12 @@ int run_adjoint(se2p_plan pl, const Job &J, const AdjIo &io)
     CKS(finish_out(pl, o_fs));
     CKS(finish_out(pl, o_fd));
     CKS(finish_out(pl, o_n));
-    if (host_io) CK(cudaStreamSynchronize(st));
-    else CK(cudaGetLastError());
+    if (host_io) {
+        CK(cudaStreamSynchronize(st));
+        CKS(tc_check(pl));
+    } else {
+        CK(cudaGetLastError());
+    }
     return SE2P_OK;
 }
 
@@ -1449,11 +1567,14 @@ int se2p_plan_create(se2p_plan *plan, int device)
         cudaEventCreateWithFlags(&pl->join, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&pl->kjoin, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&pl->cin0, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&pl->cin1, cudaEventDisableTiming) != cudaSuccess) {
+        cudaEventCreateWithFlags(&pl->cin1, cudaEventDisableTiming) != cudaSuccess ||
+        cudaHostAlloc(&pl->tc_err, sizeof(int), cudaHostAllocMapped) != cudaSuccess ||
+        cudaHostGetDevicePointer(&pl->tc_err_dev, pl->tc_err, 0) != cudaSuccess) {
         cudaGetLastError();
         se2p_plan_destroy(pl);
         return SE2P_ERR_CUDA;
     }
+    *pl->tc_err = 0;
     *plan = pl;
     return SE2P_OK;
 }
@@ -1487,6 +1608,7 @@ int se2p_plan_destroy(se2p_plan pl)
     if (pl->cin0) cudaEventDestroy(pl->cin0);
     if (pl->cin1) cudaEventDestroy(pl->cin1);
     if (pl->own) cudaStreamDestroy(pl->own);
+    if (pl->tc_err) cudaFreeHost(pl->tc_err);
     delete pl;
     return SE2P_OK;
 }
@@ -2007,6 +2129,7 @@ static int geom_kspace_multi(se2p_geom g, int nr, const double *coef, int64_t cs
     sa.w = p.w;
     sa.a = -2 * p.xi * p.xi / p.eta;
     sa.e1 = e1;
+    sa.perm = g->sperm;
     auto rhs_spread = [&](int r) {
         SpreadArgs sr = sa;
         sr.coef = coef + r * cstride;
@@ -2019,8 +2142,14 @@ static int geom_kspace_multi(se2p_geom g, int nr, const double *coef, int64_t cs
         for (int r = 0; r < nr; r++)
             CK(launch_spread_bound(rhs_spread(r), nc, kfac, mult, ws + r * bstride, ks, pl->launches));
         sa.bound = reinterpret_cast<const unsigned long long *>(ws + bslot);
-        CK(launch_spread_fix_multi(sa, nc, kY, nr, cstride, (int64_t)(nc * G), (int)bstride, ks,
-                                   pl->launches));
+        if (tc_ok(sa, nc)) {
+            TcSet t;
+            CKS(tc_sources(pl, sa, ks, t));
+            for (int r = 0; r < nr; r++) CKS(tc_spread(pl, rhs_spread(r), t, nc, ks));
+        } else {
+            CK(launch_spread_fix_multi(sa, nc, kY, nr, cstride, (int64_t)(nc * G), (int)bstride, ks,
+                                       pl->launches));
+        }
         for (int r = 0; r < nr; r++)                 // (the FP64 spread: returns at once unless crowded)
             CK(launch_spread(rhs_spread(r), nc, ks, pl->launches));
     }
@@ -2128,6 +2257,7 @@ int se2p_geom_apply(se2p_geom g, int nrhs, const double *f_slp, const double *f_
     if (!g) return SE2P_ERR_ARG;
     se2p_plan pl = g->pl;
     DeviceGuard guard(pl->device);
+    CKS(tc_check(pl));
     cudaStream_t st = pl->stream;
     const int64_t ns = g->ns, nt = g->nt;
     if (nrhs < 0) return fail(pl, SE2P_ERR_ARG, "negative nrhs");
@@ -2271,7 +2401,7 @@ int se2p_geom_apply(se2p_geom g, int nrhs, const double *f_slp, const double *f_
     if (g->dlp)
         CK(cudaMemcpyAsync(u_dlp, uo_dlp, 16 * (size_t)nt * nrhs, cudaMemcpyDefault, st));
     CK(cudaStreamSynchronize(st));
-    return SE2P_OK;
+    return tc_check(pl);
 }
 
 int64_t se2p_geom_bytes(se2p_geom g) { return g ? (int64_t)g->bytes : 0; }

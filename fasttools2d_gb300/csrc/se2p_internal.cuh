@@ -171,6 +171,30 @@ __device__ __forceinline__ void closest_node(double x, double y, double Lhx, dou
     mx = ix; my = iy; px = ox; py = oy;
 }
 
+// exp(-x) for x >= 0 by Tang's table-driven method (P. T. P. Tang, "Table-
+// driven implementation of the exponential function in IEEE floating-point
+// arithmetic", ACM TOMS 15(2), 1989): x = (n/64) ln 2 + r, |r| <= ln2/128,
+// exp(-x) = 2^-(n>>6) * 2^-((n&63)/64) * exp(-r) with a degree-5 Taylor
+// polynomial (truncation < 4e-17).  ln2/64 is split Cody-Waite style (36-bit
+// head).  Returns 0 from x = 704 on and propagates NaN.
+__device__ __forceinline__ double exp_neg(double x, const double *tab)
+{
+    const double kShift = 6755399441055744.0;   // 1.5 * 2^52
+    const double t = fma(x, 0x1.71547652b82fep+6, kShift);
+    const int n = __double2loint(t);
+    const double kd = t - kShift;
+    double r = fma(-kd, 0x1.62e42fefa0000p-7, x);
+    r = fma(-kd, 0x1.cf79abc9e3b3ap-46, r);
+    double p = fma(-r, 1.0 / 120.0, 1.0 / 24.0);
+    p = fma(-r, p, 1.0 / 6.0);
+    p = fma(-r, p, 0.5);
+    p = fma(-r, p, 1.0);
+    p = fma(-r, p, 1.0);
+    if (__double2hiint(x) >= 0x40860000) return x == x ? 0.0 : x;   // x >= 704, inf, NaN
+    const double scale = __hiloint2double((1023 - (n >> 6)) << 20, 0);
+    return p * tab[n & 63] * scale;
+}
+
 // ---------------------------------------------------------------------------
 // E1 by the reference's three-regime Pade split
 // (PE/src/mex/StokesSLP/mex_stokes_slp_real.cpp:19-47, :166-205).
@@ -309,6 +333,38 @@ struct SpreadArgs {
     // derived from *bound (the bit pattern of a positive double bounding
     // every node's sum of |contributions|).
     const unsigned long long *bound = nullptr;
+    const int *perm = nullptr;   // sorted source -> the caller's point number
+};
+
+// Tensor-core spread (se2p_tc.cu): patches of kTcX x kTcY nodes, stencil origins
+// in tiles of (kTcX - P) x (kTcY - P), items of up to kTcK sources.
+constexpr int kTcX = 64, kTcY = 32, kTcK = 64;
+constexpr int kTcMaxP = 26;         // (tiles of at least 6 stencil origins along y)
+constexpr int kTcPointBytes = 64;   // size of a point's record
+
+struct TcPointArgs {
+    const double2 *p;           // points
+    int64_t n;
+    double Lhx, Lhy, h, inv_h;
+    unsigned long long al2;     // alpha log2(e) in units of 2^-59, alpha = 2 xi^2 h^2 / eta
+    int Mx, My, P;
+    int Tx, Ty, ntx, nty;       // tile size in stencil origins, tiles per axis
+    void *fac;                  // kTcPointBytes per point
+    int *count;                 // points per tile
+    int2 *tile;                 // per point (tile, rank in it)
+};
+
+struct TcSpreadArgs {
+    const void *fac;
+    const int *list;            // tile by tile, the points' numbers
+    const int4 *items;          // (tile, first slot, count, 0)
+    const int *nitems;
+    const double *coef;         // NC coefficients per source
+    long long *grid;            // NC int64 grids at scale 2^S
+    int Mx, My, P, Tx, nty, Ty;
+    unsigned long long s;       // exp(-2 alpha) 2^64
+    const unsigned long long *bound;   // S, as in k_spread_fix
+    int *err;                   // set when a wait ran out
 };
 
 struct FilterArgs {
@@ -535,6 +591,14 @@ __device__ __forceinline__ int fix_shift(unsigned long long bits)
 // and kfac = mult 2^(2 kY).  When the bound slot ends up all ones the FP64
 // spread runs (launch it behind launch_spread_fix with a.bound set) and the
 // grids hold doubles.
+// Factor records, tiles and items of n points (kmax per item); with perm, tiles
+// of several items are put in the order of the caller's point numbers
+// (list_tmp then holds 2 n ints).
+cudaError_t launch_tc_points(const TcPointArgs &a, int kmax, const int *perm, int *start,
+                             int *istart, int *list, int *list_tmp, int4 *items, int *nitems,
+                             const unsigned long long *bound, cudaStream_t st,
+                             int64_t &launches);
+cudaError_t launch_spread_tc(const TcSpreadArgs &a, int nc, cudaStream_t st, int64_t &launches);
 int64_t spread_bound_words(int Mx, int My, int P);
 int64_t spread_bound_slot(int Mx, int My, int P);
 cudaError_t launch_spread_bound(const SpreadArgs &a, int nc, double kfac, int mult, double *ws,

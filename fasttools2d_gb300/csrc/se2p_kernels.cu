@@ -213,30 +213,6 @@ __constant__ double c_exp_tab[64] = SE2P_EXP2_TAB64;
 // The three E1 Pade sets (layout in se2p_internal.cuh).
 __constant__ double c_e1[3][22] = SE2P_E1_PADE;
 
-// exp(-x) for x >= 0 by Tang's table-driven method (P. T. P. Tang, "Table-
-// driven implementation of the exponential function in IEEE floating-point
-// arithmetic", ACM TOMS 15(2), 1989): x = (n/64) ln 2 + r, |r| <= ln2/128,
-// exp(-x) = 2^-(n>>6) * 2^-((n&63)/64) * exp(-r) with a degree-5 Taylor
-// polynomial (truncation < 4e-17).  ln2/64 is split Cody-Waite style (36-bit
-// head).  Returns 0 from x = 704 on and propagates NaN.
-__device__ __forceinline__ double exp_neg(double x, const double *tab)
-{
-    const double kShift = 6755399441055744.0;   // 1.5 * 2^52
-    const double t = fma(x, 0x1.71547652b82fep+6, kShift);
-    const int n = __double2loint(t);
-    const double kd = t - kShift;
-    double r = fma(-kd, 0x1.62e42fefa0000p-7, x);
-    r = fma(-kd, 0x1.cf79abc9e3b3ap-46, r);
-    double p = fma(-r, 1.0 / 120.0, 1.0 / 24.0);
-    p = fma(-r, p, 1.0 / 6.0);
-    p = fma(-r, p, 0.5);
-    p = fma(-r, p, 1.0);
-    p = fma(-r, p, 1.0);
-    if (__double2hiint(x) >= 0x40860000) return x == x ? 0.0 : x;   // x >= 704, inf, NaN
-    const double scale = __hiloint2double((1023 - (n >> 6)) << 20, 0);
-    return p * tab[n & 63] * scale;
-}
-
 // 1/a by the hardware approximation plus two Newton-Raphson steps
 // (r <- r + r (1 - a r)); each step doubles the correct bits.
 __device__ __forceinline__ double rcp_nr(double a)
