@@ -623,44 +623,56 @@ static bool tc_ok(const SpreadArgs &sa, int nc)
     return 24.0 * ((nc + 1) / 2) * std::min(ntile, (double)sa.ns) <= 1e5 + 1.1 * nc * (double)sa.ns;
 }
 
-static int tc_sources(se2p_plan pl, const SpreadArgs &sa, cudaStream_t ks, TcSet &t)
+// Factor records, tiles and items of n points for patches of X x Y nodes, items of
+// up to kmax points; perm and bound for the sources (launch_tc_points).  The
+// spread's set and the gather's share their slots: each is used up before the
+// next is made, in stream order.
+static int tc_points(se2p_plan pl, const double2 *p, int64_t n, const int *perm,
+                     const unsigned long long *bound, double Lhx, double Lhy, double h, double a,
+                     int Mx, int My, int P, int X, int Y, int kmax, cudaStream_t ks, TcSet &t)
 {
     TcPointArgs &pa = t.pa;
-    pa.p = sa.sp;
-    pa.n = sa.ns;
-    pa.Lhx = sa.Lhx;
-    pa.Lhy = sa.Lhy;
-    pa.h = sa.h;
-    pa.inv_h = 1.0 / sa.h;
-    const double alpha = -sa.a * sa.h * sa.h;
+    pa.p = p;
+    pa.n = n;
+    pa.Lhx = Lhx;
+    pa.Lhy = Lhy;
+    pa.h = h;
+    pa.inv_h = 1.0 / h;
+    const double alpha = -a * h * h;
     pa.al2 = (unsigned long long)std::llround(std::ldexp(alpha * 1.4426950408889634074, 59));
     t.s = (unsigned long long)std::llround(std::ldexp(std::exp(-2.0 * alpha), 62)) << 2;
-    pa.Mx = sa.Mx;
-    pa.My = sa.My;
-    pa.P = sa.P;
-    pa.Tx = kTcX - sa.P;
-    pa.Ty = kTcY - sa.P;
-    pa.ntx = (sa.Mx + pa.Tx - 1) / pa.Tx;
-    pa.nty = (sa.My + pa.Ty - 1) / pa.Ty;
+    pa.Mx = Mx;
+    pa.My = My;
+    pa.P = P;
+    pa.Tx = X - P;
+    pa.Ty = Y - P;
+    pa.ntx = (Mx + pa.Tx - 1) / pa.Tx;
+    pa.nty = (My + pa.Ty - 1) / pa.Ty;
     const int ntile = pa.ntx * pa.nty;
-    const size_t n = (size_t)(sa.ns > 0 ? sa.ns : 1);
-    // small sets: smaller items, so that every SM has one
-    const int kmax = std::min(kTcK, std::max(32, (int)((sa.ns + 2 * sm_count() - 1) / (2 * sm_count()) + 15) / 16 * 16));
+    const size_t nz = (size_t)(n > 0 ? n : 1);
+    // small sets: smaller items, so that every SM has two
+    kmax = std::min(kmax, std::max(32, (int)((n + 2 * sm_count() - 1) / (2 * sm_count()) + 15) / 16 * 16));
     char *fac = nullptr;
     int *start = nullptr, *ltmp = nullptr;
-    CKS(ensure_t(pl, S_TCFAC, n * kTcPointBytes, &fac));
-    CKS(ensure_t(pl, S_TCTILE, n, &pa.tile));
+    CKS(ensure_t(pl, S_TCFAC, nz * kTcPointBytes, &fac));
+    CKS(ensure_t(pl, S_TCTILE, nz, &pa.tile));
     CKS(ensure_t(pl, S_TCCNT, (size_t)ntile, &pa.count));
     CKS(ensure_t(pl, S_TCSTART, 2 * (size_t)ntile + 2, &start));
-    CKS(ensure_t(pl, S_TCLIST, n, &t.list));
-    CKS(ensure_t(pl, S_TCLTMP, 2 * n, &ltmp));
-    CKS(ensure_t(pl, S_TCITEMS, std::min(n, (size_t)ntile) + n / kmax + 1, &t.items));
+    CKS(ensure_t(pl, S_TCLIST, nz, &t.list));
+    if (perm) CKS(ensure_t(pl, S_TCLTMP, 2 * nz, &ltmp));
+    CKS(ensure_t(pl, S_TCITEMS, std::min(nz, (size_t)ntile) + nz / kmax + 1, &t.items));
     pa.fac = fac;
     int *istart = start + ntile + 1;
     t.nitems = istart + ntile;
-    CK(launch_tc_points(pa, kmax, sa.perm, start, istart, t.list, ltmp, t.items, t.nitems, sa.bound, ks,
+    CK(launch_tc_points(pa, kmax, perm, start, istart, t.list, ltmp, t.items, t.nitems, bound, ks,
                         pl->launches));
     return SE2P_OK;
+}
+
+static int tc_sources(se2p_plan pl, const SpreadArgs &sa, cudaStream_t ks, TcSet &t)
+{
+    return tc_points(pl, sa.sp, sa.ns, sa.perm, sa.bound, sa.Lhx, sa.Lhy, sa.h, sa.a, sa.Mx, sa.My,
+                     sa.P, kTcX, kTcY, kTcK, ks, t);
 }
 
 static int tc_spread(se2p_plan pl, const SpreadArgs &sa, const TcSet &t, int nc, cudaStream_t ks)
@@ -682,6 +694,56 @@ static int tc_spread(se2p_plan pl, const SpreadArgs &sa, const TcSet &t, int nc,
     ta.bound = sa.bound;
     ta.err = pl->tc_err_dev;
     CK(launch_spread_tc(ta, nc, ks, pl->launches));
+    return SE2P_OK;
+}
+
+// Whether the tensor-core gather runs: for the same stencils as the spread, grids of
+// at least a patch, and enough targets per tile.  It costs about 40 ns (two
+// grids) or 66 ns (four) per item, k_gather_fix 1.4 or 5.6 ns per target beside
+// a fixed 0.25 ms or so (2^16 targets, two grids: 0.97 against 0.41 ms on 2688^2
+// nodes, 0.12 against 0.21 ms on 512^2; 300,000 targets, four grids: 1.73
+// against 2.10 ms on 2688^2 nodes, 0.47 against 2.02 ms on 896^2).
+static bool tg_ok(const GatherArgs &ga, int nout)
+{
+    if (ga.P < 4 || ga.P > kTcMaxP || ga.Mx < kTgX || ga.My < kTgY ||
+        !(std::fabs(ga.w - ga.h * ga.P / 2) <= 1e-14 * ga.w))
+        return false;
+    const double ntile = std::ceil((double)ga.Mx / (kTgX - ga.P)) * std::ceil((double)ga.My / (kTgY - ga.P));
+    return (14.0 + 13.0 * nout) * std::min(ntile, (double)ga.nt) <= 2.5e5 + 0.35 * nout * nout * (double)ga.nt;
+}
+
+static int tg_targets(se2p_plan pl, const GatherArgs &ga, cudaStream_t ks, TcSet &t)
+{
+    return tc_points(pl, ga.tp, ga.nt, nullptr, nullptr, ga.Lhx, ga.Lhy, ga.h, ga.a, ga.Mx, ga.My,
+                     ga.P, kTgX, kTgY, kTgT, ks, t);
+}
+
+// The gather of nout grids (int64 at scale kTgBits): the patch sums stay below
+// 2^63 with |g| below 2^61 and the factors' sum along y below 4.
+constexpr int kTgBits = 61;
+
+static int tg_gather(se2p_plan pl, const GatherArgs &ga, const TcSet &t, int nout, cudaStream_t ks)
+{
+    TcGatherArgs ta{};
+    ta.fac = t.pa.fac;
+    ta.list = t.list;
+    ta.items = t.items;
+    ta.nitems = t.nitems;
+    ta.grid = reinterpret_cast<const long long *>(ga.grid);
+    ta.gmax = ga.gmax;
+    ta.Mx = ga.Mx;
+    ta.My = ga.My;
+    ta.P = ga.P;
+    ta.Tx = t.pa.Tx;
+    ta.Ty = t.pa.Ty;
+    ta.nty = t.pa.nty;
+    ta.Bg = kTgBits;
+    ta.s = t.s;
+    ta.nt = ga.nt;
+    ta.scale = ga.scale;
+    ta.out = ga.out;
+    ta.err = pl->tc_err_dev;
+    CK(launch_gather_tc(ta, nout, ks, pl->launches));
     return SE2P_OK;
 }
 
@@ -1201,7 +1263,14 @@ int run(se2p_plan pl, const Job &J, const Io &io)
         ga.gmax = gmax;
         ga.Bg = Bg;
         StageTimer tm(pl, T_GATHER, ks);
-        if (gmax) {
+        const bool tg = gmax && tg_ok(ga, nout);
+        if (tg) {
+            TcSet t;
+            CKS(tg_targets(pl, ga, ks, t));
+            CK(launch_grid_to_fixed(grid, nout, (int64_t)G, gmax, kTgBits, ks, pl->launches));
+            CKS(tg_gather(pl, ga, t, nout, ks));
+            CK(launch_gather_fp64_fallback(ga, nout, ks, pl->launches));
+        } else if (gmax) {
             CK(launch_grid_to_fixed(grid, nout, (int64_t)G, gmax, Bg, ks, pl->launches));
             // the box-sorted targets visited patch by patch (about kPatchNodes
             // grid nodes a side), so that a block's targets in flight share
@@ -1216,7 +1285,7 @@ int run(se2p_plan pl, const Job &J, const Io &io)
                                   pl->launches));
             ga.order = order;
         }
-        CK(launch_gather(ga, nout, ks, pl->launches));
+        if (!tg) CK(launch_gather(ga, nout, ks, pl->launches));
     }
 
     if (ks != st) {
@@ -2208,11 +2277,24 @@ static int geom_kspace_multi(se2p_geom g, int nr, const double *coef, int64_t cs
     // one slower, 4.1 against 3.57 ms for one right-hand side and 18.2 against
     // 14.5 ms for four)
     StageTimer tm(pl, T_GATHER, ks);
+    const int64_t ostride = (int64_t)(nout / 2) * g->nt;
+    const bool tg = tg_ok(ga, nout);
     for (int r = 0; r < nr; r++)
         CK(launch_grid_to_fixed(grid + (size_t)r * nc * G, nout, (int64_t)G, gmax + r * kGmaxWords,
-                                Bg, ks, pl->launches));
-    const int64_t ostride = (int64_t)(nout / 2) * g->nt;
-    CK(launch_gather_fix_multi(ga, nout, nr, (int64_t)(nc * G), ostride, ks, pl->launches));
+                                tg ? kTgBits : Bg, ks, pl->launches));
+    if (tg) {
+        TcSet t;
+        CKS(tg_targets(pl, ga, ks, t));
+        for (int r = 0; r < nr; r++) {
+            GatherArgs gr = ga;
+            gr.grid = grid + (size_t)r * nc * G;
+            gr.gmax = gmax + r * kGmaxWords;
+            gr.out = uk + r * ostride;
+            CKS(tg_gather(pl, gr, t, nout, ks));
+        }
+    } else {
+        CK(launch_gather_fix_multi(ga, nout, nr, (int64_t)(nc * G), ostride, ks, pl->launches));
+    }
     for (int r = 0; r < nr; r++) {                   // (the FP64 gather: returns at once unless non-finite)
         GatherArgs gr = ga;
         gr.grid = grid + (size_t)r * nc * G;

@@ -367,6 +367,25 @@ struct TcSpreadArgs {
     int *err;                   // set when a wait ran out
 };
 
+// Tensor-core gather: patches of kTgX x kTgY nodes, stencil origins in tiles of
+// (kTgX - P) x (kTgY - P), items of up to kTgT targets.
+constexpr int kTgX = 32, kTgY = 64, kTgT = 64;
+
+struct TcGatherArgs {
+    const void *fac;
+    const int *list;
+    const int4 *items;
+    const int *nitems;
+    const long long *grid;      // NC int64 grids (launch_grid_to_fixed with Bg)
+    const unsigned long long *gmax;
+    int Mx, My, P, Tx, Ty, nty, Bg;
+    unsigned long long s;       // exp(-2 alpha) 2^64
+    int64_t nt;
+    double scale;
+    double2 *out;               // NC/2 outputs per target, [k * nt + t]
+    int *err;
+};
+
 struct FilterArgs {
     cufftDoubleComplex *spec;   // component c at spec + c * Mx * (My/2+1)
     int Mx, My;
@@ -573,6 +592,17 @@ __device__ __forceinline__ unsigned long long gmax_all(const unsigned long long 
     return max(g[0], max(g[1], g[2]));
 }
 
+// Bit patterns of |g| at or above this are infinities and NaNs.
+constexpr unsigned long long kGridNonFinite = 0x7ff0000000000000ull;
+// Sg with max|g| 2^Sg < 2^Bg, from the bit pattern of max|g|.
+__device__ __forceinline__ int grid_shift(unsigned long long gb, int Bg)
+{
+    if (gb == 0) return 0;
+    const int e = (int)((gb >> 52) & 0x7ff) - 1022;  // max|g| < 2^e
+    const int S = Bg - e;
+    return S < -960 ? -960 : (S > 960 ? 960 : S);
+}
+
 // Scale S of the fixed-point spread's grids (int64 at 2^S, bound 2^S < 2^59),
 // from the bit pattern of the positive bound.
 __device__ __forceinline__ int fix_shift(unsigned long long bits)
@@ -598,6 +628,7 @@ cudaError_t launch_tc_points(const TcPointArgs &a, int kmax, const int *perm, in
                              int *istart, int *list, int *list_tmp, int4 *items, int *nitems,
                              const unsigned long long *bound, cudaStream_t st,
                              int64_t &launches);
+cudaError_t launch_gather_tc(const TcGatherArgs &a, int nc, cudaStream_t st, int64_t &launches);
 cudaError_t launch_spread_tc(const TcSpreadArgs &a, int nc, cudaStream_t st, int64_t &launches);
 int64_t spread_bound_words(int Mx, int My, int P);
 int64_t spread_bound_slot(int Mx, int My, int P);

@@ -1367,8 +1367,6 @@ template __global__ void k_real_adj<true, true, kFormFF>(RealArgs);
 // atomics (executed in L2, off the SM's FP64 pipe).
 // ===========================================================================
 constexpr int kSpreadWarps = 8;
-// Bit patterns of |g| at or above this are infinities and NaNs.
-constexpr unsigned long long kGridNonFinite = 0x7ff0000000000000ull;
 
 __device__ __forceinline__ int wrap_index(int i, int M)
 {
@@ -2359,15 +2357,6 @@ template __global__ void k_gather<4, 0>(GatherArgs);
 #define SE2P_GATHER_THREADS 256
 #endif
 constexpr int kGatherThreads = SE2P_GATHER_THREADS;
-
-// Sg with max|g| 2^Sg < 2^Bg, from the bit pattern of max|g|.
-__device__ __forceinline__ int grid_shift(unsigned long long gb, int Bg)
-{
-    if (gb == 0) return 0;
-    const int e = (int)((gb >> 52) & 0x7ff) - 1022;  // max|g| < 2^e
-    const int S = Bg - e;
-    return S < -960 ? -960 : (S > 960 ? 960 : S);
-}
 
 // Grid c = blockIdx.y at its pair's scale.
 __global__ void k_grid_to_fixed(double *__restrict__ grid, int64_t G,

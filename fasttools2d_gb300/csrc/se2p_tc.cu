@@ -1,4 +1,4 @@
-// se2p_tc.cu -- Gaussian spread on the tensor cores (FP64 form).
+// se2p_tc.cu -- Gaussian spread and gather on the tensor cores (FP64 form).
 //
 // The spread of a tile of sources is a contraction: with X_s[i], Y_s[j] the
 // one-dimensional Gaussian factors of source s (zero outside its P + 1
@@ -470,6 +470,7 @@ __device__ __forceinline__ void tc_ld_wait8(uint32_t (&r)[8])
 // ---------------------------------------------------------------------------
 // Digits
 // ---------------------------------------------------------------------------
+constexpr int kTcDigits = 7;
 // Base-256 digits of four numbers up to 2^63, most significant first, as FP16,
 // each number's digits times its sign: adding 128 to every byte but the top one
 // carries the digits' signs upward, so the top byte is a digit 0 .. 128 and the
@@ -512,14 +513,15 @@ __device__ __forceinline__ void store_zero_digits(char *dst, int stride)
 }
 
 // One side of one axis of a point's factors, as fractions of 2^64, from the
-// centre outward into rows i, i + di, .. (n of them) of a window of rows kTcK
+// centre outward into rows i, i + di, .. (n of them) of a window of rows STRIDE
 // apart, then zeros up to the window's end.
+template <int STRIDE>
 __device__ __forceinline__ void tc_factors(unsigned long long e, unsigned long long q,
                                            unsigned long long s, int i, int di, int n, int win,
                                            unsigned long long *out)
 {
-    unsigned long long *o = out + i * kTcK;
-    const int step = di * kTcK, left = di > 0 ? win - i - n : i + 1 - n;
+    unsigned long long *o = out + i * STRIDE;
+    const int step = di * STRIDE, left = di > 0 ? win - i - n : i + 1 - n;
     for (int k = 0; k < n; k++) {
         *o = e;
         e = mulhi_apx(e, q);
@@ -763,10 +765,10 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_spread_tc(TcSpreadArgs a)
                 const unsigned long long e = sh.seed[ax][s];
                 unsigned long long *o = (ax ? ys : xs) + s;
                 if (q < 2) {
-                    tc_factors(e, sh.seed[2 + ax][s], a.s, r + ic, 1, P1 - ic, win, o);
+                    tc_factors<kTcK>(e, sh.seed[2 + ax][s], a.s, r + ic, 1, P1 - ic, win, o);
                 } else {
                     const unsigned long long qm = sh.seed[4 + ax][s];
-                    tc_factors(mulhi_apx(e, qm), mulhi_apx(qm, a.s), a.s, r + ic - 1, -1, ic, win, o);
+                    tc_factors<kTcK>(mulhi_apx(e, qm), mulhi_apx(qm, a.s), a.s, r + ic - 1, -1, ic, win, o);
                 }
             }
             mbar_arrive(smem_u32(&sh.seedfree));
@@ -885,6 +887,301 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_spread_tc(TcSpreadArgs a)
 }
 
 // ---------------------------------------------------------------------------
+// Gather
+//
+// u_c(t) = sum_i X_t[i] sum_j G_c[i][j] Y_t[j]: the inner sums of a tile's targets
+// are a matrix product of Y (targets x nodes along y) with a patch of G_c.  An item
+// is up to kTgT targets of one tile of (kTgX - P) x (kTgY - P) stencil origins, whose
+// stencils lie in a patch of kTgX x kTgY nodes.  A = digits of Y (K-major, a row
+// per target, kept for the item; rows 64 .. 127 of the product read what follows in
+// shared memory and are ignored), B = digits of the patch of one grid, digit by
+// digit along N, D = the levels, kTgX columns each.  The levels give the inner sums as
+// int64, and each target's thread finishes with the X factors.  Warps whose TMEM
+// lanes hold targets do that while the others build the next grid's B; a ninth
+// issues the products, a tenth loads the next item's targets.
+//
+// Bound: tensor pipe (37 % active: 64 of the product's 128 rows hold targets, about
+// 46 of them at 7 nodes per target) and the latency between an item's phases, two
+// blocks per SM.  2^20 targets, 2688^2 nodes, four grids: 1.53 ms (and 0.09 ms
+// to sort the targets into tiles) against k_gather_fix's 2.94 ms, bound by L1.
+// ---------------------------------------------------------------------------
+constexpr int kTgA = kTcDigits * kTgT * kTgY * 2, kTgB = kTcDigits * kTgX * kTgY * 2;
+constexpr int kTgXs = kTgX * kTgT * 8;
+
+struct TgSmem {
+    unsigned long long seed[6][kTgT];
+    int meta[2][kTgT], idx[2][kTgT];
+    long long part[kTgT];
+    unsigned long long bfull, done, tfree, fin, ready, sfree[2], seedfree;
+    uint32_t tmem;
+    int abort_flag;
+};
+
+constexpr int kTgSmem = kTgA + kTgB + kTgXs + (int)sizeof(TgSmem) + 128;
+
+// Digits of eight signed numbers below 2^62 (all bytes biased), as store_digits.
+__device__ __forceinline__ void store_digits_signed(const long long (&v)[8], char *dst, int stride)
+{
+    const __half2 off = __float2half2_rn(-1152.0f);
+    uint32_t out[8][4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const unsigned long long a = (unsigned long long)v[2 * k] + 0x8080808080808080ull;
+        const unsigned long long b = (unsigned long long)v[2 * k + 1] + 0x8080808080808080ull;
+#pragma unroll
+        for (int w = 0; w < 2; w++) {
+            const uint32_t aw = (uint32_t)(w ? a : a >> 32), bw = (uint32_t)(w ? b : b >> 32);
+            const uint32_t z = __byte_perm(aw, bw, 0x7632), y = __byte_perm(aw, bw, 0x5410);
+            const uint32_t d[4] = {__byte_perm(z, 0x64646464u, 0x4341), __byte_perm(z, 0x64646464u, 0x4240),
+                                   __byte_perm(y, 0x64646464u, 0x4341), __byte_perm(y, 0x64646464u, 0x4240)};
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const __half2 h = __hadd2(*reinterpret_cast<const __half2 *>(&d[q]), off);
+                out[4 * w + q][k] = *reinterpret_cast<const uint32_t *>(&h);
+            }
+        }
+    }
+#pragma unroll
+    for (int p = 0; p < kTcDigits; p++)
+        *reinterpret_cast<uint4 *>(dst + p * stride) = make_uint4(out[p][0], out[p][1], out[p][2], out[p][3]);
+}
+
+template <int NC>
+__global__ void __launch_bounds__(kTcThreads, 2) k_gather_tc(TcGatherArgs a)
+{
+    extern __shared__ __align__(128) char tc_smem[];
+    if (gmax_all(a.gmax) >= kGridNonFinite) return;  // the FP64 gather runs instead
+    const int nv = *a.nitems;
+    const int v0 = (int)((int64_t)nv * blockIdx.x / gridDim.x);
+    const int v1 = (int)((int64_t)nv * (blockIdx.x + 1) / gridDim.x);
+    if (v0 == v1) return;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int P = a.P, P1 = P + 1, win = tc_window(P);
+    char *Ash = tc_smem, *Bsh = Ash + kTgA;
+    unsigned long long *xs = reinterpret_cast<unsigned long long *>(Bsh + kTgB);
+    unsigned long long *ys = reinterpret_cast<unsigned long long *>(Bsh);
+    TgSmem &sh = *reinterpret_cast<TgSmem *>(reinterpret_cast<char *>(xs) + kTgXs);
+    volatile int *ab = &sh.abort_flag;
+
+    if (tid == 0) {
+        sh.abort_flag = 0;
+        mbar_init(smem_u32(&sh.bfull), 128);
+        mbar_init(smem_u32(&sh.done), 1);
+        mbar_init(smem_u32(&sh.tfree), 128);
+        mbar_init(smem_u32(&sh.fin), 1);
+        mbar_init(smem_u32(&sh.ready), 1);
+        mbar_init(smem_u32(&sh.sfree[0]), kTcBuild);
+        mbar_init(smem_u32(&sh.sfree[1]), kTcBuild);
+        mbar_init(smem_u32(&sh.seedfree), kTcBuild);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == kTcBuild / 32) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                         smem_u32(&sh.tmem)),
+                     "n"(kTcCols)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = sh.tmem;
+
+    if (warp == kTcBuild / 32) {
+        if (lane == 0) {
+            int n = 0;
+            for (int v = v0; v < v1; v++) {
+                for (int c = 0; c < NC; c++, n++) {
+                    mbar_wait(smem_u32(&sh.bfull), n & 1, ab, a.err);
+                    if (n > 0) mbar_wait(smem_u32(&sh.tfree), (n - 1) & 1, ab, a.err);
+                    tc_fence_after();
+                    if (*ab) continue;
+#pragma unroll 1
+                    for (int k = 0; k < kTgY / 16; k++)
+#pragma unroll
+                        for (int p = 0; p < kTcDigits; p++)
+                            tc_mma(tmem + kTgX * p,
+                                   tc_desc(smem_u32(Ash) + p * (kTgT * kTgY * 2) + k * 256, 128, kTgY * 16),
+                                   tc_desc(smem_u32(Bsh) + k * 256, 128, kTgY * 16),
+                                   tc_idesc(kTgX * (kTcDigits - p), 0), k > 0 || p > 0);
+                    tc_commit(smem_u32(&sh.done));
+                }
+            }
+            // everything issued has completed before TMEM is given back
+            tc_commit(smem_u32(&sh.fin));
+            mbar_wait(smem_u32(&sh.fin), 0, ab, a.err);
+        }
+        __syncwarp();
+    } else if (warp == kTcBuild / 32 + 1) {
+        int n = 0;
+        for (int v = v0; v < v1; v++, n++) {
+            const int4 item = a.items[v];
+            const int b = n & 1;
+            const TcPoint *f[kTgT / 32];
+            int meta[kTgT / 32], idx[kTgT / 32];
+#pragma unroll
+            for (int u = 0; u < kTgT / 32; u++) {
+                const int s = lane + 32 * u;
+                f[u] = nullptr;
+                meta[u] = 0;
+                idx[u] = -1;
+                if (s < item.z) {
+                    idx[u] = a.list[item.y + s];
+                    f[u] = reinterpret_cast<const TcPoint *>(a.fac) + idx[u];
+                    meta[u] = f[u]->meta;
+                }
+            }
+            if (n > 1) mbar_wait(smem_u32(&sh.sfree[b]), (n / 2 - 1) & 1, ab, a.err);
+#pragma unroll
+            for (int u = 0; u < kTgT / 32; u++) {
+                sh.meta[b][lane + 32 * u] = meta[u];
+                sh.idx[b][lane + 32 * u] = idx[u];
+            }
+            if (n > 0) mbar_wait(smem_u32(&sh.seedfree), (n - 1) & 1, ab, a.err);
+#pragma unroll
+            for (int u = 0; u < kTgT / 32; u++) {
+                if (!f[u]) continue;
+                const int s = lane + 32 * u;
+                sh.seed[0][s] = f[u]->ex;
+                sh.seed[1][s] = f[u]->ey;
+                sh.seed[2][s] = f[u]->qpx;
+                sh.seed[3][s] = f[u]->qpy;
+                sh.seed[4][s] = f[u]->qmx;
+                sh.seed[5][s] = f[u]->qmy;
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&sh.ready));
+        }
+    } else {
+        int n = 0, nc = 0;                           // items, grids so far
+        const __half2 one = __float2half2_rn(1.0f);
+        const bool epi = (warp & 2) == 0;            // TMEM lanes 0 .. 63: targets
+        const int et = (warp & 1) * 32 + lane, eh = warp >> 2;            // target, half of the columns
+        const int bt = ((warp >> 2) * 2 + (warp & 1)) * 32 + lane;        // builder thread
+        auto bsync = [] { asm volatile("bar.sync 1, %0;" ::"n"(kTcBuild) : "memory"); };
+        for (int v = v0; v < v1; v++, n++) {
+            const int4 item = a.items[v];
+            const int cnt = item.z, b = n & 1;
+            mbar_wait(smem_u32(&sh.ready), n & 1, ab, a.err);
+            // the factors: x in the patch's coordinates (as fractions of 2^62), y in
+            // the chunk-aligned window (B's region holds them until A is built)
+            for (int t = tid; t < 4 * kTgT; t += kTcBuild) {
+                const int q = t / kTgT, ax = q & 1, s = t % kTgT;
+                if (s >= cnt) continue;
+                const int meta = sh.meta[b][s], ic = P / 2 + ((meta >> (16 + ax)) & 1);
+                const int r = ax ? (meta >> 8) & 7 : meta & 0xff, w = ax ? win : kTgX;
+                const unsigned long long e = ax ? sh.seed[1][s] : sh.seed[0][s] >> 2;
+                unsigned long long *o = (ax ? ys : xs) + s;
+                if (q < 2) {
+                    tc_factors<kTgT>(e, sh.seed[2 + ax][s], a.s, r + ic, 1, P1 - ic, w, o);
+                } else {
+                    const unsigned long long qm = sh.seed[4 + ax][s];
+                    tc_factors<kTgT>(mulhi_apx(e, qm), mulhi_apx(qm, a.s), a.s, r + ic - 1, -1, ic, w, o);
+                }
+            }
+            mbar_arrive(smem_u32(&sh.seedfree));
+            bsync();
+            for (int t = tid; t < kTgT * (kTgY / 4); t += kTcBuild) {
+                const int slot = t / (2 * kTgT), s = (t >> 1) % kTgT, half = t & 1;
+                const int ch = (((sh.meta[b][s] >> 11) & 31) + slot) & (kTgY / 8 - 1);
+                char *dst = Ash + (s >> 3) * (kTgY * 16) + ch * 128 + (s & 7) * 16 + half * 8;
+                if (s >= cnt || 8 * slot >= win) {
+                    store_zero_digits<kTcDigits>(dst, kTgT * kTgY * 2);
+                } else {
+                    unsigned long long w[4];
+#pragma unroll
+                    for (int e = 0; e < 4; e++) w[e] = ys[(8 * slot + 4 * half + e) * kTgT + s] >> 1;
+                    store_digits<kTcDigits>(w, one, dst, kTgT * kTgY * 2);
+                }
+            }
+            fence_async_shared();
+            bsync();
+            const int x0 = item.x / a.nty * a.Tx, y0 = item.x % a.nty * a.Ty;
+            long long first = 0;                     // the first of a pair's two sums
+            for (int c = 0; c < NC; c++, nc++) {
+                if (!epi) {
+                    // B: 32 columns x 8 chunks of 8 nodes
+                    if (c > 0) mbar_wait(smem_u32(&sh.done), (nc - 1) & 1, ab, a.err);
+                    const long long *grid = a.grid + (int64_t)c * a.Mx * a.My;
+#pragma unroll 1
+                    for (int t = bt; t < kTgX * (kTgY / 8); t += 128) {
+                        const int i = t % kTgX, ch = t / kTgX;
+                        int x = x0 + i, y = y0 + 8 * ch;
+                        if (x >= a.Mx) x -= a.Mx;
+                        if (y >= a.My) y -= a.My;
+                        const long long *g = grid + (int64_t)x * a.My;
+                        long long w[8];
+                        if (y + 8 <= a.My) {
+#pragma unroll
+                            for (int e = 0; e < 4; e++) {
+                                const longlong2 q = __ldg(reinterpret_cast<const longlong2 *>(g + y) + e);
+                                w[2 * e] = q.x;
+                                w[2 * e + 1] = q.y;
+                            }
+                        } else {
+#pragma unroll
+                            for (int e = 0; e < 8; e++) w[e] = __ldg(g + (y + e >= a.My ? y + e - a.My : y + e));
+                        }
+                        store_digits_signed(w, Bsh + (i >> 3) * (kTgY * 16) + ch * 128 + (i & 7) * 16, kTgX * kTgY * 2);
+                    }
+                    fence_async_shared();
+                    mbar_arrive(smem_u32(&sh.bfull));
+                } else {
+                    mbar_wait(smem_u32(&sh.done), nc & 1, ab, a.err);
+                    tc_fence_after();
+                    long long acc = 0;
+#pragma unroll 1
+                    for (int h = 0; h < kTgX / 16; h++) {
+                        const int i0 = eh * (kTgX / 2) + 8 * h;
+                        uint32_t r[kTcDigits][8];
+#pragma unroll
+                        for (int l = 0; l < kTcDigits; l++)
+                            tc_ld8(tmem + ((uint32_t)((warp & 1) * 32) << 16) + kTgX * l + i0, r[l]);
+#pragma unroll
+                        for (int l = 0; l < kTcDigits; l++) tc_ld_wait8(r[l]);
+#pragma unroll
+                        for (int e = 0; e < 8; e++) {
+                            auto d = [&](int l) { return __float2int_rn(__uint_as_float(r[l][e])); };
+                            const int p12 = d(1) * 256 + d(2), p34 = d(3) * 256 + d(4), p56 = d(5) * 256 + d(6);
+                            const unsigned hi = (unsigned)d(0) * 65536u + (unsigned)p12;
+                            const long long V = (long long)p34 * 65536 + p56 + (long long)((unsigned long long)hi << 32);
+                            const unsigned long long x = xs[(i0 + e) * kTgT + et];
+                            acc += (long long)mulhi_apx((unsigned long long)V, x) - (V < 0 ? (long long)x : 0);
+                        }
+                    }
+                    tc_fence_before();
+                    mbar_arrive(smem_u32(&sh.tfree));
+                    // the two halves of the columns
+                    if (eh) sh.part[et] = acc;
+                    asm volatile("bar.sync 2, 128;" ::: "memory");
+                    if (!eh) {
+                        acc += sh.part[et];
+                        if (c & 1) {
+                            const int j = sh.idx[b][et];
+                            const unsigned long long gb = a.gmax[c / 2];
+                            const double s = gb == 0 ? 0.0 : ldexp(a.scale, 3 - grid_shift(gb, a.Bg));
+                            if (j >= 0 && !*ab)
+                                a.out[(int64_t)(c / 2) * a.nt + j] = make_double2((double)first * s, (double)acc * s);
+                        } else {
+                            first = acc;
+                        }
+                    }
+                    asm volatile("bar.sync 2, 128;" ::: "memory");
+                }
+            }
+            mbar_arrive(smem_u32(&sh.sfree[b]));
+            // the item's last product has read A and B (the epilogue waited for it)
+            bsync();
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    if (warp == kTcBuild / 32)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(kTcCols) : "memory");
+}
+
+// ---------------------------------------------------------------------------
 // Launchers
 // ---------------------------------------------------------------------------
 cudaError_t launch_tc_points(const TcPointArgs &a, int kmax, const int *perm, int *start,
@@ -926,11 +1223,27 @@ cudaError_t launch_spread_tc(const TcSpreadArgs &a, int nc, cudaStream_t st, int
 {
     launches++;
     switch (nc) {
-    case 2: return spread_tc<2, 7>(a, st);
-    case 3: return spread_tc<3, 7>(a, st);
-    case 4: return spread_tc<4, 7>(a, st);
-    default: return spread_tc<5, 7>(a, st);
+    case 2: return spread_tc<2, kTcDigits>(a, st);
+    case 3: return spread_tc<3, kTcDigits>(a, st);
+    case 4: return spread_tc<4, kTcDigits>(a, st);
+    default: return spread_tc<5, kTcDigits>(a, st);
     }
+}
+
+template <int NC>
+static cudaError_t gather_tc(const TcGatherArgs &a, cudaStream_t st)
+{
+    const cudaError_t e =
+        cudaFuncSetAttribute(k_gather_tc<NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTgSmem);
+    if (e != cudaSuccess) return e;
+    k_gather_tc<NC><<<2 * sm_count(), kTcThreads, kTgSmem, st>>>(a);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_gather_tc(const TcGatherArgs &a, int nc, cudaStream_t st, int64_t &launches)
+{
+    launches++;
+    return nc == 2 ? gather_tc<2>(a, st) : gather_tc<4>(a, st);
 }
 
 }  // namespace se2p

@@ -1,12 +1,13 @@
-"""The tensor-core spread against the all-FP64 form, at the sizes where it can
+"""The tensor-core spread and gather against the all-FP64 form, at the sizes where they can
 go wrong: grids of one patch, sizes that no tile divides, stencils of every
 window width, items of one source and tiles of many items, sources that share a
 stencil origin, grids of very different magnitude, and the line to the direct
-spread.
+kernels; the same for the targets.
 
 Tolerance: 1e-13, as for the integer spread.  The digit sums drop 2^-56 of the
 largest coefficient per source and round once per item at the grid's unit;
-both, summed over a node's sources, are below the float-float FFT's 2^-48."""
+both, summed over a node's sources, are below the float-float FFT's 2^-48.  The
+gather's digits drop 2^-54 of the largest grid value per node."""
 import numpy as np
 import pytest
 
@@ -49,7 +50,7 @@ def _both(ft, plans, p, q, f, n, Mx, My, P, Ly=1.0, eta=0.9):
         assert relerr(a, b) < TOL, (fn.__name__, relerr(a, b))
 
 
-@pytest.mark.parametrize("Mx,My,P", [(64, 64, 24), (64, 32, 24), (66, 34, 20), (130, 98, 24),
+@pytest.mark.parametrize("Mx,My,P", [(64, 64, 24), (64, 32, 24), (32, 64, 24), (34, 66, 24), (66, 34, 20), (130, 98, 24),
                                      (104, 200, 4), (200, 104, 6), (128, 128, 10), (96, 96, 16),
                                      (122, 90, 18), (256, 64, 26), (192, 192, 22)])
 @pytest.mark.parametrize("N", [1, 17, 4001])
@@ -106,3 +107,26 @@ def test_spread_tiles_of_many_items_are_reproducible(ft, plans):
     a = [ft.mex_stokes_dlp_kspace(p, q, 60.0, 0.85, f, n, 192, 192, 1.0, 1.0, 12 / 192, 24,
                                   plan=plans[0]) for _ in range(3)]
     assert np.array_equal(a[0], a[1]) and np.array_equal(a[0], a[2])
+
+
+@pytest.mark.parametrize("nt", [1, 31, 33, 64, 65, 3000])
+def test_gather_items(ft, plans, nt):
+    """Targets over the box, and all in one grid cell (a tile of many items)."""
+    p, q, f, n = _cloud(3000, 60 + nt, nt=nt)
+    _both(ft, plans, p, q, f, n, 192, 192, 24)
+    _both(ft, plans, p, -0.2 + q / 192, f, n, 192, 192, 24)
+
+
+def test_gather_edges_and_nodes(ft, plans):
+    M = 128
+    e = np.array([-0.5, -0.5 + 1e-15, 0.0, 0.5 / M, 1.0 / M, 0.25, 0.5 - 1.0 / M, 0.5 - 1e-15,
+                  3.0 / M + 1e-14, 3.0 / M - 1e-14, 0.49])
+    q = np.array([(x, y) for x in e for y in e]).T.copy()
+    p, _, f, n = _cloud(2000, 7)
+    _both(ft, plans, p, q, f, n, M, M, 24)
+
+
+@pytest.mark.parametrize("M", [512, 1344, 2688])
+def test_gather_either_side_of_the_sparse_line(ft, plans, M):
+    p, q, f, n = _cloud(500, M, nt=65536)
+    _both(ft, plans, p, q, f, n, M, M, 24)
