@@ -257,7 +257,11 @@ __global__ void __launch_bounds__(256) k_geom_coef(RealArgs a, int64_t nnz, int 
     }
 }
 
-// y = A x for R right-hand sides at once; one lane per sorted target row.
+// y = A x for R right-hand sides at once; one lane per sorted target row, W warps
+// (1 << wlog) per slice of 32 rows, warp w taking entries w, w + W, ..  The
+// warps' sums meet in shared memory, in the order of the warps.
+// Bound: load latency with few rows: 32,768 rows of about 700 entries (boundary
+// points) are 1024 slices, 7 warps per SM with one warp each.
 // cff: per RHS, ncf float-float coefficients per sorted source (SLP f1, f2 at
 // 0, 1; DLP S11, S12+S21, S22 at doff), RHS r at cff + r * rstride.  Output
 // ur[r * nt + t] (raw sums, sorted order) per kind.
@@ -268,10 +272,12 @@ __global__ void __launch_bounds__(256) k_geom_apply(int64_t nt, int64_t nnz, con
                                                     const float2 *cff, int ncf, int doff,
                                                     int64_t rstride, const double *cfd_rhs,
                                                     int nc, int doffd, int64_t rstrided, int nr,
-                                                    double2 *ur_slp, double2 *ur_dlp)
+                                                    double2 *ur_slp, double2 *ur_dlp, int wlog)
 {
-    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= nt) return;
+    __shared__ double2 part[8][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int W = 1 << wlog, w = warp & (W - 1);
+    const int64_t t = ((int64_t)blockIdx.x * (8 >> wlog) + (warp >> wlog)) * 32 + lane;
     float su[R][4], sc[R][4];   // Dot2 accumulators: SLP u1, u2, DLP u1, u2
     double ud[R][4];            // FP64 sums of the near entries
 #pragma unroll
@@ -282,9 +288,9 @@ __global__ void __launch_bounds__(256) k_geom_apply(int64_t nt, int64_t nnz, con
             ud[r][i] = 0.0;
         }
     const double *cfd = reinterpret_cast<const double *>(cf);
-    const int n = rowptr[t + 1] - rowptr[t];
-    const int64_t e0 = (int64_t)slice[t >> 5] + (t & 31);
-    for (int k = 0; k < n; k++) {
+    const int n = t < nt ? rowptr[t + 1] - rowptr[t] : 0;
+    const int64_t e0 = t < nt ? (int64_t)slice[t >> 5] + (t & 31) : 0;
+    for (int k = w; k < n; k += W) {
         const int64_t e = e0 + ((int64_t)k << 5);
         const int sraw = src[e];
         const int s = sraw & 0x7fffffff;
@@ -355,14 +361,23 @@ __global__ void __launch_bounds__(256) k_geom_apply(int64_t nt, int64_t nnz, con
 #pragma unroll
     for (int r = 0; r < R; r++) {
         if (r >= nr) break;
-        if (SLP)
-            ur_slp[r * nt + t] =
-                make_double2(ud[r][0] + ff_to_double(ff_norm(su[r][0], sc[r][0])),
-                             ud[r][1] + ff_to_double(ff_norm(su[r][1], sc[r][1])));
-        if (DLP)
-            ur_dlp[r * nt + t] =
-                make_double2(ud[r][2] + ff_to_double(ff_norm(su[r][2], sc[r][2])),
-                             ud[r][3] + ff_to_double(ff_norm(su[r][3], sc[r][3])));
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            if (!(k ? DLP : SLP)) continue;
+            double2 v = make_double2(ud[r][2 * k] + ff_to_double(ff_norm(su[r][2 * k], sc[r][2 * k])),
+                                     ud[r][2 * k + 1] + ff_to_double(ff_norm(su[r][2 * k + 1], sc[r][2 * k + 1])));
+            if (W > 1) {
+                part[warp][lane] = v;
+                __syncthreads();
+                if (w == 0)
+                    for (int q = 1; q < W; q++) {
+                        v.x += part[warp + q][lane].x;
+                        v.y += part[warp + q][lane].y;
+                    }
+                __syncthreads();
+            }
+            if (w == 0 && t < nt) (k ? ur_dlp : ur_slp)[r * nt + t] = v;
+        }
     }
 }
 
@@ -446,11 +461,15 @@ cudaError_t launch_geom_apply(bool slp, bool dlp, int64_t nt, int64_t nnz, const
                               double2 *ur_dlp, cudaStream_t st, int64_t &launches)
 {
     if (nt <= 0 || nr <= 0) return cudaSuccess;
-    const unsigned g = geom_grid(nt, 256);
+    // warps per slice: enough for about 32 warps per SM
+    const int64_t ns = (nt + 31) / 32;
+    int wlog = 0;
+    while (wlog < 3 && (ns << wlog) < 32 * (int64_t)sm_count()) wlog++;
+    const unsigned g = (unsigned)((ns + (8 >> wlog) - 1) / (8 >> wlog));
 #define SE2P_APPLY(S, D, R)                                                                  \
     k_geom_apply<S, D, R><<<g, 256, 0, st>>>(nt, nnz, rowptr, slice, src, cf, cff, ncf, doff,   \
                                              rstride,                                          \
-                                             cfd_rhs, nc, doffd, rstrided, nr, ur_slp, ur_dlp)
+                                             cfd_rhs, nc, doffd, rstrided, nr, ur_slp, ur_dlp, wlog)
     if (nr > 2) {
         if (slp && dlp) SE2P_APPLY(true, true, 4);
         else if (slp) SE2P_APPLY(true, false, 4);
