@@ -35,7 +35,6 @@ constexpr double kPatchNodes = SE2P_PATCH_NODES;   // side of a gather patch, in
 
 enum Slot {
     S_IN_PS, S_IN_PT, S_IN_F, S_IN_FD, S_IN_N,   // staged inputs
-    S_WPS, S_WPT,                               // wrapped positions
     S_SBOX, S_SRANK, S_TBOX, S_TRANK, S_COUNT,  // binning scratch
     S_SSTART, S_TSTART, S_SPERM, S_TPERM, S_TBOXS,
     S_SP, S_TP, S_SPF, S_TPF, S_COEF,           // sorted data
@@ -934,21 +933,6 @@ int run(se2p_plan pl, const Job &J, const Io &io)
         return SE2P_OK;
     }
 
-    // Wrapped positions (driver composites); the raw sources stay for the zero mode.
-    const double2 *ws = ps, *wt = pt;
-    if (J.wrap && !J.reuse_sort) {
-        StageTimer tm(pl, T_WRAP);
-        double2 *a = nullptr, *b = nullptr;
-        if (ns > 0) {
-            CKS(ensure_t(pl, S_WPS, (size_t)ns, &a));
-            CK(launch_wrap(ns, ps, J.Lx, J.Ly, a, st, pl->launches));
-            ws = a;
-        }
-        CKS(ensure_t(pl, S_WPT, (size_t)nt, &b));
-        CK(launch_wrap(nt, pt, J.Lx, J.Ly, b, st, pl->launches));
-        wt = b;
-    }
-
     // Boxes: the real-space cell list when the real part runs, otherwise
     // tiles of about 16 grid cells (locality only).
     int nx = J.nx, ny = J.ny;
@@ -964,7 +948,7 @@ int run(se2p_plan pl, const Job &J, const Io &io)
     CKS(ensure_t(pl, S_SRANK, nsz, &srank));
     CKS(ensure_t(pl, S_TBOX, ntz, &tbox));
     CKS(ensure_t(pl, S_TRANK, ntz, &trank));
-    CKS(ensure_t(pl, S_COUNT, (size_t)nbox, &count));
+    CKS(ensure_t(pl, S_COUNT, 2 * (size_t)nbox, &count));
     CKS(ensure_t(pl, S_SSTART, (size_t)nbox + 1, &sstart));
     CKS(ensure_t(pl, S_TSTART, (size_t)nbox + 1, &tstart));
     CKS(ensure_t(pl, S_SPERM, nsz, &sperm));
@@ -984,22 +968,31 @@ int run(se2p_plan pl, const Job &J, const Io &io)
         }
     }
     if (!J.reuse_sort) {
-    StageTimer tm(pl, T_SORT);
-    BinArgs bs{ws, ns, J.Lx, J.Ly, nx, ny, sbox, srank, count};
-    CK(launch_bin(bs, sstart, nbox, sperm, nullptr, sp, spf, st, pl->launches, spl));
-    BinArgs bt{wt, nt, J.Lx, J.Ly, nx, ny, tbox, trank, count};
-    CK(launch_bin(bt, tstart, nbox, tperm, tboxs, tp, tpf, st, pl->launches, tpl));
+        // (the drivers' wrap included; the zero mode takes the raw sources)
+        StageTimer tm(pl, T_SORT);
+        const SortArgs so{{{ps, ns, sbox, srank, count, sstart, sperm, nullptr, sp, spf, spl},
+                           {pt, nt, tbox, trank, count + nbox, tstart, tperm, tboxs, tp, tpf, tpl}},
+                          J.Lx, J.Ly, 1.0 / J.Lx, 1.0 / J.Ly, nx, ny, J.wrap ? 1 : 0};
+        CK(launch_sort(so, 2, st, pl->launches));
     }
 
     const int nc = (J.slp ? 2 : 0) + (J.dlp ? 3 : 0);
     const int doff = J.slp ? 2 : 0;
+    // the sources' coefficients, and for the float-float and FP32 real space
+    // their float-float copy (the latter reads its high halves)
+    const int form = pl->precision == SE2P_PRECISION_FP32_GRID    ? kFormF32
+                     : pl->precision == SE2P_PRECISION_FP64_NATIVE ? kFormFP64
+                                                                    : kFormFF;
+    const int ncf = (J.slp ? 2 : 0) + (J.dlp ? 5 : 0);
     double *coef = nullptr;
+    float2 *cff = nullptr;
     CKS(ensure_t(pl, S_COEF, (size_t)nc * nsz, &coef));
+    if (J.real && form != kFormFP64) CKS(ensure_t(pl, S_COEF_FF, (size_t)ncf * nsz, &cff));
     CK(cudaStreamWaitEvent(st, pl->cin1, 0));        // the densities are in
     {
         StageTimer tm(pl, T_COEF);
         CK(launch_src_coef(ns, sperm, J.slp ? fs : nullptr, J.dlp ? fd : nullptr, nr, coef, nc, st,
-                           pl->launches));
+                           pl->launches, cff, ncf));
     }
 
     double2 *ur_slp = nullptr, *ur_dlp = nullptr, *uk = nullptr;
@@ -1046,23 +1039,14 @@ int run(se2p_plan pl, const Job &J, const Io &io)
             }
             ra.counters = static_cast<unsigned long long *>(pl->buf[S_COUNTERS].p);
         }
-        const int form = pl->precision == SE2P_PRECISION_FP32_GRID    ? kFormF32
-                         : pl->precision == SE2P_PRECISION_FP64_NATIVE ? kFormFP64
-                                                                        : kFormFF;
         ra.coef_ff = nullptr;
         ra.ncf = 0;
         ra.doff_ff = 0;
         ra.gtab = nullptr;
         ra.spl = spl;
         ra.tpl = tpl;
-        if (form == kFormFF || form == kFormF32) {
-            // float-float coefficients (the FP32-grid form reads their high halves)
-            const int ncf = (J.slp ? 2 : 0) + (J.dlp ? 5 : 0);
-            float2 *cff = nullptr;
-            CKS(ensure_t(pl, S_COEF_FF, (size_t)ncf * nsz, &cff));
-            if (form == kFormFF) CKS(gtab_device(pl, st, &ra.gtab));
-            StageTimer tm(pl, T_COEF);
-            CK(launch_src_coef_ff(ns, coef, nc, J.slp, J.dlp, cff, ncf, st, pl->launches));
+        if (form == kFormFF) CKS(gtab_device(pl, st, &ra.gtab));
+        if (cff) {
             ra.coef_ff = cff;
             ra.ncf = ncf;
             ra.doff_ff = J.slp ? 2 : 0;
@@ -1288,11 +1272,6 @@ int run(se2p_plan pl, const Job &J, const Io &io)
         if (!tg) CK(launch_gather(ga, nout, ks, pl->launches));
     }
 
-    if (ks != st) {
-        CK(cudaEventRecord(pl->kjoin, ks));
-        CK(cudaStreamWaitEvent(st, pl->kjoin, 0));
-    }
-
     double2 *zm = nullptr;
     if (J.zero_mode && J.dlp) {
         double2 *part = nullptr;
@@ -1303,16 +1282,20 @@ int run(se2p_plan pl, const Job &J, const Io &io)
         CK(launch_zero_mode(ns, ps, fd, nr, 1.0 / (J.Lx * J.Ly), part, zm, st, pl->launches));
     }
 
+    if (ks != st) {
+        CK(cudaEventRecord(pl->kjoin, ks));
+        CK(cudaStreamWaitEvent(st, pl->kjoin, 0));
+    }
     if (J.real && J.kspace && pl->overlap) CK(cudaStreamWaitEvent(st, pl->join, 0));
     StageTimer *t_asm = new StageTimer(pl, T_ASSEMBLE);
     const double2 *uk_slp = (J.kspace && J.slp) ? uk : nullptr;
     const double2 *uk_dlp = (J.kspace && J.dlp) ? uk + (J.slp ? nt : 0) : nullptr;
+    AssembleArgs as;
     if (J.slp && o_us.dev)
-        CK(launch_assemble(nt, io.mode_slp, tperm, J.real ? ur_slp : nullptr, uk_slp, nullptr,
-                           o_us.dev, o_urs.dev, o_uks.dev, st, pl->launches));
+        as.add(io.mode_slp, J.real ? ur_slp : nullptr, uk_slp, nullptr, o_us.dev, o_urs.dev, o_uks.dev);
     if (J.dlp && o_ud.dev)
-        CK(launch_assemble(nt, io.mode_dlp, tperm, J.real ? ur_dlp : nullptr, uk_dlp, zm,
-                           o_ud.dev, o_urd.dev, o_ukd.dev, st, pl->launches));
+        as.add(io.mode_dlp, J.real ? ur_dlp : nullptr, uk_dlp, zm, o_ud.dev, o_urd.dev, o_ukd.dev);
+    CK(launch_assemble(nt, tperm, as, st, pl->launches));
 
     delete t_asm;
     StageTimer *t_out = new StageTimer(pl, T_STAGE_OUT);
@@ -1371,12 +1354,6 @@ int run_adjoint(se2p_plan pl, const Job &J, const AdjIo &io)
     if (ns == 0) return SE2P_OK;
 
     const size_t nsz = (size_t)ns, ntz = (size_t)(nt > 0 ? nt : 1);
-    double2 *ws = nullptr, *wt = nullptr;
-    CKS(ensure_t(pl, S_WPS, nsz, &ws));
-    CKS(ensure_t(pl, S_WPT, ntz, &wt));
-    CK(launch_wrap(ns, ps, J.Lx, J.Ly, ws, st, pl->launches));
-    CK(launch_wrap(nt, pt, J.Lx, J.Ly, wt, st, pl->launches));
-
     const int nx = J.nx, ny = J.ny, nbox = nx * ny;
     int *sbox, *srank, *tbox, *trank, *count, *sstart, *tstart, *sperm, *tperm, *tboxs, *sboxs;
     double2 *sp, *tp;
@@ -1385,7 +1362,7 @@ int run_adjoint(se2p_plan pl, const Job &J, const AdjIo &io)
     CKS(ensure_t(pl, S_SRANK, nsz, &srank));
     CKS(ensure_t(pl, S_TBOX, ntz, &tbox));
     CKS(ensure_t(pl, S_TRANK, ntz, &trank));
-    CKS(ensure_t(pl, S_COUNT, (size_t)nbox, &count));
+    CKS(ensure_t(pl, S_COUNT, 2 * (size_t)nbox, &count));
     CKS(ensure_t(pl, S_SSTART, (size_t)nbox + 1, &sstart));
     CKS(ensure_t(pl, S_TSTART, (size_t)nbox + 1, &tstart));
     CKS(ensure_t(pl, S_SPERM, nsz, &sperm));
@@ -1398,10 +1375,10 @@ int run_adjoint(se2p_plan pl, const Job &J, const AdjIo &io)
     CKS(ensure_t(pl, S_TPF, ntz, &tpf));
     {
         StageTimer tm(pl, T_SORT);
-        BinArgs bs{ws, ns, J.Lx, J.Ly, nx, ny, sbox, srank, count};
-        CK(launch_bin(bs, sstart, nbox, sperm, sboxs, sp, spf, st, pl->launches));
-        BinArgs bt{wt, nt, J.Lx, J.Ly, nx, ny, tbox, trank, count};
-        CK(launch_bin(bt, tstart, nbox, tperm, tboxs, tp, tpf, st, pl->launches));
+        const SortArgs so{{{ps, ns, sbox, srank, count, sstart, sperm, sboxs, sp, spf, nullptr},
+                           {pt, nt, tbox, trank, count + nbox, tstart, tperm, tboxs, tp, tpf, nullptr}},
+                          J.Lx, J.Ly, 1.0 / J.Lx, 1.0 / J.Ly, nx, ny, 1};
+        CK(launch_sort(so, 2, st, pl->launches));
     }
     // 5 coefficients per sorted source (absent kinds as zeros) and the
     // targets' weights (w_slp, w_dlp) in sorted order.
@@ -2037,22 +2014,17 @@ static int geom_build(se2p_geom g, const double *psrc, const double *ptar, const
     CKS(geom_alloc(g, ntz + 1, &g->rowptr));
     CKS(geom_alloc(g, (ntz + 31) / 32 + 1, &g->slice));
     // wrap, then sort into the real-space boxes
-    double2 *ws = nullptr, *wt = nullptr;
     int *sbox, *srank, *tbox, *trank, *count, *tstart;
-    CKS(ensure_t(pl, S_WPS, nsz, &ws));
-    CKS(ensure_t(pl, S_WPT, ntz, &wt));
     CKS(ensure_t(pl, S_SBOX, nsz, &sbox));
     CKS(ensure_t(pl, S_SRANK, nsz, &srank));
     CKS(ensure_t(pl, S_TBOX, ntz, &tbox));
     CKS(ensure_t(pl, S_TRANK, ntz, &trank));
-    CKS(ensure_t(pl, S_COUNT, (size_t)nbox, &count));
+    CKS(ensure_t(pl, S_COUNT, 2 * (size_t)nbox, &count));
     CKS(ensure_t(pl, S_TSTART, (size_t)nbox + 1, &tstart));
-    if (ns > 0) CK(launch_wrap(ns, g->ps, p.Lx, p.Ly, ws, st, pl->launches));
-    if (nt > 0) CK(launch_wrap(nt, g->pt, p.Lx, p.Ly, wt, st, pl->launches));
-    BinArgs bs{ws, ns, p.Lx, p.Ly, nx, ny, sbox, srank, count};
-    CK(launch_bin(bs, g->sstart, nbox, g->sperm, nullptr, g->sp, g->spf, st, pl->launches));
-    BinArgs bt{wt, nt, p.Lx, p.Ly, nx, ny, tbox, trank, count};
-    CK(launch_bin(bt, tstart, nbox, g->tperm, g->tboxs, g->tp, g->tpf, st, pl->launches));
+    const SortArgs so{{{g->ps, ns, sbox, srank, count, g->sstart, g->sperm, nullptr, g->sp, g->spf, nullptr},
+                       {g->pt, nt, tbox, trank, count + nbox, tstart, g->tperm, g->tboxs, g->tp, g->tpf, nullptr}},
+                      p.Lx, p.Ly, 1.0 / p.Lx, 1.0 / p.Ly, nx, ny, 1};
+    CK(launch_sort(so, 2, st, pl->launches));
 
     RealArgs ra{};
     ra.sp = g->sp;
@@ -2388,9 +2360,8 @@ int se2p_geom_apply(se2p_geom g, int nrhs, const double *f_slp, const double *f_
             const double2 *fs = g->slp ? g->fin + (size_t)(r0 + r) * ns : nullptr;
             const double2 *fd = g->dlp ? g->din + (size_t)(r0 + r) * ns : nullptr;
             double *cr = coef + (size_t)r * nc * nsz;
-            CK(launch_src_coef(ns, g->sperm, fs, fd, g->nr, cr, nc, st, pl->launches));
-            CK(launch_src_coef_ff(ns, cr, nc, g->slp, g->dlp, cff + (size_t)r * ncf, ncf,
-                                  st, pl->launches, (int64_t)nb * ncf, false));
+            CK(launch_src_coef(ns, g->sperm, fs, fd, g->nr, cr, nc, st, pl->launches,
+                               cff + (size_t)r * ncf, (int64_t)nb * ncf, false));
         }
         CK(cudaEventRecord(pl->fork, st));
         CK(cudaStreamWaitEvent(pl->side, pl->fork, 0));
@@ -2417,17 +2388,15 @@ int se2p_geom_apply(se2p_geom g, int nrhs, const double *f_slp, const double *f_
         }
         CK(cudaStreamWaitEvent(st, pl->join, 0));
         StageTimer tm(pl, T_ASSEMBLE);
+        AssembleArgs as;
         for (int r = 0; r < nb; r++) {
             const int rr = r0 + r;
             const double2 *ukr = uk + (size_t)r * nk2 * nt;
-            if (g->slp)
-                CK(launch_assemble(nt, 3, g->tperm, ur0 + (size_t)r * nt, ukr, nullptr,
-                                   uo_slp + (size_t)rr * nt, nullptr, nullptr, st, pl->launches));
+            if (g->slp) as.add(3, ur0 + (size_t)r * nt, ukr, nullptr, uo_slp + (size_t)rr * nt);
             if (g->dlp)
-                CK(launch_assemble(nt, 4, g->tperm, ur1 + (size_t)r * nt, ukr + (g->slp ? nt : 0),
-                                   zm + r, uo_dlp + (size_t)rr * nt, nullptr, nullptr, st,
-                                   pl->launches));
+                as.add(4, ur1 + (size_t)r * nt, ukr + (g->slp ? nt : 0), zm + r, uo_dlp + (size_t)rr * nt);
         }
+        CK(launch_assemble(nt, g->tperm, as, st, pl->launches));
     }
     for (int r0 = 0; r0 < nrhs && !multi; r0 += kBatch) {
         const int nb = std::min(kBatch, nrhs - r0);
@@ -2436,9 +2405,8 @@ int se2p_geom_apply(se2p_geom g, int nrhs, const double *f_slp, const double *f_
             const double2 *fs = g->slp ? g->fin + (size_t)(r0 + r) * ns : nullptr;
             const double2 *fd = g->dlp ? g->din + (size_t)(r0 + r) * ns : nullptr;
             double *cr = coef + (size_t)r * nc * nsz;
-            CK(launch_src_coef(ns, g->sperm, fs, fd, g->nr, cr, nc, st, pl->launches));
-            CK(launch_src_coef_ff(ns, cr, nc, g->slp, g->dlp, cff + (size_t)r * ncf, ncf,
-                                  st, pl->launches, (int64_t)nb * ncf, false));
+            CK(launch_src_coef(ns, g->sperm, fs, fd, g->nr, cr, nc, st, pl->launches,
+                               cff + (size_t)r * ncf, (int64_t)nb * ncf, false));
         }
         {
             StageTimer tm(pl, T_REAL);
@@ -2624,16 +2592,14 @@ extern "C" int se2p_slp_real_noalloc(const double *psrc, int64_t ns, const doubl
     int64_t launches = 0;
     const double2 *ps = reinterpret_cast<const double2 *>(psrc);
     const double2 *pt = reinterpret_cast<const double2 *>(ptar);
-    BinArgs bs{ps, ns, Lx, Ly, nside_x, nside_y, sbox, srank, count};
-    if (launch_bin(bs, sstart, (int)nbox, sperm, nullptr, sp, spf, st, launches) != cudaSuccess)
-        return SE2P_ERR_CUDA;
-    BinArgs bt{pt, nt, Lx, Ly, nside_x, nside_y, tbox, trank, count};
-    if (launch_bin(bt, tstart, (int)nbox, tperm, tboxs, tp, tpf, st, launches) != cudaSuccess)
-        return SE2P_ERR_CUDA;
+    // (one set at a time: they share the box counts)
+    SortArgs so{{{ps, ns, sbox, srank, count, sstart, sperm, nullptr, sp, spf, nullptr}, {}},
+                Lx, Ly, 1.0 / Lx, 1.0 / Ly, nside_x, nside_y, 0};
+    if (launch_sort(so, 1, st, launches) != cudaSuccess) return SE2P_ERR_CUDA;
+    so.s[0] = SortSet{pt, nt, tbox, trank, count, tstart, tperm, tboxs, tp, tpf, nullptr};
+    if (launch_sort(so, 1, st, launches) != cudaSuccess) return SE2P_ERR_CUDA;
     if (launch_src_coef(ns, sperm, reinterpret_cast<const double2 *>(f), nullptr, nullptr, coef,
-                        2, st, launches) != cudaSuccess)
-        return SE2P_ERR_CUDA;
-    if (launch_src_coef_ff(ns, coef, 2, true, false, coef_ff, 2, st, launches) != cudaSuccess)
+                        2, st, launches, coef_ff, 2) != cudaSuccess)
         return SE2P_ERR_CUDA;
     // The same real-space arguments and form as se2p_slp_real on a plan of
     // the default precision (SE2P_PRECISION_FP64: far pairs in float-float).
@@ -2672,8 +2638,8 @@ extern "C" int se2p_slp_real_noalloc(const double *psrc, int64_t ns, const doubl
     ra.doff_ff = 0;
     ra.gtab = static_cast<const float4 *>(gt);
     if (launch_real(ra, true, false, st, launches, kFormFF) != cudaSuccess) return SE2P_ERR_CUDA;
-    if (launch_assemble(nt, 0, tperm, ur, nullptr, nullptr, reinterpret_cast<double2 *>(u), nullptr,
-                        nullptr, st, launches) != cudaSuccess)
-        return SE2P_ERR_CUDA;
+    AssembleArgs as;
+    as.add(0, ur, nullptr, nullptr, reinterpret_cast<double2 *>(u));
+    if (launch_assemble(nt, tperm, as, st, launches) != cudaSuccess) return SE2P_ERR_CUDA;
     return SE2P_OK;
 }

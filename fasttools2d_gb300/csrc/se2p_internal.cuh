@@ -258,12 +258,35 @@ __device__ __forceinline__ double e1_pade(double x, double e)
 // ---------------------------------------------------------------------------
 // Kernel argument blocks
 // ---------------------------------------------------------------------------
-struct BinArgs {
+// One or two point sets sorted into the same boxes (launch_sort).
+struct SortSet {
     const double2 *p;   // interleaved (x, y) per point
     int64_t n;
-    double Lx, Ly;
-    int nx, ny;
-    int *box, *rank, *count;
+    int *box, *rank, *count, *start;   // per point; per box (count may follow the other set's)
+    int *perm, *sorted_box;            // sorted -> caller's number; box per sorted point (or null)
+    double2 *sp;                       // sorted positions
+    float2 *spf, *spl;                 // and their FP32 high and low halves (or null)
+};
+struct SortArgs {
+    SortSet s[2];
+    double Lx, Ly, inv_Lx, inv_Ly;
+    int nx, ny, wrap;   // wrap: mod(p + L/2, L) - L/2 first
+};
+
+// Outputs of one call in the caller's order (k_assemble).
+struct AssembleOut {
+    int mode;
+    const double2 *ur, *uk, *zm;
+    double2 *u, *ur_out, *uk_out;
+};
+struct AssembleArgs {
+    AssembleOut o[8];
+    int nout = 0;
+    void add(int mode, const double2 *ur, const double2 *uk, const double2 *zm, double2 *u,
+             double2 *ur_out = nullptr, double2 *uk_out = nullptr)
+    {
+        o[nout++] = AssembleOut{mode, ur, uk, zm, u, ur_out, uk_out};
+    }
 };
 
 struct RealArgs {
@@ -455,19 +478,14 @@ struct GatherArgsF {
 // ---------------------------------------------------------------------------
 // Host launchers (se2p_kernels.cu).  Each returns the launch status.
 // ---------------------------------------------------------------------------
-cudaError_t launch_bin(const BinArgs &a, int *start, int nbox, int *perm, int *sorted_box,
-                       double2 *sorted_pos, float2 *sorted_pos_f, cudaStream_t st,
-                       int64_t &launches,
-                       float2 *sorted_pos_lo = nullptr);
+cudaError_t launch_sort(const SortArgs &a, int nsets, cudaStream_t st, int64_t &launches);
+// out: the float-float copy, ostride float2 per source (tails = false leaves out
+// the DLP pair 3 S11 + S22, 3 S22 + S11: the real-space kernels read it, the
+// geometry's stored operator does not).
 cudaError_t launch_src_coef(int64_t n, const int *perm, const double2 *f_slp,
                             const double2 *f_dlp, const double2 *nrm, double *coef, int nc,
-                            cudaStream_t st, int64_t &launches);
-// out: per source ostride float2 (ncf when 0) from out + ostride j; tails =
-// false leaves out the DLP pair 3 S11 + S22, 3 S22 + S11 (the real-space
-// kernels read it, the geometry's stored operator does not).
-cudaError_t launch_src_coef_ff(int64_t n, const double *coef, int nc, bool slp, bool dlp,
-                               float2 *out, int ncf, cudaStream_t st, int64_t &launches,
-                               int64_t ostride = 0, bool tails = true);
+                            cudaStream_t st, int64_t &launches, float2 *out = nullptr,
+                            int64_t ostride = 0, bool tails = true);
 cudaError_t launch_real(const RealArgs &a, bool slp, bool dlp, cudaStream_t st,
                         int64_t &launches, int form = kFormFP64);
 // 2D real FFT through 1D complex passes (se2p_kernels.cu): pack real grid
@@ -654,14 +672,11 @@ cudaError_t launch_filter(const FilterArgs &a, cudaStream_t st, int64_t &launche
 cudaError_t launch_filter_matrix_table(const FilterArgs &a, double *mtab, cudaStream_t st,
                                        int64_t &launches);
 cudaError_t launch_gather(const GatherArgs &a, int nc, cudaStream_t st, int64_t &launches);
-cudaError_t launch_wrap(int64_t n, const double2 *p, double Lx, double Ly, double2 *out,
-                        cudaStream_t st, int64_t &launches);
 cudaError_t launch_zero_mode(int64_t n, const double2 *p, const double2 *f, const double2 *nrm,
                              double inv_area, double2 *part, double2 *zm, cudaStream_t st,
                              int64_t &launches);
-cudaError_t launch_assemble(int64_t n, int mode, const int *perm, const double2 *ur,
-                            const double2 *uk, const double2 *zm, double2 *u, double2 *ur_out,
-                            double2 *uk_out, cudaStream_t st, int64_t &launches);
+cudaError_t launch_assemble(int64_t n, const int *perm, const AssembleArgs &a, cudaStream_t st,
+                            int64_t &launches);
 constexpr int kZeroModeParts = 304;
 
 // g(x) = exp(x) E1(x) in the reference's Pade form (mid set below 16, far

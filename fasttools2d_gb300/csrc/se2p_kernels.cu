@@ -24,20 +24,74 @@ namespace se2p {
 // atomics, so it is not the reference's input order; only FP64 summation
 // order depends on it.
 // ===========================================================================
-__global__ void k_bin_count(BinArgs a)
+// MATLAB mod(x + L/2, L) - L/2: mod(a, L) = a - floor(a/L) L computed exactly (fmod, then + L
+// when the sign differs from L): the MATLAB drivers' wrap
+// (StokesSLP_ewald_2p.m:75-78).  a within a period of [0, L) needs no fmod (a - L
+// is exact for L <= a < 2 L; fmod leaves -L < a < 0 as it is).
+// (Comparisons on the bit patterns, which order like the numbers from 0 up:
+// FP64 comparisons issue at the FP64 rate.)
+__device__ __forceinline__ double wrap_coord(double x, double L)
 {
+    const double a = xadd(x, 0.5 * L);
+    const long long ab = __double_as_longlong(a), Lb = __double_as_longlong(L);
+    double r;
+    if ((unsigned long long)ab < (unsigned long long)Lb) {             // 0 <= a < L
+        r = a;
+    } else if (ab > 0 && ab < Lb + (1ll << 52)) {                      // L <= a < 2 L
+        r = xsub(a, L);
+    } else if ((unsigned long long)ab - (1ull << 63) < (unsigned long long)Lb && ab != (long long)(1ull << 63)) {
+        r = xadd(a, L);                                                // -L < a < 0
+    } else {
+        r = fmod(a, L);
+        if (r < 0.0) r = xadd(r, L);
+        if (r == 0.0) r = 0.0;                                         // (no negative zero)
+    }
+    return xsub(r, 0.5 * L);
+}
+
+// box1 with a product in place of its division and the rest in fixed point: v = x / L
+// + 1/2 as a fraction of 2^64, nside v's integer part.  Within 2^-20 of an integer
+// (v itself is good to 2^-51, times nside below 2^26 boxes), out of [2^-40, 1)
+// and for NaN, box1 decides.
+__device__ __forceinline__ int box1_fast(double x, double L, double inv_L, int nside)
+{
+    const unsigned long long b = (unsigned long long)__double_as_longlong(fma(x, inv_L, 0.5));
+    const int sh = 1022 - (int)(b >> 52);            // (a negative v gives a huge field)
+    if ((unsigned)sh >= 40u) return box1(x, L, nside);
+    const unsigned long long u = ((b << 11) | (1ull << 63)) >> sh;
+    const unsigned long long f = u * (unsigned)nside;
+    if (f + (1ull << 44) < (1ull << 45)) return box1(x, L, nside);
+    return (int)__umul64hi(u, (unsigned)nside);
+}
+
+// x rounded to the nearest float, on the integer pipe where the float is
+// normal (conversions issue at the FP64 rate).
+__device__ __forceinline__ float f32_rn(double x)
+{
+    const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+    const int e = (int)(b >> 52) & 0x7ff;
+    if (e < 897 || e > 1149) return (float)x;
+    const unsigned long long m = (b & 0x7fffffffffffffffull) - (896ull << 52);
+    const unsigned r = (unsigned)((m + 0xfffffffull + ((m >> 29) & 1)) >> 29);
+    return __uint_as_float(r | ((unsigned)(b >> 32) & 0x80000000u));
+}
+
+// (blockIdx.y: the point set)
+__global__ void __launch_bounds__(256) k_sort_count(SortArgs a)
+{
+    const SortSet &s = a.s[blockIdx.y];
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= a.n) return;
-    const double2 q = a.p[i];
-    const int b = box1(q.y, a.Ly, a.ny) * a.nx + box1(q.x, a.Lx, a.nx);
-    a.box[i] = b;
-    a.rank[i] = atomicAdd(&a.count[b], 1);
+    if (i >= s.n) return;
+    double2 q = s.p[i];
+    if (a.wrap) q = make_double2(wrap_coord(q.x, a.Lx), wrap_coord(q.y, a.Ly));
+    const int b = box1_fast(q.y, a.Ly, a.inv_Ly, a.ny) * a.nx + box1_fast(q.x, a.Lx, a.inv_Lx, a.nx);
+    s.box[i] = b;
+    s.rank[i] = atomicAdd(&s.count[b], 1);
 }
 
 // Exclusive scan of count[0..n) into start[0..n], one block of 1024 threads,
 // 8 consecutive items per thread per chunk.
-__global__ void __launch_bounds__(1024) k_scan(const int *__restrict__ count, int n,
-                                                 int *__restrict__ start)
+__device__ __forceinline__ void scan_block(const int *__restrict__ count, int n, int *__restrict__ start)
 {
     __shared__ int warp_tot[32];
     __shared__ int carry_s;
@@ -83,26 +137,72 @@ __global__ void __launch_bounds__(1024) k_scan(const int *__restrict__ count, in
     if (tid == 0) start[n] = carry_s;
 }
 
-// Sorted slot of point i; writes the permutation and the sorted copies.
-__global__ void k_bin_place(int64_t n, const int *__restrict__ box, const int *__restrict__ rank,
-                            const int *__restrict__ start, int *__restrict__ perm,
-                            int *__restrict__ sorted_box, const double2 *__restrict__ p,
-                            double2 *__restrict__ sp, float2 *__restrict__ spf,
-                            float2 *__restrict__ spl)
+__global__ void __launch_bounds__(1024) k_scan(const int *__restrict__ count, int n,
+                                                 int *__restrict__ start)
 {
+    scan_block(count, n, start);
+}
+
+// Up to kScanWide boxes, a block scans 1024 of them and adds up the counts before
+// them itself (blockIdx.y: the point set): 31,684 boxes in 5 us, one block over
+// all of them 24 us.  The repeated reads grow with the square, so beyond that one
+// block per set.
+constexpr int kScanWide = 1 << 17;
+
+__global__ void __launch_bounds__(1024) k_sort_scan(SortArgs a)
+{
+    const int *count = a.s[blockIdx.y].count;
+    int *start = a.s[blockIdx.y].start;
+    const int n = a.nx * a.ny;
+    if (n > kScanWide) {
+        scan_block(count, n, start);
+        return;
+    }
+    __shared__ int warp_tot[32], before[32];
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const int base = blockIdx.x * 1024, i = base + tid;
+    int pre = 0;
+    for (int k = tid; k < base; k += 1024) pre += count[k];
+    const int own = i < n ? count[i] : 0;
+    int inc = own;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int x = __shfl_up_sync(~0u, inc, o);
+        if (lane >= o) inc += x;
+        pre += __shfl_xor_sync(~0u, pre, o);
+    }
+    if (lane == 31) {
+        warp_tot[wid] = inc;
+        before[wid] = pre;
+    }
+    __syncthreads();
+    int run = inc - own;
+    for (int w = 0; w < 32; w++) run += before[w] + (w < wid ? warp_tot[w] : 0);
+    if (i < n) {
+        start[i] = run;
+        if (i == n - 1) start[n] = run + own;
+    }
+}
+
+// Sorted slot of point i; writes the permutation and the sorted copies.
+__global__ void __launch_bounds__(256) k_sort_place(SortArgs a)
+{
+    const SortSet &s = a.s[blockIdx.y];
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int b = box[i];
-    const int j = start[b] + rank[i];
-    perm[j] = (int)i;
-    if (sorted_box) sorted_box[j] = b;
-    const double2 q = p[i];
-    sp[j] = q;
-    const float hx = (float)q.x, hy = (float)q.y;
-    if (spf) spf[j] = make_float2(hx, hy);
+    if (i >= s.n) return;
+    const int b = s.box[i];
+    const int j = s.start[b] + s.rank[i];
+    s.perm[j] = (int)i;
+    if (s.sorted_box) s.sorted_box[j] = b;
+    double2 q = s.p[i];
+    if (a.wrap) q = make_double2(wrap_coord(q.x, a.Lx), wrap_coord(q.y, a.Ly));
+    s.sp[j] = q;
+    if (!s.spf) return;
+    const float hx = f32_rn(q.x), hy = f32_rn(q.y);
+    s.spf[j] = make_float2(hx, hy);
     // q - hi is exact in FP64; its rounding to FP32 leaves hi + lo within
     // 2^-48 |q| of q
-    if (spl) spl[j] = make_float2((float)(q.x - (double)hx), (float)(q.y - (double)hy));
+    if (s.spl) s.spl[j] = make_float2(f32_rn(q.x - (double)hx), f32_rn(q.y - (double)hy));
 }
 
 // Per-source coefficients in sorted order, nc per source: SLP f (f1, f2),
@@ -110,51 +210,45 @@ __global__ void k_bin_place(int64_t n, const int *__restrict__ box, const int *_
 // (PE/src/mex/StokesDLP/mex_stokes_dlp_real.cpp:81-91; S12 and S21 only ever
 // enter as their sum, in the real-space contraction and as H2+H3 in the
 // DLP filter).  The same array is the spread's per-grid weights.
-__global__ void k_src_coef(int64_t n, const int *__restrict__ perm,
+//
+// With out, also the float-float copy for the far pairs of the FP64 form: SLP f1,
+// f2; DLP S11, S12+S21, S22 and (tails) the combinations 3 S11 + S22, 3 S22 + S11
+// of the stresslet contraction (formed in FP64, then split).
+__global__ void __launch_bounds__(256) k_src_coef(int64_t n, const int *__restrict__ perm,
                            const double2 *__restrict__ f_slp, const double2 *__restrict__ f_dlp,
-                           const double2 *__restrict__ nrm, double *__restrict__ coef, int nc)
+                           const double2 *__restrict__ nrm, double *__restrict__ coef, int nc,
+                           float2 *__restrict__ out, int64_t ostride, int tails)
 {
     const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= n) return;
     const int i = perm[j];
     double *c = coef + (int64_t)nc * j;
+    float2 *o = out ? out + ostride * j : nullptr;
     if (f_slp) {
         const double2 f = f_slp[i];
         c[0] = f.x;
         c[1] = f.y;
         c += 2;
+        if (o) {
+            o[0] = ff_split(f.x);
+            o[1] = ff_split(f.y);
+            o += 2;
+        }
     }
     if (f_dlp) {
         const double2 f = f_dlp[i], m = nrm[i];
-        c[0] = f.x * m.x;
-        c[1] = f.x * m.y + f.y * m.x;
-        c[2] = f.y * m.y;
-    }
-}
-
-// Float-float copy of the sorted coefficients for the far pairs of the FP64
-// form: SLP f1, f2; DLP S11, S12+S21, S22 and the combinations 3 S11 + S22,
-// 3 S22 + S11 of the stresslet contraction (formed in FP64, then split).
-__global__ void k_src_coef_ff(int64_t n, const double *__restrict__ coef, int nc, int slp,
-                              int dlp, float2 *__restrict__ out, int64_t ostride, int tails)
-{
-    const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n) return;
-    const double *c = coef + (int64_t)nc * j;
-    float2 *o = out + ostride * j;
-    if (slp) {
-        o[0] = ff_split(c[0]);
-        o[1] = ff_split(c[1]);
-        c += 2;
-        o += 2;
-    }
-    if (dlp) {
-        o[0] = ff_split(c[0]);
-        o[1] = ff_split(c[1]);
-        o[2] = ff_split(c[2]);
-        if (tails) {
-            o[3] = ff_split(fma(3.0, c[0], c[2]));
-            o[4] = ff_split(fma(3.0, c[2], c[0]));
+        const double s0 = f.x * m.x, s1 = f.x * m.y + f.y * m.x, s2 = f.y * m.y;
+        c[0] = s0;
+        c[1] = s1;
+        c[2] = s2;
+        if (o) {
+            o[0] = ff_split(s0);
+            o[1] = ff_split(s1);
+            o[2] = ff_split(s2);
+            if (tails) {
+                o[3] = ff_split(fma(3.0, s0, s2));
+                o[4] = ff_split(fma(3.0, s2, s0));
+            }
         }
     }
 }
@@ -2971,16 +3065,27 @@ __global__ void __launch_bounds__(256) k_wsum_part(int64_t n, const double *__re
     }
 }
 
-// part[nparts] = the sum of part[0 .. nparts-1], added in index order.
-__global__ void k_wsum_final(int nparts, double2 *__restrict__ part)
+// The sum of part[0 .. nparts-1] by one warp (37 us by one thread).
+__device__ __forceinline__ double2 sum_parts(int nparts, const double2 *__restrict__ part)
 {
-    if (threadIdx.x != 0) return;
     double2 t = make_double2(0.0, 0.0);
-    for (int b = 0; b < nparts; b++) {
+    for (int b = threadIdx.x; b < nparts; b += 32) {
         t.x += part[b].x;
         t.y += part[b].y;
     }
-    part[nparts] = t;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        t.x += __shfl_xor_sync(~0u, t.x, o);
+        t.y += __shfl_xor_sync(~0u, t.y, o);
+    }
+    return t;
+}
+
+// part[nparts] = the sum of part[0 .. nparts-1].
+__global__ void __launch_bounds__(32) k_wsum_final(int nparts, double2 *__restrict__ part)
+{
+    const double2 t = sum_parts(nparts, part);
+    if (threadIdx.x == 0) part[nparts] = t;
 }
 
 // Combine the real-space (gr, 7 per sorted source, unscaled) and k-space (gk,
@@ -3016,34 +3121,6 @@ __global__ void k_adj_assemble(int64_t n, const int *__restrict__ perm,
     if (g_pos) g_pos[i] = make_double2(gp1, gp2);
 }
 
-// ===========================================================================
-// Small helpers
-// ===========================================================================
-
-// x -> mod(x + L/2, L) - L/2 as numpy.mod computes it (exact fmod, then +L
-// when the sign differs from L): the MATLAB drivers' wrap
-// (StokesSLP_ewald_2p.m:75-78).
-__device__ __forceinline__ double wrap_coord(double x, double L)
-{
-    const double a = xadd(x, 0.5 * L);
-    double r = fmod(a, L);
-    if (r != 0.0) {
-        if ((r < 0.0) != (L < 0.0)) r = xadd(r, L);
-    } else {
-        r = copysign(0.0, L);
-    }
-    return xsub(r, 0.5 * L);
-}
-
-__global__ void k_wrap(int64_t n, const double2 *__restrict__ p, double Lx, double Ly,
-                       double2 *__restrict__ out)
-{
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const double2 q = p[i];
-    out[i] = make_double2(wrap_coord(q.x, Lx), wrap_coord(q.y, Ly));
-}
-
 // Partial sums of (f.n) x_src over blocks (DLP k=0 term,
 // StokesDLP_ewald_2p.m:150-151); finished by k_zero_mode_final.
 __global__ void __launch_bounds__(256) k_zero_mode_part(int64_t n, const double2 *__restrict__ p,
@@ -3077,16 +3154,11 @@ __global__ void __launch_bounds__(256) k_zero_mode_part(int64_t n, const double2
     }
 }
 
-__global__ void k_zero_mode_final(int nparts, const double2 *__restrict__ part, double inv_area,
+__global__ void __launch_bounds__(32) k_zero_mode_final(int nparts, const double2 *__restrict__ part, double inv_area,
                                   double2 *__restrict__ zm)
 {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    double2 s = make_double2(0.0, 0.0);
-    for (int i = 0; i < nparts; i++) {
-        s.x += part[i].x;
-        s.y += part[i].y;
-    }
-    *zm = make_double2(s.x * inv_area, s.y * inv_area);
+    const double2 s = sum_parts(nparts, part);
+    if (threadIdx.x == 0) *zm = make_double2(s.x * inv_area, s.y * inv_area);
 }
 
 // Final assembly in original target order.
@@ -3097,43 +3169,53 @@ __global__ void k_zero_mode_final(int nparts, const double2 *__restrict__ part, 
 //   mode 4: DLP driver        u = -(ur/4/pi + uk - zm)
 // ur (sorted order, raw sums) and uk (sorted order, scaled) may be NULL when
 // unused; ur_out / uk_out (original order) receive the parts when non-NULL.
-__global__ void k_assemble(int64_t n, int mode, const int *__restrict__ perm,
-                           const double2 *__restrict__ ur, const double2 *__restrict__ uk,
-                           const double2 *__restrict__ zm, double2 *__restrict__ u,
-                           double2 *__restrict__ ur_out, double2 *__restrict__ uk_out)
+// x / d, correctly rounded but for rare ties: the product with 1/d and one
+// residual correction (a division is ten FP64 instructions).
+__device__ __forceinline__ double div_const(double x, double d, double inv_d)
+{
+    const double q = x * inv_d, e = fma(-q, d, x);
+    return e == e ? fma(e, inv_d, q) : q;            // (an infinite q stays)
+}
+
+// (all outputs of one call, so that perm is read once)
+__global__ void __launch_bounds__(256) k_assemble(int64_t n, const int *__restrict__ perm, AssembleArgs a)
 {
     const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= n) return;
     const int i = perm[j];
-    double2 r = make_double2(0.0, 0.0), k = make_double2(0.0, 0.0);
-    if (ur) {
-        r = ur[j];
-        if (mode == 1 || mode == 4) {
-            r.x = r.x / 4.0 / kPi;
-            r.y = r.y / 4.0 / kPi;
-        } else {
-            r.x = r.x / (4.0 * kPi);
-            r.y = r.y / (4.0 * kPi);
+#pragma unroll 1
+    for (int o = 0; o < a.nout; o++) {
+        const AssembleOut &q = a.o[o];
+        double2 r = make_double2(0.0, 0.0), k = make_double2(0.0, 0.0);
+        if (q.ur) {
+            r = q.ur[j];
+            if (q.mode == 1 || q.mode == 4) {
+                r.x = div_const(0.25 * r.x, kPi, 1.0 / kPi);
+                r.y = div_const(0.25 * r.y, kPi, 1.0 / kPi);
+            } else {
+                r.x = div_const(r.x, 4.0 * kPi, 1.0 / (4.0 * kPi));
+                r.y = div_const(r.y, 4.0 * kPi, 1.0 / (4.0 * kPi));
+            }
         }
-    }
-    if (uk) {
-        k = uk[j];
-        if (mode == 4) {
-            const double2 z = *zm;
-            k.x -= z.x;
-            k.y -= z.y;
+        if (q.uk) {
+            k = q.uk[j];
+            if (q.mode == 4) {
+                const double2 z = *q.zm;
+                k.x -= z.x;
+                k.y -= z.y;
+            }
         }
+        double2 v;
+        switch (q.mode) {
+        case 0: case 1: v = r; break;
+        case 2: v = k; break;
+        case 3: v = make_double2(r.x + k.x, r.y + k.y); break;
+        default: v = make_double2(-(r.x + k.x), -(r.y + k.y)); break;
+        }
+        q.u[i] = v;
+        if (q.ur_out) q.ur_out[i] = r;
+        if (q.uk_out) q.uk_out[i] = k;
     }
-    double2 v;
-    switch (mode) {
-    case 0: case 1: v = r; break;
-    case 2: v = k; break;
-    case 3: v = make_double2(r.x + k.x, r.y + k.y); break;
-    default: v = make_double2(-(r.x + k.x), -(r.y + k.y)); break;
-    }
-    u[i] = v;
-    if (ur_out) ur_out[i] = r;
-    if (uk_out) uk_out[i] = k;
 }
 
 // ===========================================================================
@@ -3160,44 +3242,33 @@ int sm_count()
     return cache[dev];
 }
 
-cudaError_t launch_bin(const BinArgs &a, int *start, int nbox, int *perm, int *sorted_box,
-                       double2 *sorted_pos, float2 *sorted_pos_f, cudaStream_t st,
-                       int64_t &launches, float2 *sorted_pos_lo)
+cudaError_t launch_sort(const SortArgs &a, int nsets, cudaStream_t st, int64_t &launches)
 {
-    cudaError_t e = cudaMemsetAsync(a.count, 0, sizeof(int) * (size_t)nbox, st);
-    if (e != cudaSuccess) return e;
-    if (a.n > 0) {
-        k_bin_count<<<grid_for(a.n, 256), 256, 0, st>>>(a);
-        launches++;
+    const int nbox = a.nx * a.ny;
+    const bool joint = nsets == 2 && a.s[1].count == a.s[0].count + nbox;
+    int64_t n = 0;
+    for (int k = 0; k < nsets; k++) {
+        n = std::max(n, a.s[k].n);
+        if (joint && k) continue;
+        const cudaError_t e = cudaMemsetAsync(a.s[k].count, 0, sizeof(int) * (size_t)nbox * (joint ? 2 : 1), st);
+        if (e != cudaSuccess) return e;
     }
-    k_scan<<<1, 1024, 0, st>>>(a.count, nbox, start);
-    launches++;
-    if (a.n > 0) {
-        k_bin_place<<<grid_for(a.n, 256), 256, 0, st>>>(a.n, a.box, a.rank, start, perm,
-                                                         sorted_box, a.p, sorted_pos,
-                                                         sorted_pos_f, sorted_pos_lo);
-        launches++;
-    }
+    const dim3 g(grid_for(n, 256), (unsigned)nsets);
+    if (n > 0) k_sort_count<<<g, 256, 0, st>>>(a);
+    k_sort_scan<<<dim3(nbox > kScanWide ? 1 : (nbox + 1023) / 1024, nsets), 1024, 0, st>>>(a);
+    if (n > 0) k_sort_place<<<g, 256, 0, st>>>(a);
+    launches += n > 0 ? 3 : 1;
     return cudaGetLastError();
 }
 
 cudaError_t launch_src_coef(int64_t n, const int *perm, const double2 *f_slp,
                             const double2 *f_dlp, const double2 *nrm, double *coef, int nc,
-                            cudaStream_t st, int64_t &launches)
+                            cudaStream_t st, int64_t &launches, float2 *out, int64_t ostride,
+                            bool tails)
 {
     if (n <= 0) return cudaSuccess;
-    k_src_coef<<<grid_for(n, 256), 256, 0, st>>>(n, perm, f_slp, f_dlp, nrm, coef, nc);
-    launches++;
-    return cudaGetLastError();
-}
-
-cudaError_t launch_src_coef_ff(int64_t n, const double *coef, int nc, bool slp, bool dlp,
-                               float2 *out, int ncf, cudaStream_t st, int64_t &launches,
-                               int64_t ostride, bool tails)
-{
-    if (n <= 0) return cudaSuccess;
-    k_src_coef_ff<<<grid_for(n, 256), 256, 0, st>>>(n, coef, nc, slp, dlp, out,
-                                                     ostride > 0 ? ostride : ncf, tails ? 1 : 0);
+    k_src_coef<<<grid_for(n, 256), 256, 0, st>>>(n, perm, f_slp, f_dlp, nrm, coef, nc, out, ostride,
+                                                 tails ? 1 : 0);
     launches++;
     return cudaGetLastError();
 }
@@ -3301,15 +3372,6 @@ cudaError_t launch_gather(const GatherArgs &a, int nc, cudaStream_t st, int64_t 
     return cudaGetLastError();
 }
 
-cudaError_t launch_wrap(int64_t n, const double2 *p, double Lx, double Ly, double2 *out,
-                        cudaStream_t st, int64_t &launches)
-{
-    if (n <= 0) return cudaSuccess;
-    k_wrap<<<grid_for(n, 256), 256, 0, st>>>(n, p, Lx, Ly, out);
-    launches++;
-    return cudaGetLastError();
-}
-
 cudaError_t launch_zero_mode(int64_t n, const double2 *p, const double2 *f, const double2 *nrm,
                              double inv_area, double2 *part, double2 *zm, cudaStream_t st,
                              int64_t &launches)
@@ -3320,12 +3382,11 @@ cudaError_t launch_zero_mode(int64_t n, const double2 *p, const double2 *f, cons
     return cudaGetLastError();
 }
 
-cudaError_t launch_assemble(int64_t n, int mode, const int *perm, const double2 *ur,
-                            const double2 *uk, const double2 *zm, double2 *u, double2 *ur_out,
-                            double2 *uk_out, cudaStream_t st, int64_t &launches)
+cudaError_t launch_assemble(int64_t n, const int *perm, const AssembleArgs &a, cudaStream_t st,
+                            int64_t &launches)
 {
-    if (n <= 0) return cudaSuccess;
-    k_assemble<<<grid_for(n, 256), 256, 0, st>>>(n, mode, perm, ur, uk, zm, u, ur_out, uk_out);
+    if (n <= 0 || a.nout <= 0) return cudaSuccess;
+    k_assemble<<<grid_for(n, 256), 256, 0, st>>>(n, perm, a);
     launches++;
     return cudaGetLastError();
 }
