@@ -782,12 +782,12 @@ static int spread(se2p_plan pl, SpreadArgs &sa, int nc, bool allow_fixed, cudaSt
 static int fft_ff_table(se2p_plan pl, cudaStream_t st, int L, int which, const float4 **tw)
 {
     float4 *d = nullptr;
-    CKS(ensure_t(pl, which ? S_TWX : S_TWY, (size_t)L, &d));
+    CKS(ensure_t(pl, which ? S_TWX : S_TWY, 4 * (size_t)L, &d));
     if (pl->tw_len[which] != L || pl->tw_dev[which] != d) {
         std::vector<float4> &h = pl->tw_host[which];
-        h.resize((size_t)L);
+        h.resize(4 * (size_t)L);
         fft_rows_ff_twiddles(L, h.data());
-        CK(cudaMemcpyAsync(d, h.data(), sizeof(float4) * (size_t)L, cudaMemcpyHostToDevice, st));
+        CK(cudaMemcpyAsync(d, h.data(), sizeof(float4) * 4 * (size_t)L, cudaMemcpyHostToDevice, st));
         pl->tw_len[which] = L;
         pl->tw_dev[which] = d;
     }

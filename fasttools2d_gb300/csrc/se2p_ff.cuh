@@ -13,8 +13,7 @@
 // The split is exact for hi and rounds lo once: hi + lo = d (1 + delta),
 // |delta| <= 2^-48, for 2^-74 <= |d| < 2^128.  Below 2^-74 lo is flushed (the
 // relative error grows to 2^-24 there; every caller works with magnitudes
-// relative to much larger values), zero maps to (0, 0), and inf / NaN take the
-// slow conversion.
+// relative to much larger values), zero maps to (0, 0), inf and NaN stay so.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -28,7 +27,10 @@ __device__ __forceinline__ float2 ff_split(double d)
     const unsigned sign = (unsigned)hw & 0x80000000u;
     if (e <= 896) return make_float2(0.f, 0.f);      // |d| < 2^-126 (and zero)
     if (e >= 1151) {                                  // |d| >= 2^128, inf, NaN
-        return make_float2(__double2float_rn(d), 0.f);
+        // (as the conversion gives it, which the compiler would hoist above the
+        // test and issue for every value at the FP64 rate)
+        const bool nan = e == 0x7ff && (((unsigned)hw & 0xfffffu) | lw);
+        return make_float2(__uint_as_float(sign | (nan ? 0x7fffffffu : 0x7f800000u)), 0.f);
     }
     const unsigned hb = sign | ((unsigned)(e - 896) << 23) | (((unsigned)hw & 0xfffffu) << 3) |
                         (lw >> 29);

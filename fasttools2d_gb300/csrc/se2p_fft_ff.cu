@@ -33,79 +33,166 @@ namespace se2p {
 
 namespace {
 
+// Two FP32 numbers in one register pair: an instruction on pairs takes the FP32
+// pipe two cycles (65 per clock and SM measured, against 127 scalar ones) but one
+// issue slot, and the kernel is bound by issue.  A complex number is a pair (re,
+// im) of heads and one of tails, so its sums, products with a real, and shared
+// memory accesses are half as many instructions.
+typedef unsigned long long f2;
+
+__device__ __forceinline__ f2 pk(float a, float b)
+{
+    f2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float2 upk(f2 a)
+{
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a));
+    return r;
+}
+__device__ __forceinline__ f2 swap2(f2 a)
+{
+    const float2 v = upk(a);
+    return pk(v.y, v.x);
+}
+__device__ __forceinline__ f2 add2(f2 a, f2 b)
+{
+    f2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f2 mul2(f2 a, f2 b)
+{
+    f2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c)
+{
+    f2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+constexpr f2 kM1 = 0xbf800000bf800000ull;            // (-1, -1)
+// a - b, rounded once (the product with -1 is exact)
+__device__ __forceinline__ f2 sub2(f2 a, f2 b) { return fma2(b, kM1, a); }
+__device__ __forceinline__ f2 neg2(f2 a) { return mul2(a, kM1); }
+
+// TwoSum, Fast2Sum and TwoProduct of both numbers (se2p_ff.cuh has the scalar ones).
+__device__ __forceinline__ void two_sum2(f2 a, f2 b, f2 &s, f2 &e)
+{
+    s = add2(a, b);
+    const f2 bb = sub2(s, a);
+    e = add2(sub2(a, sub2(s, bb)), sub2(b, bb));
+}
+__device__ __forceinline__ void two_diff2(f2 a, f2 b, f2 &s, f2 &e)
+{
+    s = sub2(a, b);
+    const f2 bb = sub2(s, a);
+    e = sub2(sub2(a, sub2(s, bb)), add2(b, bb));
+}
+__device__ __forceinline__ void fast_two_sum2(f2 a, f2 b, f2 &s, f2 &e)
+{
+    s = add2(a, b);
+    e = sub2(b, sub2(s, a));
+}
+
 struct fc {
-    float2 r, i;   // real and imaginary parts, each (hi, lo)
+    f2 h, l;       // (re, im) heads and tails
 };
 
-__device__ __forceinline__ fc fc_add(const fc &a, const fc &b) { return {ff_add(a.r, b.r), ff_add(a.i, b.i)}; }
-__device__ __forceinline__ fc fc_sub(const fc &a, const fc &b) { return {ff_sub(a.r, b.r), ff_sub(a.i, b.i)}; }
-// a * (s i), s = +-1
-__device__ __forceinline__ fc fc_mul_si(const fc &a, float s)
+__device__ __forceinline__ fc fc_add(const fc &a, const fc &b)
 {
-    return s > 0.f ? fc{ff_neg(a.i), a.r} : fc{a.i, ff_neg(a.r)};
+    f2 s, e;
+    two_sum2(a.h, b.h, s, e);
+    e = add2(e, add2(a.l, b.l));
+    fc r;
+    fast_two_sum2(s, e, r.h, r.l);
+    return r;
 }
-__device__ __forceinline__ fc fc_mulr(const fc &a, float2 c) { return {ff_mul(a.r, c), ff_mul(a.i, c)}; }
-
-// x1 y1 - x2 y2 in float-float (products exact to the float-float level).
-__device__ __forceinline__ float2 ff_dd(float2 x1, float2 y1, float2 x2, float2 y2)
+__device__ __forceinline__ fc fc_sub(const fc &a, const fc &b)
 {
-    const float p1 = x1.x * y1.x;
-    float e1 = fmaf(x1.x, y1.x, -p1);
-    e1 = fmaf(x1.x, y1.y, e1);
-    e1 = fmaf(x1.y, y1.x, e1);
-    const float p2 = x2.x * y2.x;
-    float e2 = fmaf(x2.x, y2.x, -p2);
-    e2 = fmaf(x2.x, y2.y, e2);
-    e2 = fmaf(x2.y, y2.x, e2);
-    float s, t;
-    two_sum(p1, -p2, s, t);
-    t += e1 - e2;
-    float h, l;
-    fast_two_sum(s, t, h, l);
-    return make_float2(h, l);
+    f2 s, e;
+    two_diff2(a.h, b.h, s, e);
+    e = add2(e, sub2(a.l, b.l));
+    fc r;
+    fast_two_sum2(s, e, r.h, r.l);
+    return r;
 }
-
-// a * w, w a twiddle (already conjugated for the inverse)
-__device__ __forceinline__ fc fc_mul(const fc &a, const fc &w)
+// a * (s i), s = +-1: (-s im, s re); sg = (-s, s)
+__device__ __forceinline__ fc fc_mul_si(const fc &a, f2 sg) { return {mul2(swap2(a.h), sg), mul2(swap2(a.l), sg)}; }
+// a times the real c, cl (in both halves)
+__device__ __forceinline__ fc fc_mulr(const fc &a, f2 c, f2 cl)
 {
-    return {ff_dd(a.r, w.r, a.i, w.i), ff_dd(a.r, w.i, ff_neg(a.i), w.r)};
+    const f2 p = mul2(a.h, c);
+    f2 e = fma2(a.h, c, neg2(p));
+    e = fma2(a.h, cl, e);
+    e = fma2(a.l, c, e);
+    fc r;
+    fast_two_sum2(p, e, r.h, r.l);
+    return r;
 }
 
-__device__ __forceinline__ fc tw_load(const float4 *tw, int m, float s)
+// A twiddle (c, sn) = exp(+-2 pi i m / L) as the product takes it: c and its
+// tail in both halves, (-sn, sn) and its tails.
+struct tw2 {
+    f2 c, cl, s, sl;
+};
+
+// a * w: a c + (im, re)(-sn, sn), the two products' heads summed by TwoSum.
+__device__ __forceinline__ fc fc_mul(const fc &a, const tw2 &w)
 {
-    const float4 t = __ldg(tw + m);
-    // table holds exp(-2 pi i m / L); the inverse (s = +1) takes its conjugate
-    return s < 0.f ? fc{make_float2(t.x, t.y), make_float2(t.z, t.w)}
-                   : fc{make_float2(t.x, t.y), make_float2(-t.z, -t.w)};
+    const f2 p1 = mul2(a.h, w.c);
+    f2 e1 = fma2(a.h, w.c, neg2(p1));
+    e1 = fma2(a.h, w.cl, e1);
+    e1 = fma2(a.l, w.c, e1);
+    const f2 bh = swap2(a.h), bl = swap2(a.l);
+    const f2 p2 = mul2(bh, w.s);
+    f2 e2 = fma2(bh, w.s, neg2(p2));
+    e2 = fma2(bh, w.sl, e2);
+    e2 = fma2(bl, w.s, e2);
+    f2 s, t;
+    two_sum2(p1, p2, s, t);
+    t = add2(t, add2(e1, e2));
+    fc r;
+    fast_two_sum2(s, t, r.h, r.l);
+    return r;
 }
 
-// Shared buffer: four float arrays (re hi, re lo, im hi, im lo) of Lp =
-// sh_len(L) words each, element k at k + k/32: the padding word per 32 turns
-// the stride-R stores of the early stages (R = 2, 4, 8) into at most 2-way
-// bank conflicts.
-__host__ __device__ __forceinline__ int sh_len(int L) { return L + (L >> 5) + 1; }
-__device__ __forceinline__ fc sh_get(const float *b, int Lp, int k)
+// Entry m of the table: two 16-byte words (c, c, cl, cl), (-sn, sn, -snl, snl).
+__device__ __forceinline__ tw2 tw_load(const ulonglong2 *tw, int m)
 {
-    k += k >> 5;
-    return {make_float2(b[k], b[Lp + k]), make_float2(b[2 * Lp + k], b[3 * Lp + k])};
+    const ulonglong2 a = __ldg(tw + 2 * m), b = __ldg(tw + 2 * m + 1);
+    return {a.x, a.y, b.x, b.y};
 }
-__device__ __forceinline__ void sh_put(float *b, int Lp, int k, const fc &v)
+
+// Shared buffer: heads, then tails, of Lp = sh_len(L) pairs each, element k at k +
+// k/16: the padding pair per 16 keeps the stride-R stores of the early stages
+// (R = 2, 4, 8) free of bank conflicts.
+__host__ __device__ __forceinline__ int sh_len(int L) { return L + (L >> 4) + 1; }
+__device__ __forceinline__ fc sh_get(const f2 *b, int Lp, int k)
 {
-    k += k >> 5;
-    b[k] = v.r.x;
-    b[Lp + k] = v.r.y;
-    b[2 * Lp + k] = v.i.x;
-    b[3 * Lp + k] = v.i.y;
+    k += k >> 4;
+    return {b[k], b[Lp + k]};
 }
+__device__ __forceinline__ void sh_put(f2 *b, int Lp, int k, const fc &v)
+{
+    k += k >> 4;
+    b[k] = v.h;
+    b[Lp + k] = v.l;
+}
+__device__ __forceinline__ fc fc_make(float2 re, float2 im) { return {pk(re.x, im.x), pk(re.y, im.y)}; }
 
 // Radix-R butterflies of one Stockham stage.  Input element r of butterfly j
 // is A[j + r L/R]; it is multiplied by w^(k r L/(Ns R)), k = j mod Ns, the
 // R-point DFT is taken, and output r goes to B[(j / Ns) Ns R + k + r Ns].
 template <int R>
-__device__ __forceinline__ void dft(fc *v, float s, const fc *cst);
+__device__ __forceinline__ void dft(fc *v, f2 sg, const tw2 *cst);
 
 template <>
-__device__ __forceinline__ void dft<2>(fc *v, float, const fc *)
+__device__ __forceinline__ void dft<2>(fc *v, f2, const tw2 *)
 {
     const fc a = v[0], b = v[1];
     v[0] = fc_add(a, b);
@@ -113,28 +200,27 @@ __device__ __forceinline__ void dft<2>(fc *v, float, const fc *)
 }
 
 template <>
-__device__ __forceinline__ void dft<4>(fc *v, float s, const fc *)
+__device__ __forceinline__ void dft<4>(fc *v, f2 sg, const tw2 *)
 {
     const fc t0 = fc_add(v[0], v[2]), t1 = fc_sub(v[0], v[2]);
-    const fc t2 = fc_add(v[1], v[3]), t3 = fc_mul_si(fc_sub(v[1], v[3]), s);   // W4 = s i
+    const fc t2 = fc_add(v[1], v[3]), t3 = fc_mul_si(fc_sub(v[1], v[3]), sg);   // W4 = s i
     v[0] = fc_add(t0, t2);
     v[2] = fc_sub(t0, t2);
     v[1] = fc_add(t1, t3);
     v[3] = fc_sub(t1, t3);
 }
 
-// cst[0].r = sqrt(1/2)
+// cst[0].c = sqrt(1/2)
 template <>
-__device__ __forceinline__ void dft<8>(fc *v, float s, const fc *cst)
+__device__ __forceinline__ void dft<8>(fc *v, f2 sg, const tw2 *cst)
 {
     fc e[4] = {v[0], v[2], v[4], v[6]}, o[4] = {v[1], v[3], v[5], v[7]};
-    dft<4>(e, s, nullptr);
-    dft<4>(o, s, nullptr);
-    const float2 h = cst[0].r;
+    dft<4>(e, sg, nullptr);
+    dft<4>(o, sg, nullptr);
     // W8 = (1 + s i) sqrt(1/2), W8^2 = s i, W8^3 = (-1 + s i) sqrt(1/2)
-    const fc o1 = fc_mulr(fc_add(o[1], fc_mul_si(o[1], s)), h);
-    const fc o2 = fc_mul_si(o[2], s);
-    const fc o3 = fc_mulr(fc_sub(fc_mul_si(o[3], s), o[3]), h);
+    const fc o1 = fc_mulr(fc_add(o[1], fc_mul_si(o[1], sg)), cst[0].c, cst[0].cl);
+    const fc o2 = fc_mul_si(o[2], sg);
+    const fc o3 = fc_mulr(fc_sub(fc_mul_si(o[3], sg), o[3]), cst[0].c, cst[0].cl);
     v[0] = fc_add(e[0], o[0]);
     v[4] = fc_sub(e[0], o[0]);
     v[1] = fc_add(e[1], o1);
@@ -150,41 +236,37 @@ __device__ __forceinline__ void dft<8>(fc *v, float s, const fc *cst)
 // into an unnormalised tail; one normalisation at the end.  A term costs 12
 // FP32 operations against 18 for a product and an add normalised separately.
 struct ffacc {
-    float s, t;
+    f2 s, t;
 };
-__device__ __forceinline__ ffacc acc_from(float2 x) { return {x.x, x.y}; }
-__device__ __forceinline__ ffacc acc_prod(float2 c, float2 x)
+__device__ __forceinline__ ffacc acc_prod(f2 c, f2 cl, const fc &x)
 {
-    const float p = c.x * x.x;
-    float e = fmaf(c.x, x.x, -p);
-    e = fmaf(c.x, x.y, e);
-    e = fmaf(c.y, x.x, e);
+    const f2 p = mul2(c, x.h);
+    f2 e = fma2(c, x.h, neg2(p));
+    e = fma2(c, x.l, e);
+    e = fma2(cl, x.h, e);
     return {p, e};
 }
-__device__ __forceinline__ void acc_add(ffacc &a, float2 x)
+__device__ __forceinline__ void acc_add(ffacc &a, f2 h, f2 l)
 {
-    float s, q;
-    two_sum(a.s, x.x, s, q);
+    f2 s, q;
+    two_sum2(a.s, h, s, q);
     a.s = s;
-    a.t += q + x.y;
+    a.t = add2(a.t, add2(q, l));
 }
-__device__ __forceinline__ void acc_fma(ffacc &a, float2 c, float2 x)
+__device__ __forceinline__ fc acc_get(const ffacc &a)
 {
-    const ffacc p = acc_prod(c, x);
-    float s, q;
-    two_sum(a.s, p.s, s, q);
-    a.s = s;
-    a.t += q + p.t;
+    fc r;
+    two_sum2(a.s, a.t, r.h, r.l);
+    return r;
 }
-__device__ __forceinline__ float2 acc_get(const ffacc &a) { return ff_norm(a.s, a.t); }
 
 // Odd R: with s_n = a_n + a_(R-n), d_n = a_n - a_(R-n),
 // A_k = a_0 + sum_n cos(2 pi n k / R) s_n, B_k = sum_n sin(2 pi n k / R) d_n,
 // X_k = A_k + s i B_k, X_(R-k) = A_k - s i B_k.  cst[m] = (cos, sin)(2 pi m / R),
-// m = 1 .. (R-1)/2, as the .r and .i fields.  The sums X_0, A_k and B_k are
-// float-float dot products (ffacc).
+// m = 1 .. (R-1)/2, each in both halves of .c and .s.  The sums X_0, A_k and B_k
+// are float-float dot products (ffacc).
 template <int R>
-__device__ __forceinline__ void dft_odd(fc *v, float s, const fc *cst)
+__device__ __forceinline__ void dft_odd(fc *v, f2 sg, const tw2 *cst)
 {
     constexpr int h = (R - 1) / 2;
     fc sm[h], df[h];
@@ -194,56 +276,48 @@ __device__ __forceinline__ void dft_odd(fc *v, float s, const fc *cst)
         df[n - 1] = fc_sub(v[n], v[R - n]);
     }
     const fc a0 = v[0];
-    ffacc x0r = acc_from(a0.r), x0i = acc_from(a0.i);
+    ffacc x0 = {a0.h, a0.l};
 #pragma unroll
-    for (int n = 0; n < h; n++) {
-        acc_add(x0r, sm[n].r);
-        acc_add(x0i, sm[n].i);
-    }
+    for (int n = 0; n < h; n++) acc_add(x0, sm[n].h, sm[n].l);
 #pragma unroll
     for (int k = 1; k <= h; k++) {
-        ffacc Ar = acc_from(a0.r), Ai = acc_from(a0.i), Br = {0.f, 0.f}, Bi = {0.f, 0.f};
+        ffacc A = {a0.h, a0.l}, B = {0, 0};
 #pragma unroll
         for (int n = 1; n <= h; n++) {
             int m = (n * k) % R;
             const bool neg = m > h;                  // sin(2 pi (R-m)/R) = -sin(2 pi m/R)
             if (neg) m = R - m;
-            const float2 c = cst[m - 1].r;
-            const float2 sn = neg ? ff_neg(cst[m - 1].i) : cst[m - 1].i;
-            acc_fma(Ar, c, sm[n - 1].r);
-            acc_fma(Ai, c, sm[n - 1].i);
-            if (n == 1) {
-                Br = acc_prod(sn, df[0].r);
-                Bi = acc_prod(sn, df[0].i);
-            } else {
-                acc_fma(Br, sn, df[n - 1].r);
-                acc_fma(Bi, sn, df[n - 1].i);
-            }
+            const tw2 &w = cst[m - 1];
+            const ffacc pa = acc_prod(w.c, w.cl, sm[n - 1]);
+            acc_add(A, pa.s, pa.t);
+            ffacc pb = acc_prod(w.s, w.sl, df[n - 1]);
+            if (neg) pb = {neg2(pb.s), neg2(pb.t)};
+            if (n == 1) B = pb;
+            else acc_add(B, pb.s, pb.t);
         }
-        const fc A = {acc_get(Ar), acc_get(Ai)};
-        const fc iB = fc_mul_si(fc{acc_get(Br), acc_get(Bi)}, s);
-        v[k] = fc_add(A, iB);
-        v[R - k] = fc_sub(A, iB);
+        const fc a = acc_get(A), b = fc_mul_si(acc_get(B), sg);
+        v[k] = fc_add(a, b);
+        v[R - k] = fc_sub(a, b);
     }
-    v[0] = {acc_get(x0r), acc_get(x0i)};
+    v[0] = acc_get(x0);
 }
 
 template <>
-__device__ __forceinline__ void dft<3>(fc *v, float s, const fc *cst) { dft_odd<3>(v, s, cst); }
+__device__ __forceinline__ void dft<3>(fc *v, f2 sg, const tw2 *cst) { dft_odd<3>(v, sg, cst); }
 template <>
-__device__ __forceinline__ void dft<5>(fc *v, float s, const fc *cst) { dft_odd<5>(v, s, cst); }
+__device__ __forceinline__ void dft<5>(fc *v, f2 sg, const tw2 *cst) { dft_odd<5>(v, sg, cst); }
 template <>
-__device__ __forceinline__ void dft<7>(fc *v, float s, const fc *cst) { dft_odd<7>(v, s, cst); }
+__device__ __forceinline__ void dft<7>(fc *v, f2 sg, const tw2 *cst) { dft_odd<7>(v, sg, cst); }
 
 // R = 6 = 2 x 3 by the prime-factor (Good-Thomas) split, with no inner
 // twiddles: 3-point DFTs of inputs (0, 2, 4) and (3, 5, 1), then 2-point
 // DFTs of their outputs, which land at (3 k1 + 4 k2) mod 6.  cst as for R = 3.
 template <>
-__device__ __forceinline__ void dft<6>(fc *v, float s, const fc *cst)
+__device__ __forceinline__ void dft<6>(fc *v, f2 sg, const tw2 *cst)
 {
     fc a[3] = {v[0], v[2], v[4]}, b[3] = {v[3], v[5], v[1]};
-    dft_odd<3>(a, s, cst);
-    dft_odd<3>(b, s, cst);
+    dft_odd<3>(a, sg, cst);
+    dft_odd<3>(b, sg, cst);
     v[0] = fc_add(a[0], b[0]);
     v[3] = fc_sub(a[0], b[0]);
     v[4] = fc_add(a[1], b[1]);
@@ -252,24 +326,24 @@ __device__ __forceinline__ void dft<6>(fc *v, float s, const fc *cst)
     v[5] = fc_sub(a[2], b[2]);
 }
 
+// tw: the table of the transform's sign; tw0: the forward one, whose entries m L / R
+// give the butterflies' constants.
 template <int R>
-__device__ void stage(const float *A, float *B, int L, int Ns, unsigned magic, float s,
-                      const float4 *tw)
+__device__ void stage(const f2 *A, f2 *B, int L, int Ns, unsigned magic, f2 sg,
+                      const ulonglong2 *tw, const ulonglong2 *tw0)
 {
     // the constants of the R-point DFT from the twiddle table
-    fc cst[R / 2 > 0 ? R / 2 : 1];
+    constexpr f2 kPM = 0xbf8000003f800000ull;        // (1, -1)
+    tw2 cst[R / 2 > 0 ? R / 2 : 1];
     if (R == 8) {
-        const fc w = tw_load(tw, L / 8, -1.f);       // exp(-i pi/4): re = sqrt(1/2)
-        cst[0] = w;
-    } else if (R & 1) {
+        cst[0] = tw_load(tw0, L / 8);                // exp(-i pi/4): re = sqrt(1/2)
+    } else if ((R & 1) || R == 6) {
+        constexpr int O = R == 6 ? 3 : R;
 #pragma unroll
-        for (int m = 1; m <= R / 2; m++) {
-            const fc w = tw_load(tw, m * (L / R), -1.f);   // cos - i sin
-            cst[m - 1] = {w.r, ff_neg(w.i)};
+        for (int m = 1; m <= O / 2; m++) {
+            const tw2 w = tw_load(tw0, m * (L / O));   // sn = -sin: (-sn, sn) = (sin, -sin)
+            cst[m - 1] = {w.c, w.cl, mul2(w.s, kPM), mul2(w.sl, kPM)};
         }
-    } else if (R == 6) {
-        const fc w = tw_load(tw, L / 3, -1.f);       // the 3-point constants
-        cst[0] = {w.r, ff_neg(w.i)};
     }
     const int nb = L / R, stride = L / (Ns * R), Lp = sh_len(L);
     for (int j = threadIdx.x; j < nb; j += blockDim.x) {
@@ -279,9 +353,9 @@ __device__ void stage(const float *A, float *B, int L, int Ns, unsigned magic, f
         for (int r = 0; r < R; r++) v[r] = sh_get(A, Lp, j + r * nb);
         if (Ns > 1) {
 #pragma unroll
-            for (int r = 1; r < R; r++) v[r] = fc_mul(v[r], tw_load(tw, k * r * stride, s));
+            for (int r = 1; r < R; r++) v[r] = fc_mul(v[r], tw_load(tw, k * r * stride));
         }
-        dft<R>(v, s, cst);
+        dft<R>(v, sg, cst);
         const int o = (j - k) * R + k;
 #pragma unroll
         for (int r = 0; r < R; r++) sh_put(B, Lp, o + r * Ns, v[r]);
@@ -296,7 +370,9 @@ __device__ __forceinline__ double ff_to_double_scaled(float hi, float lo, int e)
     const unsigned hb = __float_as_uint(hi), lb = __float_as_uint(lo);
     const int eh = (int)((hb >> 23) & 0xff);
     if (eh == 0) return 0.0;
-    if (eh == 0xff) return (double)hi;               // inf, NaN (rare: the slow conversion)
+    if (eh == 0xff)                                  // inf, NaN (no conversion: it would be hoisted)
+        return __longlong_as_double((long long)((unsigned long long)(hb >> 31) << 63 | 0x7ffull << 52 |
+                                                (unsigned long long)(hb & 0x7fffffu) << 29));
     long long m = (long long)((hb & 0x7fffffu) | 0x800000u) << 29;   // units 2^(eh-179)
     const int el = (int)((lb >> 23) & 0xff);
     if (el != 0) {
@@ -371,14 +447,18 @@ __device__ __forceinline__ float2 ff_split_scaled(double d, int e)
     return ff_split(__longlong_as_double(nb));
 }
 
-__global__ void __launch_bounds__(256) k_fft_rows_ff(double2 *__restrict__ data, int64_t rows,
-                                                     FftRowsFF p, const float4 *__restrict__ tw)
+__global__ void __launch_bounds__(256, 2) k_fft_rows_ff(double2 *__restrict__ data, int64_t rows,
+                                                        FftRowsFF p, const float4 *__restrict__ tab)
 {
-    extern __shared__ float fsh[];
+    extern __shared__ __align__(16) f2 fsh[];
     __shared__ int emax_w[8];
     const int L = p.L, Lp = sh_len(L);
-    const float s = (float)p.sign;
-    float *A = fsh, *B = fsh + 4 * Lp;
+    const float sf = (float)p.sign;
+    const f2 s = pk(-sf, sf);
+    const ulonglong2 *tw0 = reinterpret_cast<const ulonglong2 *>(tab);
+    const ulonglong2 *tw = p.sign < 0 ? tw0 : tw0 + 2 * L;
+    const int half = 2 * Lp + (2 * Lp & 1);
+    f2 *A = fsh, *B = fsh + half;
     // fused pack from int64 planes: the values need no row scaling (|v| <
     // 2^60 stays far inside the float range after the transform's growth by
     // at most L); the 2^-S of the fixed-point grid is applied on the way out
@@ -399,11 +479,11 @@ __global__ void __launch_bounds__(256) k_fft_rows_ff(double2 *__restrict__ data,
             const long long *g = static_cast<const long long *>(p.pack_in);
             for (int k = threadIdx.x; k < L; k += blockDim.x) {
                 const long long vr = g[off_re + k], vi = has_im ? g[off_im + k] : 0;
-                sh_put(A, Lp, k, fc{ll_to_ff(vr), ll_to_ff(vi)});
+                sh_put(A, Lp, k, fc_make(ll_to_ff(vr), ll_to_ff(vi)));
             }
             e = -S;
         } else {
-            // the row as doubles into B (4 Lp floats >= L double2), and its
+            // the row as doubles into B (2 Lp pairs >= L double2), and its
             // largest exponent
             double2 *raw = reinterpret_cast<double2 *>(B);
             int em = 0;
@@ -429,7 +509,7 @@ __global__ void __launch_bounds__(256) k_fft_rows_ff(double2 *__restrict__ data,
             e = (em == 0 || em == 0x7ff) ? 0 : em - 1023 - 63;
             for (int k = threadIdx.x; k < L; k += blockDim.x) {
                 const double2 v = raw[k];
-                sh_put(A, Lp, k, fc{ff_split_scaled(v.x, e), ff_split_scaled(v.y, e)});
+                sh_put(A, Lp, k, fc_make(ff_split_scaled(v.x, e), ff_split_scaled(v.y, e)));
             }
         }
         __syncthreads();
@@ -438,16 +518,16 @@ __global__ void __launch_bounds__(256) k_fft_rows_ff(double2 *__restrict__ data,
             const int R = p.radix[st];
             const unsigned mg = p.magic[st];
             switch (R) {
-            case 8: stage<8>(A, B, L, Ns, mg, s, tw); break;
-            case 4: stage<4>(A, B, L, Ns, mg, s, tw); break;
-            case 6: stage<6>(A, B, L, Ns, mg, s, tw); break;
-            case 2: stage<2>(A, B, L, Ns, mg, s, tw); break;
-            case 7: stage<7>(A, B, L, Ns, mg, s, tw); break;
-            case 5: stage<5>(A, B, L, Ns, mg, s, tw); break;
-            default: stage<3>(A, B, L, Ns, mg, s, tw); break;
+            case 8: stage<8>(A, B, L, Ns, mg, s, tw, tw0); break;
+            case 4: stage<4>(A, B, L, Ns, mg, s, tw, tw0); break;
+            case 6: stage<6>(A, B, L, Ns, mg, s, tw, tw0); break;
+            case 2: stage<2>(A, B, L, Ns, mg, s, tw, tw0); break;
+            case 7: stage<7>(A, B, L, Ns, mg, s, tw, tw0); break;
+            case 5: stage<5>(A, B, L, Ns, mg, s, tw, tw0); break;
+            default: stage<3>(A, B, L, Ns, mg, s, tw, tw0); break;
             }
             Ns *= R;
-            float *t = A;
+            f2 *t = A;
             A = B;
             B = t;
             __syncthreads();
@@ -459,11 +539,12 @@ __global__ void __launch_bounds__(256) k_fft_rows_ff(double2 *__restrict__ data,
             unsigned long long m = 0;
             for (int k = threadIdx.x; k < L; k += blockDim.x) {
                 const fc v = sh_get(A, Lp, k);
-                const double re = ff_to_double_scaled(v.r.x, v.r.y, e);
+                const float2 vh = upk(v.h), vl = upk(v.l);
+                const double re = ff_to_double_scaled(vh.x, vl.x, e);
                 p.unpack_out[off_re + k] = re;
                 m = max(m, (unsigned long long)__double_as_longlong(fabs(re)));
                 if (has_im) {
-                    const double im = ff_to_double_scaled(v.i.x, v.i.y, e);
+                    const double im = ff_to_double_scaled(vh.y, vl.y, e);
                     p.unpack_out[off_im + k] = im;
                     m = max(m, (unsigned long long)__double_as_longlong(fabs(im)));
                 }
@@ -475,13 +556,14 @@ __global__ void __launch_bounds__(256) k_fft_rows_ff(double2 *__restrict__ data,
         } else {
             for (int k = threadIdx.x; k < L; k += blockDim.x) {
                 const fc v = sh_get(A, Lp, k);
-                d[k] = make_double2(ff_to_double_scaled(v.r.x, v.r.y, e),
-                                    ff_to_double_scaled(v.i.x, v.i.y, e));
+                const float2 vh = upk(v.h), vl = upk(v.l);
+                d[k] = make_double2(ff_to_double_scaled(vh.x, vl.x, e),
+                                    ff_to_double_scaled(vh.y, vl.y, e));
             }
         }
         // the next row reuses both buffers and emax_w
         A = fsh;
-        B = fsh + 4 * Lp;
+        B = fsh + half;
         __syncthreads();
     }
 }
@@ -516,7 +598,10 @@ void fft_rows_ff_twiddles(int L, float4 *host)
         const long double a = -2.0L * pi * (long double)m / (long double)L;
         const long double c = cosl(a), sn = sinl(a);
         const float ch = (float)c, sh = (float)sn;
-        host[m] = make_float4(ch, (float)(c - (long double)ch), sh, (float)(sn - (long double)sh));
+        const float cl = (float)(c - (long double)ch), sl = (float)(sn - (long double)sh);
+        host[2 * m] = host[2 * (L + m)] = make_float4(ch, ch, cl, cl);
+        host[2 * m + 1] = make_float4(-sh, sh, -sl, sl);
+        host[2 * (L + m) + 1] = make_float4(sh, -sh, sl, -sl);
     }
 }
 
@@ -524,7 +609,7 @@ cudaError_t launch_fft_rows_ff(double2 *data, int64_t rows, const FftRowsFF &p, 
                                cudaStream_t st, int64_t &launches)
 {
     if (rows <= 0) return cudaSuccess;
-    const size_t smem = sizeof(float) * 8 * (size_t)sh_len(p.L);
+    const size_t smem = sizeof(f2) * 2 * ((size_t)(2 * sh_len(p.L) + 1) & ~(size_t)1);
     cudaError_t e = cudaFuncSetAttribute(k_fft_rows_ff, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)smem);
     if (e != cudaSuccess) return e;

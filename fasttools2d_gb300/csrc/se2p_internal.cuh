@@ -545,7 +545,8 @@ struct FftRowsFF {
     unsigned long long *gmax = nullptr;   // largest |value| unpacked per pair q (bit pattern), optional
 };
 bool fft_rows_ff_plan(int L, FftRowsFF &p);
-void fft_rows_ff_twiddles(int L, float4 *host);   // exp(-2 pi i m/L), m < L, float-float
+// exp(-2 pi i m/L), then exp(+2 pi i m/L), m < L: 2 float4 each, 4 L in all
+void fft_rows_ff_twiddles(int L, float4 *host);
 cudaError_t launch_fft_rows_ff(double2 *data, int64_t rows, const FftRowsFF &p, const float4 *tw,
                                cudaStream_t st, int64_t &launches);
 // Real-space operator of a fixed geometry (se2p_geom.cu).
