@@ -1549,6 +1549,48 @@ int run_adjoint(se2p_plan pl, const Job &J, const AdjIo &io)
     }
     {
         StageTimer tm(pl, T_GATHER, ks);
+        GatherArgs gt;                               // the sources as gather points
+        gt.tp = sp;
+        gt.nt = ns;
+        gt.Mx = Mx;
+        gt.My = My;
+        gt.P = P;
+        gt.Lhx = ga.Lhx;
+        gt.Lhy = ga.Lhy;
+        gt.h = h;
+        gt.w = J.w;
+        gt.a = ga.a;
+        if (ffg && tg_ok(gt, 5)) {
+            TcSet t;
+            CKS(tg_targets(pl, gt, ks, t));
+            CK(launch_grid_to_fixed(grid, 5, (int64_t)G, gmax, kTgBits, ks, pl->launches));
+            TcGatherAdjArgs ta{};
+            ta.fac = t.pa.fac;
+            ta.list = t.list;
+            ta.items = t.items;
+            ta.nitems = t.nitems;
+            ta.grid = reinterpret_cast<const long long *>(grid);
+            ta.gmax = gmax;
+            ta.Mx = Mx;
+            ta.My = My;
+            ta.P = P;
+            ta.Tx = t.pa.Tx;
+            ta.Ty = t.pa.Ty;
+            ta.nty = t.pa.nty;
+            ta.Bg = kTgBits;
+            ta.s = t.s;
+            ta.sp = sp;
+            ta.coef = coef;
+            ta.Lhx = ga.Lhx;
+            ta.Lhy = ga.Lhy;
+            ta.h = h;
+            ta.scale = ga.scale;
+            ta.dscale = 2.0 * ga.a * h;
+            ta.out = gk;
+            ta.err = pl->tc_err_dev;
+            CK(launch_gather_adj_tc(ta, ks, pl->launches));
+            ga.tc = true;
+        }
         CK(launch_gather_adj(ga, ks, pl->launches));
     }
     if (ks != st) {

@@ -342,6 +342,8 @@ struct GatherAdjArgs {
     // planes; null for the FP64 gather alone
     unsigned long long *gmax = nullptr;
     float2 *gff = nullptr;
+    // the tensor-core gather ran instead of k_gather_adj_ff
+    bool tc = false;
 };
 
 struct SpreadArgs {
@@ -406,6 +408,24 @@ struct TcGatherArgs {
     int64_t nt;
     double scale;
     double2 *out;               // NC/2 outputs per target, [k * nt + t]
+    int *err;
+};
+
+// Tensor-core adjoint gather: the gather's tiles and items, the points being the
+// forward sources.
+struct TcGatherAdjArgs {
+    const void *fac;
+    const int *list;
+    const int4 *items;
+    const int *nitems;
+    const long long *grid;      // 5 int64 grids (launch_grid_to_fixed with Bg)
+    const unsigned long long *gmax;
+    int Mx, My, P, Tx, Ty, nty, Bg;
+    unsigned long long s;       // exp(-2 alpha) 2^64
+    const double2 *sp;          // sorted sources
+    const double *coef;         // 5 per source
+    double Lhx, Lhy, h, scale, dscale;   // dscale = 2 a h: the derivative's factor
+    double *out;                // 7 per source: 5 values, gradient x, y
     int *err;
 };
 
@@ -648,6 +668,7 @@ cudaError_t launch_tc_points(const TcPointArgs &a, int kmax, const int *perm, in
                              const unsigned long long *bound, cudaStream_t st,
                              int64_t &launches);
 cudaError_t launch_gather_tc(const TcGatherArgs &a, int nc, cudaStream_t st, int64_t &launches);
+cudaError_t launch_gather_adj_tc(const TcGatherAdjArgs &a, cudaStream_t st, int64_t &launches);
 cudaError_t launch_spread_tc(const TcSpreadArgs &a, int nc, cudaStream_t st, int64_t &launches);
 int64_t spread_bound_words(int Mx, int My, int P);
 int64_t spread_bound_slot(int Mx, int My, int P);

@@ -2753,7 +2753,7 @@ template <int PT>
 __global__ void __launch_bounds__(256) k_gather_adj(GatherAdjArgs a)
 {
     // behind k_gather_adj_ff: runs only when a grid held a non-finite value
-    if (a.gff && gmax_all(a.gmax) < kGridNonFinite) return;
+    if ((a.gff || a.tc) && gmax_all(a.gmax) < kGridNonFinite) return;
     const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= a.ns) return;
     const int P = PT > 0 ? PT : a.P;
@@ -3459,7 +3459,7 @@ cudaError_t launch_probe_red64(unsigned long long *a, int64_t n, int iters, int6
 cudaError_t launch_gather_adj(const GatherAdjArgs &a, cudaStream_t st, int64_t &launches)
 {
     if (a.ns <= 0) return cudaSuccess;
-    if (a.gff) {
+    if (a.gff && !a.tc) {
         const int64_t n = 5 * (int64_t)a.Mx * a.My;
         k_grid_to_ff<<<grid_for(n, 256), 256, 0, st>>>(a.grid, n, a.gmax, a.gff);
         const int64_t warps = (a.ns + 31) / 32;

@@ -935,6 +935,33 @@ __device__ __forceinline__ void store_digits_signed(const long long (&v)[8], cha
         *reinterpret_cast<uint4 *>(dst + p * stride) = make_uint4(out[p][0], out[p][1], out[p][2], out[p][3]);
 }
 
+// The same for four.
+__device__ __forceinline__ void store_digits_signed4(const long long (&v)[4], char *dst, int stride)
+{
+    const __half2 off = __float2half2_rn(-1152.0f);
+    uint32_t out[8][2];
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        const unsigned long long a = (unsigned long long)v[2 * k] + 0x8080808080808080ull;
+        const unsigned long long b = (unsigned long long)v[2 * k + 1] + 0x8080808080808080ull;
+#pragma unroll
+        for (int w = 0; w < 2; w++) {
+            const uint32_t aw = (uint32_t)(w ? a : a >> 32), bw = (uint32_t)(w ? b : b >> 32);
+            const uint32_t z = __byte_perm(aw, bw, 0x7632), y = __byte_perm(aw, bw, 0x5410);
+            const uint32_t d[4] = {__byte_perm(z, 0x64646464u, 0x4341), __byte_perm(z, 0x64646464u, 0x4240),
+                                   __byte_perm(y, 0x64646464u, 0x4341), __byte_perm(y, 0x64646464u, 0x4240)};
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const __half2 h = __hadd2(*reinterpret_cast<const __half2 *>(&d[q]), off);
+                out[4 * w + q][k] = *reinterpret_cast<const uint32_t *>(&h);
+            }
+        }
+    }
+#pragma unroll
+    for (int p = 0; p < kTcDigits; p++)
+        *reinterpret_cast<uint2 *>(dst + p * stride) = make_uint2(out[p][0], out[p][1]);
+}
+
 template <int NC>
 __global__ void __launch_bounds__(kTcThreads, 2) k_gather_tc(TcGatherArgs a)
 {
@@ -1171,6 +1198,292 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_gather_tc(TcGatherArgs a)
 }
 
 // ---------------------------------------------------------------------------
+// Adjoint gather
+//
+// At each forward source, for the five adjoint grids: the value sum_ij X_i Y_j g and the
+// sums with the weights' position derivatives, X'_i = 2 a h (u_x - i') X_i with i' the
+// node's offset from the stencil's middle and u_x the point's in nodes, and the
+// same in y.  Rows 0 .. 63 of the product are Y, rows 64 .. 127 are j' Y for the same
+// points, so one product gives sum_j Y_j g and sum_j j' Y_j g; the threads of the
+// first rows also add i' X_i times their sums.  One block per SM, the accumulators
+// and B doubled: while one grid is multiplied, the previous one's sums are
+// finished and the next one's B is built.
+//
+// Bound: latency (one block of 18 warps per SM).  2^18 sources, 1344^2 nodes: 0.74 ms
+// (and 0.09 ms for the tiles and the int64 grids) against 2.17 ms for
+// k_gather_adj_ff with its float-float grids, bound by issue; 1500 sources on 96^2
+// nodes 0.027 against 0.375 ms.  The gradients' error falls from 6e-14 to 4e-15
+// with it, the weights no longer being float-float.
+// ---------------------------------------------------------------------------
+constexpr int kGaThreads = 18 * 32;
+constexpr int kGaA = kTcDigits * 128 * kTgY * 2;
+
+struct GaSmem {
+    unsigned long long seed[6][kTgT];
+    double coef[2][5][kTgT], ux[2][kTgT], uy[2][kTgT];
+    int meta[2][kTgT], idx[2][kTgT];
+    long long sum[2][5][128], sumx[2][5][kTgT];      // per half of the columns
+    unsigned long long bfull[2], done[2], tfree[2], fin, ready, sfree[2], seedfree;
+    uint32_t tmem;
+    int abort_flag;
+};
+
+constexpr int kGaSmem = kGaA + 2 * kTgB + kTgXs + (int)sizeof(GaSmem) + 128;
+
+__global__ void __launch_bounds__(kGaThreads, 1) k_gather_adj_tc(TcGatherAdjArgs a)
+{
+    extern __shared__ __align__(128) char tc_smem[];
+    if (gmax_all(a.gmax) >= kGridNonFinite) return;  // the FP64 gather runs instead
+    const int nv = *a.nitems;
+    const int v0 = (int)((int64_t)nv * blockIdx.x / gridDim.x);
+    const int v1 = (int)((int64_t)nv * (blockIdx.x + 1) / gridDim.x);
+    if (v0 == v1) return;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int P = a.P, P1 = P + 1, win = tc_window(P);
+    char *Ash = tc_smem, *Bsh = Ash + kGaA;
+    unsigned long long *xs = reinterpret_cast<unsigned long long *>(Bsh + 2 * kTgB);
+    unsigned long long *ys = reinterpret_cast<unsigned long long *>(Bsh);
+    GaSmem &sh = *reinterpret_cast<GaSmem *>(reinterpret_cast<char *>(xs) + kTgXs);
+    volatile int *ab = &sh.abort_flag;
+
+    if (tid == 0) {
+        sh.abort_flag = 0;
+        for (int b = 0; b < 2; b++) {
+            mbar_init(smem_u32(&sh.bfull[b]), 256);
+            mbar_init(smem_u32(&sh.done[b]), 1);
+            mbar_init(smem_u32(&sh.tfree[b]), 256);
+            mbar_init(smem_u32(&sh.sfree[b]), 512);
+        }
+        mbar_init(smem_u32(&sh.fin), 1);
+        mbar_init(smem_u32(&sh.ready), 1);
+        mbar_init(smem_u32(&sh.seedfree), 256);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 16) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(&sh.tmem))
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = sh.tmem;
+
+    if (warp == 16) {
+        if (lane == 0) {
+            int n = 0;
+            for (int v = v0; v < v1; v++) {
+                for (int c = 0; c < 5; c++, n++) {
+                    const int b = n & 1;
+                    mbar_wait(smem_u32(&sh.bfull[b]), (n >> 1) & 1, ab, a.err);
+                    if (n > 1) mbar_wait(smem_u32(&sh.tfree[b]), ((n >> 1) - 1) & 1, ab, a.err);
+                    tc_fence_after();
+                    if (*ab) continue;
+#pragma unroll 1
+                    for (int k = 0; k < kTgY / 16; k++)
+#pragma unroll
+                        for (int p = 0; p < kTcDigits; p++)
+                            tc_mma(tmem + 256 * b + kTgX * p,
+                                   tc_desc(smem_u32(Ash) + p * (128 * kTgY * 2) + k * 256, 128, kTgY * 16),
+                                   tc_desc(smem_u32(Bsh) + b * kTgB + k * 256, 128, kTgY * 16),
+                                   tc_idesc(kTgX * (kTcDigits - p), 0), k > 0 || p > 0);
+                    tc_commit(smem_u32(&sh.done[b]));
+                }
+            }
+            // everything issued has completed before TMEM is given back
+            tc_commit(smem_u32(&sh.fin));
+            mbar_wait(smem_u32(&sh.fin), 0, ab, a.err);
+        }
+        __syncwarp();
+    } else if (warp == 17) {
+        int n = 0;
+        for (int v = v0; v < v1; v++, n++) {
+            const int4 item = a.items[v];
+            const int b = n & 1;
+            if (n > 1) mbar_wait(smem_u32(&sh.sfree[b]), (n / 2 - 1) & 1, ab, a.err);
+            const TcPoint *f[kTgT / 32];
+#pragma unroll
+            for (int u = 0; u < kTgT / 32; u++) {
+                const int s = lane + 32 * u;
+                f[u] = nullptr;
+                int j = -1, meta = 0;
+                if (s < item.z) {
+                    j = a.list[item.y + s];
+                    f[u] = reinterpret_cast<const TcPoint *>(a.fac) + j;
+                    meta = f[u]->meta;
+#pragma unroll
+                    for (int c = 0; c < 5; c++) sh.coef[b][c][s] = a.coef[5 * (int64_t)j + c];
+                    const double2 S = a.sp[j];
+                    int mx, my;
+                    double px, py;
+                    closest_node(S.x, S.y, a.Lhx, a.Lhy, a.h, P, mx, my, px, py);
+                    sh.ux[b][s] = px / a.h;
+                    sh.uy[b][s] = py / a.h;
+                }
+                sh.meta[b][s] = meta;
+                sh.idx[b][s] = j;
+            }
+            if (n > 0) mbar_wait(smem_u32(&sh.seedfree), (n - 1) & 1, ab, a.err);
+#pragma unroll
+            for (int u = 0; u < kTgT / 32; u++) {
+                if (!f[u]) continue;
+                const int s = lane + 32 * u;
+                sh.seed[0][s] = f[u]->ex;
+                sh.seed[1][s] = f[u]->ey;
+                sh.seed[2][s] = f[u]->qpx;
+                sh.seed[3][s] = f[u]->qpy;
+                sh.seed[4][s] = f[u]->qmx;
+                sh.seed[5][s] = f[u]->qmy;
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&sh.ready));
+        }
+    } else {
+        int n = 0, nc = 0;                           // items, grids so far
+        const __half2 one = __float2half2_rn(1.0f);
+        auto bsync = [] { asm volatile("bar.sync 1, 512;" ::: "memory"); };
+        for (int v = v0; v < v1; v++, n++) {
+            const int4 item = a.items[v];
+            const int cnt = item.z, b = n & 1;
+            mbar_wait(smem_u32(&sh.ready), n & 1, ab, a.err);
+            if (tid < 4 * kTgT) {
+                const int q = tid / kTgT, ax = q & 1, s = tid % kTgT;
+                if (s < cnt) {
+                    const int meta = sh.meta[b][s], ic = P / 2 + ((meta >> (16 + ax)) & 1);
+                    const int r = ax ? (meta >> 8) & 7 : meta & 0xff, w = ax ? win : kTgX;
+                    const unsigned long long e = ax ? sh.seed[1][s] : sh.seed[0][s] >> 2;
+                    unsigned long long *o = (ax ? ys : xs) + s;
+                    if (q < 2) {
+                        tc_factors<kTgT>(e, sh.seed[2 + ax][s], a.s, r + ic, 1, P1 - ic, w, o);
+                    } else {
+                        const unsigned long long qm = sh.seed[4 + ax][s];
+                        tc_factors<kTgT>(mulhi_apx(e, qm), mulhi_apx(qm, a.s), a.s, r + ic - 1, -1, ic, w, o);
+                    }
+                }
+                mbar_arrive(smem_u32(&sh.seedfree));
+            }
+            bsync();
+            for (int t = tid; t < 2 * kTgT * (kTgY / 4); t += 512) {
+                const int der = t / (kTgT * (kTgY / 4)), t1 = t % (kTgT * (kTgY / 4));
+                const int slot = t1 / (2 * kTgT), s = (t1 >> 1) % kTgT, half = t1 & 1, row = 64 * der + s;
+                const int oy = (sh.meta[b][s] >> 8) & 0xff;
+                const int ch = ((oy >> 3) + slot) & (kTgY / 8 - 1);
+                char *dst = Ash + (row >> 3) * (kTgY * 16) + ch * 128 + (row & 7) * 16 + half * 8;
+                if (s >= cnt || 8 * slot >= win) {
+                    store_zero_digits<kTcDigits>(dst, 128 * kTgY * 2);
+                } else {
+                    unsigned long long w[4];
+                    const int r0 = 8 * slot + 4 * half;
+#pragma unroll
+                    for (int e = 0; e < 4; e++) w[e] = ys[(r0 + e) * kTgT + s] >> 1;
+                    if (der) {
+                        // j' Y as fractions of 2^61 (|j' Y| < 2)
+                        const int j0 = r0 - (oy & 7) - P / 2;
+                        long long z[4];
+#pragma unroll
+                        for (int e = 0; e < 4; e++) z[e] = (long long)(w[e] >> 2) * (j0 + e);
+                        store_digits_signed4(z, dst, 128 * kTgY * 2);
+                    } else {
+                        store_digits<kTcDigits>(w, one, dst, 128 * kTgY * 2);
+                    }
+                }
+            }
+            fence_async_shared();
+            bsync();
+            const int x0 = item.x / a.nty * a.Tx, y0 = item.x % a.nty * a.Ty;
+            for (int c = 0; c < 5; c++, nc++) {
+                const int tb = nc & 1;
+                if (warp >= 8) {
+                    // B: 32 columns x 8 chunks of 8 nodes, one each
+                    if (nc > 1) mbar_wait(smem_u32(&sh.done[tb]), ((nc >> 1) - 1) & 1, ab, a.err);
+                    const int bt = tid - 256, i = bt % kTgX, ch = bt / kTgX;
+                    int x = x0 + i, y = y0 + 8 * ch;
+                    if (x >= a.Mx) x -= a.Mx;
+                    if (y >= a.My) y -= a.My;
+                    const long long *g = a.grid + ((int64_t)c * a.Mx + x) * a.My;
+                    long long w[8];
+                    if (y + 8 <= a.My) {
+#pragma unroll
+                        for (int e = 0; e < 4; e++) {
+                            const longlong2 q = __ldg(reinterpret_cast<const longlong2 *>(g + y) + e);
+                            w[2 * e] = q.x;
+                            w[2 * e + 1] = q.y;
+                        }
+                    } else {
+#pragma unroll
+                        for (int e = 0; e < 8; e++) w[e] = __ldg(g + (y + e >= a.My ? y + e - a.My : y + e));
+                    }
+                    store_digits_signed(w, Bsh + tb * kTgB + (i >> 3) * (kTgY * 16) + ch * 128 + (i & 7) * 16,
+                                        kTgX * kTgY * 2);
+                    fence_async_shared();
+                    mbar_arrive(smem_u32(&sh.bfull[tb]));
+                } else {
+                    const int quad = warp & 3, eh = warp >> 2, t = (quad & 1) * 32 + lane;
+                    const int mid = (sh.meta[b][t] & 0xff) + P / 2;
+                    mbar_wait(smem_u32(&sh.done[tb]), (nc >> 1) & 1, ab, a.err);
+                    tc_fence_after();
+                    long long acc = 0, accx = 0;
+#pragma unroll 1
+                    for (int h = 0; h < kTgX / 16; h++) {
+                        const int i0 = eh * (kTgX / 2) + 8 * h;
+                        uint32_t r[kTcDigits][8];
+#pragma unroll
+                        for (int l = 0; l < kTcDigits; l++)
+                            tc_ld8(tmem + 256 * tb + ((uint32_t)(quad * 32) << 16) + kTgX * l + i0, r[l]);
+#pragma unroll
+                        for (int l = 0; l < kTcDigits; l++) tc_ld_wait8(r[l]);
+#pragma unroll
+                        for (int e = 0; e < 8; e++) {
+                            auto d = [&](int l) { return __float2int_rn(__uint_as_float(r[l][e])); };
+                            const int p12 = d(1) * 256 + d(2), p34 = d(3) * 256 + d(4), p56 = d(5) * 256 + d(6);
+                            const unsigned hi = (unsigned)d(0) * 65536u + (unsigned)p12;
+                            const long long V = (long long)p34 * 65536 + p56 + (long long)((unsigned long long)hi << 32);
+                            const unsigned long long x = xs[(i0 + e) * kTgT + t];
+                            const long long m = (long long)mulhi_apx((unsigned long long)V, x) - (V < 0 ? (long long)x : 0);
+                            acc += m;
+                            accx += (m >> 3) * (i0 + e - mid);
+                        }
+                    }
+                    tc_fence_before();
+                    mbar_arrive(smem_u32(&sh.tfree[tb]));
+                    sh.sum[eh][c][quad * 32 + lane] = acc;
+                    if (quad < 2) sh.sumx[eh][c][t] = accx;
+                }
+            }
+            // (the item's last products have read A: the epilogue waited for them)
+            bsync();
+            if (tid < cnt && !*ab) {
+                const int j = sh.idx[b][tid];
+                const double ux = sh.ux[b][tid], uy = sh.uy[b][tid];
+                double gx = 0.0, gy = 0.0;
+                double *o = a.out + 7 * (int64_t)j;
+#pragma unroll
+                for (int c = 0; c < 5; c++) {
+                    const unsigned long long gb = a.gmax[c / 2];
+                    const double s = gb == 0 ? 0.0 : ldexp(a.scale, 3 - grid_shift(gb, a.Bg));
+                    const double V = (double)(sh.sum[0][c][tid] + sh.sum[1][c][tid]) * s;
+                    const double Ix = (double)(sh.sumx[0][c][tid] + sh.sumx[1][c][tid]) * (8.0 * s);
+                    const double Iy = (double)(sh.sum[0][c][64 + tid] + sh.sum[1][c][64 + tid]) * (4.0 * s);
+                    const double cf = sh.coef[b][c][tid];
+                    o[c] = V;
+                    gx = fma(cf, fma(ux, V, -Ix), gx);
+                    gy = fma(cf, fma(uy, V, -Iy), gy);
+                }
+                o[5] = gx * a.dscale;
+                o[6] = gy * a.dscale;
+            }
+            mbar_arrive(smem_u32(&sh.sfree[b]));
+            bsync();
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    if (warp == 16)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
+}
+
+// ---------------------------------------------------------------------------
 // Launchers
 // ---------------------------------------------------------------------------
 cudaError_t launch_tc_points(const TcPointArgs &a, int kmax, const int *perm, int *start,
@@ -1233,6 +1546,16 @@ cudaError_t launch_gather_tc(const TcGatherArgs &a, int nc, cudaStream_t st, int
 {
     launches++;
     return nc == 2 ? gather_tc<2>(a, st) : gather_tc<4>(a, st);
+}
+
+cudaError_t launch_gather_adj_tc(const TcGatherAdjArgs &a, cudaStream_t st, int64_t &launches)
+{
+    const cudaError_t e =
+        cudaFuncSetAttribute(k_gather_adj_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, kGaSmem);
+    if (e != cudaSuccess) return e;
+    k_gather_adj_tc<<<sm_count(), kGaThreads, kGaSmem, st>>>(a);
+    launches++;
+    return cudaGetLastError();
 }
 
 }  // namespace se2p

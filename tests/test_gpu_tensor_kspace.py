@@ -130,3 +130,18 @@ def test_gather_edges_and_nodes(ft, plans):
 def test_gather_either_side_of_the_sparse_line(ft, plans, M):
     p, q, f, n = _cloud(500, M, nt=65536)
     _both(ft, plans, p, q, f, n, M, M, 24)
+
+
+@pytest.mark.parametrize("M,P,N,xi,nside", [(64, 24, 40, 20.0, 4), (96, 24, 1500, 30.0, 6), (98, 20, 65, 30.0, 6),
+                                            (130, 10, 700, 40.0, 8), (192, 26, 3000, 55.0, 11)])
+def test_adjoint_gather(ft, plans, M, P, N, xi, nside):
+    """Gradients of the tensor-core adjoint gather against the all-FP64 form, at the
+    1e-11 of the float-float adjoint's test."""
+    rng = np.random.default_rng(M + N)
+    p, q, f, n = _cloud(N, M, nt=300)
+    g, w1, w2 = rng.standard_normal((2, N)), rng.standard_normal((2, 300)), rng.standard_normal((2, 300))
+    p[:, : N // 4] = 0.05 + p[:, : N // 4] / M       # one grid cell: a tile of many items
+    prm = ft.EwaldParams.derived(xi, nside, nside, M, M, P, 1.0, 1.0)
+    a, b = (ft.stokes_ewald_adjoint(p, q, f, g, n, w1, w2, prm, plan=pl) for pl in plans)
+    for x, y in zip(a, b):
+        assert relerr(x, y) < 1e-11, relerr(x, y)
