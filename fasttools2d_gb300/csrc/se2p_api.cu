@@ -992,7 +992,7 @@ int run(se2p_plan pl, const Job &J, const Io &io)
     {
         StageTimer tm(pl, T_COEF);
         CK(launch_src_coef(ns, sperm, J.slp ? fs : nullptr, J.dlp ? fd : nullptr, nr, coef, nc, st,
-                           pl->launches, cff, ncf));
+                           pl->launches, cff, ncf, true, J.real ? count : nullptr));
     }
 
     double2 *ur_slp = nullptr, *ur_dlp = nullptr, *uk = nullptr;
@@ -1010,6 +1010,8 @@ int run(se2p_plan pl, const Job &J, const Io &io)
         ra.tp = tp;
         ra.tbox = tboxs;
         ra.ntar = nt;
+        ra.ns = ns;
+        ra.next = count;   // (the box counts are done with: zeroed beside the coefficients)
         ra.nx = nx;
         ra.ny = ny;
         ra.Lx = J.Lx;
@@ -1391,7 +1393,7 @@ int run_adjoint(se2p_plan pl, const Job &J, const AdjIo &io)
     {
         StageTimer tm(pl, T_COEF);
         CK(launch_src_coef(ns, sperm, slp ? fs : zeros, dlp ? fd : zeros, dlp ? nr : zeros, coef, 5,
-                           st, pl->launches));
+                           st, pl->launches, nullptr, 0, true, count));
         CK(launch_sorted_pair(nt, tperm, w1, w2, wcoef, st, pl->launches));
     }
     double *gr = nullptr, *gk = nullptr;
@@ -1406,6 +1408,7 @@ int run_adjoint(se2p_plan pl, const Job &J, const AdjIo &io)
     ra.nc = 5;
     ra.doff = 2;
     ra.sstart = tstart;            // candidate (inner) cell list: the targets
+    ra.next = count;
     ra.tp = tp;
     ra.tpf = tpf;
     ra.tbox = tboxs;
@@ -2641,7 +2644,7 @@ extern "C" int se2p_slp_real_noalloc(const double *psrc, int64_t ns, const doubl
     so.s[0] = SortSet{pt, nt, tbox, trank, count, tstart, tperm, tboxs, tp, tpf, nullptr};
     if (launch_sort(so, 1, st, launches) != cudaSuccess) return SE2P_ERR_CUDA;
     if (launch_src_coef(ns, sperm, reinterpret_cast<const double2 *>(f), nullptr, nullptr, coef,
-                        2, st, launches, coef_ff, 2) != cudaSuccess)
+                        2, st, launches, coef_ff, 2, true, count) != cudaSuccess)
         return SE2P_ERR_CUDA;
     // The same real-space arguments and form as se2p_slp_real on a plan of
     // the default precision (SE2P_PRECISION_FP64: far pairs in float-float).
@@ -2656,6 +2659,8 @@ extern "C" int se2p_slp_real_noalloc(const double *psrc, int64_t ns, const doubl
     ra.tp = tp;
     ra.tbox = tboxs;
     ra.ntar = nt;
+    ra.ns = ns;
+    ra.next = count;
     ra.nx = nside_x;
     ra.ny = nside_y;
     ra.Lx = Lx;

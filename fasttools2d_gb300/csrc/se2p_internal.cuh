@@ -300,6 +300,9 @@ struct RealArgs {
     const float2 *tpf;
     const int *tbox;      // box of each sorted target
     int64_t ntar;
+    int64_t ns;           // number of sources
+    int run;              // points per run of the outer loop (set by the launch)
+    int *next;            // counter of the runs taken beyond each warp's first, zeroed before
     int nx, ny;
     double Lx, Ly, xi, xi2, cut2, self_c;
     double inv_xi2, pf;   // 1/xi^2, 2 xi^2
@@ -505,7 +508,7 @@ cudaError_t launch_sort(const SortArgs &a, int nsets, cudaStream_t st, int64_t &
 cudaError_t launch_src_coef(int64_t n, const int *perm, const double2 *f_slp,
                             const double2 *f_dlp, const double2 *nrm, double *coef, int nc,
                             cudaStream_t st, int64_t &launches, float2 *out = nullptr,
-                            int64_t ostride = 0, bool tails = true);
+                            int64_t ostride = 0, bool tails = true, int *zero = nullptr);
 cudaError_t launch_real(const RealArgs &a, bool slp, bool dlp, cudaStream_t st,
                         int64_t &launches, int form = kFormFP64);
 // 2D real FFT through 1D complex passes (se2p_kernels.cu): pack real grid

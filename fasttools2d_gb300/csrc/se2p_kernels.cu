@@ -210,6 +210,7 @@ __global__ void __launch_bounds__(256) k_sort_place(SortArgs a)
 // (PE/src/mex/StokesDLP/mex_stokes_dlp_real.cpp:81-91; S12 and S21 only ever
 // enter as their sum, in the real-space contraction and as H2+H3 in the
 // DLP filter).  The same array is the spread's per-grid weights.
+// zero: a word to clear (the real space's run counter), or null.
 //
 // With out, also the float-float copy for the far pairs of the FP64 form: SLP f1,
 // f2; DLP S11, S12+S21, S22 and (tails) the combinations 3 S11 + S22, 3 S22 + S11
@@ -217,9 +218,11 @@ __global__ void __launch_bounds__(256) k_sort_place(SortArgs a)
 __global__ void __launch_bounds__(256) k_src_coef(int64_t n, const int *__restrict__ perm,
                            const double2 *__restrict__ f_slp, const double2 *__restrict__ f_dlp,
                            const double2 *__restrict__ nrm, double *__restrict__ coef, int nc,
-                           float2 *__restrict__ out, int64_t ostride, int tails)
+                           float2 *__restrict__ out, int64_t ostride, int tails,
+                           int *__restrict__ zero)
 {
     const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (zero && j == 0) *zero = 0;
     if (j >= n) return;
     const int i = perm[j];
     double *c = coef + (int64_t)nc * j;
@@ -679,6 +682,7 @@ __global__ void __launch_bounds__(kRealWarps * 32, SE2P_REAL_MINB) k_real(RealAr
     __shared__ float e1f[MIXED ? 66 : 1];
     // FP32-grid form: target positions as float-float (hi.x, hi.y, lo.x, lo.y)
     __shared__ float4 tposff_s[kRealWarps][MIXED ? kRing : 1];
+    __shared__ int run_s;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     float4 *tposff = tposff_s[wid];
     for (int i = threadIdx.x; i < 64; i += blockDim.x) {
@@ -785,179 +789,185 @@ __global__ void __launch_bounds__(kRealWarps * 32, SE2P_REAL_MINB) k_real(RealAr
         retire(true);
     };
 
-    // Each block takes one contiguous run of the box-sorted targets, and its
-    // warps interleave over it: a warp's consecutive targets mostly share a
-    // box (so its neighbour-box set is built once per box), and the block's
-    // warps read the same sources at the same time.
+    // Runs of kRealWarps * a.run box-sorted targets: a block's first run by its number,
+    // the next from the counter whenever it is done.  The block's warps interleave over
+    // the run: a warp's consecutive targets mostly share a box (so its neighbour-box set
+    // is built once per box), and the block's warps read the same sources at the same
+    // time.  The FIFOs go on from run to run.
     // (the cell lists hold int indices, so ntar < 2^31)
-    const int per = (int)((a.ntar + gridDim.x - 1) / gridDim.x);
-    const int t_end = (int)min(a.ntar, (int64_t)blockIdx.x * per + per);
+    const int64_t len = (int64_t)kRealWarps * a.run;
     if (lane == 0) W.curbox = -1;
     __syncwarp();
-    for (int t = (int)blockIdx.x * per + wid; t < t_end; t += kRealWarps) {
-        if (nfl == kRing) drain();
-        const int slot = (head + nfl) % kRing;
-        nfl++;
-        gseq++;
-        const int tb = a.tbox[t];
-        const double2 T = a.tp[t];
-        const float2 Tf = a.tpf[t];
-        const bool newbox = tb != W.curbox;                // (warp-uniform)
-        if (newbox) {
-            __syncwarp();
+    for (int64_t t0 = (int64_t)blockIdx.x * len; t0 < a.ntar; t0 = run_s * len) {
+        const int t_end = (int)min(t0 + len, a.ntar);
+        for (int t = (int)t0 + wid; t < t_end; t += kRealWarps) {
+            if (nfl == kRing) drain();
+            const int slot = (head + nfl) % kRing;
+            nfl++;
+            gseq++;
+            const int tb = a.tbox[t];
+            const double2 T = a.tp[t];
+            const float2 Tf = a.tpf[t];
+            const bool newbox = tb != W.curbox;                // (warp-uniform)
+            if (newbox) {
+                __syncwarp();
+                if (lane == 0) {
+                    W.curbox = tb;
+                    W.curbxy = make_int2(tb % a.nx, tb / a.nx);
+                }
+                __syncwarp();
+            }
+            const int2 cur_bxy = W.curbxy;
+            if (lane < 4) {
+                W.acc[slot][lane] = 0.0;
+                W.accf[slot][lane] = make_float2(0.f, 0.f);
+            }
             if (lane == 0) {
-                W.curbox = tb;
-                W.curbxy = make_int2(tb % a.nx, tb / a.nx);
+                W.tpos[slot] = T;
+                W.tbxy[slot] = cur_bxy;
+                W.tidx[slot] = t;
+                if (MIXED) {
+                    const float2 tl = a.tpl[t];
+                    tposff[slot] = make_float4(Tf.x, Tf.y, tl.x, tl.y);
+                }
             }
-            __syncwarp();
-        }
-        const int2 cur_bxy = W.curbxy;
-        if (lane < 4) {
-            W.acc[slot][lane] = 0.0;
-            W.accf[slot][lane] = make_float2(0.f, 0.f);
-        }
-        if (lane == 0) {
-            W.tpos[slot] = T;
-            W.tbxy[slot] = cur_bxy;
-            W.tidx[slot] = t;
-            if (MIXED) {
-                const float2 tl = a.tpl[t];
-                tposff[slot] = make_float4(Tf.x, Tf.y, tl.x, tl.y);
-            }
-        }
-        // neighbour boxes: first source, counts -> list prefix, image shift
-        // (once per box), and the pre-test band, which depends on the target
-        if (newbox) {
-            int cntk = 0;
-            if (lane < 9) {
-                const int ux = cur_bxy.x + c_nb_dx[lane], uy = cur_bxy.y + c_nb_dy[lane];
-                const int wx = (ux + a.nx) % a.nx, wy = (uy + a.ny) % a.ny;
-                const int sb = wy * a.nx + wx;
-                const int b0 = a.sstart[sb];
-                cntk = a.sstart[sb + 1] - b0;
-                W.nbs[lane] = b0;
-                const double zx = ux < 0 ? a.zxm : (ux >= a.nx ? a.zxp : 0.0);
-                const double zy = uy < 0 ? a.zym : (uy >= a.ny ? a.zyp : 0.0);
-                W.nbz[lane] = make_double2(zx, zy);
-                W.nbzf[lane] = make_float2((float)zx, (float)zy);
-            }
-            int incl = cntk;
+            // neighbour boxes: first source, counts -> list prefix, image shift
+            // (once per box), and the pre-test band, which depends on the target
+            if (newbox) {
+                int cntk = 0;
+                if (lane < 9) {
+                    const int ux = cur_bxy.x + c_nb_dx[lane], uy = cur_bxy.y + c_nb_dy[lane];
+                    const int wx = (ux + a.nx) % a.nx, wy = (uy + a.ny) % a.ny;
+                    const int sb = wy * a.nx + wx;
+                    const int b0 = a.sstart[sb];
+                    cntk = a.sstart[sb + 1] - b0;
+                    W.nbs[lane] = b0;
+                    const double zx = ux < 0 ? a.zxm : (ux >= a.nx ? a.zxp : 0.0);
+                    const double zy = uy < 0 ? a.zym : (uy >= a.ny ? a.zyp : 0.0);
+                    W.nbz[lane] = make_double2(zx, zy);
+                    W.nbzf[lane] = make_float2((float)zx, (float)zy);
+                }
+                int incl = cntk;
 #pragma unroll
-            for (int o = 1; o < 16; o <<= 1) {
-                const int v = __shfl_up_sync(~0u, incl, o);
-                if (lane >= o) incl += v;
+                for (int o = 1; o < 16; o <<= 1) {
+                    const int v = __shfl_up_sync(~0u, incl, o);
+                    if (lane >= o) incl += v;
+                }
+                if (lane < 9) W.nbp[lane + 1] = incl;
+                if (lane == 0) W.nbp[0] = 0;
+                __syncwarp();
             }
-            if (lane < 9) W.nbp[lane + 1] = incl;
-            if (lane == 0) W.nbp[0] = 0;
+            if (lane < 9) {
+                const float2 zf = W.nbzf[lane];
+                W.nbe[lane] = make_float2(0x1p-22f * (fabsf(Tf.x) + fabsf(zf.x)),
+                                          0x1p-22f * (fabsf(Tf.y) + fabsf(zf.y)));
+            }
             __syncwarp();
-        }
-        if (lane < 9) {
-            const float2 zf = W.nbzf[lane];
-            W.nbe[lane] = make_float2(0x1p-22f * (fabsf(Tf.x) + fabsf(zf.x)),
-                                      0x1p-22f * (fabsf(Tf.y) + fabsf(zf.y)));
-        }
-        __syncwarp();
-        const int total = W.nbp[9];
-        unsigned nslp = 0, ndlp = 0;
-        int kc = 0;   // neighbour box of this lane's candidate (v only grows)
-        for (int v0 = 0; v0 < total; v0 += 32) {
-            const int v = v0 + lane;
-            int fl = 0, s = 0, k = kc;
-            bool nearp = false;
-            if (v < total) {
-                while (v >= W.nbp[k + 1]) k++;
-                kc = k;
-                s = W.nbs[k] + (v - W.nbp[k]);
-                if (k == 0) {
-                    // own box, no cutoff.  Distinct FP32 images imply an FP64
-                    // r2 > 0 (the offset is then >= 2^-150, its square normal),
-                    // so only r2f == 0 (or NaN) needs the reference's exact r2.
-                    const float2 Sf = a.spf[s];
-                    const float dxf = Tf.x - Sf.x, dyf = Tf.y - Sf.y;
-                    float r2f = dxf * dxf + dyf * dyf;
-                    bool self = false;
-                    if (!(r2f > 0.0f)) {
-                        const double2 S = a.sp[s];
-                        const double dx = xsub(T.x, S.x), dy = xsub(T.y, S.y);
-                        const double r2 = xadd(xmul(dx, dx), xmul(dy, dy));
-                        self = r2 == 0.0;
-                        r2f = (float)r2;
-                    }
-                    if (self) {
-                        // SLP self term (mex_stokes_slp_real.cpp:161-163); DLP skips r2 == 0.
-                        if (SLP) {
-                            const double *f = a.coef + (int64_t)a.nc * s;
-                            atomicAdd(&W.acc[slot][0], a.self_c * f[0]);
-                            atomicAdd(&W.acc[slot][1], a.self_c * f[1]);
+            const int total = W.nbp[9];
+            unsigned nslp = 0, ndlp = 0;
+            int kc = 0;   // neighbour box of this lane's candidate (v only grows)
+            for (int v0 = 0; v0 < total; v0 += 32) {
+                const int v = v0 + lane;
+                int fl = 0, s = 0, k = kc;
+                bool nearp = false;
+                if (v < total) {
+                    while (v >= W.nbp[k + 1]) k++;
+                    kc = k;
+                    s = W.nbs[k] + (v - W.nbp[k]);
+                    if (k == 0) {
+                        // own box, no cutoff.  Distinct FP32 images imply an FP64
+                        // r2 > 0 (the offset is then >= 2^-150, its square normal),
+                        // so only r2f == 0 (or NaN) needs the reference's exact r2.
+                        const float2 Sf = a.spf[s];
+                        const float dxf = Tf.x - Sf.x, dyf = Tf.y - Sf.y;
+                        float r2f = dxf * dxf + dyf * dyf;
+                        bool self = false;
+                        if (!(r2f > 0.0f)) {
+                            const double2 S = a.sp[s];
+                            const double dx = xsub(T.x, S.x), dy = xsub(T.y, S.y);
+                            const double r2 = xadd(xmul(dx, dx), xmul(dy, dy));
+                            self = r2 == 0.0;
+                            r2f = (float)r2;
+                        }
+                        if (self) {
+                            // SLP self term (mex_stokes_slp_real.cpp:161-163); DLP skips r2 == 0.
+                            if (SLP) {
+                                const double *f = a.coef + (int64_t)a.nc * s;
+                                atomicAdd(&W.acc[slot][0], a.self_c * f[0]);
+                                atomicAdd(&W.acc[slot][1], a.self_c * f[1]);
+                            }
+                        } else {
+                            fl = 3;
+                            const float xf = r2f * a.xi2f;
+                            nearp = !(xf > xlo && xf < xhi);
                         }
                     } else {
-                        fl = 3;
+                        const float2 Sf = a.spf[s];
+                        const float2 zf = W.nbzf[k];
+                        const float dxf = Sf.x - (Tf.x - zf.x), dyf = Sf.y - (Tf.y - zf.y);
+                        const float r2f = dxf * dxf + dyf * dyf;
+                        // |r2f - r2| bound for both offset forms (3 roundings per
+                        // coordinate, then squaring and summing), doubled.
+                        const float2 nbe = W.nbe[k];
+                        const float ex = fmaf(0x1p-22f, fabsf(Sf.x), nbe.x);
+                        const float ey = fmaf(0x1p-22f, fabsf(Sf.y), nbe.y);
+                        const float band = 2.0f * (ex * (2.0f * fabsf(dxf) + ex) +
+                                                   ey * (2.0f * fabsf(dyf) + ey) + 0x1p-22f * r2f);
                         const float xf = r2f * a.xi2f;
                         nearp = !(xf > xlo && xf < xhi);
-                    }
-                } else {
-                    const float2 Sf = a.spf[s];
-                    const float2 zf = W.nbzf[k];
-                    const float dxf = Sf.x - (Tf.x - zf.x), dyf = Sf.y - (Tf.y - zf.y);
-                    const float r2f = dxf * dxf + dyf * dyf;
-                    // |r2f - r2| bound for both offset forms (3 roundings per
-                    // coordinate, then squaring and summing), doubled.
-                    const float2 nbe = W.nbe[k];
-                    const float ex = fmaf(0x1p-22f, fabsf(Sf.x), nbe.x);
-                    const float ey = fmaf(0x1p-22f, fabsf(Sf.y), nbe.y);
-                    const float band = 2.0f * (ex * (2.0f * fabsf(dxf) + ex) +
-                                               ey * (2.0f * fabsf(dyf) + ey) + 0x1p-22f * r2f);
-                    const float xf = r2f * a.xi2f;
-                    nearp = !(xf > xlo && xf < xhi);
-                    if (r2f + band < a.cut2f) {
-                        fl = 3;
-                    } else if (!(r2f - band >= a.cut2f)) {
-                        // near the cutoff (or non-finite): the reference's exact tests
-                        const double2 S = a.sp[s];
-                        const double2 z = W.nbz[k];
-                        if (SLP) {
-                            const double dx = xsub(S.x, xsub(T.x, z.x));
-                            const double dy = xsub(S.y, xsub(T.y, z.y));
-                            if (xadd(xmul(dx, dx), xmul(dy, dy)) < a.cut2) fl |= 1;
-                        }
-                        if (DLP) {
-                            const double x1 = xadd(xsub(S.x, T.x), z.x);
-                            const double x2 = xadd(xsub(S.y, T.y), z.y);
-                            if (xadd(xmul(x1, x1), xmul(x2, x2)) < a.cut2) fl |= 2;
+                        if (r2f + band < a.cut2f) {
+                            fl = 3;
+                        } else if (!(r2f - band >= a.cut2f)) {
+                            // near the cutoff (or non-finite): the reference's exact tests
+                            const double2 S = a.sp[s];
+                            const double2 z = W.nbz[k];
+                            if (SLP) {
+                                const double dx = xsub(S.x, xsub(T.x, z.x));
+                                const double dy = xsub(S.y, xsub(T.y, z.y));
+                                if (xadd(xmul(dx, dx), xmul(dy, dy)) < a.cut2) fl |= 1;
+                            }
+                            if (DLP) {
+                                const double x1 = xadd(xsub(S.x, T.x), z.x);
+                                const double x2 = xadd(xsub(S.y, T.y), z.y);
+                                if (xadd(xmul(x1, x1), xmul(x2, x2)) < a.cut2) fl |= 2;
+                            }
                         }
                     }
                 }
-            }
-            if (!SLP) fl &= 2;
-            if (!DLP) fl &= 1;
-            if (a.counters) {                        // (warp-uniform)
-                nslp += __popc(__ballot_sync(~0u, (fl & 1) != 0));
-                ndlp += __popc(__ballot_sync(~0u, (fl & 2) != 0));
-            }
-            const int2 ent = make_int2(s, slot | (k << 8) | (fl << 12));
+                if (!SLP) fl &= 2;
+                if (!DLP) fl &= 1;
+                if (a.counters) {                        // (warp-uniform)
+                    nslp += __popc(__ballot_sync(~0u, (fl & 1) != 0));
+                    ndlp += __popc(__ballot_sync(~0u, (fl & 2) != 0));
+                }
+                const int2 ent = make_int2(s, slot | (k << 8) | (fl << 12));
 #pragma unroll
-            for (int j = 0; j < 2; j++) {
-                const bool mine = fl != 0 && nearp == (j == 1);
-                const unsigned m = __ballot_sync(~0u, mine);
-                if (mine) W.q[j][Q[j].qn + __popc(m & ((1u << lane) - 1u))] = ent;
-                Q[j].qn += __popc(m);
-                Q[j].enq += __popc(m);
+                for (int j = 0; j < 2; j++) {
+                    const bool mine = fl != 0 && nearp == (j == 1);
+                    const unsigned m = __ballot_sync(~0u, mine);
+                    if (mine) W.q[j][Q[j].qn + __popc(m & ((1u << lane) - 1u))] = ent;
+                    Q[j].qn += __popc(m);
+                    Q[j].enq += __popc(m);
+                }
+                __syncwarp();
+                if (Q[0].qn >= 32) batch(0, 32);
+                if (Q[1].qn >= 32) batch(1, 32);
+            }
+            if (lane == 0) {
+                W.tend[0][slot] = Q[0].enq;
+                W.tend[1][slot] = Q[1].enq;
+                if (a.counters) {                        // (diagnostic counts, per target)
+                    atomicAdd(a.counters, (unsigned long long)total);
+                    if (SLP) atomicAdd(a.counters + 1, (unsigned long long)nslp);
+                    if (DLP) atomicAdd(a.counters + 2, (unsigned long long)ndlp);
+                }
             }
             __syncwarp();
-            if (Q[0].qn >= 32) batch(0, 32);
-            if (Q[1].qn >= 32) batch(1, 32);
+            retire(false);
         }
-        if (lane == 0) {
-            W.tend[0][slot] = Q[0].enq;
-            W.tend[1][slot] = Q[1].enq;
-            if (a.counters) {                        // (diagnostic counts, per target)
-                atomicAdd(a.counters, (unsigned long long)total);
-                if (SLP) atomicAdd(a.counters + 1, (unsigned long long)nslp);
-                if (DLP) atomicAdd(a.counters + 2, (unsigned long long)ndlp);
-            }
-        }
-        __syncwarp();
-        retire(false);
+        __syncthreads();
+        if (threadIdx.x == 0) run_s = (int)gridDim.x + atomicAdd(a.next, 1);
+        __syncthreads();
     }
     drain();
 }
@@ -998,8 +1008,10 @@ struct AdjWarp {
     double2 pos[kRing];
     int2 bxy[kRing];            // the source's box as (column, row)
     long long idx[kRing];
-    long long tend[2][kRing];
+    unsigned tend[2][kRing];    // FIFO position after the source's last pair (mod 2^32)
     int nbs[9], nbp[10];
+    int curbox;                 // the box those describe (-1: none yet)
+    int2 curbxy;                // and its (column, row)
     double2 nbz[9];
     float2 nbzf[9];
 };
@@ -1027,34 +1039,33 @@ __device__ __forceinline__ void seg_flush_n(Acc &accs, int lane, int key, double
     __syncwarp();
 }
 
-// seg_flush_n for float-float sums, into the float-float ring.
-template <int NV, class Acc>
-__device__ __forceinline__ void seg_flush_n_ff(Acc &accs, int lane, int key, float2 *v)
+// The flush of the far pairs' seven sums per source (as flush_ff, an eighth value
+// of zero beside them): 4 + 2 + 1 exchanges, then 2 of the one value left per lane.
+// Lanes 4 i end with value i, its three bits taken from the top.
+__device__ __forceinline__ void flush_adj_ff(AdjWarp &W, int lane, bool fl, int tag, const float2 *v)
 {
+    const bool b2 = lane & 16, b1 = lane & 8, b0 = lane & 4;
+    const float2 z = make_float2(0.f, 0.f);
+    for (unsigned left = __ballot_sync(~0u, fl); left;) {
+        const int key = __shfl_sync(~0u, tag, __ffs(left) - 1);
+        const bool mine = fl && tag == key;
+        left &= ~__ballot_sync(~0u, mine);
+        float2 a[4], b[2];
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int ko = __shfl_up_sync(~0u, key, o);
-        float2 a[NV];
-#pragma unroll
-        for (int i = 0; i < NV; i++) {
-            a[i].x = __shfl_up_sync(~0u, v[i].x, o);
-            a[i].y = __shfl_up_sync(~0u, v[i].y, o);
+        for (int i = 0; i < 4; i++) {
+            const float2 lo = mine ? v[i] : z, hi = i < 3 && mine ? v[4 + (i < 3 ? i : 0)] : z;
+            a[i] = ff_tree_add(b2 ? hi : lo, ff_shfl_xor(b2 ? lo : hi, 16));
         }
-        if (lane >= o && ko == key) {
-            // heads by TwoSum, tails and errors carried unnormalised (as in seg_flush_ff)
 #pragma unroll
-            for (int i = 0; i < NV; i++) {
-                float s, e;
-                two_sum(v[i].x, a[i].x, s, e);
-                v[i] = make_float2(s, v[i].y + a[i].y + e);
-            }
+        for (int i = 0; i < 2; i++)
+            b[i] = ff_tree_add(b1 ? a[2 + i] : a[i], ff_shfl_xor(b1 ? a[i] : a[2 + i], 8));
+        float2 c = ff_tree_add(b0 ? b[1] : b[0], ff_shfl_xor(b0 ? b[0] : b[1], 4));
+        c = ff_tree_add(c, ff_shfl_xor(c, 2));
+        c = ff_tree_add(c, ff_shfl_xor(c, 1));
+        if ((lane & 3) == 0 && lane < 4 * kAdjVals) {
+            float2 &acc = W.accf[key % kRing][lane >> 2];
+            acc = ff_add(acc, ff_norm(c.x, c.y));
         }
-    }
-    const int kn = __shfl_down_sync(~0u, key, 1);
-    if (key >= 0 && key != 0x7fffffff && (lane == 31 || kn != key)) {
-        float2 *a = accs[key % kRing];
-#pragma unroll
-        for (int i = 0; i < NV; i++) a[i] = ff_add(a[i], ff_norm(v[i].x, v[i].y));
     }
     __syncwarp();
 }
@@ -1229,6 +1240,7 @@ __global__ void __launch_bounds__(kAdjWarps * 32, 5) k_real_adj(RealArgs a)
 {
     constexpr bool FF = FORM == kFormFF;
     __shared__ AdjWarp warps[kAdjWarps];
+    __shared__ int run_s;
     __shared__ double tab[64];
     __shared__ float2 tabff[64];
     __shared__ double e1s[66];
@@ -1243,10 +1255,9 @@ __global__ void __launch_bounds__(kAdjWarps * 32, 5) k_real_adj(RealArgs a)
     // queue 0: far pairs (float-float in the FF form), queue 1: the rest in FP64
     const float xlo = FF ? 1.0001f : 1.0f, xhi = FF ? 63.9f : INFINITY;
     AdjWarp &W = warps[wid];
-    const int64_t nw = (int64_t)gridDim.x * kAdjWarps;
     int head = 0, nfl = 0, gseq = 0;
     int qn[2] = {0, 0}, tag[2] = {-1, -1};
-    long long enq[2] = {0, 0}, proc[2] = {0, 0};
+    unsigned enq[2] = {0, 0}, proc[2] = {0, 0};   // (mod 2^32)
     double v[2][kAdjVals];
     float2 vf[kAdjVals];
 #pragma unroll
@@ -1268,10 +1279,7 @@ __global__ void __launch_bounds__(kAdjWarps * 32, 5) k_real_adj(RealArgs a)
         const bool ffq = FF && j == 0;
         if (__any_sync(~0u, fl)) {
             if (ffq) {
-                float2 tf[kAdjVals];
-#pragma unroll
-                for (int i = 0; i < kAdjVals; i++) tf[i] = fl ? vf[i] : make_float2(0.f, 0.f);
-                seg_flush_n_ff<kAdjVals>(W.accf, lane, tag[j], tf);
+                flush_adj_ff(W, lane, fl, tag[j], vf);
             } else {
                 double tmp[kAdjVals];
 #pragma unroll
@@ -1294,8 +1302,8 @@ __global__ void __launch_bounds__(kAdjWarps * 32, 5) k_real_adj(RealArgs a)
         }
     };
     auto retire = [&](bool all) {
-        while (nfl > 0 && (all || (proc[0] >= W.tend[0][head] + 32 &&
-                                   proc[1] >= W.tend[1][head] + 32))) {
+        while (nfl > 0 && (all || ((int)(proc[0] - W.tend[0][head]) >= 32 &&
+                                   (int)(proc[1] - W.tend[1][head]) >= 32))) {
             if (lane < kAdjVals) {
                 double v = W.acc[head][lane];
                 if (FF) v += ff_to_double(W.accf[head][lane]);
@@ -1306,74 +1314,89 @@ __global__ void __launch_bounds__(kAdjWarps * 32, 5) k_real_adj(RealArgs a)
         }
         __syncwarp();
     };
-    auto drain = [&]() {
-#pragma unroll
-        for (int j = 0; j < 2; j++) {
-            batch(j, qn[j]);
-            const int key = tag[j] >= 0 ? tag[j] : 0x7fffffff;
-            if (FF && j == 0) {
-                seg_flush_n_ff<kAdjVals>(W.accf, lane, key, vf);
-            } else {
-                seg_flush_n<kAdjVals>(W.acc, lane, key, v[j]);
-            }
-#pragma unroll
-            for (int i = 0; i < kAdjVals; i++) {
-                v[j][i] = 0.0;
-                vf[i] = make_float2(0.f, 0.f);
-            }
-            tag[j] = -1;
+    // Outer loop over forward sources (sorted), inner candidates are forward targets:
+    // runs as in k_real.  One pass per source, and one that drains the FIFOs when the
+    // ring is full or all runs are taken: its first step evaluates what is queued, its
+    // second (with no pairs) flushes every lane.  All passes go through the same two
+    // calls of batch, so that the pair arithmetic is in the instruction cache once
+    // (stalls for instructions were 5.8 of 13 cycles per issue with three copies).
+    const int64_t len = (int64_t)kAdjWarps * a.run;
+    int64_t s0 = (int64_t)blockIdx.x * len;
+    int s = (int)s0 + wid, s_end = (int)min(s0 + len, a.nouter);
+    if (lane == 0) W.curbox = -1;
+    __syncwarp();
+    for (;;) {
+        while (s >= s_end && s0 < a.nouter) {              // (the same for all warps)
+            __syncthreads();
+            if (threadIdx.x == 0) run_s = (int)gridDim.x + atomicAdd(a.next, 1);
+            __syncthreads();
+            s0 = run_s * len;
+            s = (int)min(s0, a.nouter) + wid;
+            s_end = (int)min(s0 + len, a.nouter);
         }
-        retire(true);
-    };
-
-    // outer loop over forward sources (sorted), inner candidates are forward targets
-    for (int64_t s = (int64_t)blockIdx.x * kAdjWarps + wid; s < a.nouter; s += nw) {
-        if (nfl == kRing) drain();
+        const bool dr = nfl == kRing || s0 >= a.nouter;    // (warp-uniform)
         const int slot = (head + nfl) % kRing;
-        nfl++;
-        gseq++;
-        const int sbx = a.obox[s];
-        const double2 Sp = a.sp[s];
-        const float2 Sf = a.spf[s];
-        if (lane < kAdjVals + 1) W.acc[slot][lane] = 0.0;
-        if (lane < kAdjVals) W.accf[slot][lane] = make_float2(0.f, 0.f);
-        if (lane == 0) {
-            W.pos[slot] = Sp;
-            W.bxy[slot] = make_int2(sbx % a.nx, sbx / a.nx);
-            W.idx[slot] = s;
-        }
-        int cntk = 0;
-        if (lane < 9) {
-            // target box at offset k from the source box
-            const int ux = sbx % a.nx + c_nb_dx[lane], uy = sbx / a.nx + c_nb_dy[lane];
-            const int wx = (ux + a.nx) % a.nx, wy = (uy + a.ny) % a.ny;
-            const int tb = wy * a.nx + wx;
-            const int b0 = a.sstart[tb];           // target cell list
-            cntk = a.sstart[tb + 1] - b0;
-            W.nbs[lane] = b0;
-            // source image shift seen from that target box (box tb, offset -k)
-            const int vx = wx - c_nb_dx[lane], vy = wy - c_nb_dy[lane];
-            const double zx = vx < 0 ? a.zxm : (vx >= a.nx ? a.zxp : 0.0);
-            const double zy = vy < 0 ? a.zym : (vy >= a.ny ? a.zyp : 0.0);
-            W.nbz[lane] = make_double2(zx, zy);
-            W.nbzf[lane] = make_float2((float)zx, (float)zy);
-        }
-        int incl = cntk;
+        int total = 64;
+        double2 Sp = make_double2(0.0, 0.0);
+        float2 Sf = make_float2(0.f, 0.f);
+        if (!dr) {
+            nfl++;
+            gseq++;
+            const int sbx = a.obox[s];
+            Sp = a.sp[s];
+            Sf = a.spf[s];
+            const bool newbox = sbx != W.curbox;           // (warp-uniform)
+            if (newbox) {
+                __syncwarp();
+                if (lane == 0) {
+                    W.curbox = sbx;
+                    W.curbxy = make_int2(sbx % a.nx, sbx / a.nx);
+                }
+                __syncwarp();
+            }
+            const int2 b = W.curbxy;
+            if (lane < kAdjVals + 1) W.acc[slot][lane] = 0.0;
+            if (lane < kAdjVals) W.accf[slot][lane] = make_float2(0.f, 0.f);
+            if (lane == 0) {
+                W.pos[slot] = Sp;
+                W.bxy[slot] = b;
+                W.idx[slot] = s;
+            }
+            if (newbox) {
+                int cntk = 0;
+                if (lane < 9) {
+                    // target box at offset k from the source box
+                    const int ux = b.x + c_nb_dx[lane], uy = b.y + c_nb_dy[lane];
+                    const int wx = (ux + a.nx) % a.nx, wy = (uy + a.ny) % a.ny;
+                    const int tb = wy * a.nx + wx;
+                    const int b0 = a.sstart[tb];           // target cell list
+                    cntk = a.sstart[tb + 1] - b0;
+                    W.nbs[lane] = b0;
+                    // source image shift seen from that target box (box tb, offset -k)
+                    const int vx = wx - c_nb_dx[lane], vy = wy - c_nb_dy[lane];
+                    const double zx = vx < 0 ? a.zxm : (vx >= a.nx ? a.zxp : 0.0);
+                    const double zy = vy < 0 ? a.zym : (vy >= a.ny ? a.zyp : 0.0);
+                    W.nbz[lane] = make_double2(zx, zy);
+                    W.nbzf[lane] = make_float2((float)zx, (float)zy);
+                }
+                int incl = cntk;
 #pragma unroll
-        for (int o = 1; o < 16; o <<= 1) {
-            const int vv = __shfl_up_sync(~0u, incl, o);
-            if (lane >= o) incl += vv;
+                for (int o = 1; o < 16; o <<= 1) {
+                    const int vv = __shfl_up_sync(~0u, incl, o);
+                    if (lane >= o) incl += vv;
+                }
+                if (lane < 9) W.nbp[lane + 1] = incl;
+                if (lane == 0) W.nbp[0] = 0;
+            }
+            __syncwarp();
+            total = W.nbp[9];
         }
-        if (lane < 9) W.nbp[lane + 1] = incl;
-        if (lane == 0) W.nbp[0] = 0;
-        __syncwarp();
-        const int total = W.nbp[9];
         int kc = 0;   // neighbour box of this lane's candidate (vi only grows)
         for (int v0 = 0; v0 < total; v0 += 32) {
             const int vi = v0 + lane;
             int fl = 0, t = 0, k = kc;
             bool nearp = false;
-            if (vi < total) {
+            if (!dr && vi < total) {
                 while (vi >= W.nbp[k + 1]) k++;
                 kc = k;
                 t = W.nbs[k] + (vi - W.nbp[k]);
@@ -1433,8 +1456,14 @@ __global__ void __launch_bounds__(kAdjWarps * 32, 5) k_real_adj(RealArgs a)
                 enq[j] += __popc(m);
             }
             __syncwarp();
-            if (qn[0] >= 32) batch(0, 32);
-            if (qn[1] >= 32) batch(1, 32);
+#pragma unroll
+            for (int j = 0; j < 2; j++)
+                if (dr || qn[j] >= 32) batch(j, dr ? qn[j] : 32);
+        }
+        if (dr) {
+            retire(true);
+            if (s0 >= a.nouter) return;
+            continue;
         }
         if (lane == 0) {
             W.tend[0][slot] = enq[0];
@@ -1442,8 +1471,8 @@ __global__ void __launch_bounds__(kAdjWarps * 32, 5) k_real_adj(RealArgs a)
         }
         __syncwarp();
         retire(false);
+        s += kAdjWarps;
     }
-    drain();
 }
 
 template __global__ void k_real_adj<true, false, kFormFP64>(RealArgs);
@@ -3271,13 +3300,29 @@ cudaError_t launch_sort(const SortArgs &a, int nsets, cudaStream_t st, int64_t &
 cudaError_t launch_src_coef(int64_t n, const int *perm, const double2 *f_slp,
                             const double2 *f_dlp, const double2 *nrm, double *coef, int nc,
                             cudaStream_t st, int64_t &launches, float2 *out, int64_t ostride,
-                            bool tails)
+                            bool tails, int *zero)
 {
-    if (n <= 0) return cudaSuccess;
-    k_src_coef<<<grid_for(n, 256), 256, 0, st>>>(n, perm, f_slp, f_dlp, nrm, coef, nc, out, ostride,
-                                                 tails ? 1 : 0);
+    if (n <= 0 && !zero) return cudaSuccess;
+    k_src_coef<<<grid_for(n > 0 ? n : 1, 256), 256, 0, st>>>(n, perm, f_slp, f_dlp, nrm, coef, nc, out,
+                                                             ostride, tails ? 1 : 0, zero);
     launches++;
     return cudaGetLastError();
+}
+
+// Points per warp and run of the real-space kernels' outer loop, for n points over
+// nwarps warps and ninner candidates in nbox boxes: an eighth of a warp's points (32
+// at most), but at least 256 points at one candidate per box (8 at 32 candidates: below
+// that the barrier and the neighbour set of every run cost more than they even out).
+// Microseconds per evaluation with runs of 1, 2, 4, 8, 16, 32 points and one run per
+// warp: 2^20 uniform points 12582, 12020, 11612, 11387, 11291, 11307, 11505; 2^17
+// (36 per warp) 1743, 1685, 1646, 1634, 1673, 1787, 1645; 2^16 points by circles
+// (455 candidates per box) 2275, 2284, 2490, 3258, 5255, 9629, 5870.
+static int real_run(int64_t n, int64_t ninner, int64_t nbox, int64_t nwarps)
+{
+    const int64_t all = (n + nwarps - 1) / nwarps, eighth = all / 8 < 32 ? all / 8 : 32;
+    const int64_t least = ninner > 0 && 256 * nbox / ninner < all ? 256 * nbox / ninner : all;
+    const int64_t r = eighth > least ? eighth : least;
+    return (int)(r > 1 ? r : 1);
 }
 
 template <int FORM>
@@ -3288,10 +3333,11 @@ static void launch_real_form(const RealArgs &a, bool slp, bool dlp, unsigned g, 
     else k_real<false, true, FORM><<<g, kRealWarps * 32, 0, st>>>(a);
 }
 
-cudaError_t launch_real(const RealArgs &a, bool slp, bool dlp, cudaStream_t st,
+cudaError_t launch_real(const RealArgs &args, bool slp, bool dlp, cudaStream_t st,
                         int64_t &launches, int form)
 {
-    if (a.ntar <= 0) return cudaSuccess;
+    if (args.ntar <= 0) return cudaSuccess;
+    RealArgs a = args;
     const int64_t want = (a.ntar + kRealWarps - 1) / kRealWarps;
     // Six 4-warp blocks per SM (the launch bound holds 80 registers: 24 warps
     // resident), persistent over the sorted targets.  The k-space chain
@@ -3300,6 +3346,7 @@ cudaError_t launch_real(const RealArgs &a, bool slp, bool dlp, cudaStream_t st,
     // against 18.6 with 20 warps and 18.45 with 24.
     const int64_t cap = (int64_t)sm_count() * SE2P_REAL_MINB;
     const unsigned g = (unsigned)(want < cap ? want : cap);
+    a.run = real_run(a.ntar, a.ns, (int64_t)a.nx * a.ny, (int64_t)g * kRealWarps);
     if (form == kFormF32) launch_real_form<kFormF32>(a, slp, dlp, g, st);
     else if (form == kFormFF) launch_real_form<kFormFF>(a, slp, dlp, g, st);
     else launch_real_form<kFormFP64>(a, slp, dlp, g, st);
@@ -3416,15 +3463,17 @@ static void launch_real_adj_form(const RealArgs &a, bool slp, bool dlp, unsigned
     else k_real_adj<false, true, FORM><<<g, kAdjWarps * 32, 0, st>>>(a);
 }
 
-cudaError_t launch_real_adj(const RealArgs &a, bool slp, bool dlp, cudaStream_t st,
+cudaError_t launch_real_adj(const RealArgs &args, bool slp, bool dlp, cudaStream_t st,
                             int64_t &launches, int form)
 {
-    if (a.nouter <= 0) return cudaSuccess;
+    if (args.nouter <= 0) return cudaSuccess;
+    RealArgs a = args;
     const int64_t want = (a.nouter + kAdjWarps - 1) / kAdjWarps;
     // as many 4-warp blocks as fit at once (5 per SM at the launch bound), so
     // that no second wave of persistent blocks trails the first
     const int64_t cap = (int64_t)sm_count() * 5;
     const unsigned g = (unsigned)(want < cap ? want : cap);
+    a.run = real_run(a.nouter, a.ntar, (int64_t)a.nx * a.ny, (int64_t)g * kAdjWarps);
     if (form == kFormFF) launch_real_adj_form<kFormFF>(a, slp, dlp, g, st);
     else launch_real_adj_form<kFormFP64>(a, slp, dlp, g, st);
     launches++;
