@@ -322,21 +322,127 @@ __device__ __forceinline__ double rcp_nr(double a)
     return fma(r, e, r);
 }
 
+// The candidates of one outer point: the points of its 3x3 boxes in up to nine pieces.
+// Boxes of a row are consecutive in the cell list, so away from the first and last
+// column three pieces hold the nine boxes, the own row first.
+// The scan is issue-bound like the rest of the kernel (about a third of its instructions):
+// what a candidate's test needs is the same for a piece, and the cutoff's error band for a
+// point.  With a band, an image lookup and a search of nine boxes per candidate instead,
+// k_real took 2.15 ms on 2^16 points by circles (now 1.84) and k_real_adj 3.5 ms at 2^18
+// points (now 3.07).
+struct Nbhd {
+    int4 seg[9];                // first point and end of the piece, image code
+    float2 z[9];                // the piece's image shift, rounded, to take off the outer point
+    int own0, ownn;             // the own box's points (in piece 0)
+    int nseg, total;            // pieces, points
+    int box;                    // the box these describe (-1: none yet)
+    float2 zmax;                // largest |image shift| of a piece
+    float2 p, cut;              // of the outer point: rounded position, cutoff pre-test
+};
+
+// Image codes: x in bits 0-1, y in bits 2-3; 0 none, 1 the shift zxm (zym), 2 zxp (zyp).
+__device__ __forceinline__ double2 image_shift(const RealArgs &a, int code)
+{
+    const int cx = code & 3, cy = code >> 2;
+    return make_double2(cx == 0 ? 0.0 : cx == 1 ? a.zxm : a.zxp, cy == 0 ? 0.0 : cy == 1 ? a.zym : a.zyp);
+}
+
+// FLIP: the shift of the outer point seen from the candidate's box (the adjoint's outer
+// points are the forward sources), in place of the candidate's seen from the outer box.
+template <bool FLIP>
+__device__ __forceinline__ void nbhd_build(Nbhd &N, const RealArgs &a, int lane, int box)
+{
+    const int bx = box % a.nx, by = box / a.nx;
+    const bool row = bx > 0 && bx < a.nx - 1;              // a row's three boxes are one piece
+    const int nseg = row ? 3 : 9;
+    int cnt = 0, p0 = 0, code = 0;
+    if (lane < nseg) {
+        const int ux = bx + (row ? 0 : c_nb_dx[lane]);
+        const int uy = by + (row ? (lane == 0 ? 0 : 2 * lane - 3) : c_nb_dy[lane]);
+        const int wx = ux < 0 ? ux + a.nx : ux >= a.nx ? ux - a.nx : ux;
+        const int wy = uy < 0 ? uy + a.ny : uy >= a.ny ? uy - a.ny : uy;
+        const int b = wy * a.nx + wx;
+        p0 = a.sstart[b - row];
+        cnt = a.sstart[b + 1 + row] - p0;
+        int cx = ux < 0 ? 1 : ux >= a.nx ? 2 : 0, cy = uy < 0 ? 1 : uy >= a.ny ? 2 : 0;
+        if (FLIP) {
+            cx = cx ? 3 - cx : 0;
+            cy = cy ? 3 - cy : 0;
+        }
+        code = cx | cy << 2;
+    }
+    int end = cnt;
+#pragma unroll
+    for (int o = 1; o < 16; o <<= 1) {
+        const int v = __shfl_up_sync(~0u, end, o);
+        if (lane >= o) end += v;
+    }
+    __syncwarp();
+    if (lane < 9) {
+        const double2 z = image_shift(a, code);
+        const float sgn = FLIP ? -1.f : 1.f;
+        N.seg[lane] = make_int4(p0, p0 + cnt, code, 0);
+        N.z[lane] = make_float2(sgn * (float)z.x, sgn * (float)z.y);
+    }
+    if (lane == 8) N.total = end;
+    if (lane == 0) {
+        N.own0 = a.sstart[box];
+        N.ownn = a.sstart[box + 1] - N.own0;
+        N.nseg = nseg;
+        N.box = box;
+        N.zmax = make_float2(row ? 0.f : fmaxf(fabsf((float)a.zxm), fabsf((float)a.zxp)),
+                             by > 0 && by < a.ny - 1 ? 0.f
+                                                     : fmaxf(fabsf((float)a.zym), fabsf((float)a.zyp)));
+    }
+    __syncwarp();
+}
+
+// The FP32 pre-test of the cutoff r2 < cut2 for an outer point at P (rounded from
+// FP64): an FP32 r2f below x is inside in the exact test, one at y or above outside, and
+// the rest take the exact test.  With u = 2^-24 the rounded positions, the shift and the
+// two subtractions put a coordinate difference d of the list within
+// u (2 |d| + 3 (|P| + |z|)) < e = 2^-22 (R + max(|P| + |z|)) where |d| < R = 1.25 rc, so
+// r2f within e (3 R + 2 e) + 3 u r2f; for the rest (r2f > 1.5 cut2) the same bound
+// relative to d leaves r2 > cut2 as long as e < R / 20.  Where that does not hold
+// (coordinates far outside the cell, or cut2 near the end of the FP32 range) every
+// candidate takes the exact test.
+__device__ __forceinline__ float2 cut_band(const Nbhd &N, float2 P, float cut2f)
+{
+    const float R = 1.25f * sqrtf(cut2f);
+    const float e = 0x1p-22f * (R + fmaxf(fabsf(P.x) + N.zmax.x, fabsf(P.y) + N.zmax.y));
+    const float band = 1.1f * (e * (3.0f * R + 2.0f * e) + 0x1p-21f * R * R);
+    const bool ok = e < 0.05f * R && cut2f > 1e-30f && cut2f < 1e30f;
+    return ok ? make_float2(cut2f - band, cut2f + band) : make_float2(-1.f, INFINITY);
+}
+
+// A piece as the test of its candidates needs it (the same in every lane).
+struct Piece {
+    int begin, end, ey;         // points; the FIFO entry's second word
+    int own0;
+    unsigned ownn;              // own box's points, no cutoff there
+    float ox, oy;               // the outer point seen from the piece
+    __device__ __forceinline__ Piece(const Nbhd &N, int q, int base)
+    {
+        const int4 sg = N.seg[q];
+        begin = sg.x;
+        end = sg.y;
+        ey = base | sg.z << 8;
+        ox = N.p.x - N.z[q].x;
+        oy = N.p.y - N.z[q].y;
+        own0 = N.own0;
+        ownn = q == 0 ? N.ownn : 0;
+    }
+};
+
 struct RealWarp {
     int2 q[2][64];              // pair FIFOs: [0] main, [1] near field (x <= 1)
-                                // entry = (sorted source, slot | k << 8 | flags << 12)
+                                // entry = (sorted source, slot | image code << 8 | flags << 12)
     double acc[kRing][4];       // per-target sums: SLP u1, u2, DLP u1, u2
     float2 accf[kRing][4];      // the same from float-float pairs (FP64 form, queue 0)
     double2 tpos[kRing];
-    int2 tbxy[kRing];           // the target's box as (column, row)
     int tidx[kRing];
     unsigned tend[2][kRing];    // FIFO position after the target's last pair (mod 2^32)
-    int nbs[9], nbp[10];        // neighbour box: first sorted source, list prefix
-    int curbox;                 // the box those describe (-1: none yet)
-    int2 curbxy;                // and its (column, row)
-    double2 nbz[9];
-    float2 nbzf[9];
-    float2 nbe[9];              // 2^-22 (|t| + |z|) per neighbour box (the pre-test band)
+    Nbhd nb;
 };
 
 // Segmented warp reduction of (v0..v3) by nondecreasing key; the last lane
@@ -435,24 +541,20 @@ __device__ __forceinline__ void real_pair(const RealArgs &a, const RealWarp &W, 
                                           const double *tab, const double *e1s, double &s1,
                                           double &s2, double &d1, double &d2)
 {
-    const int s = e.x, slot = e.y & 0xff, k = (e.y >> 8) & 0xf, fl = e.y >> 12;
+    const int s = e.x, slot = e.y & 0xff, img = (e.y >> 8) & 0xf, fl = e.y >> 12;
     const double2 S = a.sp[s];
     const double2 T = W.tpos[slot];
-    // image shift of neighbour k: 0 or the reference's (L*(+-nside))/nside
-    const int2 tb = W.tbxy[slot];
-    const int ux = tb.x + c_nb_dx[k], uy = tb.y + c_nb_dy[k];
+    // image shift: 0 or the reference's (L*(+-nside))/nside
     // Without a periodic image both offset forms are exactly s - t; across an
     // image (rare) the SLP form s-(t-z) and the DLP form (s-t)+z are formed
     // separately and each kernel keeps its own r2, as the reference does.
-    const bool img = ux < 0 || ux >= a.nx || uy < 0 || uy >= a.ny;
     double x1 = S.x - T.x, x2 = S.y - T.y, dxs = x1, dys = x2;
     if (img) {
-        const double zx = ux < 0 ? a.zxm : (ux >= a.nx ? a.zxp : 0.0);
-        const double zy = uy < 0 ? a.zym : (uy >= a.ny ? a.zyp : 0.0);
-        x1 += zx;
-        x2 += zy;
-        dxs = S.x - (T.x - zx);
-        dys = S.y - (T.y - zy);
+        const double2 z = image_shift(a, img);
+        x1 += z.x;
+        x2 += z.y;
+        dxs = S.x - (T.x - z.x);
+        dys = S.y - (T.y - z.y);
     }
     const double r2 = fma(dxs, dxs, dys * dys);
     const double x = r2 * a.xi2;
@@ -534,9 +636,7 @@ __device__ __forceinline__ void real_pair_f32(const RealArgs &a, const RealWarp 
                                               const float4 &zyf, float &s1, float &s2, float &d1,
                                               float &d2)
 {
-    const int s = e.x, slot = e.y & 0xff, k = (e.y >> 8) & 0xf, fl = e.y >> 12;
-    const int2 tb = W.tbxy[slot];
-    const int ux = tb.x + c_nb_dx[k], uy = tb.y + c_nb_dy[k];
+    const int s = e.x, slot = e.y & 0xff, cx = (e.y >> 8) & 3, cy = (e.y >> 10) & 3, fl = e.y >> 12;
     // The offset s - t + z from float-float positions, on the FP32 pipe: the
     // TwoSum of the high halves is exact, the image shift z (zxf = (z-.hi,
     // z-.lo, z+.hi, z+.lo)) cancels its head exactly (Sterbenz: the two are
@@ -544,10 +644,10 @@ __device__ __forceinline__ void real_pair_f32(const RealArgs &a, const RealWarp 
     // follow; one rounding to FP32 at the end.
     const float2 Sh = a.spf[s], Sl = a.spl[s];
     const float4 Tq = tposff[slot];
-    const float2 zx = ux < 0 ? make_float2(zxf.x, zxf.y)
-                             : (ux >= a.nx ? make_float2(zxf.z, zxf.w) : make_float2(0.f, 0.f));
-    const float2 zy = uy < 0 ? make_float2(zyf.x, zyf.y)
-                             : (uy >= a.ny ? make_float2(zyf.z, zyf.w) : make_float2(0.f, 0.f));
+    const float2 zx = cx == 1 ? make_float2(zxf.x, zxf.y)
+                              : (cx == 2 ? make_float2(zxf.z, zxf.w) : make_float2(0.f, 0.f));
+    const float2 zy = cy == 1 ? make_float2(zyf.x, zyf.y)
+                              : (cy == 2 ? make_float2(zyf.z, zyf.w) : make_float2(0.f, 0.f));
     float px, ex, py, ey;
     two_sum(Sh.x, -Tq.x, px, ex);
     two_sum(Sh.y, -Tq.y, py, ey);
@@ -604,16 +704,14 @@ __device__ __forceinline__ void real_pair_ff(const RealArgs &a, const RealWarp &
                                              const float2 *tabff, float2 xi2, float2 pf,
                                              float2 &s1, float2 &s2, float2 &d1, float2 &d2)
 {
-    const int s = e.x, slot = e.y & 0xff, k = (e.y >> 8) & 0xf, fl = e.y >> 12;
+    const int s = e.x, slot = e.y & 0xff, img = (e.y >> 8) & 0xf, fl = e.y >> 12;
     const double2 S = a.sp[s];
     const double2 T = W.tpos[slot];
-    // image shift of neighbour k of this pair's target (the FIFO outlives W.nbz)
-    const int2 tb = W.tbxy[slot];
-    const int ux = tb.x + c_nb_dx[k], uy = tb.y + c_nb_dy[k];
     double dx = S.x - T.x, dy = S.y - T.y;
-    if (ux < 0 || ux >= a.nx || uy < 0 || uy >= a.ny) {   // across a periodic image
-        dx += ux < 0 ? a.zxm : (ux >= a.nx ? a.zxp : 0.0);
-        dy += uy < 0 ? a.zym : (uy >= a.ny ? a.zyp : 0.0);
+    if (img) {                                            // across a periodic image
+        const double2 z = image_shift(a, img);
+        dx += z.x;
+        dy += z.y;
     }
     const float2 x1 = ff_split(dx), x2 = ff_split(dy);
     const float2 r2 = ff_add(ff_sqr(x1), ff_sqr(x2));
@@ -656,7 +754,6 @@ __device__ __forceinline__ void real_pair_ff(const RealArgs &a, const RealWarp &
 
 // Lane-side state of one pair FIFO.
 struct PairQueue {
-    int qn;               // entries queued (warp-uniform)
     unsigned enq, proc;   // entries enqueued / processed so far, mod 2^32 (warp-uniform)
     int tag;              // sequence number of the target this lane's sums belong to
     double s1, s2, d1, d2;
@@ -698,7 +795,7 @@ __global__ void __launch_bounds__(kRealWarps * 32, SE2P_REAL_MINB) k_real(RealAr
     // Queue 0 (the fast pairs): float-float pairs 1 < x < 64 with margins
     // for the FP32 pre-test; FP32-grid form, x > 1 (near pairs, E1 at small
     // argument, stay FP64 in both forms).
-    const float xlo = FF ? 1.0001f : 1.0f, xhi = FF ? 63.9f : INFINITY;
+    const float rlo = (FF ? 1.0001f : 1.0f) / a.xi2f, rhi = FF ? 63.9f / a.xi2f : INFINITY;
     for (int i = threadIdx.x; i < 66; i += blockDim.x) {
         e1s[i] = (&c_e1[0][0])[i];
         if (MIXED) e1f[i] = (&c_e1f[0][0])[i];
@@ -710,7 +807,7 @@ __global__ void __launch_bounds__(kRealWarps * 32, SE2P_REAL_MINB) k_real(RealAr
     PairQueue Q[2];
 #pragma unroll
     for (int j = 0; j < 2; j++) {
-        Q[j].qn = 0; Q[j].enq = 0; Q[j].proc = 0; Q[j].tag = -1;
+        Q[j].enq = 0; Q[j].proc = 0; Q[j].tag = -1;
         Q[j].s1 = Q[j].s2 = Q[j].d1 = Q[j].d2 = 0.0;
         Q[j].f1 = Q[j].f2 = Q[j].g1 = Q[j].g2 = 0.f;
         Q[j].h1 = Q[j].h2 = Q[j].k1 = Q[j].k2 = make_float2(0.f, 0.f);
@@ -720,13 +817,11 @@ __global__ void __launch_bounds__(kRealWarps * 32, SE2P_REAL_MINB) k_real(RealAr
     // sums belong to another target flush first.
     auto batch = [&](int j, int cnt) {
         PairQueue &P = Q[j];
-        const int2 e = lane < cnt ? W.q[j][lane] : make_int2(0, -1);
+        const int2 e = lane < cnt ? W.q[j][(P.proc + lane) & 63] : make_int2(0, -1);
         __syncwarp();
-        if (lane < P.qn - cnt) W.q[j][lane] = W.q[j][lane + cnt];
-        P.qn -= cnt;
         P.proc += cnt;
         int eseq = -1;
-        if (e.y >= 0) eseq = gseq - nfl + (((e.y & 0xff) - head + kRing) % kRing);
+        if (e.y >= 0) eseq = gseq - nfl + (((e.y & 0xff) - head) & (kRing - 1));
         const bool fl = P.tag >= 0 && (lane >= cnt || P.tag != eseq);
         const bool f32 = MIXED && j == 0;
         const bool ffp = FF && j == 0;
@@ -773,7 +868,7 @@ __global__ void __launch_bounds__(kRealWarps * 32, SE2P_REAL_MINB) k_real(RealAr
     auto drain = [&]() {
 #pragma unroll
         for (int j = 0; j < 2; j++) {
-            batch(j, Q[j].qn);
+            batch(j, (int)(Q[j].enq - Q[j].proc));
             const int key = Q[j].tag >= 0 ? Q[j].tag : 0x7fffffff;
             if (MIXED && j == 0)
                 flush_f(W, lane, Q[j].tag >= 0, Q[j].tag, Q[j].f1, Q[j].f2, Q[j].g1, Q[j].g2);
@@ -796,7 +891,7 @@ __global__ void __launch_bounds__(kRealWarps * 32, SE2P_REAL_MINB) k_real(RealAr
     // time.  The FIFOs go on from run to run.
     // (the cell lists hold int indices, so ntar < 2^31)
     const int64_t len = (int64_t)kRealWarps * a.run;
-    if (lane == 0) W.curbox = -1;
+    if (lane == 0) W.nb.box = -1;
     __syncwarp();
     for (int64_t t0 = (int64_t)blockIdx.x * len; t0 < a.ntar; t0 = run_s * len) {
         const int t_end = (int)min(t0 + len, a.ntar);
@@ -806,158 +901,99 @@ __global__ void __launch_bounds__(kRealWarps * 32, SE2P_REAL_MINB) k_real(RealAr
             nfl++;
             gseq++;
             const int tb = a.tbox[t];
-            const double2 T = a.tp[t];
-            const float2 Tf = a.tpf[t];
-            const bool newbox = tb != W.curbox;                // (warp-uniform)
-            if (newbox) {
-                __syncwarp();
-                if (lane == 0) {
-                    W.curbox = tb;
-                    W.curbxy = make_int2(tb % a.nx, tb / a.nx);
-                }
-                __syncwarp();
-            }
-            const int2 cur_bxy = W.curbxy;
+            if (tb != W.nb.box) nbhd_build<false>(W.nb, a, lane, tb);   // (warp-uniform)
             if (lane < 4) {
                 W.acc[slot][lane] = 0.0;
                 W.accf[slot][lane] = make_float2(0.f, 0.f);
             }
             if (lane == 0) {
-                W.tpos[slot] = T;
-                W.tbxy[slot] = cur_bxy;
+                W.tpos[slot] = a.tp[t];
                 W.tidx[slot] = t;
+                const float2 Tf = a.tpf[t];
+                W.nb.p = Tf;
+                W.nb.cut = cut_band(W.nb, Tf, a.cut2f);
                 if (MIXED) {
                     const float2 tl = a.tpl[t];
                     tposff[slot] = make_float4(Tf.x, Tf.y, tl.x, tl.y);
                 }
             }
-            // neighbour boxes: first source, counts -> list prefix, image shift
-            // (once per box), and the pre-test band, which depends on the target
-            if (newbox) {
-                int cntk = 0;
-                if (lane < 9) {
-                    const int ux = cur_bxy.x + c_nb_dx[lane], uy = cur_bxy.y + c_nb_dy[lane];
-                    const int wx = (ux + a.nx) % a.nx, wy = (uy + a.ny) % a.ny;
-                    const int sb = wy * a.nx + wx;
-                    const int b0 = a.sstart[sb];
-                    cntk = a.sstart[sb + 1] - b0;
-                    W.nbs[lane] = b0;
-                    const double zx = ux < 0 ? a.zxm : (ux >= a.nx ? a.zxp : 0.0);
-                    const double zy = uy < 0 ? a.zym : (uy >= a.ny ? a.zyp : 0.0);
-                    W.nbz[lane] = make_double2(zx, zy);
-                    W.nbzf[lane] = make_float2((float)zx, (float)zy);
-                }
-                int incl = cntk;
-#pragma unroll
-                for (int o = 1; o < 16; o <<= 1) {
-                    const int v = __shfl_up_sync(~0u, incl, o);
-                    if (lane >= o) incl += v;
-                }
-                if (lane < 9) W.nbp[lane + 1] = incl;
-                if (lane == 0) W.nbp[0] = 0;
-                __syncwarp();
-            }
-            if (lane < 9) {
-                const float2 zf = W.nbzf[lane];
-                W.nbe[lane] = make_float2(0x1p-22f * (fabsf(Tf.x) + fabsf(zf.x)),
-                                          0x1p-22f * (fabsf(Tf.y) + fabsf(zf.y)));
-            }
             __syncwarp();
-            const int total = W.nbp[9];
+            const float2 cut = W.nb.cut;
+            const int nseg = W.nb.nseg, base = slot | (SLP ? 0x1000 : 0) | (DLP ? 0x2000 : 0);
             unsigned nslp = 0, ndlp = 0;
-            int kc = 0;   // neighbour box of this lane's candidate (v only grows)
-            for (int v0 = 0; v0 < total; v0 += 32) {
-                const int v = v0 + lane;
-                int fl = 0, s = 0, k = kc;
-                bool nearp = false;
-                if (v < total) {
-                    while (v >= W.nbp[k + 1]) k++;
-                    kc = k;
-                    s = W.nbs[k] + (v - W.nbp[k]);
-                    if (k == 0) {
-                        // own box, no cutoff.  Distinct FP32 images imply an FP64
-                        // r2 > 0 (the offset is then >= 2^-150, its square normal),
-                        // so only r2f == 0 (or NaN) needs the reference's exact r2.
+            for (int q = 0; q < nseg; q++) {
+                const Piece C(W.nb, q, base);
+                for (int s0 = C.begin; s0 < C.end; s0 += 32) {
+                    const int s = s0 + lane;
+                    int y = C.ey;
+                    bool in = false, nearp = false;
+                    if (s < C.end) {
                         const float2 Sf = a.spf[s];
-                        const float dxf = Tf.x - Sf.x, dyf = Tf.y - Sf.y;
+                        const float dxf = Sf.x - C.ox, dyf = Sf.y - C.oy;
                         float r2f = dxf * dxf + dyf * dyf;
-                        bool self = false;
-                        if (!(r2f > 0.0f)) {
-                            const double2 S = a.sp[s];
-                            const double dx = xsub(T.x, S.x), dy = xsub(T.y, S.y);
-                            const double r2 = xadd(xmul(dx, dx), xmul(dy, dy));
-                            self = r2 == 0.0;
-                            r2f = (float)r2;
-                        }
-                        if (self) {
-                            // SLP self term (mex_stokes_slp_real.cpp:161-163); DLP skips r2 == 0.
-                            if (SLP) {
-                                const double *f = a.coef + (int64_t)a.nc * s;
-                                atomicAdd(&W.acc[slot][0], a.self_c * f[0]);
-                                atomicAdd(&W.acc[slot][1], a.self_c * f[1]);
+                        const bool own = (unsigned)(s - C.own0) < C.ownn;
+                        in = r2f > 0.f && r2f < (own ? INFINITY : cut.x);
+                        if (!in && (own || !(r2f >= cut.y))) {
+                            const double2 S = a.sp[s], T = W.tpos[slot];
+                            y = base & 0xff | C.ey & 0xf00;
+                            if (own) {
+                                // own box.  Distinct FP32 images imply an FP64 r2 > 0 (the
+                                // offset is then >= 2^-150, its square normal), so only
+                                // r2f == 0 (or not finite) needs the reference's exact r2.
+                                const double dx = xsub(T.x, S.x), dy = xsub(T.y, S.y);
+                                const double r2 = xadd(xmul(dx, dx), xmul(dy, dy));
+                                r2f = (float)r2;
+                                if (r2 == 0.0) {
+                                    // SLP self term (mex_stokes_slp_real.cpp:161-163); DLP skips r2 == 0.
+                                    if (SLP) {
+                                        const double *f = a.coef + (int64_t)a.nc * s;
+                                        atomicAdd(&W.acc[slot][0], a.self_c * f[0]);
+                                        atomicAdd(&W.acc[slot][1], a.self_c * f[1]);
+                                    }
+                                } else {
+                                    y = C.ey;
+                                }
+                            } else {
+                                // near the cutoff (or not finite): the reference's exact tests
+                                const double2 z = image_shift(a, (C.ey >> 8) & 0xf);
+                                if (SLP) {
+                                    const double dx = xsub(S.x, xsub(T.x, z.x));
+                                    const double dy = xsub(S.y, xsub(T.y, z.y));
+                                    if (xadd(xmul(dx, dx), xmul(dy, dy)) < a.cut2) y |= 0x1000;
+                                }
+                                if (DLP) {
+                                    const double x1 = xadd(xsub(S.x, T.x), z.x);
+                                    const double x2 = xadd(xsub(S.y, T.y), z.y);
+                                    if (xadd(xmul(x1, x1), xmul(x2, x2)) < a.cut2) y |= 0x2000;
+                                }
                             }
-                        } else {
-                            fl = 3;
-                            const float xf = r2f * a.xi2f;
-                            nearp = !(xf > xlo && xf < xhi);
+                            in = y >> 12;
                         }
-                    } else {
-                        const float2 Sf = a.spf[s];
-                        const float2 zf = W.nbzf[k];
-                        const float dxf = Sf.x - (Tf.x - zf.x), dyf = Sf.y - (Tf.y - zf.y);
-                        const float r2f = dxf * dxf + dyf * dyf;
-                        // |r2f - r2| bound for both offset forms (3 roundings per
-                        // coordinate, then squaring and summing), doubled.
-                        const float2 nbe = W.nbe[k];
-                        const float ex = fmaf(0x1p-22f, fabsf(Sf.x), nbe.x);
-                        const float ey = fmaf(0x1p-22f, fabsf(Sf.y), nbe.y);
-                        const float band = 2.0f * (ex * (2.0f * fabsf(dxf) + ex) +
-                                                   ey * (2.0f * fabsf(dyf) + ey) + 0x1p-22f * r2f);
-                        const float xf = r2f * a.xi2f;
-                        nearp = !(xf > xlo && xf < xhi);
-                        if (r2f + band < a.cut2f) {
-                            fl = 3;
-                        } else if (!(r2f - band >= a.cut2f)) {
-                            // near the cutoff (or non-finite): the reference's exact tests
-                            const double2 S = a.sp[s];
-                            const double2 z = W.nbz[k];
-                            if (SLP) {
-                                const double dx = xsub(S.x, xsub(T.x, z.x));
-                                const double dy = xsub(S.y, xsub(T.y, z.y));
-                                if (xadd(xmul(dx, dx), xmul(dy, dy)) < a.cut2) fl |= 1;
-                            }
-                            if (DLP) {
-                                const double x1 = xadd(xsub(S.x, T.x), z.x);
-                                const double x2 = xadd(xsub(S.y, T.y), z.y);
-                                if (xadd(xmul(x1, x1), xmul(x2, x2)) < a.cut2) fl |= 2;
-                            }
-                        }
+                        nearp = !(r2f > rlo && r2f < rhi);
                     }
+                    if (a.counters) {                        // (warp-uniform)
+                        nslp += __popc(__ballot_sync(~0u, in && (y & 0x1000)));
+                        ndlp += __popc(__ballot_sync(~0u, in && (y & 0x2000)));
+                    }
+                    const unsigned below = (1u << lane) - 1u;
+                    const unsigned m0 = __ballot_sync(~0u, in && !nearp), m1 = __ballot_sync(~0u, in && nearp);
+                    if (in && !nearp) W.q[0][(Q[0].enq + __popc(m0 & below)) & 63] = make_int2(s, y);
+                    Q[0].enq += __popc(m0);
+                    if (m1) {                                // (warp-uniform)
+                        if (in && nearp) W.q[1][(Q[1].enq + __popc(m1 & below)) & 63] = make_int2(s, y);
+                        Q[1].enq += __popc(m1);
+                        __syncwarp();
+                        if (Q[1].enq - Q[1].proc >= 32) batch(1, 32);
+                    }
+                    __syncwarp();
+                    if (Q[0].enq - Q[0].proc >= 32) batch(0, 32);
                 }
-                if (!SLP) fl &= 2;
-                if (!DLP) fl &= 1;
-                if (a.counters) {                        // (warp-uniform)
-                    nslp += __popc(__ballot_sync(~0u, (fl & 1) != 0));
-                    ndlp += __popc(__ballot_sync(~0u, (fl & 2) != 0));
-                }
-                const int2 ent = make_int2(s, slot | (k << 8) | (fl << 12));
-#pragma unroll
-                for (int j = 0; j < 2; j++) {
-                    const bool mine = fl != 0 && nearp == (j == 1);
-                    const unsigned m = __ballot_sync(~0u, mine);
-                    if (mine) W.q[j][Q[j].qn + __popc(m & ((1u << lane) - 1u))] = ent;
-                    Q[j].qn += __popc(m);
-                    Q[j].enq += __popc(m);
-                }
-                __syncwarp();
-                if (Q[0].qn >= 32) batch(0, 32);
-                if (Q[1].qn >= 32) batch(1, 32);
             }
             if (lane == 0) {
                 W.tend[0][slot] = Q[0].enq;
                 W.tend[1][slot] = Q[1].enq;
                 if (a.counters) {                        // (diagnostic counts, per target)
-                    atomicAdd(a.counters, (unsigned long long)total);
+                    atomicAdd(a.counters, (unsigned long long)W.nb.total);
                     if (SLP) atomicAdd(a.counters + 1, (unsigned long long)nslp);
                     if (DLP) atomicAdd(a.counters + 2, (unsigned long long)ndlp);
                 }
@@ -1006,14 +1042,9 @@ struct AdjWarp {
     double acc[kRing][kAdjVals + 1];
     float2 accf[kRing][kAdjVals];    // the same from float-float pairs (FP64 form, queue 0)
     double2 pos[kRing];
-    int2 bxy[kRing];            // the source's box as (column, row)
-    long long idx[kRing];
+    int idx[kRing];
     unsigned tend[2][kRing];    // FIFO position after the source's last pair (mod 2^32)
-    int nbs[9], nbp[10];
-    int curbox;                 // the box those describe (-1: none yet)
-    int2 curbxy;                // and its (column, row)
-    double2 nbz[9];
-    float2 nbzf[9];
+    Nbhd nb;
 };
 
 template <int NV, class Acc>
@@ -1074,19 +1105,12 @@ template <bool SLP, bool DLP>
 __device__ __forceinline__ void adj_pair(const RealArgs &a, const AdjWarp &W, int2 e,
                                          const double *tab, const double *e1s, double *g)
 {
-    const int t = e.x, slot = e.y & 0xff, k = (e.y >> 8) & 0xf, fl = e.y >> 12;
+    const int t = e.x, slot = e.y & 0xff, fl = e.y >> 12;
     const double2 T = a.tp[t];                  // forward target (inner point)
     const double2 S = W.pos[slot];              // forward source (outer point)
-    // image shift of the source seen from the target's box: the target sits
-    // in box wrap(source box + offset k), so the unwrapped source box
-    // (target box - offset k) lies below 0 exactly when source box + offset
-    // reached past the last box, and beyond it when that went below 0
-    const int2 b = W.bxy[slot];
-    const int tx = b.x + c_nb_dx[k], ty = b.y + c_nb_dy[k];
-    const double zx = tx >= a.nx ? a.zxm : (tx < 0 ? a.zxp : 0.0);
-    const double zy = ty >= a.ny ? a.zym : (ty < 0 ? a.zyp : 0.0);
-    const double x1 = (S.x - T.x) + zx, x2 = (S.y - T.y) + zy;          // DLP form
-    const double d1 = S.x - (T.x - zx), d2 = S.y - (T.y - zy);          // SLP form
+    const double2 z = image_shift(a, (e.y >> 8) & 0xf);
+    const double x1 = (S.x - T.x) + z.x, x2 = (S.y - T.y) + z.y;        // DLP form
+    const double d1 = S.x - (T.x - z.x), d2 = S.y - (T.y - z.y);        // SLP form
     const double *wt = a.wcoef + 4 * (int64_t)t;                         // w_slp, w_dlp of t
     const double *cs = a.coef + (int64_t)a.nc * W.idx[slot];            // outer coefficients
     if (SLP && (fl & 1)) {
@@ -1096,16 +1120,16 @@ __device__ __forceinline__ void adj_pair(const RealArgs &a, const AdjWarp &W, in
         const double ir2 = rcp_nr(r2);
         const int set = x >= 16.0 ? 0 : (x > 1.0 ? 1 : 2);
         const double *c = e1s + 22 * set;
-        const double z = set == 2 ? x : ir2 * a.inv_xi2;
+        const double y = set == 2 ? x : ir2 * a.inv_xi2;
         double pa = c[0], pb = c[1];
 #pragma unroll
         for (int i = 2; i < 22; i += 2) {
-            pa = fma(z, pa, c[i]);
-            pb = fma(z, pb, c[i + 1]);
+            pa = fma(y, pa, c[i]);
+            pb = fma(y, pb, c[i + 1]);
         }
         const double den = set == 2 ? pb : pb + x;
         const double qv = pa * rcp_nr(den);
-        const double E = set == 2 ? qv + x - log(x) - 0.66373538970947265625 : ex * (z + qv);
+        const double E = set == 2 ? qv + x - log(x) - 0.66373538970947265625 : ex * (y + qv);
         const double w1 = wt[0], w2 = wt[1], f1 = cs[0], f2 = cs[1];
         const double h = 0.5 * E, gg = ex * ir2;
         const double gq = gg * fma(d1, w2, -d2 * w1);
@@ -1156,15 +1180,16 @@ __device__ __forceinline__ void adj_pair_ff(const RealArgs &a, const AdjWarp &W,
                                             const float2 *tabff, float2 xi2, float2 pf,
                                             float2 *g)
 {
-    const int t = e.x, slot = e.y & 0xff, k = (e.y >> 8) & 0xf, fl = e.y >> 12;
+    const int t = e.x, slot = e.y & 0xff, img = (e.y >> 8) & 0xf, fl = e.y >> 12;
     const double2 T = a.tp[t];
     const double2 S = W.pos[slot];
-    // (the image shift as in adj_pair)
-    const int2 b = W.bxy[slot];
-    const int tx = b.x + c_nb_dx[k], ty = b.y + c_nb_dy[k];
-    const double zx = tx >= a.nx ? a.zxm : (tx < 0 ? a.zxp : 0.0);
-    const double zy = ty >= a.ny ? a.zym : (ty < 0 ? a.zyp : 0.0);
-    const float2 x1 = ff_split((S.x - T.x) + zx), x2 = ff_split((S.y - T.y) + zy);
+    double dx = S.x - T.x, dy = S.y - T.y;
+    if (img) {                                            // across a periodic image
+        const double2 z = image_shift(a, img);
+        dx += z.x;
+        dy += z.y;
+    }
+    const float2 x1 = ff_split(dx), x2 = ff_split(dy);
     const float2 r2 = ff_add(ff_sqr(x1), ff_sqr(x2));
     const float2 x = ff_mul(r2, xi2);
     const float2 ex = ff_exp_neg(x, tabff);
@@ -1253,10 +1278,10 @@ __global__ void __launch_bounds__(kAdjWarps * 32, 5) k_real_adj(RealArgs a)
     __syncthreads();
     const float2 xi2ff = ff_split(a.xi2), pfff = ff_split(a.pf);
     // queue 0: far pairs (float-float in the FF form), queue 1: the rest in FP64
-    const float xlo = FF ? 1.0001f : 1.0f, xhi = FF ? 63.9f : INFINITY;
+    const float rlo = (FF ? 1.0001f : 1.0f) / a.xi2f, rhi = FF ? 63.9f / a.xi2f : INFINITY;
     AdjWarp &W = warps[wid];
     int head = 0, nfl = 0, gseq = 0;
-    int qn[2] = {0, 0}, tag[2] = {-1, -1};
+    int tag[2] = {-1, -1};
     unsigned enq[2] = {0, 0}, proc[2] = {0, 0};   // (mod 2^32)
     double v[2][kAdjVals];
     float2 vf[kAdjVals];
@@ -1268,13 +1293,11 @@ __global__ void __launch_bounds__(kAdjWarps * 32, 5) k_real_adj(RealArgs a)
         for (int i = 0; i < kAdjVals; i++) v[j][i] = 0.0;
 
     auto batch = [&](int j, int cnt) {
-        const int2 e = lane < cnt ? W.q[j][lane] : make_int2(0, -1);
+        const int2 e = lane < cnt ? W.q[j][(proc[j] + lane) & 63] : make_int2(0, -1);
         __syncwarp();
-        if (lane < qn[j] - cnt) W.q[j][lane] = W.q[j][lane + cnt];
-        qn[j] -= cnt;
         proc[j] += cnt;
         int eseq = -1;
-        if (e.y >= 0) eseq = gseq - nfl + (((e.y & 0xff) - head + kRing) % kRing);
+        if (e.y >= 0) eseq = gseq - nfl + (((e.y & 0xff) - head) & (kRing - 1));
         const bool fl = tag[j] >= 0 && (lane >= cnt || tag[j] != eseq);
         const bool ffq = FF && j == 0;
         if (__any_sync(~0u, fl)) {
@@ -1307,7 +1330,7 @@ __global__ void __launch_bounds__(kAdjWarps * 32, 5) k_real_adj(RealArgs a)
             if (lane < kAdjVals) {
                 double v = W.acc[head][lane];
                 if (FF) v += ff_to_double(W.accf[head][lane]);
-                a.gout[kAdjVals * W.idx[head] + lane] = v;
+                a.gout[kAdjVals * (int64_t)W.idx[head] + lane] = v;
             }
             head = (head + 1) % kRing;
             nfl--;
@@ -1323,7 +1346,7 @@ __global__ void __launch_bounds__(kAdjWarps * 32, 5) k_real_adj(RealArgs a)
     const int64_t len = (int64_t)kAdjWarps * a.run;
     int64_t s0 = (int64_t)blockIdx.x * len;
     int s = (int)s0 + wid, s_end = (int)min(s0 + len, a.nouter);
-    if (lane == 0) W.curbox = -1;
+    if (lane == 0) W.nb.box = -1;
     __syncwarp();
     for (;;) {
         while (s >= s_end && s0 < a.nouter) {              // (the same for all warps)
@@ -1336,129 +1359,89 @@ __global__ void __launch_bounds__(kAdjWarps * 32, 5) k_real_adj(RealArgs a)
         }
         const bool dr = nfl == kRing || s0 >= a.nouter;    // (warp-uniform)
         const int slot = (head + nfl) % kRing;
-        int total = 64;
-        double2 Sp = make_double2(0.0, 0.0);
-        float2 Sf = make_float2(0.f, 0.f);
+        int nseg = 1;
         if (!dr) {
             nfl++;
             gseq++;
-            const int sbx = a.obox[s];
-            Sp = a.sp[s];
-            Sf = a.spf[s];
-            const bool newbox = sbx != W.curbox;           // (warp-uniform)
-            if (newbox) {
-                __syncwarp();
-                if (lane == 0) {
-                    W.curbox = sbx;
-                    W.curbxy = make_int2(sbx % a.nx, sbx / a.nx);
-                }
-                __syncwarp();
-            }
-            const int2 b = W.curbxy;
+            const int sb = a.obox[s];
+            if (sb != W.nb.box) nbhd_build<true>(W.nb, a, lane, sb);   // (warp-uniform)
             if (lane < kAdjVals + 1) W.acc[slot][lane] = 0.0;
             if (lane < kAdjVals) W.accf[slot][lane] = make_float2(0.f, 0.f);
             if (lane == 0) {
-                W.pos[slot] = Sp;
-                W.bxy[slot] = b;
+                const float2 Sf = a.spf[s];
+                W.pos[slot] = a.sp[s];
                 W.idx[slot] = s;
-            }
-            if (newbox) {
-                int cntk = 0;
-                if (lane < 9) {
-                    // target box at offset k from the source box
-                    const int ux = b.x + c_nb_dx[lane], uy = b.y + c_nb_dy[lane];
-                    const int wx = (ux + a.nx) % a.nx, wy = (uy + a.ny) % a.ny;
-                    const int tb = wy * a.nx + wx;
-                    const int b0 = a.sstart[tb];           // target cell list
-                    cntk = a.sstart[tb + 1] - b0;
-                    W.nbs[lane] = b0;
-                    // source image shift seen from that target box (box tb, offset -k)
-                    const int vx = wx - c_nb_dx[lane], vy = wy - c_nb_dy[lane];
-                    const double zx = vx < 0 ? a.zxm : (vx >= a.nx ? a.zxp : 0.0);
-                    const double zy = vy < 0 ? a.zym : (vy >= a.ny ? a.zyp : 0.0);
-                    W.nbz[lane] = make_double2(zx, zy);
-                    W.nbzf[lane] = make_float2((float)zx, (float)zy);
-                }
-                int incl = cntk;
-#pragma unroll
-                for (int o = 1; o < 16; o <<= 1) {
-                    const int vv = __shfl_up_sync(~0u, incl, o);
-                    if (lane >= o) incl += vv;
-                }
-                if (lane < 9) W.nbp[lane + 1] = incl;
-                if (lane == 0) W.nbp[0] = 0;
+                W.nb.p = Sf;
+                W.nb.cut = cut_band(W.nb, Sf, a.cut2f);
             }
             __syncwarp();
-            total = W.nbp[9];
+            nseg = W.nb.nseg;
         }
-        int kc = 0;   // neighbour box of this lane's candidate (vi only grows)
-        for (int v0 = 0; v0 < total; v0 += 32) {
-            const int vi = v0 + lane;
-            int fl = 0, t = 0, k = kc;
-            bool nearp = false;
-            if (!dr && vi < total) {
-                while (vi >= W.nbp[k + 1]) k++;
-                kc = k;
-                t = W.nbs[k] + (vi - W.nbp[k]);
-                if (k == 0) {
-                    const double2 T = a.tp[t];
-                    const double dx = xsub(T.x, Sp.x), dy = xsub(T.y, Sp.y);
-                    const double r2 = xadd(xmul(dx, dx), xmul(dy, dy));
-                    if (r2 == 0.0) {
-                        // SLP self term: d/df of self_c f.w (mex_stokes_slp_real.cpp:161-163)
-                        if (SLP) {
-                            atomicAdd(&W.acc[slot][0], a.self_c * a.wcoef[4 * (int64_t)t]);
-                            atomicAdd(&W.acc[slot][1], a.self_c * a.wcoef[4 * (int64_t)t + 1]);
-                        }
-                    } else {
-                        fl = 3;
-                        const float xf = (float)r2 * a.xi2f;
-                        nearp = !(xf > xlo && xf < xhi);
-                    }
-                } else {
+        const int base = slot | (SLP ? 0x1000 : 0) | (DLP ? 0x2000 : 0);
+        const float2 cut = W.nb.cut;
+        for (int q = 0; q < nseg; q++) {
+            Piece C(W.nb, q, base);
+            if (dr) {                                          // (two steps)
+                C.begin = 0;
+                C.end = 64;
+            }
+            for (int t0 = C.begin; t0 < C.end; t0 += 32) {
+                const int t = t0 + lane;
+                int y = C.ey;
+                bool in = false, nearp = false;
+                if (!dr && t < C.end) {
                     const float2 Tf = a.tpf[t];
-                    const float2 zf = W.nbzf[k];
-                    const float dxf = Sf.x - (Tf.x - zf.x), dyf = Sf.y - (Tf.y - zf.y);
-                    const float r2f = dxf * dxf + dyf * dyf;
-                    const float ex = 0x1p-22f * (fabsf(Sf.x) + fabsf(Tf.x) + fabsf(zf.x));
-                    const float ey = 0x1p-22f * (fabsf(Sf.y) + fabsf(Tf.y) + fabsf(zf.y));
-                    const float band = 2.0f * (ex * (2.0f * fabsf(dxf) + ex) +
-                                               ey * (2.0f * fabsf(dyf) + ey) + 0x1p-22f * r2f);
-                    const float xf = r2f * a.xi2f;
-                    nearp = !(xf > xlo && xf < xhi);
-                    if (r2f + band < a.cut2f) {
-                        fl = 3;
-                    } else if (!(r2f - band >= a.cut2f)) {
-                        const double2 T = a.tp[t];
-                        const double2 z = W.nbz[k];
-                        if (SLP) {
-                            const double dx = xsub(Sp.x, xsub(T.x, z.x));
-                            const double dy = xsub(Sp.y, xsub(T.y, z.y));
-                            if (xadd(xmul(dx, dx), xmul(dy, dy)) < a.cut2) fl |= 1;
+                    const float dxf = Tf.x - C.ox, dyf = Tf.y - C.oy;
+                    float r2f = dxf * dxf + dyf * dyf;
+                    const bool own = (unsigned)(t - C.own0) < C.ownn;
+                    in = r2f > 0.f && r2f < (own ? INFINITY : cut.x);
+                    if (!in && (own || !(r2f >= cut.y))) {
+                        const double2 T = a.tp[t], Sp = W.pos[slot];
+                        y = base & 0xff | C.ey & 0xf00;
+                        if (own) {
+                            const double dx = xsub(T.x, Sp.x), dy = xsub(T.y, Sp.y);
+                            const double r2 = xadd(xmul(dx, dx), xmul(dy, dy));
+                            r2f = (float)r2;
+                            if (r2 == 0.0) {
+                                // SLP self term: d/df of self_c f.w (mex_stokes_slp_real.cpp:161-163)
+                                if (SLP) {
+                                    atomicAdd(&W.acc[slot][0], a.self_c * a.wcoef[4 * (int64_t)t]);
+                                    atomicAdd(&W.acc[slot][1], a.self_c * a.wcoef[4 * (int64_t)t + 1]);
+                                }
+                            } else {
+                                y = C.ey;
+                            }
+                        } else {
+                            // near the cutoff (or not finite): the reference's exact tests
+                            const double2 z = image_shift(a, (C.ey >> 8) & 0xf);
+                            if (SLP) {
+                                const double dx = xsub(Sp.x, xsub(T.x, z.x));
+                                const double dy = xsub(Sp.y, xsub(T.y, z.y));
+                                if (xadd(xmul(dx, dx), xmul(dy, dy)) < a.cut2) y |= 0x1000;
+                            }
+                            if (DLP) {
+                                const double x1 = xadd(xsub(Sp.x, T.x), z.x);
+                                const double x2 = xadd(xsub(Sp.y, T.y), z.y);
+                                if (xadd(xmul(x1, x1), xmul(x2, x2)) < a.cut2) y |= 0x2000;
+                            }
                         }
-                        if (DLP) {
-                            const double x1 = xadd(xsub(Sp.x, T.x), z.x);
-                            const double x2 = xadd(xsub(Sp.y, T.y), z.y);
-                            if (xadd(xmul(x1, x1), xmul(x2, x2)) < a.cut2) fl |= 2;
-                        }
+                        in = y >> 12;
                     }
+                    nearp = !(r2f > rlo && r2f < rhi);
+                }
+                const unsigned below = (1u << lane) - 1u;
+                const unsigned m0 = __ballot_sync(~0u, in && !nearp), m1 = __ballot_sync(~0u, in && nearp);
+                if (in && !nearp) W.q[0][(enq[0] + __popc(m0 & below)) & 63] = make_int2(t, y);
+                if (in && nearp) W.q[1][(enq[1] + __popc(m1 & below)) & 63] = make_int2(t, y);
+                enq[0] += __popc(m0);
+                enq[1] += __popc(m1);
+                __syncwarp();
+#pragma unroll
+                for (int j = 0; j < 2; j++) {
+                    const int n = (int)(enq[j] - proc[j]);
+                    if (dr || n >= 32) batch(j, min(n, 32));
                 }
             }
-            if (!SLP) fl &= 2;
-            if (!DLP) fl &= 1;
-            const int2 ent = make_int2(t, slot | (k << 8) | (fl << 12));
-#pragma unroll
-            for (int j = 0; j < 2; j++) {
-                const bool mine = fl != 0 && nearp == (j == 1);
-                const unsigned m = __ballot_sync(~0u, mine);
-                if (mine) W.q[j][qn[j] + __popc(m & ((1u << lane) - 1u))] = ent;
-                qn[j] += __popc(m);
-                enq[j] += __popc(m);
-            }
-            __syncwarp();
-#pragma unroll
-            for (int j = 0; j < 2; j++)
-                if (dr || qn[j] >= 32) batch(j, dr ? qn[j] : 32);
         }
         if (dr) {
             retire(true);

@@ -65,3 +65,31 @@ def test_gradients_do_not_depend_on_the_runs(ft, precision):
             assert np.abs(a[:, few] - b).max() <= TOL * np.abs(a).max()
     finally:
         plan.close()
+
+
+@pytest.mark.parametrize("far", [3.0e4, 1.5e7])
+@pytest.mark.parametrize("box", [(1.0, 1.0, 1, 1), (1.0, 2.0, 1, 2)])
+def test_pairs_far_outside_the_cell(ft, far, box):
+    """All points far outside the cell (the reference puts them into one edge box), where
+    the FP32 pre-test of the cutoff cannot decide for their images: the oracle's pair set
+    and sums (1e-12, as the other comparisons with it: the same FP64 offsets, then at
+    most 400 terms).  In FP64 throughout: the float-float form takes its pairs by the
+    FP32 distance, which has no digits left there."""
+    from oracle import oracle as O
+    Lx, Ly, nx, ny = box
+    rng = np.random.default_rng(int(far) + ny)
+    ps, pt = (np.vstack([far + (rng.random(400) - 0.5) * Lx, (rng.random(400) - 0.5) * Ly - far])
+              for _ in range(2))
+    f, g = rng.standard_normal((2, 400)), rng.standard_normal((2, 400))
+    xi = 3.0 * max(nx / Lx, ny / Ly)
+    plan = ft.Plan(0)
+    try:
+        plan.set_precision("fp64_native")
+        for got, ref in ((ft.mex_stokes_slp_real(ps, pt, f, xi, nx, ny, Lx, Ly, plan=plan),
+                          O.mex_stokes_slp_real(ps, pt, f, xi, nx, ny, Lx, Ly)),
+                         (ft.mex_stokes_dlp_real(ps, pt, f, g, xi, nx, ny, Lx, Ly, plan=plan),
+                          O.mex_stokes_dlp_real(ps, pt, f, g, xi, nx, ny, Lx, Ly))):
+            assert np.isfinite(ref).all()
+            assert np.abs(got - ref).max() <= TOL * np.abs(ref).max()
+    finally:
+        plan.close()
