@@ -41,7 +41,7 @@ enum Slot {
     S_UR_SLP, S_UR_DLP, S_UK,                   // partial results (sorted order)
     S_GRID, S_SPEC, S_E1, S_ZPART, S_ZM, S_COUNTERS,
     S_OUT0, S_OUT1, S_OUT2, S_OUT3,             // staged outputs
-    S_IN_W1, S_IN_W2, S_WCOEF, S_GR, S_GK, S_SBOXS, S_ZEROS,   // adjoint
+    S_IN_W1, S_IN_W2, S_WCOEF, S_WCOEF_FF, S_GR, S_GK, S_SBOXS, S_ZEROS,   // adjoint
     S_GTAB, S_COEF_FF,                          // float-float real space
     S_ZGRID,                                    // complex pairs of grids (1D-pass FFT)
     S_GCOUNT, S_GTGT, S_GMETA,                  // geometry build scratch
@@ -983,7 +983,7 @@ int run(se2p_plan pl, const Job &J, const Io &io)
     const int form = pl->precision == SE2P_PRECISION_FP32_GRID    ? kFormF32
                      : pl->precision == SE2P_PRECISION_FP64_NATIVE ? kFormFP64
                                                                     : kFormFF;
-    const int ncf = (J.slp ? 2 : 0) + (J.dlp ? 5 : 0);
+    const int ncf = (J.slp ? 2 : 0) + (J.dlp ? 4 : 0);
     double *coef = nullptr;
     float2 *cff = nullptr;
     CKS(ensure_t(pl, S_COEF, (size_t)nc * nsz, &coef));
@@ -1390,11 +1390,17 @@ int run_adjoint(se2p_plan pl, const Job &J, const AdjIo &io)
     CKS(ensure_t(pl, S_WCOEF, 4 * ntz, &wcoef));
     CKS(ensure_t(pl, S_ZEROS, nsz, &zeros));
     CK(cudaMemsetAsync(zeros, 0, sizeof(double2) * nsz, st));
+    const int form = pl->precision == SE2P_PRECISION_FP64_NATIVE ? kFormFP64 : kFormFF;
+    float2 *cff = nullptr, *wff = nullptr;     // float-float copies for the real space
+    if (form == kFormFF) {
+        CKS(ensure_t(pl, S_COEF_FF, 6 * nsz, &cff));
+        CKS(ensure_t(pl, S_WCOEF_FF, 4 * ntz, &wff));
+    }
     {
         StageTimer tm(pl, T_COEF);
         CK(launch_src_coef(ns, sperm, slp ? fs : zeros, dlp ? fd : zeros, dlp ? nr : zeros, coef, 5,
-                           st, pl->launches, nullptr, 0, true, count));
-        CK(launch_sorted_pair(nt, tperm, w1, w2, wcoef, st, pl->launches));
+                           st, pl->launches, cff, 6, true, count));
+        CK(launch_sorted_pair(nt, tperm, w1, w2, wcoef, wff, st, pl->launches));
     }
     double *gr = nullptr, *gk = nullptr;
     CKS(ensure_t(pl, S_GR, 7 * nsz, &gr));
@@ -1432,6 +1438,10 @@ int run_adjoint(se2p_plan pl, const Job &J, const AdjIo &io)
     ra.nouter = ns;
     ra.obox = sboxs;
     ra.wcoef = wcoef;
+    ra.coef_ff = cff;
+    ra.ncf = 6;
+    ra.doff_ff = 2;
+    ra.wcoef_ff = wff;
     ra.gout = gr;
     const bool side = pl->overlap;
     cudaStream_t rs = side ? pl->side : st;
@@ -1439,7 +1449,6 @@ int run_adjoint(se2p_plan pl, const Job &J, const AdjIo &io)
         CK(cudaEventRecord(pl->fork, st));
         CK(cudaStreamWaitEvent(rs, pl->fork, 0));
     }
-    const int form = pl->precision == SE2P_PRECISION_FP64_NATIVE ? kFormFP64 : kFormFF;
     ra.gtab = nullptr;
     if (form == kFormFF) CKS(gtab_device(pl, st, &ra.gtab));
     {

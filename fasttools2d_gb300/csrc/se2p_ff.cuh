@@ -151,6 +151,43 @@ __device__ __forceinline__ void ff_dot_acc(float2 a, float2 b, float &s, float &
     c += err + e;
 }
 
+// The same for one addend.
+__device__ __forceinline__ void ff_sum_acc(float2 a, float &s, float &c)
+{
+    float t, err;
+    two_sum(s, a.x, t, err);
+    s = t;
+    c += err + a.y;
+}
+
+// Moves what the compensation c can give to s.  Where cancellation has left |s| < |c|
+// the Fast2Sum is not exact, by at most an ulp of c (2^-24 of what a rounding of the sum
+// already was).
+__device__ __forceinline__ void ff_acc_norm(float &s, float &c)
+{
+    float h, l;
+    fast_two_sum(s, c, h, l);
+    s = h;
+    c = l;
+}
+
+// a1^2 + a2^2.
+__device__ __forceinline__ float2 ff_sqr2(float2 a1, float2 a2)
+{
+    const float p1 = a1.x * a1.x;
+    float e1 = fmaf(a1.x, a1.x, -p1);
+    e1 = fmaf(2.0f * a1.x, a1.y, e1);
+    const float p2 = a2.x * a2.x;
+    float e2 = fmaf(a2.x, a2.x, -p2);
+    e2 = fmaf(2.0f * a2.x, a2.y, e2);
+    float s, t;
+    two_sum(p1, p2, s, t);
+    t += e1 + e2;
+    float h, l;
+    fast_two_sum(s, t, h, l);
+    return make_float2(h, l);
+}
+
 __device__ __forceinline__ float2 ff_neg(float2 a) { return make_float2(-a.x, -a.y); }
 
 __device__ __forceinline__ float2 ff_sub(float2 a, float2 b) { return ff_add(a, ff_neg(b)); }

@@ -312,7 +312,7 @@ struct RealArgs {
     double2 *u_dlp;
     unsigned long long *counters;   // [candidates, SLP pairs, DLP pairs] (may be NULL)
     // float-float form only: per sorted source ncf coefficient pairs (SLP f1,
-    // f2; DLP S11, S12+S21, S22, 3 S11 + S22, 3 S22 + S11 from doff_ff) and
+    // f2; DLP S11, S12+S21, S22, S11 + S22 from doff_ff) and
     // the piecewise fit of the E1 Pade form (kGPieces x 3 float4)
     const float2 *coef_ff;
     int ncf, doff_ff;
@@ -328,6 +328,7 @@ struct RealArgs {
     int64_t nouter;
     const int *obox;
     const double *wcoef;
+    const float2 *wcoef_ff;   // and as float-float (float-float form)
     double *gout;
 };
 
@@ -503,7 +504,7 @@ struct GatherArgsF {
 // ---------------------------------------------------------------------------
 cudaError_t launch_sort(const SortArgs &a, int nsets, cudaStream_t st, int64_t &launches);
 // out: the float-float copy, ostride float2 per source (tails = false leaves out
-// the DLP pair 3 S11 + S22, 3 S22 + S11: the real-space kernels read it, the
+// the DLP sum S11 + S22: the real-space kernels read it, the
 // geometry's stored operator does not).
 cudaError_t launch_src_coef(int64_t n, const int *perm, const double2 *f_slp,
                             const double2 *f_dlp, const double2 *nrm, double *coef, int nc,
@@ -597,7 +598,7 @@ int sm_count();
 cudaError_t launch_real_adj(const RealArgs &a, bool slp, bool dlp, cudaStream_t st,
                             int64_t &launches, int form = kFormFP64);
 cudaError_t launch_sorted_pair(int64_t n, const int *perm, const double2 *a, const double2 *b,
-                               double *out, cudaStream_t st, int64_t &launches);
+                               double *out, float2 *ff, cudaStream_t st, int64_t &launches);
 cudaError_t launch_filter_adj(const FilterArgs &a, cudaStream_t st, int64_t &launches);
 // With a.gff set (adj_gather_ff_ok), the float-float gather runs, and the
 // FP64 one only when the grid holds a non-finite value.

@@ -213,8 +213,7 @@ __global__ void __launch_bounds__(256) k_sort_place(SortArgs a)
 // zero: a word to clear (the real space's run counter), or null.
 //
 // With out, also the float-float copy for the far pairs of the FP64 form: SLP f1,
-// f2; DLP S11, S12+S21, S22 and (tails) the combinations 3 S11 + S22, 3 S22 + S11
-// of the stresslet contraction (formed in FP64, then split).
+// f2; DLP S11, S12+S21, S22 and (tails) S11 + S22 (formed in FP64, then split).
 __global__ void __launch_bounds__(256) k_src_coef(int64_t n, const int *__restrict__ perm,
                            const double2 *__restrict__ f_slp, const double2 *__restrict__ f_dlp,
                            const double2 *__restrict__ nrm, double *__restrict__ coef, int nc,
@@ -248,19 +247,16 @@ __global__ void __launch_bounds__(256) k_src_coef(int64_t n, const int *__restri
             o[0] = ff_split(s0);
             o[1] = ff_split(s1);
             o[2] = ff_split(s2);
-            if (tails) {
-                o[3] = ff_split(fma(3.0, s0, s2));
-                o[4] = ff_split(fma(3.0, s2, s0));
-            }
+            if (tails) o[3] = ff_split(s0 + s2);
         }
     }
 }
 
 // Sorted copy of two per-point 2-vectors (either may be NULL -> zeros):
-// out[4 j .. 4 j + 3] = (a[perm[j]], b[perm[j]]).
+// out[4 j .. 4 j + 3] = (a[perm[j]], b[perm[j]]), and with ff their float-float split.
 __global__ void k_sorted_pair(int64_t n, const int *__restrict__ perm,
                               const double2 *__restrict__ a, const double2 *__restrict__ b,
-                              double *__restrict__ out)
+                              double *__restrict__ out, float2 *__restrict__ ff)
 {
     const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= n) return;
@@ -272,6 +268,11 @@ __global__ void k_sorted_pair(int64_t n, const int *__restrict__ perm,
     o[1] = x.y;
     o[2] = y.x;
     o[3] = y.y;
+    if (!ff) return;
+    ff[4 * j] = ff_split(x.x);
+    ff[4 * j + 1] = ff_split(x.y);
+    ff[4 * j + 2] = ff_split(y.x);
+    ff[4 * j + 3] = ff_split(y.y);
 }
 
 // ===========================================================================
@@ -680,7 +681,7 @@ __device__ __forceinline__ void real_pair_f32(const RealArgs &a, const RealWarp 
     if (DLP && (fl & 2)) {
         const float2 *Sc = a.coef_ff + (int64_t)a.ncf * s + a.doff_ff;
         const float S11 = Sc[0].x, S1221 = Sc[1].x, S22 = Sc[2].x;
-        const float T1 = Sc[3].x, T2 = Sc[4].x;   // 3 S11 + S22, 3 S22 + S11
+        const float T1 = fmaf(3.f, S11, S22), T2 = fmaf(3.f, S22, S11);
         const float r2 = fmaf(x1, x1, x2 * x2);
         const float x = r2 * xi2;
         const float ex = __expf(-x);
@@ -714,7 +715,7 @@ __device__ __forceinline__ void real_pair_ff(const RealArgs &a, const RealWarp &
         dy += z.y;
     }
     const float2 x1 = ff_split(dx), x2 = ff_split(dy);
-    const float2 r2 = ff_add(ff_sqr(x1), ff_sqr(x2));
+    const float2 r2 = ff_sqr2(x1, x2);
     const float2 x = ff_mul(r2, xi2);
     const float2 ex = ff_exp_neg(x, tabff);
     const float2 ir2 = ff_rcp(r2);
@@ -731,24 +732,24 @@ __device__ __forceinline__ void real_pair_ff(const RealArgs &a, const RealWarp &
         ff_dot_acc(gq, x2, s1.x, s1.y);
         ff_dot_acc(h, f2, s2.x, s2.y);
         ff_dot_acc(ff_neg(gq), x1, s2.x, s2.y);
-        s1 = ff_norm(s1.x, s1.y);
-        s2 = ff_norm(s2.x, s2.y);
+        ff_acc_norm(s1.x, s1.y);
+        ff_acc_norm(s2.x, s2.y);
     }
     if (DLP && (fl & 2)) {
         const float2 *Sc = cf + a.doff_ff;
-        const float2 S11 = Sc[0], S1221 = Sc[1], S22 = Sc[2], T1 = Sc[3], T2 = Sc[4];
-        const float2 fb = ff_scale(ff_mul(ff_add_f(x, 1.0f), ff_sqr(ir2)), -4.0f);
-        const float2 Q = ff_dot3(ff_sqr(x1), S11, ff_mul(x1, x2), S1221, ff_sqr(x2), S22);
-        const float2 A1 = ff_dot2(x1, T1, x2, S1221);
-        const float2 A2 = ff_dot2(x2, T2, x1, S1221);
-        const float2 fq = ff_mul(fb, Q);
-        const float2 efq = ff_mul(ex, fq), epf = ff_mul(ex, pf);
-        ff_dot_acc(efq, x1, d1.x, d1.y);
-        ff_dot_acc(epf, A1, d1.x, d1.y);
-        ff_dot_acc(efq, x2, d2.x, d2.y);
-        ff_dot_acc(epf, A2, d2.x, d2.y);
-        d1 = ff_norm(d1.x, d1.y);
-        d2 = ff_norm(d2.x, d2.y);
+        const float2 S11 = Sc[0], S1221 = Sc[1], S22 = Sc[2], tr = Sc[3];
+        // with q = grad (x.S x), 2 Q = x.q: fb Q x + pf A = (fb Q + pf tr) x + pf q
+        const float2 fbh = ff_scale(ff_mul(ff_add_f(x, 1.0f), ff_sqr(ir2)), -2.0f);
+        const float2 q1 = ff_dot2(S11, ff_scale(x1, 2.0f), S1221, x2);
+        const float2 q2 = ff_dot2(S22, ff_scale(x2, 2.0f), S1221, x1);
+        const float2 Q2 = ff_dot2(x1, q1, x2, q2);
+        const float2 ec = ff_mul(ex, ff_dot2(fbh, Q2, pf, tr)), epf = ff_mul(ex, pf);
+        ff_dot_acc(ec, x1, d1.x, d1.y);
+        ff_dot_acc(epf, q1, d1.x, d1.y);
+        ff_dot_acc(ec, x2, d2.x, d2.y);
+        ff_dot_acc(epf, q2, d2.x, d2.y);
+        ff_acc_norm(d1.x, d1.y);
+        ff_acc_norm(d2.x, d2.y);
     }
 }
 
@@ -1173,11 +1174,20 @@ __device__ __forceinline__ void adj_pair(const RealArgs &a, const AdjWarp &W, in
     }
 }
 
-// adj_pair in float-float for the far pairs (1 < xi^2 r^2 < 64) of the FP64
-// form: same terms, same pair, evaluated as in real_pair_ff.
+// adj_pair in float-float for the far pairs (1 < xi^2 r^2 < 64) of the FP64 form: the
+// same terms, evaluated as in real_pair_ff, every sum of products by its heads and
+// errors.  With gg = ex / r2, a = x.w, b = x.f, c = w.f:
+//   SLP  grad = (c (pf ex - gg) - 2 a b gg (xi^2 + 1/r2)) x + gg b w + gg a f
+// and with q = grad (x.S x) = 2 S x, d = x.w, B = fb x.S x + pf tr S:
+//   DLP  y = ex fb d x + 2 ex pf w,  dS = (x1 y1 + ex pf d, (x1 y2 + x2 y1) / 2, x2 y2 + ex pf d)
+//        grad = ex ((x.q d (fbp - pf fb / 2) - pf^2 (w.q + tr S d)) x + fb d q + B w + pf 2 S w)
+// g[3] is kept without its 1/2.  966 FP32 operations per pair of both kinds (1500 in
+// float-float products and sums one by one), and the code is that much shorter, which
+// counts: the kernel waits for instructions.  k_real_adj at 2^18 points and 80
+// neighbours: 2.11 ms (3.07 before).
 template <bool SLP, bool DLP>
 __device__ __forceinline__ void adj_pair_ff(const RealArgs &a, const AdjWarp &W, int2 e,
-                                            const float2 *tabff, float2 xi2, float2 pf,
+                                            const float2 *tabff, float2 xi2, float2 pf, float2 pf2,
                                             float2 *g)
 {
     const int t = e.x, slot = e.y & 0xff, img = (e.y >> 8) & 0xf, fl = e.y >> 12;
@@ -1190,74 +1200,77 @@ __device__ __forceinline__ void adj_pair_ff(const RealArgs &a, const AdjWarp &W,
         dy += z.y;
     }
     const float2 x1 = ff_split(dx), x2 = ff_split(dy);
-    const float2 r2 = ff_add(ff_sqr(x1), ff_sqr(x2));
+    const float2 r2 = ff_sqr2(x1, x2);
     const float2 x = ff_mul(r2, xi2);
     const float2 ex = ff_exp_neg(x, tabff);
     const float2 ir2 = ff_rcp(r2);
-    const double *wt = a.wcoef + 4 * (int64_t)t;
-    const double *cs = a.coef + (int64_t)a.nc * W.idx[slot];
+    const float2 epf = ff_mul(ex, pf);
+    const float2 *wt = a.wcoef_ff + 4 * (int64_t)t;
+    const float2 *cs = a.coef_ff + (int64_t)a.ncf * W.idx[slot];
+    float2 rad = make_float2(0.f, 0.f);                   // the gradient's part along x
     if (SLP && (fl & 1)) {
-        const float2 w1 = ff_split(wt[0]), w2 = ff_split(wt[1]);
-        const float2 f1 = ff_split(cs[0]), f2 = ff_split(cs[1]);
+        const float2 w1 = wt[0], w2 = wt[1], f1 = cs[0], f2 = cs[1];
         const float2 h = ff_scale(ff_mul(ex, ff_g_e1(x, a.gtab)), 0.5f);
         const float2 gg = ff_mul(ex, ir2);
-        const float2 gq = ff_mul(gg, ff_sub(ff_mul(x1, w2), ff_mul(x2, w1)));
-        g[0] = ff_add(g[0], ff_add(ff_mul(h, w1), ff_mul(gq, x2)));
-        g[1] = ff_add(g[1], ff_sub(ff_mul(h, w2), ff_mul(gq, x1)));
-        const float2 aa = ff_add(ff_mul(x1, w1), ff_mul(x2, w2));
-        const float2 bb = ff_add(ff_mul(x1, f1), ff_mul(x2, f2));
-        const float2 cc = ff_add(ff_mul(w1, f1), ff_mul(w2, f2));
-        const float2 ab = ff_mul(aa, bb);
-        const float2 abr = ff_mul(ab, ir2);
-        // kap = ex (-cc ir2 - 2 xi2 (ab ir2 - cc) - 2 ab ir2^2)
-        float2 kp = ff_neg(ff_mul(cc, ir2));
-        kp = ff_sub(kp, ff_scale(ff_mul(xi2, ff_sub(abr, cc)), 2.0f));
-        kp = ff_sub(kp, ff_scale(ff_mul(abr, ir2), 2.0f));
-        const float2 kap = ff_mul(ex, kp);
-        g[5] = ff_add(g[5], ff_add(ff_mul(kap, x1),
-                                   ff_mul(gg, ff_add(ff_mul(bb, w1), ff_mul(aa, f1)))));
-        g[6] = ff_add(g[6], ff_add(ff_mul(kap, x2),
-                                   ff_mul(gg, ff_add(ff_mul(bb, w2), ff_mul(aa, f2)))));
+        const float2 gq = ff_mul(gg, ff_dot2(x1, w2, ff_neg(x2), w1));
+        ff_dot_acc(h, w1, g[0].x, g[0].y);
+        ff_dot_acc(gq, x2, g[0].x, g[0].y);
+        ff_dot_acc(h, w2, g[1].x, g[1].y);
+        ff_dot_acc(ff_neg(gq), x1, g[1].x, g[1].y);
+        ff_acc_norm(g[0].x, g[0].y);
+        ff_acc_norm(g[1].x, g[1].y);
+        const float2 aa = ff_dot2(x1, w1, x2, w2), bb = ff_dot2(x1, f1, x2, f2);
+        const float2 cc = ff_dot2(w1, f1, w2, f2);
+        const float2 p2 = ff_scale(ff_mul(gg, ff_add(xi2, ir2)), -2.0f);
+        rad = ff_dot2(cc, ff_sub(epf, gg), ff_mul(aa, bb), p2);
+        const float2 gb = ff_mul(gg, bb), ga = ff_mul(gg, aa);
+        ff_dot_acc(gb, w1, g[5].x, g[5].y);
+        ff_dot_acc(ga, f1, g[5].x, g[5].y);
+        ff_dot_acc(gb, w2, g[6].x, g[6].y);
+        ff_dot_acc(ga, f2, g[6].x, g[6].y);
     }
     if (DLP && (fl & 2)) {
-        const float2 w1 = ff_split(wt[2]), w2 = ff_split(wt[3]);
-        const double *Sc = cs + a.doff;
-        const float2 S11 = ff_split(Sc[0]), S1221 = ff_split(Sc[1]), S22 = ff_split(Sc[2]);
+        const float2 w1 = wt[2], w2 = wt[3];
+        const float2 *Sc = cs + a.doff_ff;
+        const float2 S11 = Sc[0], S1221 = Sc[1], S22 = Sc[2], tr = Sc[3];
+        const float2 wd = ff_dot2(w1, x1, w2, x2);
         const float2 ir4 = ff_sqr(ir2);
-        const float2 fb = ff_scale(ff_mul(ff_add_f(x, 1.0f), ir4), -4.0f);
+        const float2 fbh = ff_scale(ff_mul(ff_add_f(x, 1.0f), ir4), -2.0f);           // fb / 2
         const float2 fbp = ff_scale(ff_mul(ff_add_f(x, 2.0f), ff_mul(ir4, ir2)), 4.0f);
-        const float2 wd = ff_add(ff_mul(w1, x1), ff_mul(w2, x2));
-        const float2 fw = ff_mul(fb, wd);
-        const float2 fwx1 = ff_mul(fw, x1), fwx2 = ff_mul(fw, x2);
-        const float2 w1x1 = ff_mul(w1, x1), w2x2 = ff_mul(w2, x2);
-        const float2 w1x2 = ff_mul(w1, x2), w2x1 = ff_mul(w2, x1);
+        const float2 e1 = ff_scale(ff_mul(ex, ff_mul(fbh, wd)), 2.0f);
         // d(w.v)/dS
-        g[2] = ff_add(g[2], ff_mul(ex, ff_add(ff_mul(fwx1, x1),
-                                              ff_mul(pf, ff_add(ff_mul_f(w1x1, 3.0f), w2x2)))));
-        g[3] = ff_add(g[3], ff_mul(ex, ff_add(ff_mul(fwx1, x2), ff_mul(pf, ff_add(w1x2, w2x1)))));
-        g[4] = ff_add(g[4], ff_mul(ex, ff_add(ff_mul(fwx2, x2),
-                                              ff_mul(pf, ff_add(w1x1, ff_mul_f(w2x2, 3.0f))))));
+        const float2 epf2 = ff_scale(epf, 2.0f), c = ff_mul(epf, wd);
+        const float2 y1 = ff_dot2(e1, x1, epf2, w1), y2 = ff_dot2(e1, x2, epf2, w2);
+        ff_dot_acc(x1, y1, g[2].x, g[2].y);
+        ff_sum_acc(c, g[2].x, g[2].y);
+        ff_dot_acc(x1, y2, g[3].x, g[3].y);
+        ff_dot_acc(x2, y1, g[3].x, g[3].y);
+        ff_dot_acc(x2, y2, g[4].x, g[4].y);
+        ff_sum_acc(c, g[4].x, g[4].y);
+#pragma unroll
+        for (int i = 2; i < 5; i++) ff_acc_norm(g[i].x, g[i].y);
         // grad_d [w.v(d; S)], subtracted
-        const float2 B11 = ff_add(ff_mul_f(S11, 3.0f), S22), B22 = ff_add(ff_mul_f(S22, 3.0f), S11);
-        const float2 Q = ff_add(ff_add(ff_mul(ff_sqr(x1), S11), ff_mul(ff_mul(x1, x2), S1221)),
-                                ff_mul(ff_sqr(x2), S22));
-        const float2 A1 = ff_add(ff_mul(B11, x1), ff_mul(S1221, x2));
-        const float2 A2 = ff_add(ff_mul(S1221, x1), ff_mul(B22, x2));
-        const float2 wA = ff_add(ff_mul(w1, A1), ff_mul(w2, A2));
-        const float2 Bw1 = ff_add(ff_mul(B11, w1), ff_mul(S1221, w2));
-        const float2 Bw2 = ff_add(ff_mul(S1221, w1), ff_mul(B22, w2));
-        const float2 Sd1 = ff_add(ff_scale(ff_mul(S11, x1), 2.0f), ff_mul(S1221, x2));
-        const float2 Sd2 = ff_add(ff_mul(S1221, x1), ff_scale(ff_mul(S22, x2), 2.0f));
-        const float2 fbQ = ff_mul(fb, Q);
-        const float2 radial = ff_add(ff_scale(ff_mul(xi2, ff_add(ff_mul(fbQ, wd), ff_mul(pf, wA))), -2.0f),
-                                     ff_scale(ff_mul(ff_mul(fbp, Q), wd), 2.0f));
-        const float2 r1 = ff_add(ff_add(ff_mul(radial, x1), ff_mul(fw, Sd1)),
-                                 ff_add(ff_mul(fbQ, w1), ff_mul(pf, Bw1)));
-        const float2 r2b = ff_add(ff_add(ff_mul(radial, x2), ff_mul(fw, Sd2)),
-                                  ff_add(ff_mul(fbQ, w2), ff_mul(pf, Bw2)));
-        g[5] = ff_sub(g[5], ff_mul(ex, r1));
-        g[6] = ff_sub(g[6], ff_mul(ex, r2b));
+        const float2 q1 = ff_dot2(S11, ff_scale(x1, 2.0f), S1221, x2);
+        const float2 q2 = ff_dot2(S22, ff_scale(x2, 2.0f), S1221, x1);
+        const float2 Q2 = ff_dot2(x1, q1, x2, q2);
+        const float2 wA = ff_dot3(w1, q1, w2, q2, tr, wd);
+        const float2 K = ff_sub(fbp, ff_mul(pf, fbh));
+        rad = ff_sub(rad, ff_mul(ex, ff_dot2(ff_mul(Q2, wd), K, ff_neg(pf2), wA)));
+        const float2 nB = ff_neg(ff_mul(ex, ff_dot2(fbh, Q2, pf, tr)));
+        const float2 s1 = ff_dot2(S11, ff_scale(w1, 2.0f), S1221, w2);
+        const float2 s2 = ff_dot2(S22, ff_scale(w2, 2.0f), S1221, w1);
+        const float2 ne1 = ff_neg(e1), nep = ff_neg(epf);
+        ff_dot_acc(ne1, q1, g[5].x, g[5].y);
+        ff_dot_acc(nB, w1, g[5].x, g[5].y);
+        ff_dot_acc(nep, s1, g[5].x, g[5].y);
+        ff_dot_acc(ne1, q2, g[6].x, g[6].y);
+        ff_dot_acc(nB, w2, g[6].x, g[6].y);
+        ff_dot_acc(nep, s2, g[6].x, g[6].y);
     }
+    ff_dot_acc(rad, x1, g[5].x, g[5].y);
+    ff_dot_acc(rad, x2, g[6].x, g[6].y);
+    ff_acc_norm(g[5].x, g[5].y);
+    ff_acc_norm(g[6].x, g[6].y);
 }
 
 template <bool SLP, bool DLP, int FORM>
@@ -1276,7 +1289,7 @@ __global__ void __launch_bounds__(kAdjWarps * 32, 5) k_real_adj(RealArgs a)
     }
     for (int i = threadIdx.x; i < 66; i += blockDim.x) e1s[i] = (&c_e1[0][0])[i];
     __syncthreads();
-    const float2 xi2ff = ff_split(a.xi2), pfff = ff_split(a.pf);
+    const float2 xi2ff = ff_split(a.xi2), pfff = ff_split(a.pf), pf2ff = ff_split(a.pf * a.pf);
     // queue 0: far pairs (float-float in the FF form), queue 1: the rest in FP64
     const float rlo = (FF ? 1.0001f : 1.0f) / a.xi2f, rhi = FF ? 63.9f / a.xi2f : INFINITY;
     AdjWarp &W = warps[wid];
@@ -1319,7 +1332,7 @@ __global__ void __launch_bounds__(kAdjWarps * 32, 5) k_real_adj(RealArgs a)
             }
         }
         if (lane < cnt) {
-            if (ffq) adj_pair_ff<SLP, DLP>(a, W, e, tabff, xi2ff, pfff, vf);
+            if (ffq) adj_pair_ff<SLP, DLP>(a, W, e, tabff, xi2ff, pfff, pf2ff, vf);
             else adj_pair<SLP, DLP>(a, W, e, tab, e1s, v[j]);
             tag[j] = eseq;
         }
@@ -1329,7 +1342,7 @@ __global__ void __launch_bounds__(kAdjWarps * 32, 5) k_real_adj(RealArgs a)
                                    (int)(proc[1] - W.tend[1][head]) >= 32))) {
             if (lane < kAdjVals) {
                 double v = W.acc[head][lane];
-                if (FF) v += ff_to_double(W.accf[head][lane]);
+                if (FF) v += (lane == 3 ? 0.5 : 1.0) * ff_to_double(W.accf[head][lane]);
                 a.gout[kAdjVals * (int64_t)W.idx[head] + lane] = v;
             }
             head = (head + 1) % kRing;
@@ -3429,10 +3442,10 @@ cudaError_t launch_assemble(int64_t n, const int *perm, const AssembleArgs &a, c
 }
 
 cudaError_t launch_sorted_pair(int64_t n, const int *perm, const double2 *a, const double2 *b,
-                               double *out, cudaStream_t st, int64_t &launches)
+                               double *out, float2 *ff, cudaStream_t st, int64_t &launches)
 {
     if (n <= 0) return cudaSuccess;
-    k_sorted_pair<<<grid_for(n, 256), 256, 0, st>>>(n, perm, a, b, out);
+    k_sorted_pair<<<grid_for(n, 256), 256, 0, st>>>(n, perm, a, b, out, ff);
     launches++;
     return cudaGetLastError();
 }
