@@ -17,8 +17,8 @@
 // for the exponent scan), scaled by a power of two that
 // puts its largest entry near 2^64 (exact; the FFT of a row of L <= 2^13
 // values grows it by at most L), split into float-float pairs with integer
-// operations, transformed by mixed-radix Stockham stages (radices 8, 4, 6, 2,
-// 7, 5, 3, ping-pong between two shared buffers), and written back as doubles
+// operations, transformed by mixed-radix Stockham stages (radices 12, 8, 7,
+// 6, 5, 4, 3, 2, ping-pong between two shared buffers), and written back as doubles
 // rebuilt with integer operations (float <-> double conversions run at the
 // FP64 rate on GB300).  Twiddles exp(-2 pi i m / L) come from a per-length
 // table built in long double on the host; the odd radices take their
@@ -27,6 +27,8 @@
 // The transform is unnormalised with cuFFT's sign convention (forward
 // exp(-2 pi i j k / L)), so it replaces cufftExecZ2Z on the same layout.
 #include "se2p_internal.cuh"
+#include <algorithm>
+#include <climits>
 #include <math_constants.h>
 
 namespace se2p {
@@ -326,6 +328,26 @@ __device__ __forceinline__ void dft<6>(fc *v, f2 sg, const tw2 *cst)
     v[5] = fc_sub(a[2], b[2]);
 }
 
+// R = 12 = 4 x 3: inputs (3 n1 + 4 n2) mod 12, outputs (9 k1 + 4 k2) mod 12.
+template <>
+__device__ __forceinline__ void dft<12>(fc *v, f2 sg, const tw2 *cst)
+{
+    fc t[4][3];
+#pragma unroll
+    for (int n = 0; n < 4; n++) {
+#pragma unroll
+        for (int m = 0; m < 3; m++) t[n][m] = v[(3 * n + 4 * m) % 12];
+        dft_odd<3>(t[n], sg, cst);
+    }
+#pragma unroll
+    for (int m = 0; m < 3; m++) {
+        fc u[4] = {t[0][m], t[1][m], t[2][m], t[3][m]};
+        dft<4>(u, sg, nullptr);
+#pragma unroll
+        for (int n = 0; n < 4; n++) v[(9 * n + 4 * m) % 12] = u[n];
+    }
+}
+
 // tw: the table of the transform's sign; tw0: the forward one, whose entries m L / R
 // give the butterflies' constants.
 template <int R>
@@ -334,11 +356,12 @@ __device__ void stage(const f2 *A, f2 *B, int L, int Ns, unsigned magic, f2 sg,
 {
     // the constants of the R-point DFT from the twiddle table
     constexpr f2 kPM = 0xbf8000003f800000ull;        // (1, -1)
-    tw2 cst[R / 2 > 0 ? R / 2 : 1];
+    constexpr int O = R % 3 == 0 ? 3 : R;
+    constexpr int NC = O & 1 ? O / 2 : 1;
+    tw2 cst[NC];
     if (R == 8) {
         cst[0] = tw_load(tw0, L / 8);                // exp(-i pi/4): re = sqrt(1/2)
-    } else if ((R & 1) || R == 6) {
-        constexpr int O = R == 6 ? 3 : R;
+    } else if (O & 1) {
 #pragma unroll
         for (int m = 1; m <= O / 2; m++) {
             const tw2 w = tw_load(tw0, m * (L / O));   // sn = -sin: (-sn, sn) = (sin, -sin)
@@ -518,6 +541,7 @@ __global__ void __launch_bounds__(256, 2) k_fft_rows_ff(double2 *__restrict__ da
             const int R = p.radix[st];
             const unsigned mg = p.magic[st];
             switch (R) {
+            case 12: stage<12>(A, B, L, Ns, mg, s, tw, tw0); break;
             case 8: stage<8>(A, B, L, Ns, mg, s, tw, tw0); break;
             case 4: stage<4>(A, B, L, Ns, mg, s, tw, tw0); break;
             case 6: stage<6>(A, B, L, Ns, mg, s, tw, tw0); break;
@@ -575,20 +599,49 @@ bool fft_rows_ff_plan(int L, FftRowsFF &p)
     p.L = L;
     p.nst = 0;
     if (L < 2 || L > kFftFFMaxLen) return false;
+    // The factorisation into the butterflies at hand that costs least: per point and
+    // stage the butterfly's instructions (counted from the code) and 55 for the
+    // twiddle, shared memory and the barrier.  2688 = 8 4 12 7: 2^20 points 11.21 ms
+    // against 11.33 as 8 8 6 7 (14, 16, 10 as butterflies spill registers: 11.24 to 11.72).
+    static const int kR[] = {12, 8, 7, 6, 5, 4, 3, 2};
+    static const int kC[] = {55, 38, 55, 44, 43, 22, 33, 11};
+    constexpr int NR = sizeof kR / sizeof *kR;
     int n = L;
-    while (n % 8 == 0 && p.nst < kFftFFMaxStages) { p.radix[p.nst++] = 8; n /= 8; }
-    while (n % 4 == 0 && p.nst < kFftFFMaxStages) { p.radix[p.nst++] = 4; n /= 4; }
-    while (n % 6 == 0 && p.nst < kFftFFMaxStages) { p.radix[p.nst++] = 6; n /= 6; }
-    while (n % 2 == 0 && p.nst < kFftFFMaxStages) { p.radix[p.nst++] = 2; n /= 2; }
-    for (int r : {7, 5, 3})
-        while (n % r == 0 && p.nst < kFftFFMaxStages) { p.radix[p.nst++] = r; n /= r; }
+    int best = INT_MAX, pick[kFftFFMaxStages], at = 0, depth = 0, cost = 0;
+    // (depth first, each factor no larger than the one before; at: the next to try)
+    for (;;) {
+        if (n == 1 && cost < best) {
+            best = cost;
+            p.nst = depth;
+            for (int i = 0; i < depth; i++) p.radix[i] = kR[pick[i]];
+        }
+        while (at < NR && !(n % kR[at] == 0 && n > 1 && depth < kFftFFMaxStages &&
+                            cost + kC[at] + 55 < best))
+            at++;
+        if (at < NR) {
+            pick[depth++] = at;
+            n /= kR[at];
+            cost += kC[at] + 55;
+        } else if (depth > 0) {
+            at = pick[--depth];
+            n *= kR[at];
+            cost -= kC[at] + 55;
+            at++;
+        } else {
+            break;
+        }
+    }
+    if (best == INT_MAX) return false;
+    // powers of two first: the early stages' strided stores are free of bank conflicts
+    // for them
+    std::stable_partition(p.radix, p.radix + p.nst, [](int r) { return (r & (r - 1)) == 0; });
     unsigned long long Ns = 1;
     for (int st = 0; st < p.nst; st++) {
         // (the first stage, Ns = 1, takes k = 0 without it)
         p.magic[st] = Ns == 1 ? 0u : (unsigned)(((1ull << 32) + Ns - 1) / Ns);
         Ns *= (unsigned long long)p.radix[st];
     }
-    return n == 1;
+    return true;
 }
 
 void fft_rows_ff_twiddles(int L, float4 *host)
@@ -616,7 +669,12 @@ cudaError_t launch_fft_rows_ff(double2 *data, int64_t rows, const FftRowsFF &p, 
     const int per_sm = (int)std::max<size_t>(1, (size_t)(200 * 1024) / (smem + 1024));
     const int64_t cap = (int64_t)sm_count() * per_sm;
     const unsigned g = (unsigned)(rows < cap ? rows : cap);
-    k_fft_rows_ff<<<g, 256, smem, st>>>(data, rows, p, tw);
+    // The registers hold 512 threads on an SM: where the shared memory takes more than two
+    // rows, smaller blocks, so that one row's barriers are another's work (2^18 points,
+    // L = 1344: 7.43 ms per gradient with 256 threads, 7.14 with 128; L = 640: 50,000 points
+    // 733 us with 256, 694 with 128).
+    const int threads = per_sm >= 4 ? 128 : per_sm == 3 ? 160 : 256;
+    k_fft_rows_ff<<<g, threads, smem, st>>>(data, rows, p, tw);
     launches++;
     return cudaGetLastError();
 }

@@ -542,8 +542,8 @@ cudaError_t launch_join_half_spectra_t(const double2 *specT, int nout, int Mx, i
                                        cudaStream_t st, int64_t &launches);
 // Float-float row FFTs (se2p_fft_ff.cu): unnormalised C2C of `rows`
 // contiguous rows of L complex doubles, in place, sign -1 forward / +1
-// inverse (cuFFT's convention).  Lengths 8^a 4^b 2^c 7^d 5^e 3^f up to
-// kFftFFMaxLen; fft_rows_ff_plan says whether L is one.
+// inverse (cuFFT's convention).  Lengths 2^a 3^b 5^c 7^d up to kFftFFMaxLen;
+// fft_rows_ff_plan says whether L is one.
 constexpr int kFftFFMaxLen = 6144;
 constexpr int kFftFFMaxStages = 16;
 struct FftRowsFF {
