@@ -10,8 +10,8 @@
 //
 // Conversions between double and float run at the FP64 rate on GB300, so the
 // double -> (hi, lo) split is done with integer operations on the bit pattern.
-// The split is exact for hi and rounds lo once: hi + lo = d (1 + delta),
-// |delta| <= 2^-48, for 2^-74 <= |d| < 2^128.  Below 2^-74 lo is flushed (the
+// hi is d to the nearest float and lo the rest rounded once: hi + lo = d (1 + delta),
+// |delta| <= 2^-49, for 2^-74 <= |d| < 2^128.  Below 2^-74 lo is flushed (the
 // relative error grows to 2^-24 there; every caller works with magnitudes
 // relative to much larger values), zero maps to (0, 0), inf and NaN stay so.
 #pragma once
@@ -32,14 +32,16 @@ __device__ __forceinline__ float2 ff_split(double d)
         const bool nan = e == 0x7ff && (((unsigned)hw & 0xfffffu) | lw);
         return make_float2(__uint_as_float(sign | (nan ? 0x7fffffffu : 0x7f800000u)), 0.f);
     }
-    const unsigned hb = sign | ((unsigned)(e - 896) << 23) | (((unsigned)hw & 0xfffffu) << 3) |
-                        (lw >> 29);
-    const float hi = __uint_as_float(hb);
-    // lo = low 29 mantissa bits * 2^(e - 1075), with the sign of d
+    // the bits rounded to 24 of the mantissa (half up; a carry runs into the exponent),
+    // the exponent field moved by 896 and the fields by 29 places
+    const unsigned lr = lw + 0x10000000u;
+    const unsigned hr = (unsigned)hw + (lr < lw);
+    const float hi = __uint_as_float(sign | ((__funnelshift_l(lr, hr, 3) - (896u << 23)) & 0x7fffffffu));
+    // lo = what is left, the low 29 mantissa bits as a signed number * 2^(e - 1075),
+    // with the sign of d
     const int se = e - 948;                           // float exponent field of 2^(e-1075)
     const float scale = __uint_as_float((unsigned)max(se, 0) << 23);
-    const float lo = __uint_as_float(__float_as_uint(__uint2float_rn(lw & 0x1fffffffu) * scale) ^
-                                     sign);
+    const float lo = __uint_as_float(__float_as_uint(__int2float_rn((int)(lw << 3) >> 3) * scale) ^ sign);
     return make_float2(hi, lo);
 }
 
