@@ -55,6 +55,7 @@ enum Slot {
     S_GORDER, S_GPCNT, S_GPSTART,               // patch-major target order of the gather
     // tensor-core k space: factor records, tiles and items of the points spread
     S_TCFAC, S_TCTILE, S_TCCNT, S_TCSTART, S_TCLIST, S_TCLTMP, S_TCITEMS,
+    S_TGFAC, S_TGTILE, S_TGSTART, S_TGLIST, S_TGITEMS,
     S_COUNT_SLOTS
 };
 
@@ -604,6 +605,7 @@ struct TcSet {
     int *list = nullptr, *nitems = nullptr;
     int4 *items = nullptr;
     unsigned long long s = 0;            // exp(-2 alpha) 2^64
+    bool ready = false;
 };
 
 // Whether the tensor-core spread runs.  It can for w = h P/2, where both axes'
@@ -622,56 +624,68 @@ static bool tc_ok(const SpreadArgs &sa, int nc)
     return 24.0 * ((nc + 1) / 2) * std::min(ntile, (double)sa.ns) <= 1e5 + 1.1 * nc * (double)sa.ns;
 }
 
-// Factor records, tiles and items of n points for patches of X x Y nodes, items of
-// up to kmax points; perm and bound for the sources (launch_tc_points).  The
-// spread's set and the gather's share their slots: each is used up before the
-// next is made, in stream order.
-static int tc_points(se2p_plan pl, const double2 *p, int64_t n, const int *perm,
-                     const unsigned long long *bound, double Lhx, double Lhy, double h, double a,
-                     int Mx, int My, int P, int X, int Y, int kmax, cudaStream_t ks, TcSet &t)
+// Factor records, tiles and items of a set of points (which = 0: the spread's, 1: the
+// gather's) for patches of X x Y nodes, items of up to kmax points.
+template <class Args>                            // SpreadArgs or GatherArgs
+static int tc_set(se2p_plan pl, int which, const double2 *p, int64_t n, const Args &g, const int *perm,
+                  int X, int Y, int kmax, TcSet &t, TcSetArgs &o)
 {
     TcPointArgs &pa = t.pa;
     pa.p = p;
     pa.n = n;
-    pa.Lhx = Lhx;
-    pa.Lhy = Lhy;
-    pa.h = h;
-    pa.inv_h = 1.0 / h;
-    const double alpha = -a * h * h;
+    pa.Lhx = g.Lhx;
+    pa.Lhy = g.Lhy;
+    pa.h = g.h;
+    pa.inv_h = 1.0 / g.h;
+    const double alpha = -g.a * g.h * g.h;
     pa.al2 = (unsigned long long)std::llround(std::ldexp(alpha * 1.4426950408889634074, 59));
     t.s = (unsigned long long)std::llround(std::ldexp(std::exp(-2.0 * alpha), 62)) << 2;
-    pa.Mx = Mx;
-    pa.My = My;
-    pa.P = P;
-    pa.Tx = X - P;
-    pa.Ty = Y - P;
-    pa.ntx = (Mx + pa.Tx - 1) / pa.Tx;
-    pa.nty = (My + pa.Ty - 1) / pa.Ty;
+    pa.Mx = g.Mx;
+    pa.My = g.My;
+    pa.P = g.P;
+    pa.Tx = X - g.P;
+    pa.Ty = Y - g.P;
+    pa.ntx = (g.Mx + pa.Tx - 1) / pa.Tx;
+    pa.nty = (g.My + pa.Ty - 1) / pa.Ty;
     const int ntile = pa.ntx * pa.nty;
     const size_t nz = (size_t)(n > 0 ? n : 1);
     // small sets: smaller items, so that every SM has two
     kmax = std::min(kmax, std::max(32, (int)((n + 2 * sm_count() - 1) / (2 * sm_count()) + 15) / 16 * 16));
     char *fac = nullptr;
     int *start = nullptr, *ltmp = nullptr;
-    CKS(ensure_t(pl, S_TCFAC, nz * kTcPointBytes, &fac));
-    CKS(ensure_t(pl, S_TCTILE, nz, &pa.tile));
-    CKS(ensure_t(pl, S_TCCNT, (size_t)ntile, &pa.count));
-    CKS(ensure_t(pl, S_TCSTART, 2 * (size_t)ntile + 2, &start));
-    CKS(ensure_t(pl, S_TCLIST, nz, &t.list));
+    CKS(ensure_t(pl, which ? S_TGFAC : S_TCFAC, nz * kTcPointBytes, &fac));
+    CKS(ensure_t(pl, which ? S_TGTILE : S_TCTILE, nz, &pa.tile));
+    CKS(ensure_t(pl, which ? S_TGSTART : S_TCSTART, 2 * (size_t)ntile + 2, &start));
+    CKS(ensure_t(pl, which ? S_TGLIST : S_TCLIST, nz, &t.list));
     if (perm) CKS(ensure_t(pl, S_TCLTMP, 2 * nz, &ltmp));
-    CKS(ensure_t(pl, S_TCITEMS, std::min(nz, (size_t)ntile) + nz / kmax + 1, &t.items));
+    CKS(ensure_t(pl, which ? S_TGITEMS : S_TCITEMS, std::min(nz, (size_t)ntile) + nz / kmax + 1, &t.items));
     pa.fac = fac;
     int *istart = start + ntile + 1;
     t.nitems = istart + ntile;
-    CK(launch_tc_points(pa, kmax, perm, start, istart, t.list, ltmp, t.items, t.nitems, bound, ks,
-                        pl->launches));
+    t.ready = true;
+    o = TcSetArgs{pa, kmax, ntile, perm, start, istart, perm ? ltmp : t.list, perm ? ltmp + n : nullptr,
+                  t.list, t.items, t.nitems};
     return SE2P_OK;
 }
 
-static int tc_sources(se2p_plan pl, const SpreadArgs &sa, cudaStream_t ks, TcSet &t)
+// The sources' set for the spread and / or the points' of the gather, in the same
+// launches (a set of its own took 15 us more at small sizes: 1000 sources on themselves
+// 164 us with both at once, 182 without).
+static int tc_prepare(se2p_plan pl, const SpreadArgs *sa, TcSet *ts, const GatherArgs *ga, TcSet *tt,
+                      cudaStream_t ks)
 {
-    return tc_points(pl, sa.sp, sa.ns, sa.perm, sa.bound, sa.Lhx, sa.Lhy, sa.h, sa.a, sa.Mx, sa.My,
-                     sa.P, kTcX, kTcY, kTcK, ks, t);
+    TcPrepArgs b{};
+    int nset = 0;
+    if (sa) CKS(tc_set(pl, 0, sa->sp, sa->ns, *sa, sa->perm, kTcX, kTcY, kTcK, *ts, b.s[nset++]));
+    if (ga) CKS(tc_set(pl, 1, ga->tp, ga->nt, *ga, nullptr, kTgX, kTgY, kTgT, *tt, b.s[nset++]));
+    int *count = nullptr;
+    CKS(ensure_t(pl, S_TCCNT, (size_t)b.s[0].ntile + b.s[1].ntile, &count));
+    for (int k = 0; k < nset; k++) {
+        b.s[k].a.count = count;
+        count += b.s[k].ntile;
+    }
+    CK(launch_tc_points(b, nset, sa ? sa->bound : nullptr, ks, pl->launches));
+    return SE2P_OK;
 }
 
 static int tc_spread(se2p_plan pl, const SpreadArgs &sa, const TcSet &t, int nc, cudaStream_t ks)
@@ -711,12 +725,6 @@ static bool tg_ok(const GatherArgs &ga, int nout)
     return (14.0 + 13.0 * nout) * std::min(ntile, (double)ga.nt) <= 2.5e5 + 0.35 * nout * nout * (double)ga.nt;
 }
 
-static int tg_targets(se2p_plan pl, const GatherArgs &ga, cudaStream_t ks, TcSet &t)
-{
-    return tc_points(pl, ga.tp, ga.nt, nullptr, nullptr, ga.Lhx, ga.Lhy, ga.h, ga.a, ga.Mx, ga.My,
-                     ga.P, kTgX, kTgY, kTgT, ks, t);
-}
-
 // The gather of nout grids (int64 at scale kTgBits): the patch sums stay below
 // 2^63 with |g| below 2^61 and the factors' sum along y below 4.
 constexpr int kTgBits = 61;
@@ -750,9 +758,10 @@ static int tg_gather(se2p_plan pl, const GatherArgs &ga, const TcSet &t, int nou
 // on return, the grid holds the integers of the tensor-core spread or of
 // k_spread_fix, or (when the bound slot *fixb is all ones: crowded sources)
 // the FP64 spread's doubles, and the pack of fft_fwd_1d reads which; with
-// *fixb null it holds doubles.
+// *fixb null it holds doubles.  The tensor-core spread's preparation does that of a
+// gather's points too, into tt, if ga is one that the tensor-core gather will take.
 static int spread(se2p_plan pl, SpreadArgs &sa, int nc, bool allow_fixed, cudaStream_t ks,
-                  const unsigned long long **fixb)
+                  const unsigned long long **fixb, const GatherArgs *ga, TcSet *tt)
 {
     int kY = 0, mult = 1;
     double kfac = 1.0;
@@ -766,7 +775,7 @@ static int spread(se2p_plan pl, SpreadArgs &sa, int nc, bool allow_fixed, cudaSt
         CK(launch_spread_bound(sa, nc, kfac, mult, ws, ks, pl->launches));
         if (tc_ok(sa, nc)) {
             TcSet t;
-            CKS(tc_sources(pl, sa, ks, t));
+            CKS(tc_prepare(pl, &sa, &t, ga, tt, ks));
             CKS(tc_spread(pl, sa, t, nc, ks));
         } else {
             CK(launch_spread_fix(sa, nc, kY, ks, pl->launches));
@@ -1171,10 +1180,30 @@ int run(se2p_plan pl, const Job &J, const Io &io)
         sa.a = -2 * J.xi * J.xi / J.eta;
         sa.e1 = e1;
         sa.perm = sperm;
+        GatherArgs ga;
+        ga.tp = tp;
+        ga.nt = nt;
+        ga.Mx = Mx;
+        ga.My = My;
+        ga.P = P;
+        ga.Lhx = sa.Lhx;
+        ga.Lhy = sa.Lhy;
+        ga.h = h;
+        ga.w = J.w;
+        ga.a = sa.a;
+        // FP64 form: the fixed-point gather, whenever the spread could run
+        // fixed-point (the same Gaussian-factor condition)
+        int kYg = 0, multg = 1;
+        double kfacg = 1.0;
+        const bool fixg = pl->precision == SE2P_PRECISION_FP64 && spread_fixed_ok(sa, kYg, kfacg, multg) &&
+                          kYg == 0;
+        const bool tg = fixg && tg_ok(ga, nout);
+        TcSet tset;
         const unsigned long long *fixb = nullptr;
         {
             StageTimer tm(pl, T_SPREAD, ks);
-            CKS(spread(pl, sa, nc, pl->precision == SE2P_PRECISION_FP64, ks, &fixb));
+            CKS(spread(pl, sa, nc, pl->precision == SE2P_PRECISION_FP64, ks, &fixb, tg ? &ga : nullptr,
+                       &tset));
         }
         const bool ffft = pl->precision == SE2P_PRECISION_FP64 && fft_ff_ok(Mx, My);
 
@@ -1210,51 +1239,30 @@ int run(se2p_plan pl, const Job &J, const Io &io)
         }
 
         // Z2D as 1D complex passes: C2C along x, Hermitian join, C2C along y, unpack
-        // FP64 form: the fixed-point gather, whenever the spread could run
-        // fixed-point (the same Gaussian-factor condition)
         unsigned long long *gmax = nullptr;
-        int Bg = 0;
-        {
-            int kY = 0, mult = 1;
-            double kfac = 1.0;
-            if (pl->precision == SE2P_PRECISION_FP64 && spread_fixed_ok(sa, kY, kfac, mult) &&
-                kY == 0) {
-                CKS(ensure_t(pl, S_GMAX, kGmaxWords, &gmax));
-                CK(cudaMemsetAsync(gmax, 0, sizeof(unsigned long long) * kGmaxWords, ks));
-                Bg = gather_fixed_bits(sa);
-            }
+        if (fixg) {
+            CKS(ensure_t(pl, S_GMAX, kGmaxWords, &gmax));
+            CK(cudaMemsetAsync(gmax, 0, sizeof(unsigned long long) * kGmaxWords, ks));
         }
         {
             StageTimer tm(pl, T_FFT_INV, ks);
             CKS(fft_inv_1d(pl, ks, Mx, My, spec, nout, zg, grid, ffft, gmax));
         }
 
-        GatherArgs ga;
-        ga.tp = tp;
-        ga.nt = nt;
         ga.grid = grid;
-        ga.Mx = Mx;
-        ga.My = My;
-        ga.P = P;
-        ga.Lhx = J.Lx / 2.0;
-        ga.Lhy = J.Ly / 2.0;
-        ga.h = h;
-        ga.w = J.w;
-        ga.a = -2 * J.xi * J.xi / J.eta;
         double s = 4 * J.xi * J.xi / J.eta;               // mex_stokes_slp_kspace.cpp:325-328
         s = s * s * h * h / kPi;
         ga.scale = s / (4 * kPi);
         ga.e1 = e1;
         ga.out = uk;
         ga.gmax = gmax;
+        const int Bg = fixg ? gather_fixed_bits(sa) : 0;
         ga.Bg = Bg;
         StageTimer tm(pl, T_GATHER, ks);
-        const bool tg = gmax && tg_ok(ga, nout);
         if (tg) {
-            TcSet t;
-            CKS(tg_targets(pl, ga, ks, t));
+            if (!tset.ready) CKS(tc_prepare(pl, nullptr, nullptr, &ga, &tset, ks));
             CK(launch_grid_to_fixed(grid, nout, (int64_t)G, gmax, kTgBits, ks, pl->launches));
-            CKS(tg_gather(pl, ga, t, nout, ks));
+            CKS(tg_gather(pl, ga, tset, nout, ks));
             CK(launch_gather_fp64_fallback(ga, nout, ks, pl->launches));
         } else if (gmax) {
             CK(launch_grid_to_fixed(grid, nout, (int64_t)G, gmax, Bg, ks, pl->launches));
@@ -1493,10 +1501,27 @@ int run_adjoint(se2p_plan pl, const Job &J, const AdjIo &io)
     sa.a = -2 * J.xi * J.xi / J.eta;
     sa.e1 = e1;
     sa.perm = tperm;
+    // float-float gather (FP64 form) when float's range holds the weights;
+    // it needs the grid maximum from the unpack and reuses zg for its planes
+    const double a_gauss = -2 * J.xi * J.xi / J.eta;
+    const bool ffg = form == kFormFF && adj_gather_ff_ok(a_gauss, h, J.w, P);
+    GatherArgs gt;                                   // the sources as gather points
+    gt.tp = sp;
+    gt.nt = ns;
+    gt.Mx = Mx;
+    gt.My = My;
+    gt.P = P;
+    gt.Lhx = sa.Lhx;
+    gt.Lhy = sa.Lhy;
+    gt.h = h;
+    gt.w = J.w;
+    gt.a = sa.a;
+    const bool tg = ffg && tg_ok(gt, 5);
+    TcSet tset;
     const unsigned long long *fixb = nullptr;
     {
         StageTimer tm(pl, T_SPREAD, ks);
-        CKS(spread(pl, sa, 4, form == kFormFF, ks, &fixb));
+        CKS(spread(pl, sa, 4, form == kFormFF, ks, &fixb, tg ? &gt : nullptr, &tset));
     }
     const bool ffft = form == kFormFF && fft_ff_ok(Mx, My);
     cufftDoubleComplex *zg = nullptr;
@@ -1524,11 +1549,7 @@ int run_adjoint(se2p_plan pl, const Job &J, const AdjIo &io)
         CKS(filter_matrix(pl, fa, ks));
         CK(launch_filter_adj(fa, ks, pl->launches));
     }
-    // float-float gather (FP64 form) when float's range holds the weights;
-    // it needs the grid maximum from the unpack and reuses zg for its planes
     unsigned long long *gmax = nullptr;
-    const double a_gauss = -2 * J.xi * J.xi / J.eta;
-    const bool ffg = form == kFormFF && adj_gather_ff_ok(a_gauss, h, J.w, P);
     if (ffg) {
         CKS(ensure_t(pl, S_GMAX, kGmaxWords, &gmax));
         CK(cudaMemsetAsync(gmax, 0, sizeof(unsigned long long) * kGmaxWords, ks));
@@ -1561,36 +1582,24 @@ int run_adjoint(se2p_plan pl, const Job &J, const AdjIo &io)
     }
     {
         StageTimer tm(pl, T_GATHER, ks);
-        GatherArgs gt;                               // the sources as gather points
-        gt.tp = sp;
-        gt.nt = ns;
-        gt.Mx = Mx;
-        gt.My = My;
-        gt.P = P;
-        gt.Lhx = ga.Lhx;
-        gt.Lhy = ga.Lhy;
-        gt.h = h;
-        gt.w = J.w;
-        gt.a = ga.a;
-        if (ffg && tg_ok(gt, 5)) {
-            TcSet t;
-            CKS(tg_targets(pl, gt, ks, t));
+        if (tg) {
+            if (!tset.ready) CKS(tc_prepare(pl, nullptr, nullptr, &gt, &tset, ks));
             CK(launch_grid_to_fixed(grid, 5, (int64_t)G, gmax, kTgBits, ks, pl->launches));
             TcGatherAdjArgs ta{};
-            ta.fac = t.pa.fac;
-            ta.list = t.list;
-            ta.items = t.items;
-            ta.nitems = t.nitems;
+            ta.fac = tset.pa.fac;
+            ta.list = tset.list;
+            ta.items = tset.items;
+            ta.nitems = tset.nitems;
             ta.grid = reinterpret_cast<const long long *>(grid);
             ta.gmax = gmax;
             ta.Mx = Mx;
             ta.My = My;
             ta.P = P;
-            ta.Tx = t.pa.Tx;
-            ta.Ty = t.pa.Ty;
-            ta.nty = t.pa.nty;
+            ta.Tx = tset.pa.Tx;
+            ta.Ty = tset.pa.Ty;
+            ta.nty = tset.pa.nty;
             ta.Bg = kTgBits;
-            ta.s = t.s;
+            ta.s = tset.s;
             ta.sp = sp;
             ta.coef = coef;
             ta.Lhx = ga.Lhx;
@@ -2225,6 +2234,19 @@ static int geom_kspace_multi(se2p_geom g, int nr, const double *coef, int64_t cs
     sa.a = -2 * p.xi * p.xi / p.eta;
     sa.e1 = e1;
     sa.perm = g->sperm;
+    GatherArgs ga;
+    ga.tp = g->tp;
+    ga.nt = g->nt;
+    ga.Mx = Mx;
+    ga.My = My;
+    ga.P = P;
+    ga.Lhx = p.Lx / 2.0;
+    ga.Lhy = p.Ly / 2.0;
+    ga.h = h;
+    ga.w = p.w;
+    ga.a = -2 * p.xi * p.xi / p.eta;
+    const bool tg = tg_ok(ga, nout);
+    TcSet tset;
     auto rhs_spread = [&](int r) {
         SpreadArgs sr = sa;
         sr.coef = coef + r * cstride;
@@ -2239,7 +2261,7 @@ static int geom_kspace_multi(se2p_geom g, int nr, const double *coef, int64_t cs
         sa.bound = reinterpret_cast<const unsigned long long *>(ws + bslot);
         if (tc_ok(sa, nc)) {
             TcSet t;
-            CKS(tc_sources(pl, sa, ks, t));
+            CKS(tc_prepare(pl, &sa, &t, tg ? &ga : nullptr, &tset, ks));
             for (int r = 0; r < nr; r++) CKS(tc_spread(pl, rhs_spread(r), t, nc, ks));
         } else {
             CK(launch_spread_fix_multi(sa, nc, kY, nr, cstride, (int64_t)(nc * G), (int)bstride, ks,
@@ -2280,18 +2302,7 @@ static int geom_kspace_multi(se2p_geom g, int nr, const double *coef, int64_t cs
             CKS(fft_inv_1d(pl, ks, Mx, My, spec, nout, zg, gr, true, gmax + r * kGmaxWords));
         }
     }
-    GatherArgs ga;
-    ga.tp = g->tp;
-    ga.nt = g->nt;
     ga.grid = grid;
-    ga.Mx = Mx;
-    ga.My = My;
-    ga.P = P;
-    ga.Lhx = p.Lx / 2.0;
-    ga.Lhy = p.Ly / 2.0;
-    ga.h = h;
-    ga.w = p.w;
-    ga.a = -2 * p.xi * p.xi / p.eta;
     double sc = 4 * p.xi * p.xi / p.eta;             // mex_stokes_slp_kspace.cpp:325-328
     sc = sc * sc * h * h / kPi;
     ga.scale = sc / (4 * kPi);
@@ -2304,19 +2315,17 @@ static int geom_kspace_multi(se2p_geom g, int nr, const double *coef, int64_t cs
     // 14.5 ms for four)
     StageTimer tm(pl, T_GATHER, ks);
     const int64_t ostride = (int64_t)(nout / 2) * g->nt;
-    const bool tg = tg_ok(ga, nout);
     for (int r = 0; r < nr; r++)
         CK(launch_grid_to_fixed(grid + (size_t)r * nc * G, nout, (int64_t)G, gmax + r * kGmaxWords,
                                 tg ? kTgBits : Bg, ks, pl->launches));
     if (tg) {
-        TcSet t;
-        CKS(tg_targets(pl, ga, ks, t));
+        if (!tset.ready) CKS(tc_prepare(pl, nullptr, nullptr, &ga, &tset, ks));
         for (int r = 0; r < nr; r++) {
             GatherArgs gr = ga;
             gr.grid = grid + (size_t)r * nc * G;
             gr.gmax = gmax + r * kGmaxWords;
             gr.out = uk + r * ostride;
-            CKS(tg_gather(pl, gr, t, nout, ks));
+            CKS(tg_gather(pl, gr, tset, nout, ks));
         }
     } else {
         CK(launch_gather_fix_multi(ga, nout, nr, (int64_t)(nc * G), ostride, ks, pl->launches));

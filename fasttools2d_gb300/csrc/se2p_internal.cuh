@@ -383,6 +383,22 @@ struct TcPointArgs {
     int2 *tile;                 // per point (tile, rank in it)
 };
 
+// One or two sets of points on their way into tiles: their records, and from the tiles'
+// counts the scans, the list of slots and the items.
+struct TcSetArgs {
+    TcPointArgs a;
+    int kmax, ntile;
+    const int *perm;            // sorted -> caller's number (sources), or null
+    int *start, *istart;        // per tile: first slot, first item
+    int *list, *key;            // slot -> point; with perm, slot -> caller's number
+    int *ordered;               // with perm: list with the slots of long tiles in the caller's order
+    int4 *items;
+    int *nitems;
+};
+struct TcPrepArgs {
+    TcSetArgs s[2];
+};
+
 struct TcSpreadArgs {
     const void *fac;
     const int *list;            // tile by tile, the points' numbers
@@ -667,10 +683,8 @@ __device__ __forceinline__ int fix_shift(unsigned long long bits)
 // Factor records, tiles and items of n points (kmax per item); with perm, tiles
 // of several items are put in the order of the caller's point numbers
 // (list_tmp then holds 2 n ints).
-cudaError_t launch_tc_points(const TcPointArgs &a, int kmax, const int *perm, int *start,
-                             int *istart, int *list, int *list_tmp, int4 *items, int *nitems,
-                             const unsigned long long *bound, cudaStream_t st,
-                             int64_t &launches);
+cudaError_t launch_tc_points(const TcPrepArgs &b, int nset, const unsigned long long *bound,
+                             cudaStream_t st, int64_t &launches);
 cudaError_t launch_gather_tc(const TcGatherArgs &a, int nc, cudaStream_t st, int64_t &launches);
 cudaError_t launch_gather_adj_tc(const TcGatherAdjArgs &a, cudaStream_t st, int64_t &launches);
 cudaError_t launch_spread_tc(const TcSpreadArgs &a, int nc, cudaStream_t st, int64_t &launches);

@@ -179,8 +179,9 @@ __device__ __forceinline__ void tc_seed(unsigned long long u, unsigned long long
 
 // Bound: issue (about 400 integer instructions per point).  With the exponentials,
 // divisions and conversions in FP64 it took 310 us for 2^20 points, bound by the FP64 pipe.
-__global__ void __launch_bounds__(256) k_tc_points(TcPointArgs a)
+__global__ void __launch_bounds__(256) k_tc_points(TcPrepArgs b)
 {
+    const TcPointArgs &a = b.s[blockIdx.y].a;
     __shared__ unsigned long long tab[256];
     tab[threadIdx.x] = c_exp2_tab[threadIdx.x];
     __syncthreads();
@@ -220,11 +221,12 @@ __global__ void __launch_bounds__(256) k_tc_points(TcPointArgs a)
 // Exclusive scans of the tiles' counts and of their numbers of items,
 // ceil(count / kmax) each: a block scans 1024 tiles and adds up the counts before
 // them itself (23 blocks at 2688^2 nodes: 4 us; one block over all of them, 30 us).
-__global__ void __launch_bounds__(1024) k_tc_items(const int *__restrict__ count, int ntile,
-                                                   int kmax, int *__restrict__ start,
-                                                   int *__restrict__ istart,
-                                                   int *__restrict__ nitems)
+__global__ void __launch_bounds__(1024) k_tc_items(TcPrepArgs b)
 {
+    const TcSetArgs &t = b.s[blockIdx.y];
+    const int *__restrict__ count = t.a.count;
+    const int ntile = t.ntile, kmax = t.kmax;
+    if ((int)blockIdx.x * 1024 >= ntile) return;
     // ceil(v / kmax) by a product with ceil(2^32 / kmax), exact for kmax <= 64 and v
     // below 2^25; larger counts divide
     const unsigned inv = 0xffffffffu / (unsigned)kmax + 1;
@@ -265,11 +267,11 @@ __global__ void __launch_bounds__(1024) k_tc_items(const int *__restrict__ count
         run.y += before[w].y + (w < wid ? warp_tot[w].y : 0);
     }
     if (i < ntile) {
-        start[i] = run.x;
-        istart[i] = run.y;
+        t.start[i] = run.x;
+        t.istart[i] = run.y;
         if (i == ntile - 1) {
-            start[ntile] = run.x + own.x;
-            *nitems = run.y + own.y;
+            t.start[ntile] = run.x + own.x;
+            *t.nitems = run.y + own.y;
         }
     }
 }
@@ -277,24 +279,20 @@ __global__ void __launch_bounds__(1024) k_tc_items(const int *__restrict__ count
 // Slot -> sorted point, tile by tile, and the items: a tile's points cut into
 // nearly equal runs, items[k] = (tile, first slot, count, 0).  key: the
 // points' numbers in the caller's order, by slot (with perm).
-__global__ void __launch_bounds__(256) k_tc_list(int64_t n, const int2 *__restrict__ tile,
-                                                 const int *__restrict__ start,
-                                                 const int *__restrict__ istart, int kmax,
-                                                 const int *__restrict__ perm,
-                                                 int *__restrict__ list, int *__restrict__ key,
-                                                 int4 *__restrict__ items)
+__global__ void __launch_bounds__(256) k_tc_list(TcPrepArgs b)
 {
+    const TcSetArgs &w = b.s[blockIdx.y];
     const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n) return;
-    const int2 t = tile[j];
-    const int a = start[t.x], v = start[t.x + 1] - a;
-    list[a + t.y] = (int)j;
-    if (perm) key[a + t.y] = perm[j];
-    const int nch = (v + kmax - 1) / kmax;
+    if (j >= w.a.n) return;
+    const int2 t = w.a.tile[j];
+    const int a = w.start[t.x], v = w.start[t.x + 1] - a;
+    w.list[a + t.y] = (int)j;
+    if (w.perm) w.key[a + t.y] = w.perm[j];
+    const int nch = (v + w.kmax - 1) / w.kmax;
     const int c = (int)(((int64_t)t.y * nch + nch - 1) / v);
     const int first = (int)((int64_t)v * c / nch);
     if (c < nch && first == t.y)
-        items[istart[t.x] + c] = make_int4(t.x, a + first, (int)((int64_t)v * (c + 1) / nch) - first, 0);
+        w.items[w.istart[t.x] + c] = make_int4(t.x, a + first, (int)((int64_t)v * (c + 1) / nch) - first, 0);
 }
 
 // A tile of more than one item: its slots in the order of the caller's point
@@ -1486,24 +1484,29 @@ __global__ void __launch_bounds__(kGaThreads, 1) k_gather_adj_tc(TcGatherAdjArgs
 // ---------------------------------------------------------------------------
 // Launchers
 // ---------------------------------------------------------------------------
-cudaError_t launch_tc_points(const TcPointArgs &a, int kmax, const int *perm, int *start,
-                             int *istart, int *list, int *list_tmp, int4 *items, int *nitems,
-                             const unsigned long long *bound, cudaStream_t st,
-                             int64_t &launches)
+cudaError_t launch_tc_points(const TcPrepArgs &b, int nset, const unsigned long long *bound,
+                             cudaStream_t st, int64_t &launches)
 {
-    const int ntile = a.ntx * a.nty;
-    cudaError_t e = cudaMemsetAsync(a.count, 0, sizeof(int) * (size_t)ntile, st);
+    // (the sets' counts are one array)
+    int64_t n = 0;
+    int ntile = 0, total = 0;
+    for (int k = 0; k < nset; k++) {
+        n = b.s[k].a.n > n ? b.s[k].a.n : n;
+        ntile = b.s[k].ntile > ntile ? b.s[k].ntile : ntile;
+        total += b.s[k].ntile;
+    }
+    const cudaError_t e = cudaMemsetAsync(b.s[0].a.count, 0, sizeof(int) * (size_t)total, st);
     if (e != cudaSuccess) return e;
-    const unsigned g = (unsigned)((a.n + 255) / 256);
-    if (a.n > 0) k_tc_points<<<g, 256, 0, st>>>(a);
-    k_tc_items<<<(ntile + 1023) / 1024, 1024, 0, st>>>(a.count, ntile, kmax, start, istart, nitems);
-    launches += a.n > 0 ? 2 : 1;
-    if (a.n > 0) {
-        k_tc_list<<<g, 256, 0, st>>>(a.n, a.tile, start, istart, kmax, perm, perm ? list_tmp : list,
-                                     perm ? list_tmp + a.n : nullptr, items);
-        launches++;
-        if (perm) {
-            k_tc_order<<<g, 256, 0, st>>>(a.n, a.tile, start, kmax, list_tmp + a.n, list_tmp, list, bound);
+    const dim3 g((unsigned)((n + 255) / 256), nset);
+    if (n > 0) k_tc_points<<<g, 256, 0, st>>>(b);
+    k_tc_items<<<dim3((ntile + 1023) / 1024, nset), 1024, 0, st>>>(b);
+    if (n > 0) k_tc_list<<<g, 256, 0, st>>>(b);
+    launches += n > 0 ? 3 : 1;
+    for (int k = 0; k < nset; k++) {
+        const TcSetArgs &t = b.s[k];
+        if (t.perm && t.a.n > 0) {
+            k_tc_order<<<(unsigned)((t.a.n + 255) / 256), 256, 0, st>>>(t.a.n, t.a.tile, t.start, t.kmax, t.key,
+                                                                       t.list, t.ordered, bound);
             launches++;
         }
     }
