@@ -668,6 +668,20 @@ static int tc_set(se2p_plan pl, int which, const double2 *p, int64_t n, const Ar
     return SE2P_OK;
 }
 
+// The sets' counts per tile, zeroed (ahead of other kernels: a memset between two kernels
+// keeps the second from being chained to the first).
+static int tc_counts(se2p_plan pl, const SpreadArgs *sa, const GatherArgs *ga, cudaStream_t ks, int **count)
+{
+    size_t n = 0;
+    auto tiles = [](int M, int T) { return (size_t)((M + T - 1) / T); };
+    if (sa) n += tiles(sa->Mx, kTcX - sa->P) * tiles(sa->My, kTcY - sa->P);
+    if (ga) n += tiles(ga->Mx, kTgX - ga->P) * tiles(ga->My, kTgY - ga->P);
+    CKS(ensure_t(pl, S_TCCNT, n, count));
+    CK(cudaMemsetAsync(*count, 0, sizeof(int) * n, ks));
+    return SE2P_OK;
+}
+
+// (with sa, after tc_counts)
 // The sources' set for the spread and / or the points' of the gather, in the same
 // launches (a set of its own took 15 us more at small sizes: 1000 sources on themselves
 // 164 us with both at once, 182 without).
@@ -676,10 +690,11 @@ static int tc_prepare(se2p_plan pl, const SpreadArgs *sa, TcSet *ts, const Gathe
 {
     TcPrepArgs b{};
     int nset = 0;
+    int *count = nullptr;
+    if (!sa) CKS(tc_counts(pl, nullptr, ga, ks, &count));
     if (sa) CKS(tc_set(pl, 0, sa->sp, sa->ns, *sa, sa->perm, kTcX, kTcY, kTcK, *ts, b.s[nset++]));
     if (ga) CKS(tc_set(pl, 1, ga->tp, ga->nt, *ga, nullptr, kTgX, kTgY, kTgT, *tt, b.s[nset++]));
-    int *count = nullptr;
-    CKS(ensure_t(pl, S_TCCNT, (size_t)b.s[0].ntile + b.s[1].ntile, &count));
+    count = static_cast<int *>(pl->buf[S_TCCNT].p);
     for (int k = 0; k < nset; k++) {
         b.s[k].a.count = count;
         count += b.s[k].ntile;
@@ -772,8 +787,11 @@ static int spread(se2p_plan pl, SpreadArgs &sa, int nc, bool allow_fixed, cudaSt
         CKS(ensure_t(pl, S_SBINS, (size_t)spread_bound_words(sa.Mx, sa.My, sa.P), &ws));
         sa.bound = reinterpret_cast<const unsigned long long *>(
             ws + spread_bound_slot(sa.Mx, sa.My, sa.P));
+        const bool tc = tc_ok(sa, nc);
+        int *count = nullptr;
+        if (tc) CKS(tc_counts(pl, &sa, ga, ks, &count));
         CK(launch_spread_bound(sa, nc, kfac, mult, ws, ks, pl->launches));
-        if (tc_ok(sa, nc)) {
+        if (tc) {
             TcSet t;
             CKS(tc_prepare(pl, &sa, &t, ga, tt, ks));
             CKS(tc_spread(pl, sa, t, nc, ks));
@@ -1199,6 +1217,11 @@ int run(se2p_plan pl, const Job &J, const Io &io)
                           kYg == 0;
         const bool tg = fixg && tg_ok(ga, nout);
         TcSet tset;
+        unsigned long long *gmax = nullptr;
+        if (fixg) {
+            CKS(ensure_t(pl, S_GMAX, kGmaxWords, &gmax));
+            CK(cudaMemsetAsync(gmax, 0, sizeof(unsigned long long) * kGmaxWords, ks));
+        }
         const unsigned long long *fixb = nullptr;
         {
             StageTimer tm(pl, T_SPREAD, ks);
@@ -1239,11 +1262,6 @@ int run(se2p_plan pl, const Job &J, const Io &io)
         }
 
         // Z2D as 1D complex passes: C2C along x, Hermitian join, C2C along y, unpack
-        unsigned long long *gmax = nullptr;
-        if (fixg) {
-            CKS(ensure_t(pl, S_GMAX, kGmaxWords, &gmax));
-            CK(cudaMemsetAsync(gmax, 0, sizeof(unsigned long long) * kGmaxWords, ks));
-        }
         {
             StageTimer tm(pl, T_FFT_INV, ks);
             CKS(fft_inv_1d(pl, ks, Mx, My, spec, nout, zg, grid, ffft, gmax));
@@ -1518,6 +1536,11 @@ int run_adjoint(se2p_plan pl, const Job &J, const AdjIo &io)
     gt.a = sa.a;
     const bool tg = ffg && tg_ok(gt, 5);
     TcSet tset;
+    unsigned long long *gmax = nullptr;
+    if (ffg) {
+        CKS(ensure_t(pl, S_GMAX, kGmaxWords, &gmax));
+        CK(cudaMemsetAsync(gmax, 0, sizeof(unsigned long long) * kGmaxWords, ks));
+    }
     const unsigned long long *fixb = nullptr;
     {
         StageTimer tm(pl, T_SPREAD, ks);
@@ -1548,11 +1571,6 @@ int run_adjoint(se2p_plan pl, const Job &J, const AdjIo &io)
         StageTimer tm(pl, T_FILTER, ks);
         CKS(filter_matrix(pl, fa, ks));
         CK(launch_filter_adj(fa, ks, pl->launches));
-    }
-    unsigned long long *gmax = nullptr;
-    if (ffg) {
-        CKS(ensure_t(pl, S_GMAX, kGmaxWords, &gmax));
-        CK(cudaMemsetAsync(gmax, 0, sizeof(unsigned long long) * kGmaxWords, ks));
     }
     {
         StageTimer tm(pl, T_FFT_INV, ks);
@@ -2256,10 +2274,13 @@ static int geom_kspace_multi(se2p_geom g, int nr, const double *coef, int64_t cs
     };
     {
         StageTimer tm(pl, T_SPREAD, ks);
+        const bool tc = tc_ok(sa, nc);
+        int *count = nullptr;
+        if (tc) CKS(tc_counts(pl, &sa, tg ? &ga : nullptr, ks, &count));
         for (int r = 0; r < nr; r++)
             CK(launch_spread_bound(rhs_spread(r), nc, kfac, mult, ws + r * bstride, ks, pl->launches));
         sa.bound = reinterpret_cast<const unsigned long long *>(ws + bslot);
-        if (tc_ok(sa, nc)) {
+        if (tc) {
             TcSet t;
             CKS(tc_prepare(pl, &sa, &t, tg ? &ga : nullptr, &tset, ks));
             for (int r = 0; r < nr; r++) CKS(tc_spread(pl, rhs_spread(r), t, nc, ks));

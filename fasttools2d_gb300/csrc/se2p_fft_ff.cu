@@ -473,6 +473,7 @@ __device__ __forceinline__ float2 ff_split_scaled(double d, int e)
 __global__ void __launch_bounds__(256, 2) k_fft_rows_ff(double2 *__restrict__ data, int64_t rows,
                                                         FftRowsFF p, const float4 *__restrict__ tab)
 {
+    chain_enter();
     extern __shared__ __align__(16) f2 fsh[];
     __shared__ int emax_w[8];
     const int L = p.L, Lp = sh_len(L);
@@ -674,7 +675,7 @@ cudaError_t launch_fft_rows_ff(double2 *data, int64_t rows, const FftRowsFF &p, 
     // L = 1344: 7.43 ms per gradient with 256 threads, 7.14 with 128; L = 640: 50,000 points
     // 733 us with 256, 694 with 128).
     const int threads = per_sm >= 4 ? 128 : per_sm == 3 ? 160 : 256;
-    k_fft_rows_ff<<<g, threads, smem, st>>>(data, rows, p, tw);
+    launch_chained(k_fft_rows_ff, g, threads, smem, st, data, rows, p, tw);
     launches++;
     return cudaGetLastError();
 }

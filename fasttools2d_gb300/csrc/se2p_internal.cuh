@@ -516,6 +516,39 @@ struct GatherArgsF {
 };
 
 // ---------------------------------------------------------------------------
+// Chained launches (programmatic dependent launch): a kernel launched by
+// launch_chained may have its blocks in place while the stream's previous kernel
+// still runs; chain_enter, the first statement of every such kernel, waits until that
+// one has completed and its writes are visible, and lets the next one's blocks in.  As
+// every kernel of a chain waits before it does anything, completion stays in stream
+// order.  Small evaluations are a chain of 25 kernels of a few microseconds each
+// (1000 sources on themselves: 123 us, 164 without).  After a memset, a copy or an event
+// the launch is an ordinary one, and so it is on the default stream and under capture.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ void chain_enter()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+template <class... P, class... A>
+inline void launch_chained(void (*k)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t st, A... a)
+{
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c{};
+    c.gridDim = grid;
+    c.blockDim = dim3(threads);
+    c.dynamicSmemBytes = smem;
+    c.stream = st;
+    c.attrs = &at;
+    c.numAttrs = st && cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
+    cudaLaunchKernelEx(&c, k, static_cast<P>(a)...);   // (an error stays for cudaGetLastError)
+}
+
+// ---------------------------------------------------------------------------
 // Host launchers (se2p_kernels.cu).  Each returns the launch status.
 // ---------------------------------------------------------------------------
 cudaError_t launch_sort(const SortArgs &a, int nsets, cudaStream_t st, int64_t &launches);
@@ -683,6 +716,7 @@ __device__ __forceinline__ int fix_shift(unsigned long long bits)
 // Factor records, tiles and items of n points (kmax per item); with perm, tiles
 // of several items are put in the order of the caller's point numbers
 // (list_tmp then holds 2 n ints).
+// (a.count of the sets zeroed before)
 cudaError_t launch_tc_points(const TcPrepArgs &b, int nset, const unsigned long long *bound,
                              cudaStream_t st, int64_t &launches);
 cudaError_t launch_gather_tc(const TcGatherArgs &a, int nc, cudaStream_t st, int64_t &launches);

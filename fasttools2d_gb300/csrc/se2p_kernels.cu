@@ -151,6 +151,7 @@ constexpr int kScanWide = 1 << 17;
 
 __global__ void __launch_bounds__(1024) k_sort_scan(SortArgs a)
 {
+    chain_enter();
     const int *count = a.s[blockIdx.y].count;
     int *start = a.s[blockIdx.y].start;
     const int n = a.nx * a.ny;
@@ -187,6 +188,7 @@ __global__ void __launch_bounds__(1024) k_sort_scan(SortArgs a)
 // Sorted slot of point i; writes the permutation and the sorted copies.
 __global__ void __launch_bounds__(256) k_sort_place(SortArgs a)
 {
+    chain_enter();
     const SortSet &s = a.s[blockIdx.y];
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= s.n) return;
@@ -220,6 +222,7 @@ __global__ void __launch_bounds__(256) k_src_coef(int64_t n, const int *__restri
                            float2 *__restrict__ out, int64_t ostride, int tails,
                            int *__restrict__ zero)
 {
+    chain_enter();
     const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (zero && j == 0) *zero = 0;
     if (j >= n) return;
@@ -258,6 +261,7 @@ __global__ void k_sorted_pair(int64_t n, const int *__restrict__ perm,
                               const double2 *__restrict__ a, const double2 *__restrict__ b,
                               double *__restrict__ out, float2 *__restrict__ ff)
 {
+    chain_enter();
     const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= n) return;
     const int i = perm[j];
@@ -1503,6 +1507,7 @@ __device__ __forceinline__ int wrap_index(int i, int M)
 template <int NC>
 __global__ void __launch_bounds__(kSpreadWarps * 32) k_spread(SpreadArgs a)
 {
+    chain_enter();
     // behind k_spread_fix: runs only when the bound slot says kFixedOff
     if (a.bound && *a.bound != kFixedOff) return;
     __shared__ double wsh[kSpreadWarps][NC + 1][32];
@@ -1685,6 +1690,7 @@ static BoundAxis bound_axis(int M, int P, double a, double h)
 __global__ void k_spread_bin_sum(SpreadArgs a, int nc, int nbx, int nby, double *__restrict__ bins,
                                  int *__restrict__ cnt, unsigned long long *__restrict__ bound)
 {
+    chain_enter();
     const double inv_h = 1.0 / a.h;
     for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < a.ns;
          s += (int64_t)gridDim.x * blockDim.x) {
@@ -1711,6 +1717,7 @@ __global__ void k_spread_bin_sum(SpreadArgs a, int nc, int nbx, int nby, double 
 __global__ void k_bound_x(const double *__restrict__ bins, const int *__restrict__ cnt,
                           BoundAxis ax, int nby, double *__restrict__ t, int *__restrict__ tc)
 {
+    chain_enter();
     const int nbx = ax.nb;
     const int64_t nb = (int64_t)nbx * nby;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nb;
@@ -1741,6 +1748,7 @@ __global__ void k_bound_y_max(const double *__restrict__ t, const int *__restric
                               BoundAxis ay, int nbx, double kfac, int mult,
                               unsigned long long *__restrict__ bound)
 {
+    chain_enter();
     const int nby = ay.nb;
     const int64_t nb = (int64_t)nbx * nby;
     double best = 0.0;
@@ -2093,6 +2101,7 @@ __global__ void __launch_bounds__(256) k_split_half_spectra_t(const double2 *__r
                                                               double2 *__restrict__ specT,
                                                               int fold)
 {
+    chain_enter();
     __shared__ double2 sa[kTT][kTT + 1], sb[kTT][kTT + 1];
     const int H1 = My / 2 + 1;
     const int64_t G = (int64_t)Mx * My, HT = (int64_t)H1 * Mx;
@@ -2130,6 +2139,7 @@ __global__ void __launch_bounds__(256) k_join_half_spectra_t(const double2 *__re
                                                              int nout, int Mx, int My,
                                                              double2 *__restrict__ z)
 {
+    chain_enter();
     __shared__ double2 sa[kTT][kTT + 1], sb[kTT][kTT + 1];
     const int H1 = My / 2 + 1;
     const int64_t G = (int64_t)Mx * My, HT = (int64_t)H1 * Mx;
@@ -2233,6 +2243,7 @@ __device__ __forceinline__ void dlp_mode(double k1, double k2, double xi, double
 
 __global__ void k_filter(FilterArgs a)
 {
+    chain_enter();
     const int H = a.My / 2 + 1;
     const int64_t G = (int64_t)a.Mx * H;
     const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -2378,6 +2389,7 @@ __global__ void k_filter_matrix_table(FilterArgs a, double *__restrict__ mtab)
 template <int NC, int PT>
 __global__ void __launch_bounds__(256) k_gather(GatherArgs a)
 {
+    chain_enter();
     // behind k_gather_fix: runs only when a grid held a non-finite value
     if (a.gmax && gmax_all(a.gmax) < kGridNonFinite) return;
     for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < a.nt;
@@ -2488,6 +2500,7 @@ constexpr int kGatherThreads = SE2P_GATHER_THREADS;
 __global__ void k_grid_to_fixed(double *__restrict__ grid, int64_t G,
                                 const unsigned long long *__restrict__ gmax, int Bg)
 {
+    chain_enter();
     if (gmax_all(gmax) >= kGridNonFinite) return;
     const int c = blockIdx.y;
     const double s = ldexp(1.0, grid_shift(gmax[c / 2], Bg));
@@ -2697,6 +2710,7 @@ __device__ __forceinline__ void dlp_matrix(double k1, double k2, double xi, doub
 
 __global__ void k_filter_adj(FilterArgs a)
 {
+    chain_enter();
     const int H = a.My / 2 + 1;
     const int64_t G = (int64_t)a.Mx * H;
     const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -3116,6 +3130,7 @@ __device__ __forceinline__ double2 sum_parts(int nparts, const double2 *__restri
 // part[nparts] = the sum of part[0 .. nparts-1].
 __global__ void __launch_bounds__(32) k_wsum_final(int nparts, double2 *__restrict__ part)
 {
+    chain_enter();
     const double2 t = sum_parts(nparts, part);
     if (threadIdx.x == 0) part[nparts] = t;
 }
@@ -3131,6 +3146,7 @@ __global__ void k_adj_assemble(int64_t n, const int *__restrict__ perm,
                                double2 *__restrict__ g_pos, double2 *__restrict__ g_fs,
                                double2 *__restrict__ g_fd, double2 *__restrict__ g_n)
 {
+    chain_enter();
     const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= n) return;
     const int i = perm[j];
@@ -3189,6 +3205,7 @@ __global__ void __launch_bounds__(256) k_zero_mode_part(int64_t n, const double2
 __global__ void __launch_bounds__(32) k_zero_mode_final(int nparts, const double2 *__restrict__ part, double inv_area,
                                   double2 *__restrict__ zm)
 {
+    chain_enter();
     const double2 s = sum_parts(nparts, part);
     if (threadIdx.x == 0) *zm = make_double2(s.x * inv_area, s.y * inv_area);
 }
@@ -3212,6 +3229,7 @@ __device__ __forceinline__ double div_const(double x, double d, double inv_d)
 // (all outputs of one call, so that perm is read once)
 __global__ void __launch_bounds__(256) k_assemble(int64_t n, const int *__restrict__ perm, AssembleArgs a)
 {
+    chain_enter();
     const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= n) return;
     const int i = perm[j];
@@ -3287,8 +3305,8 @@ cudaError_t launch_sort(const SortArgs &a, int nsets, cudaStream_t st, int64_t &
     }
     const dim3 g(grid_for(n, 256), (unsigned)nsets);
     if (n > 0) k_sort_count<<<g, 256, 0, st>>>(a);
-    k_sort_scan<<<dim3(nbox > kScanWide ? 1 : (nbox + 1023) / 1024, nsets), 1024, 0, st>>>(a);
-    if (n > 0) k_sort_place<<<g, 256, 0, st>>>(a);
+    launch_chained(k_sort_scan, dim3(nbox > kScanWide ? 1 : (nbox + 1023) / 1024, nsets), 1024, 0, st, a);
+    if (n > 0) launch_chained(k_sort_place, g, 256, 0, st, a);
     launches += n > 0 ? 3 : 1;
     return cudaGetLastError();
 }
@@ -3299,7 +3317,7 @@ cudaError_t launch_src_coef(int64_t n, const int *perm, const double2 *f_slp,
                             bool tails, int *zero)
 {
     if (n <= 0 && !zero) return cudaSuccess;
-    k_src_coef<<<grid_for(n > 0 ? n : 1, 256), 256, 0, st>>>(n, perm, f_slp, f_dlp, nrm, coef, nc, out,
+    launch_chained(k_src_coef, grid_for(n > 0 ? n : 1, 256), 256, 0, st, n, perm, f_slp, f_dlp, nrm, coef, nc, out,
                                                              ostride, tails ? 1 : 0, zero);
     launches++;
     return cudaGetLastError();
@@ -3358,10 +3376,10 @@ cudaError_t launch_spread(const SpreadArgs &a, int nc, cudaStream_t st, int64_t 
     const int64_t cap = (int64_t)sm_count() * 8;
     const unsigned g = (unsigned)(want < cap ? want : cap);
     switch (nc) {
-    case 2: k_spread<2><<<g, kSpreadWarps * 32, 0, st>>>(a); break;
-    case 3: k_spread<3><<<g, kSpreadWarps * 32, 0, st>>>(a); break;
-    case 4: k_spread<4><<<g, kSpreadWarps * 32, 0, st>>>(a); break;
-    default: k_spread<5><<<g, kSpreadWarps * 32, 0, st>>>(a); break;
+    case 2: launch_chained(k_spread<2>, g, kSpreadWarps * 32, 0, st, a); break;
+    case 3: launch_chained(k_spread<3>, g, kSpreadWarps * 32, 0, st, a); break;
+    case 4: launch_chained(k_spread<4>, g, kSpreadWarps * 32, 0, st, a); break;
+    default: launch_chained(k_spread<5>, g, kSpreadWarps * 32, 0, st, a); break;
     }
     launches++;
     return cudaGetLastError();
@@ -3379,7 +3397,7 @@ cudaError_t launch_filter_matrix_table(const FilterArgs &a, double *mtab, cudaSt
 cudaError_t launch_filter(const FilterArgs &a, cudaStream_t st, int64_t &launches)
 {
     const int64_t n = (int64_t)a.Mx * (a.My / 2 + 1);
-    k_filter<<<grid_for(n, 256), 256, 0, st>>>(a);
+    launch_chained(k_filter, grid_for(n, 256), 256, 0, st, a);
     launches++;
     return cudaGetLastError();
 }
@@ -3410,13 +3428,13 @@ cudaError_t launch_gather(const GatherArgs &a, int nc, cudaStream_t st, int64_t 
         if (e != cudaSuccess) return e;
     }
     if (nc == 2) {
-        if (a.P == 24) k_gather<2, 24><<<g, 256, 0, st>>>(a);
-        else if (a.P == 12) k_gather<2, 12><<<g, 256, 0, st>>>(a);
-        else k_gather<2, 0><<<g, 256, 0, st>>>(a);
+        if (a.P == 24) launch_chained(k_gather<2, 24>, g, 256, 0, st, a);
+        else if (a.P == 12) launch_chained(k_gather<2, 12>, g, 256, 0, st, a);
+        else launch_chained(k_gather<2, 0>, g, 256, 0, st, a);
     } else {
-        if (a.P == 24) k_gather<4, 24><<<g, 256, 0, st>>>(a);
-        else if (a.P == 12) k_gather<4, 12><<<g, 256, 0, st>>>(a);
-        else k_gather<4, 0><<<g, 256, 0, st>>>(a);
+        if (a.P == 24) launch_chained(k_gather<4, 24>, g, 256, 0, st, a);
+        else if (a.P == 12) launch_chained(k_gather<4, 12>, g, 256, 0, st, a);
+        else launch_chained(k_gather<4, 0>, g, 256, 0, st, a);
     }
     launches++;
     return cudaGetLastError();
@@ -3427,7 +3445,7 @@ cudaError_t launch_zero_mode(int64_t n, const double2 *p, const double2 *f, cons
                              int64_t &launches)
 {
     k_zero_mode_part<<<kZeroModeParts, 256, 0, st>>>(n, p, f, nrm, part);
-    k_zero_mode_final<<<1, 32, 0, st>>>(kZeroModeParts, part, inv_area, zm);
+    launch_chained(k_zero_mode_final, 1, 32, 0, st, kZeroModeParts, part, inv_area, zm);
     launches += 2;
     return cudaGetLastError();
 }
@@ -3436,7 +3454,7 @@ cudaError_t launch_assemble(int64_t n, const int *perm, const AssembleArgs &a, c
                             int64_t &launches)
 {
     if (n <= 0 || a.nout <= 0) return cudaSuccess;
-    k_assemble<<<grid_for(n, 256), 256, 0, st>>>(n, perm, a);
+    launch_chained(k_assemble, grid_for(n, 256), 256, 0, st, n, perm, a);
     launches++;
     return cudaGetLastError();
 }
@@ -3445,7 +3463,7 @@ cudaError_t launch_sorted_pair(int64_t n, const int *perm, const double2 *a, con
                                double *out, float2 *ff, cudaStream_t st, int64_t &launches)
 {
     if (n <= 0) return cudaSuccess;
-    k_sorted_pair<<<grid_for(n, 256), 256, 0, st>>>(n, perm, a, b, out, ff);
+    launch_chained(k_sorted_pair, grid_for(n, 256), 256, 0, st, n, perm, a, b, out, ff);
     launches++;
     return cudaGetLastError();
 }
@@ -3479,7 +3497,7 @@ cudaError_t launch_real_adj(const RealArgs &args, bool slp, bool dlp, cudaStream
 cudaError_t launch_filter_adj(const FilterArgs &a, cudaStream_t st, int64_t &launches)
 {
     const int64_t n = (int64_t)a.Mx * (a.My / 2 + 1);
-    k_filter_adj<<<grid_for(n, 256), 256, 0, st>>>(a);
+    launch_chained(k_filter_adj, grid_for(n, 256), 256, 0, st, a);
     launches++;
     return cudaGetLastError();
 }
@@ -3538,11 +3556,11 @@ cudaError_t launch_adj_assemble(int64_t n, const int *perm, const double *gr, co
 {
     if (dlp) {
         k_wsum_part<<<kZeroModeParts, 256, 0, st>>>(nt, w, 4, 2, part);
-        k_wsum_final<<<1, 32, 0, st>>>(kZeroModeParts, part);
+        launch_chained(k_wsum_final, 1, 32, 0, st, kZeroModeParts, part);
         launches += 2;
     }
     if (n > 0) {
-        k_adj_assemble<<<grid_for(n, 256), 256, 0, st>>>(n, perm, gr, gk, part + kZeroModeParts,
+        launch_chained(k_adj_assemble, grid_for(n, 256), 256, 0, st, n, perm, gr, gk, part + kZeroModeParts,
                                                          praw, fd, nrm, inv_area, slp, dlp,
                                                          g_pos, g_fs, g_fd, g_n);
         launches++;
@@ -3581,11 +3599,11 @@ cudaError_t launch_spread_bound(const SpreadArgs &a, int nc, double kfac, int mu
     unsigned long long *bound = reinterpret_cast<unsigned long long *>(ws + 2 * nb);
     int *cnt = reinterpret_cast<int *>(ws + 2 * nb + 1), *tc = cnt + nb;
     if (a.ns > 0) {
-        k_spread_bin_sum<<<stream_grid(a.ns), 256, 0, st>>>(a, nc, ax.nb, ay.nb, bins, cnt, bound);
+        launch_chained(k_spread_bin_sum, stream_grid(a.ns), 256, 0, st, a, nc, ax.nb, ay.nb, bins, cnt, bound);
         launches++;
     }
-    k_bound_x<<<stream_grid(nb), 256, 0, st>>>(bins, cnt, ax, ay.nb, t, tc);
-    k_bound_y_max<<<stream_grid(nb), 256, 0, st>>>(t, tc, ay, ax.nb, kfac, mult, bound);
+    launch_chained(k_bound_x, stream_grid(nb), 256, 0, st, bins, cnt, ax, ay.nb, t, tc);
+    launch_chained(k_bound_y_max, stream_grid(nb), 256, 0, st, t, tc, ay, ax.nb, kfac, mult, bound);
     launches += 2;
     return cudaGetLastError();
 }
@@ -3613,13 +3631,13 @@ cudaError_t launch_gather_fp64_fallback(const GatherArgs &a, int nc, cudaStream_
     unsigned g = grid_for(a.nt, 256);
     if (g > (unsigned)sm_count()) g = (unsigned)sm_count();
     if (nc == 2) {
-        if (a.P == 24) k_gather<2, 24><<<g, 256, 0, st>>>(a);
-        else if (a.P == 12) k_gather<2, 12><<<g, 256, 0, st>>>(a);
-        else k_gather<2, 0><<<g, 256, 0, st>>>(a);
+        if (a.P == 24) launch_chained(k_gather<2, 24>, g, 256, 0, st, a);
+        else if (a.P == 12) launch_chained(k_gather<2, 12>, g, 256, 0, st, a);
+        else launch_chained(k_gather<2, 0>, g, 256, 0, st, a);
     } else {
-        if (a.P == 24) k_gather<4, 24><<<g, 256, 0, st>>>(a);
-        else if (a.P == 12) k_gather<4, 12><<<g, 256, 0, st>>>(a);
-        else k_gather<4, 0><<<g, 256, 0, st>>>(a);
+        if (a.P == 24) launch_chained(k_gather<4, 24>, g, 256, 0, st, a);
+        else if (a.P == 12) launch_chained(k_gather<4, 12>, g, 256, 0, st, a);
+        else launch_chained(k_gather<4, 0>, g, 256, 0, st, a);
     }
     launches++;
     return cudaGetLastError();
@@ -3728,7 +3746,7 @@ cudaError_t launch_grid_to_fixed(double *grid, int nout, int64_t G, const unsign
 {
     if (nout <= 0) return cudaSuccess;
     const dim3 grd(stream_grid(G), (unsigned)nout);
-    k_grid_to_fixed<<<grd, 256, 0, st>>>(grid, G, gmax, Bg);
+    launch_chained(k_grid_to_fixed, grd, 256, 0, st, grid, G, gmax, Bg);
     launches++;
     return cudaGetLastError();
 }
@@ -3754,7 +3772,7 @@ cudaError_t launch_split_half_spectra_t(const double2 *z, int nc, int Mx, int My
 {
     const int H1 = My / 2 + 1;
     const dim3 g((H1 + kTT - 1) / kTT, (Mx + kTT - 1) / kTT, (nc + 1) / 2);
-    k_split_half_spectra_t<<<g, 256, 0, st>>>(z, nc, Mx, My, specT, fold && (nc & 1) ? 1 : 0);
+    launch_chained(k_split_half_spectra_t, g, 256, 0, st, z, nc, Mx, My, specT, fold && (nc & 1) ? 1 : 0);
     launches++;
     return cudaGetLastError();
 }
@@ -3763,7 +3781,7 @@ cudaError_t launch_join_half_spectra_t(const double2 *specT, int nout, int Mx, i
                                        cudaStream_t st, int64_t &launches)
 {
     const dim3 g((My + kTT - 1) / kTT, (Mx + kTT - 1) / kTT, (nout + 1) / 2);
-    k_join_half_spectra_t<<<g, 256, 0, st>>>(specT, nout, Mx, My, z);
+    launch_chained(k_join_half_spectra_t, g, 256, 0, st, specT, nout, Mx, My, z);
     launches++;
     return cudaGetLastError();
 }

@@ -181,6 +181,7 @@ __device__ __forceinline__ void tc_seed(unsigned long long u, unsigned long long
 // divisions and conversions in FP64 it took 310 us for 2^20 points, bound by the FP64 pipe.
 __global__ void __launch_bounds__(256) k_tc_points(TcPrepArgs b)
 {
+    chain_enter();
     const TcPointArgs &a = b.s[blockIdx.y].a;
     __shared__ unsigned long long tab[256];
     tab[threadIdx.x] = c_exp2_tab[threadIdx.x];
@@ -223,6 +224,7 @@ __global__ void __launch_bounds__(256) k_tc_points(TcPrepArgs b)
 // them itself (23 blocks at 2688^2 nodes: 4 us; one block over all of them, 30 us).
 __global__ void __launch_bounds__(1024) k_tc_items(TcPrepArgs b)
 {
+    chain_enter();
     const TcSetArgs &t = b.s[blockIdx.y];
     const int *__restrict__ count = t.a.count;
     const int ntile = t.ntile, kmax = t.kmax;
@@ -281,6 +283,7 @@ __global__ void __launch_bounds__(1024) k_tc_items(TcPrepArgs b)
 // points' numbers in the caller's order, by slot (with perm).
 __global__ void __launch_bounds__(256) k_tc_list(TcPrepArgs b)
 {
+    chain_enter();
     const TcSetArgs &w = b.s[blockIdx.y];
     const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= w.a.n) return;
@@ -307,6 +310,7 @@ __global__ void __launch_bounds__(256) k_tc_order(int64_t n, const int2 *__restr
                                                   int *__restrict__ out,
                                                   const unsigned long long *__restrict__ bound)
 {
+    chain_enter();
     if (*bound == kFixedOff) return;                 // crowded: the FP64 spread runs instead
     __shared__ __align__(16) int ks[256];
     __shared__ int range[2];
@@ -581,6 +585,7 @@ static int tc_spread_smem(int NS, int P)
 template <int NC, int NS>
 __global__ void __launch_bounds__(kTcThreads, 2) k_spread_tc(TcSpreadArgs a)
 {
+    chain_enter();
     constexpr int NG = (NC + 1) / 2;
     constexpr int kBK = NS * (kTcY / 8) * 128;       // B: bytes per 8 sources
     extern __shared__ __align__(128) char tc_smem[];
@@ -963,6 +968,7 @@ __device__ __forceinline__ void store_digits_signed4(const long long (&v)[4], ch
 template <int NC>
 __global__ void __launch_bounds__(kTcThreads, 2) k_gather_tc(TcGatherArgs a)
 {
+    chain_enter();
     extern __shared__ __align__(128) char tc_smem[];
     if (gmax_all(a.gmax) >= kGridNonFinite) return;  // the FP64 gather runs instead
     const int nv = *a.nitems;
@@ -1230,6 +1236,7 @@ constexpr int kGaSmem = kGaA + 2 * kTgB + kTgXs + (int)sizeof(GaSmem) + 128;
 
 __global__ void __launch_bounds__(kGaThreads, 1) k_gather_adj_tc(TcGatherAdjArgs a)
 {
+    chain_enter();
     extern __shared__ __align__(128) char tc_smem[];
     if (gmax_all(a.gmax) >= kGridNonFinite) return;  // the FP64 gather runs instead
     const int nv = *a.nitems;
@@ -1487,25 +1494,21 @@ __global__ void __launch_bounds__(kGaThreads, 1) k_gather_adj_tc(TcGatherAdjArgs
 cudaError_t launch_tc_points(const TcPrepArgs &b, int nset, const unsigned long long *bound,
                              cudaStream_t st, int64_t &launches)
 {
-    // (the sets' counts are one array)
     int64_t n = 0;
-    int ntile = 0, total = 0;
+    int ntile = 0;
     for (int k = 0; k < nset; k++) {
         n = b.s[k].a.n > n ? b.s[k].a.n : n;
         ntile = b.s[k].ntile > ntile ? b.s[k].ntile : ntile;
-        total += b.s[k].ntile;
     }
-    const cudaError_t e = cudaMemsetAsync(b.s[0].a.count, 0, sizeof(int) * (size_t)total, st);
-    if (e != cudaSuccess) return e;
     const dim3 g((unsigned)((n + 255) / 256), nset);
-    if (n > 0) k_tc_points<<<g, 256, 0, st>>>(b);
-    k_tc_items<<<dim3((ntile + 1023) / 1024, nset), 1024, 0, st>>>(b);
-    if (n > 0) k_tc_list<<<g, 256, 0, st>>>(b);
+    if (n > 0) launch_chained(k_tc_points, g, 256, 0, st, b);
+    launch_chained(k_tc_items, dim3((ntile + 1023) / 1024, nset), 1024, 0, st, b);
+    if (n > 0) launch_chained(k_tc_list, g, 256, 0, st, b);
     launches += n > 0 ? 3 : 1;
     for (int k = 0; k < nset; k++) {
         const TcSetArgs &t = b.s[k];
         if (t.perm && t.a.n > 0) {
-            k_tc_order<<<(unsigned)((t.a.n + 255) / 256), 256, 0, st>>>(t.a.n, t.a.tile, t.start, t.kmax, t.key,
+            launch_chained(k_tc_order, (unsigned)((t.a.n + 255) / 256), 256, 0, st, t.a.n, t.a.tile, t.start, t.kmax, t.key,
                                                                        t.list, t.ordered, bound);
             launches++;
         }
@@ -1520,7 +1523,7 @@ static cudaError_t spread_tc(const TcSpreadArgs &a, cudaStream_t st)
     const cudaError_t e =
         cudaFuncSetAttribute(k_spread_tc<NC, NS>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e != cudaSuccess) return e;
-    k_spread_tc<NC, NS><<<2 * sm_count(), kTcThreads, bytes, st>>>(a);
+    launch_chained(k_spread_tc<NC, NS>, 2 * sm_count(), kTcThreads, bytes, st, a);
     return cudaGetLastError();
 }
 
@@ -1541,7 +1544,7 @@ static cudaError_t gather_tc(const TcGatherArgs &a, cudaStream_t st)
     const cudaError_t e =
         cudaFuncSetAttribute(k_gather_tc<NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTgSmem);
     if (e != cudaSuccess) return e;
-    k_gather_tc<NC><<<2 * sm_count(), kTcThreads, kTgSmem, st>>>(a);
+    launch_chained(k_gather_tc<NC>, 2 * sm_count(), kTcThreads, kTgSmem, st, a);
     return cudaGetLastError();
 }
 
@@ -1556,7 +1559,7 @@ cudaError_t launch_gather_adj_tc(const TcGatherAdjArgs &a, cudaStream_t st, int6
     const cudaError_t e =
         cudaFuncSetAttribute(k_gather_adj_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, kGaSmem);
     if (e != cudaSuccess) return e;
-    k_gather_adj_tc<<<sm_count(), kGaThreads, kGaSmem, st>>>(a);
+    launch_chained(k_gather_adj_tc, sm_count(), kGaThreads, kGaSmem, st, a);
     launches++;
     return cudaGetLastError();
 }
