@@ -333,8 +333,9 @@ __device__ __forceinline__ double rcp_nr(double a)
 // The scan is issue-bound like the rest of the kernel (about a third of its instructions):
 // what a candidate's test needs is the same for a piece, and the cutoff's error band for a
 // point.  With a band, an image lookup and a search of nine boxes per candidate instead,
-// k_real took 2.15 ms on 2^16 points by circles (now 1.84) and k_real_adj 3.5 ms at 2^18
-// points (now 3.07).
+// k_real took 2.15 ms on 2^16 points by circles (then 1.84) and k_real_adj 3.5 ms at 2^18
+// points (then 3.07); with the common case free of divergent branches, the exact tests
+// behind one vote, 1.68 and 2.03 (2^20 uniform points 4.20 -> 4.06 ms).
 struct Nbhd {
     int4 seg[9];                // first point and end of the piece, image code
     float2 z[9];                // the piece's image shift, rounded, to take off the outer point
@@ -766,11 +767,13 @@ struct PairQueue {
     float2 h1, h2, k1, k2; // float-float sums of the FP64 form's far pairs
 };
 
-#ifndef SE2P_REAL_MINB
-#define SE2P_REAL_MINB 6
-#endif
+// Blocks of k_real per SM (the launch bound): 24 warps at 80 registers, and for the
+// double layer alone in float-float 28 at 72 (2^16 points by circles 1.92 ms against
+// 2.03; both kinds 11.15 against 11.16 ms at 2^20 points, FP32-grid form 3.88 against
+// 3.81, where the registers no longer hold a pair).
+constexpr int real_blocks(bool slp, int form) { return !slp && form == kFormFF ? 7 : 6; }
 template <bool SLP, bool DLP, int FORM>
-__global__ void __launch_bounds__(kRealWarps * 32, SE2P_REAL_MINB) k_real(RealArgs a)
+__global__ void __launch_bounds__(kRealWarps * 32, real_blocks(SLP, FORM)) k_real(RealArgs a)
 {
     constexpr bool MIXED = FORM == kFormF32;
     constexpr bool FF = FORM == kFormFF;
@@ -898,6 +901,7 @@ __global__ void __launch_bounds__(kRealWarps * 32, SE2P_REAL_MINB) k_real(RealAr
     const int64_t len = (int64_t)kRealWarps * a.run;
     if (lane == 0) W.nb.box = -1;
     __syncwarp();
+    const bool counting = a.counters;
     for (int64_t t0 = (int64_t)blockIdx.x * len; t0 < a.ntar; t0 = run_s * len) {
         const int t_end = (int)min(t0 + len, a.ntar);
         for (int t = (int)t0 + wid; t < t_end; t += kRealWarps) {
@@ -930,17 +934,18 @@ __global__ void __launch_bounds__(kRealWarps * 32, SE2P_REAL_MINB) k_real(RealAr
                 const Piece C(W.nb, q, base);
                 for (int s0 = C.begin; s0 < C.end; s0 += 32) {
                     const int s = s0 + lane;
+                    const float2 Sf = a.spf[min(s, C.end - 1)];
+                    const float dxf = Sf.x - C.ox, dyf = Sf.y - C.oy;
+                    float r2f = dxf * dxf + dyf * dyf;
+                    const bool act = s < C.end, own = (unsigned)(s - C.own0) < C.ownn;
+                    bool in = act && r2f > 0.f && r2f < (own ? INFINITY : cut.x);
                     int y = C.ey;
-                    bool in = false, nearp = false;
-                    if (s < C.end) {
-                        const float2 Sf = a.spf[s];
-                        const float dxf = Sf.x - C.ox, dyf = Sf.y - C.oy;
-                        float r2f = dxf * dxf + dyf * dyf;
-                        const bool own = (unsigned)(s - C.own0) < C.ownn;
-                        in = r2f > 0.f && r2f < (own ? INFINITY : cut.x);
-                        if (!in && (own || !(r2f >= cut.y))) {
+                    // (rare)
+                    const bool odd = act && !in && (own || !(r2f >= cut.y));
+                    if (__any_sync(~0u, odd)) {
+                        if (odd) {
                             const double2 S = a.sp[s], T = W.tpos[slot];
-                            y = base & 0xff | C.ey & 0xf00;
+                            y = (base & 0xff) | (C.ey & 0xf00);
                             if (own) {
                                 // own box.  Distinct FP32 images imply an FP64 r2 > 0 (the
                                 // offset is then >= 2^-150, its square normal), so only
@@ -974,24 +979,29 @@ __global__ void __launch_bounds__(kRealWarps * 32, SE2P_REAL_MINB) k_real(RealAr
                             }
                             in = y >> 12;
                         }
-                        nearp = !(r2f > rlo && r2f < rhi);
+                        __syncwarp();
                     }
-                    if (a.counters) {                        // (warp-uniform)
+                    const bool far = r2f > rlo && r2f < rhi;
+                    if (counting) {                          // (warp-uniform)
                         nslp += __popc(__ballot_sync(~0u, in && (y & 0x1000)));
                         ndlp += __popc(__ballot_sync(~0u, in && (y & 0x2000)));
                     }
                     const unsigned below = (1u << lane) - 1u;
-                    const unsigned m0 = __ballot_sync(~0u, in && !nearp), m1 = __ballot_sync(~0u, in && nearp);
-                    if (in && !nearp) W.q[0][(Q[0].enq + __popc(m0 & below)) & 63] = make_int2(s, y);
+                    const unsigned m0 = __ballot_sync(~0u, in && far), m1 = __ballot_sync(~0u, in && !far);
+                    if (in && far) W.q[0][(Q[0].enq + __popc(m0 & below)) & 63] = make_int2(s, y);
                     Q[0].enq += __popc(m0);
                     if (m1) {                                // (warp-uniform)
-                        if (in && nearp) W.q[1][(Q[1].enq + __popc(m1 & below)) & 63] = make_int2(s, y);
+                        if (in && !far) W.q[1][(Q[1].enq + __popc(m1 & below)) & 63] = make_int2(s, y);
                         Q[1].enq += __popc(m1);
-                        __syncwarp();
-                        if (Q[1].enq - Q[1].proc >= 32) batch(1, 32);
+                        if (Q[1].enq - Q[1].proc >= 32) {
+                            __syncwarp();
+                            batch(1, 32);
+                        }
                     }
-                    __syncwarp();
-                    if (Q[0].enq - Q[0].proc >= 32) batch(0, 32);
+                    if (Q[0].enq - Q[0].proc >= 32) {
+                        __syncwarp();
+                        batch(0, 32);
+                    }
                 }
             }
             if (lane == 0) {
@@ -1278,7 +1288,7 @@ __device__ __forceinline__ void adj_pair_ff(const RealArgs &a, const AdjWarp &W,
 }
 
 template <bool SLP, bool DLP, int FORM>
-__global__ void __launch_bounds__(kAdjWarps * 32, 5) k_real_adj(RealArgs a)
+__global__ void __launch_bounds__(kAdjWarps * 32, 4) k_real_adj(RealArgs a)
 {
     constexpr bool FF = FORM == kFormFF;
     __shared__ AdjWarp warps[kAdjWarps];
@@ -1404,17 +1414,18 @@ __global__ void __launch_bounds__(kAdjWarps * 32, 5) k_real_adj(RealArgs a)
             }
             for (int t0 = C.begin; t0 < C.end; t0 += 32) {
                 const int t = t0 + lane;
+                float2 Tf = make_float2(0.f, 0.f);
+                if (!dr) Tf = a.tpf[min(t, C.end - 1)];
+                const float dxf = Tf.x - C.ox, dyf = Tf.y - C.oy;
+                float r2f = dxf * dxf + dyf * dyf;
+                const bool act = !dr && t < C.end, own = (unsigned)(t - C.own0) < C.ownn;
+                bool in = act && r2f > 0.f && r2f < (own ? INFINITY : cut.x);
                 int y = C.ey;
-                bool in = false, nearp = false;
-                if (!dr && t < C.end) {
-                    const float2 Tf = a.tpf[t];
-                    const float dxf = Tf.x - C.ox, dyf = Tf.y - C.oy;
-                    float r2f = dxf * dxf + dyf * dyf;
-                    const bool own = (unsigned)(t - C.own0) < C.ownn;
-                    in = r2f > 0.f && r2f < (own ? INFINITY : cut.x);
-                    if (!in && (own || !(r2f >= cut.y))) {
+                const bool odd = act && !in && (own || !(r2f >= cut.y));
+                if (__any_sync(~0u, odd)) {
+                    if (odd) {
                         const double2 T = a.tp[t], Sp = W.pos[slot];
-                        y = base & 0xff | C.ey & 0xf00;
+                        y = (base & 0xff) | (C.ey & 0xf00);
                         if (own) {
                             const double dx = xsub(T.x, Sp.x), dy = xsub(T.y, Sp.y);
                             const double r2 = xadd(xmul(dx, dx), xmul(dy, dy));
@@ -1444,19 +1455,22 @@ __global__ void __launch_bounds__(kAdjWarps * 32, 5) k_real_adj(RealArgs a)
                         }
                         in = y >> 12;
                     }
-                    nearp = !(r2f > rlo && r2f < rhi);
+                    __syncwarp();
                 }
+                const bool far = r2f > rlo && r2f < rhi;
                 const unsigned below = (1u << lane) - 1u;
-                const unsigned m0 = __ballot_sync(~0u, in && !nearp), m1 = __ballot_sync(~0u, in && nearp);
-                if (in && !nearp) W.q[0][(enq[0] + __popc(m0 & below)) & 63] = make_int2(t, y);
-                if (in && nearp) W.q[1][(enq[1] + __popc(m1 & below)) & 63] = make_int2(t, y);
+                const unsigned m0 = __ballot_sync(~0u, in && far), m1 = __ballot_sync(~0u, in && !far);
+                if (in && far) W.q[0][(enq[0] + __popc(m0 & below)) & 63] = make_int2(t, y);
+                if (in && !far) W.q[1][(enq[1] + __popc(m1 & below)) & 63] = make_int2(t, y);
                 enq[0] += __popc(m0);
                 enq[1] += __popc(m1);
-                __syncwarp();
 #pragma unroll
                 for (int j = 0; j < 2; j++) {
                     const int n = (int)(enq[j] - proc[j]);
-                    if (dr || n >= 32) batch(j, min(n, 32));
+                    if (dr || n >= 32) {
+                        __syncwarp();
+                        batch(j, min(n, 32));
+                    }
                 }
             }
         }
@@ -3353,12 +3367,11 @@ cudaError_t launch_real(const RealArgs &args, bool slp, bool dlp, cudaStream_t s
     if (args.ntar <= 0) return cudaSuccess;
     RealArgs a = args;
     const int64_t want = (a.ntar + kRealWarps - 1) / kRealWarps;
-    // Six 4-warp blocks per SM (the launch bound holds 80 registers: 24 warps
-    // resident), persistent over the sorted targets.  The k-space chain
-    // (high-priority stream) takes what is left.  With 8-warp blocks at 94
+    // Persistent blocks of 4 warps, as many as are resident (real_blocks).  The k-space
+    // chain (high-priority stream) takes what is left.  With 8-warp blocks at 94
     // registers only 16 warps fitted: 19.9 ms per evaluation at 2^20 points,
     // against 18.6 with 20 warps and 18.45 with 24.
-    const int64_t cap = (int64_t)sm_count() * SE2P_REAL_MINB;
+    const int64_t cap = (int64_t)sm_count() * real_blocks(slp, form);
     const unsigned g = (unsigned)(want < cap ? want : cap);
     a.run = real_run(a.ntar, a.ns, (int64_t)a.nx * a.ny, (int64_t)g * kRealWarps);
     if (form == kFormF32) launch_real_form<kFormF32>(a, slp, dlp, g, st);
@@ -3483,9 +3496,9 @@ cudaError_t launch_real_adj(const RealArgs &args, bool slp, bool dlp, cudaStream
     if (args.nouter <= 0) return cudaSuccess;
     RealArgs a = args;
     const int64_t want = (a.nouter + kAdjWarps - 1) / kAdjWarps;
-    // as many 4-warp blocks as fit at once (5 per SM at the launch bound), so
-    // that no second wave of persistent blocks trails the first
-    const int64_t cap = (int64_t)sm_count() * 5;
+    // as many 4-warp blocks as fit at once: 4 per SM at 128 registers (a gradient of
+    // 2^18 points 6.95 ms, 7.01 with 5, whose 96 registers do not hold a pair)
+    const int64_t cap = (int64_t)sm_count() * 4;
     const unsigned g = (unsigned)(want < cap ? want : cap);
     a.run = real_run(a.nouter, a.ntar, (int64_t)a.nx * a.ny, (int64_t)g * kAdjWarps);
     if (form == kFormFF) launch_real_adj_form<kFormFF>(a, slp, dlp, g, st);
