@@ -229,6 +229,40 @@ __device__ __forceinline__ float2 ff_add_f(float2 a, float b)
     return make_float2(h, l);
 }
 
+// a + b with b a float, |a.x| >= |b|.
+__device__ __forceinline__ float2 ff_add_small_f(float2 a, float b)
+{
+    float s, e;
+    fast_two_sum(a.x, b, s, e);
+    e += a.y;
+    float h, l;
+    fast_two_sum(s, e, h, l);
+    return make_float2(h, l);
+}
+
+// c + a b for |c| well above |a b| (a Horner step of a local expansion).
+__device__ __forceinline__ float2 ff_horner(float2 c, float2 a, float2 b)
+{
+    const float p = a.x * b.x;
+    float e = fmaf(a.x, b.x, -p);
+    e = fmaf(a.x, b.y, e);
+    e = fmaf(a.y, b.x, e);
+    float s, t, h, l;
+    fast_two_sum(c.x, p, s, t);
+    fast_two_sum(s, t + (e + c.y), h, l);
+    return make_float2(h, l);
+}
+__device__ __forceinline__ float2 ff_horner_f(float2 c, float2 a, float b)
+{
+    const float p = a.x * b;
+    float e = fmaf(a.x, b, -p);
+    e = fmaf(a.y, b, e);
+    float s, t, h, l;
+    fast_two_sum(c.x, p, s, t);
+    fast_two_sum(s, t + (e + c.y), h, l);
+    return make_float2(h, l);
+}
+
 // 1/a: the correctly rounded float reciprocal of the head, then one Newton
 // step r + r (1 - a r) with the residual formed by FMAs (relative error
 // about 2^-47).
@@ -261,16 +295,16 @@ __device__ __forceinline__ float2 ff_exp_neg(float2 x, const float2 *tab)
     float s, e;
     two_sum(t1, -p2, s, e);
     e += (x.y - e2) - kd * C3;
-    float rh, rl;
-    two_sum(s, e, rh, rl);
+    float rh, rl;                                    // (near r = 0 inexact by an ulp of e < 2^-30)
+    fast_two_sum(s, e, rh, rl);
     const float q = fmaf(fmaf(rh, 1.0f / 120.0f, -1.0f / 24.0f), rh, 1.0f / 6.0f);
     const float t3 = rh * rh * rh * q;
     const float p = rh * rh;
     float pe = fmaf(rh, rh, -p);
     pe = fmaf(2.0f * rh, rl, pe);
     float s1, e1, s2, e2b;
-    two_sum(1.0f, -rh, s1, e1);
-    two_sum(s1, 0.5f * p, s2, e2b);
+    fast_two_sum(1.0f, -rh, s1, e1);
+    fast_two_sum(s1, 0.5f * p, s2, e2b);
     const float lo = (e1 + e2b) + ((0.5f * pe - rl) - t3);
     float h, l;
     fast_two_sum(s2, lo, h, l);

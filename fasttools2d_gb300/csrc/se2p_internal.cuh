@@ -773,10 +773,12 @@ __device__ __forceinline__ float2 ff_g_e1(float2 x, const float4 *__restrict__ g
     const float4 *cf = gtab + 3 * (oct * kGPiecesPerOctave + m);
     const float4 A = __ldg(cf), B = __ldg(cf + 1), C = __ldg(cf + 2);
     const float t = fmaf(fmaf(C.z, dh, C.y), dh, C.x);
-    float2 p = ff_add(make_float2(B.z, B.w), ff_mul_f(d, t));
-    p = ff_add(make_float2(B.x, B.y), ff_mul(p, d));
-    p = ff_add(make_float2(A.z, A.w), ff_mul(p, d));
-    return ff_add(make_float2(A.x, A.y), ff_mul(p, d));
+    // (|d| <= x / 128, and each coefficient is about x times the next: the sums need no
+    // TwoSum; with the same in ff_exp_neg k_real 4.06 -> 3.98 ms at 2^20 points)
+    float2 p = ff_horner_f(make_float2(B.z, B.w), d, t);
+    p = ff_horner(make_float2(B.x, B.y), p, d);
+    p = ff_horner(make_float2(A.z, A.w), p, d);
+    return ff_horner(make_float2(A.x, A.y), p, d);
 }
 
 }  // namespace se2p

@@ -744,7 +744,7 @@ __device__ __forceinline__ void real_pair_ff(const RealArgs &a, const RealWarp &
         const float2 *Sc = cf + a.doff_ff;
         const float2 S11 = Sc[0], S1221 = Sc[1], S22 = Sc[2], tr = Sc[3];
         // with q = grad (x.S x), 2 Q = x.q: fb Q x + pf A = (fb Q + pf tr) x + pf q
-        const float2 fbh = ff_scale(ff_mul(ff_add_f(x, 1.0f), ff_sqr(ir2)), -2.0f);
+        const float2 fbh = ff_scale(ff_mul(ff_add_small_f(x, 1.0f), ff_sqr(ir2)), -2.0f);
         const float2 q1 = ff_dot2(S11, ff_scale(x1, 2.0f), S1221, x2);
         const float2 q2 = ff_dot2(S22, ff_scale(x2, 2.0f), S1221, x1);
         const float2 Q2 = ff_dot2(x1, q1, x2, q2);
@@ -1198,7 +1198,7 @@ __device__ __forceinline__ void adj_pair(const RealArgs &a, const AdjWarp &W, in
 // g[3] is kept without its 1/2.  966 FP32 operations per pair of both kinds (1500 in
 // float-float products and sums one by one), and the code is that much shorter, which
 // counts: the kernel waits for instructions.  k_real_adj at 2^18 points and 80
-// neighbours: 2.11 ms (3.07 before).
+// neighbours: 2.11 ms (3.07 before; 1.94 with the later changes of the scan and exp).
 template <bool SLP, bool DLP>
 __device__ __forceinline__ void adj_pair_ff(const RealArgs &a, const AdjWarp &W, int2 e,
                                             const float2 *tabff, float2 xi2, float2 pf, float2 pf2,
@@ -1249,7 +1249,7 @@ __device__ __forceinline__ void adj_pair_ff(const RealArgs &a, const AdjWarp &W,
         const float2 S11 = Sc[0], S1221 = Sc[1], S22 = Sc[2], tr = Sc[3];
         const float2 wd = ff_dot2(w1, x1, w2, x2);
         const float2 ir4 = ff_sqr(ir2);
-        const float2 fbh = ff_scale(ff_mul(ff_add_f(x, 1.0f), ir4), -2.0f);           // fb / 2
+        const float2 fbh = ff_scale(ff_mul(ff_add_small_f(x, 1.0f), ir4), -2.0f);           // fb / 2
         const float2 fbp = ff_scale(ff_mul(ff_add_f(x, 2.0f), ff_mul(ir4, ir2)), 4.0f);
         const float2 e1 = ff_scale(ff_mul(ex, ff_mul(fbh, wd)), 2.0f);
         // d(w.v)/dS
