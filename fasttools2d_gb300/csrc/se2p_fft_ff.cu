@@ -470,12 +470,14 @@ __device__ __forceinline__ float2 ff_split_scaled(double d, int e)
     return ff_split(__longlong_as_double(nb));
 }
 
-__global__ void __launch_bounds__(256, 2) k_fft_rows_ff(double2 *__restrict__ data, int64_t rows,
+constexpr int kFftThreads = 384;   // at most, 24 warps on an SM (80 registers)
+
+__global__ void __launch_bounds__(kFftThreads, 2) k_fft_rows_ff(double2 *__restrict__ data, int64_t rows,
                                                         FftRowsFF p, const float4 *__restrict__ tab)
 {
     chain_enter();
     extern __shared__ __align__(16) f2 fsh[];
-    __shared__ int emax_w[8];
+    __shared__ int emax_w[kFftThreads / 32];
     const int L = p.L, Lp = sh_len(L);
     const float sf = (float)p.sign;
     const f2 s = pk(-sf, sf);
@@ -670,11 +672,13 @@ cudaError_t launch_fft_rows_ff(double2 *data, int64_t rows, const FftRowsFF &p, 
     const int per_sm = (int)std::max<size_t>(1, (size_t)(200 * 1024) / (smem + 1024));
     const int64_t cap = (int64_t)sm_count() * per_sm;
     const unsigned g = (unsigned)(rows < cap ? rows : cap);
-    // The registers hold 512 threads on an SM: where the shared memory takes more than two
-    // rows, smaller blocks, so that one row's barriers are another's work (2^18 points,
-    // L = 1344: 7.43 ms per gradient with 256 threads, 7.14 with 128; L = 640: 50,000 points
-    // 733 us with 256, 694 with 128).
-    const int threads = per_sm >= 4 ? 128 : per_sm == 3 ? 160 : 256;
+    // 768 threads on an SM over the rows its shared memory holds, at least 128 a row, so
+    // that one row's barriers are another's work.  L = 1344 (four rows): a gradient of
+    // 2^18 points 7.43 ms with 256 threads at 16 warps per SM, 7.14 with 128, and at 24
+    // warps 6.89 with 128, 6.78 with 192, 7.20 with 256 (later code); L = 640: 50,000
+    // points 733, 694, then 650 us at 16 warps and 634 at 24; L = 2688 (two rows): 2^20
+    // points 10.97 ms with 256 threads at 16 warps, 10.92 with 384 at 24.
+    const int threads = std::max(128, std::min(kFftThreads, 768 / per_sm / 32 * 32));
     launch_chained(k_fft_rows_ff, g, threads, smem, st, data, rows, p, tw);
     launches++;
     return cudaGetLastError();
