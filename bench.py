@@ -72,22 +72,29 @@ UNIT = "evals/s"
 #   this run; peak = 128 FP32 lanes x SMs x the SM clock sampled in this run.
 #   Issue utilisation (warp instructions per evaluation, ncu) is reported
 #   beside it.
-# * spread (k_spread_fix, exact int64 sums): bound by L2 atomics; work = one
-#   64-bit reduction per stencil node and grid, (P+1)^2 C_in per source with
-#   C_in = 5 grids (SLP f1, f2; DLP S11, S12+S21, S22); peak = coalesced int64
-#   atomics measured in this run (se2p_plan_probe_atomics).
-# * gather (k_gather_fix, int64 sums of exact products): bound by issue and
-#   load latency; work = warp instructions per target (ncu).
+# * spread (k_spread_tc, exact integer sums on the tensor cores): each tile of
+#   stencil origins (40 x 8 at P = 24) adds its 64 x 32 node patch to the C_in = 5
+#   grids (SLP f1, f2; DLP S11, S12+S21, S22) by 64-bit L2 reductions; work = those;
+#   peak = coalesced int64 atomics measured in this run (se2p_plan_probe_atomics).
+#   The kernel is bound by the latency of a tile's phases, not by this rate.
+# * gather (k_gather_tc, the transposed contraction): bound by issue and the
+#   latency of a tile's phases; work = warp instructions per target (ncu).
 # * filter: FP64 FLOP against cuBLAS DGEMM.
 # DRAM bytes per launch are ncu's dram__bytes_read + _write of one launch
 # (profiles/).
 C_IN, C_OUT = 5, 4
-SPREAD_RED_PER_SOURCE = (P + 1) ** 2 * C_IN
+
+
+def spread_reductions():
+    """64-bit reductions of one spread (M may have been shrunk)."""
+    return -(-M // (64 - P)) * -(-M // (32 - P)) * 64 * 32 * C_IN
+
+
 FILTER_FLOP_PER_MODE = 60
-DRAM_BYTES = {"spread": 1.925e9, "gather": 0.281e9, "real": 0.213e9}
-REAL_WARP_INST_PER_PAIR = 39.7     # ncu smsp__inst_executed / SLP+DLP pair evaluations
-REAL_FP32_INST_PER_EVAL = 556.0    # ncu FADD 374 + FFMA 130 + FMUL 52 thread instructions per evaluation
-GATHER_WARP_INST_PER_TARGET = 1508.0   # ncu smsp__inst_executed / targets (k_gather_fix<4,24>)
+DRAM_BYTES = {"spread": 1.080e9, "gather": 0.755e9, "real": 0.171e9}
+REAL_WARP_INST_PER_PAIR = 31.1     # ncu smsp__inst_executed / SLP+DLP pair evaluations
+REAL_FP32_INST_PER_EVAL = 420.0    # ncu FADD 265 + FFMA 110 + FMUL 45 thread instructions per evaluation
+GATHER_WARP_INST_PER_TARGET = 476.0    # ncu smsp__inst_executed / targets (k_gather_tc<4>)
 # Algorithmic HBM bytes of one launch, each array read or written once:
 # real space reads per sorted source its position (16 B), FP32 copy (8 B), 5
 # FP64 coefficients and 7 float-float ones (96 B), and per target its
@@ -731,12 +738,12 @@ def gpu_arm(args, rank, world, local_rank):
     issue_src = "4 warp instructions per clock per SM x SMs x measured SM clock"
     fp32_peak = 128 * sms * clock_ghz * 1e9 / 1e12
     hbm, hbm_src = measured_hbm_gbs()
-    # the integer spread against the L2 atomic rate, whichever kernel is on top
+    # the spread's reductions against the L2 atomic rate, whichever kernel is on top
     spread_atomics = None
     if "spread" in per:
         red_peak = plan.probe_atomics()
-        red_done = N * SPREAD_RED_PER_SOURCE / (per["spread"] * 1e-3) / 1e9
-        spread_atomics = {"kernel": "k_spread_fix<5>", "achieved": red_done, "peak": red_peak,
+        red_done = spread_reductions() / (per["spread"] * 1e-3) / 1e9
+        spread_atomics = {"kernel": "k_spread_tc<5>", "achieved": red_done, "peak": red_peak,
                           "unit": "G int64 atomics/s", "frac": red_done / red_peak,
                           "ms_per_launch": per["spread"],
                           "hbm_side": {"traffic": DRAM_BYTES["spread"],
@@ -771,12 +778,12 @@ def gpu_arm(args, rank, world, local_rank):
                 "work": f"{REAL_FP32_INST_PER_EVAL:.0f} FP32 thread instructions (FADD+FFMA+FMUL, ncu) "
                         "per SLP+DLP pair evaluation x evaluations counted in this run"}
     elif top == "gather":
-        roof = {"kernel": "k_gather_fix<4,24> (integer gather, 4 grids)", "bound": "issue",
+        roof = {"kernel": "k_gather_tc<4> (tensor-core integer gather, 4 grids)", "bound": "issue",
                 "achieved": N * GATHER_WARP_INST_PER_TARGET / (top_ms * 1e-3) / 1e12,
                 "peak": issue_peak, "unit": "T warp-inst/s", "peak_source": issue_src}
     elif top == "spread":
-        roof = {"kernel": "k_spread_fix<5> (integer spread, 5 grids)", "bound": "l2_atomics",
-                "achieved": N * SPREAD_RED_PER_SOURCE / (top_ms * 1e-3) / 1e9,
+        roof = {"kernel": "k_spread_tc<5> (tensor-core integer spread, 5 grids)", "bound": "l2_atomics",
+                "achieved": spread_reductions() / (top_ms * 1e-3) / 1e9,
                 "peak": spread_atomics["peak"], "unit": "G int64 atomics/s",
                 "peak_source": "coalesced 64-bit integer atomics into an L2-resident array, "
                                "se2p_plan_probe_atomics in this run "

@@ -523,7 +523,7 @@ struct GatherArgsF {
 // every kernel of a chain waits before it does anything, completion stays in stream
 // order.  Small evaluations are a chain of 25 kernels of a few microseconds each
 // (1000 sources on themselves: 123 us, 164 without).  After a memset, a copy or an event
-// the launch is an ordinary one, and so it is on the default stream and under capture.
+// the launch is an ordinary one, and so it is on a default stream and under capture.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void chain_enter()
 {
@@ -544,7 +544,8 @@ inline void launch_chained(void (*k)(P...), dim3 grid, unsigned threads, size_t 
     c.dynamicSmemBytes = smem;
     c.stream = st;
     c.attrs = &at;
-    c.numAttrs = st && cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
+    c.numAttrs = st && st != cudaStreamLegacy && st != cudaStreamPerThread &&
+                 cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
     cudaLaunchKernelEx(&c, k, static_cast<P>(a)...);   // (an error stays for cudaGetLastError)
 }
 

@@ -7,7 +7,8 @@
 // default form runs in the narrowest arithmetic that keeps results within
 // 1e-12 of the reference: real-space far pairs in float-float on the FP32
 // pipe (near pairs, the self term and the cutoff decisions in FP64), the
-// spread and gather as exact int64 sums of rounded products, the filter in
+// spread and gather as exact integer sums (on the tensor cores, se2p_tc.cu, or
+// where few points share a grid tile by the int64 kernels here), the filter in
 // FP64.  The all-FP64 versions of these kernels serve the FP64_NATIVE form
 // and the fallbacks; they keep every FP64 warp instruction fully populated
 // (accepted pairs compacted before the Pade/exp work, a flattened (P+1)^2
