@@ -571,9 +571,19 @@ __device__ __forceinline__ void real_pair(const RealArgs &a, const RealWarp &W, 
     const int set = x >= 16.0 ? 0 : (x > 1.0 ? 1 : 2);
     const double *c = e1s + 22 * set;
     const double z = set == 2 ? x : ir2 * a.inv_xi2;
-    double pa = c[0], pb = c[1];
+    // (the far and the near set start with five zero pairs: near batches skip them)
+    double pa = 0.0, pb = 0.0;
+    if (__any_sync(__activemask(), set == 1)) {
+        pa = c[0];
+        pb = c[1];
 #pragma unroll
-    for (int i = 2; i < 22; i += 2) {
+        for (int i = 2; i < 10; i += 2) {
+            pa = fma(z, pa, c[i]);
+            pb = fma(z, pb, c[i + 1]);
+        }
+    }
+#pragma unroll
+    for (int i = 10; i < 22; i += 2) {
         pa = fma(z, pa, c[i]);
         pb = fma(z, pb, c[i + 1]);
     }
@@ -858,19 +868,28 @@ __global__ void __launch_bounds__(kRealWarps * 32, real_blocks(SLP, FORM)) k_rea
             P.tag = eseq;
         }
     };
-    // Retire finished targets in order (all of them after a full flush).
+    // Retire finished targets in order (all of them after a full flush), up to eight at
+    // once, four lanes each: their conversions run at the FP64 rate whatever lanes take
+    // part, so the loop leaves targets waiting while the ring has room (one target at a
+    // time, with all Horner steps for the near pairs: 3.98 against 3.87 ms at 2^20 points,
+    // FP32-grid form 2.20 against 2.02).
     auto retire = [&](bool all) {
-        while (nfl > 0 && (all || ((int)(Q[0].proc - W.tend[0][head]) >= 32 &&
-                                   (int)(Q[1].proc - W.tend[1][head]) >= 32))) {
-            if (lane < 4 && (lane < 2 ? SLP : DLP)) {
-                const int64_t t = W.tidx[head];
-                double v = W.acc[head][lane];
-                if (FF || MIXED) v += ff_to_double(W.accf[head][lane]);
-                double *u = reinterpret_cast<double *>(lane < 2 ? a.u_slp : a.u_dlp);
-                u[2 * t + (lane & 1)] = v;
+        while (nfl > (all ? 0 : kRing - 12)) {
+            const int g = lane >> 2, c = lane & 3, slot = (head + g) % kRing;
+            const bool done = g < nfl && (all || ((int)(Q[0].proc - W.tend[0][slot]) >= 32 &&
+                                                  (int)(Q[1].proc - W.tend[1][slot]) >= 32));
+            const unsigned m = __ballot_sync(~0u, done);
+            const int n = m == ~0u ? 8 : (__ffs(~m) - 1) >> 2;   // (the first that is not)
+            if (n == 0) break;
+            if (g < n && (c < 2 ? SLP : DLP)) {
+                const int64_t t = W.tidx[slot];
+                double v = W.acc[slot][c];
+                if (FF || MIXED) v += ff_to_double(W.accf[slot][c]);
+                double *u = reinterpret_cast<double *>(c < 2 ? a.u_slp : a.u_dlp);
+                u[2 * t + (c & 1)] = v;
             }
-            head = (head + 1) % kRing;
-            nfl--;
+            head = (head + n) % kRing;
+            nfl -= n;
         }
         __syncwarp();
     };
@@ -1137,9 +1156,18 @@ __device__ __forceinline__ void adj_pair(const RealArgs &a, const AdjWarp &W, in
         const int set = x >= 16.0 ? 0 : (x > 1.0 ? 1 : 2);
         const double *c = e1s + 22 * set;
         const double y = set == 2 ? x : ir2 * a.inv_xi2;
-        double pa = c[0], pb = c[1];
+        double pa = 0.0, pb = 0.0;                        // (as in real_pair)
+        if (__any_sync(__activemask(), set == 1)) {
+            pa = c[0];
+            pb = c[1];
 #pragma unroll
-        for (int i = 2; i < 22; i += 2) {
+            for (int i = 2; i < 10; i += 2) {
+                pa = fma(y, pa, c[i]);
+                pb = fma(y, pb, c[i + 1]);
+            }
+        }
+#pragma unroll
+        for (int i = 10; i < 22; i += 2) {
             pa = fma(y, pa, c[i]);
             pb = fma(y, pb, c[i + 1]);
         }
@@ -1352,16 +1380,21 @@ __global__ void __launch_bounds__(kAdjWarps * 32, 4) k_real_adj(RealArgs a)
             tag[j] = eseq;
         }
     };
-    auto retire = [&](bool all) {
-        while (nfl > 0 && (all || ((int)(proc[0] - W.tend[0][head]) >= 32 &&
-                                   (int)(proc[1] - W.tend[1][head]) >= 32))) {
-            if (lane < kAdjVals) {
-                double v = W.acc[head][lane];
-                if (FF) v += (lane == 3 ? 0.5 : 1.0) * ff_to_double(W.accf[head][lane]);
-                a.gout[kAdjVals * (int64_t)W.idx[head] + lane] = v;
+    auto retire = [&](bool all) {                          // (as in k_real, four at once)
+        while (nfl > (all ? 0 : kRing - 12)) {
+            const int g = lane >> 3, c = lane & 7, slot = (head + g) % kRing;
+            const bool done = g < nfl && (all || ((int)(proc[0] - W.tend[0][slot]) >= 32 &&
+                                                  (int)(proc[1] - W.tend[1][slot]) >= 32));
+            const unsigned m = __ballot_sync(~0u, done);
+            const int n = m == ~0u ? 4 : (__ffs(~m) - 1) >> 3;
+            if (n == 0) break;
+            if (g < n && c < kAdjVals) {
+                double v = W.acc[slot][c];
+                if (FF) v += (c == 3 ? 0.5 : 1.0) * ff_to_double(W.accf[slot][c]);
+                a.gout[kAdjVals * (int64_t)W.idx[slot] + c] = v;
             }
-            head = (head + 1) % kRing;
-            nfl--;
+            head = (head + n) % kRing;
+            nfl -= n;
         }
         __syncwarp();
     };
