@@ -441,6 +441,14 @@ struct Piece {
     }
 };
 
+// The E1 set of x >= 0: 0 from 16 on, 1 above 1, 2 to 1 (compared as bit patterns, which
+// order like the numbers: FP64 comparisons issue at the FP64 rate; NaN takes set 0 or 2).
+__device__ __forceinline__ int e1_set(double x)
+{
+    const long long b = __double_as_longlong(x);
+    return b >= 0x4030000000000000ll ? 0 : b > 0x3ff0000000000000ll ? 1 : 2;
+}
+
 struct RealWarp {
     int2 q[2][64];              // pair FIFOs: [0] main, [1] near field (x <= 1)
                                 // entry = (sorted source, slot | image code << 8 | flags << 12)
@@ -460,6 +468,7 @@ __device__ __forceinline__ void seg_flush(RealWarp &W, int lane, int key, double
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const int ko = __shfl_up_sync(~0u, key, o);
+        if (!__any_sync(~0u, lane >= o && ko == key)) break;   // (no longer segment)
         const double a0 = __shfl_up_sync(~0u, v0, o), a1 = __shfl_up_sync(~0u, v1, o);
         const double a2 = __shfl_up_sync(~0u, v2, o), a3 = __shfl_up_sync(~0u, v3, o);
         if (lane >= o && ko == key) {
@@ -568,7 +577,7 @@ __device__ __forceinline__ void real_pair(const RealArgs &a, const RealWarp &W, 
     const double ex = exp_neg(x, tab);
     const double ir2 = rcp_nr(r2);
     // E1 (unified Horner over the three Pade forms)
-    const int set = x >= 16.0 ? 0 : (x > 1.0 ? 1 : 2);
+    const int set = e1_set(x);
     const double *c = e1s + 22 * set;
     const double z = set == 2 ? x : ir2 * a.inv_xi2;
     // (the far and the near set start with five zero pairs: near batches skip them)
@@ -1088,6 +1097,7 @@ __device__ __forceinline__ void seg_flush_n(Acc &accs, int lane, int key, double
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const int ko = __shfl_up_sync(~0u, key, o);
+        if (!__any_sync(~0u, lane >= o && ko == key)) break;   // (no longer segment)
         double a[NV];
 #pragma unroll
         for (int i = 0; i < NV; i++) a[i] = __shfl_up_sync(~0u, v[i], o);
@@ -1153,7 +1163,7 @@ __device__ __forceinline__ void adj_pair(const RealArgs &a, const AdjWarp &W, in
         const double x = r2 * a.xi2;
         const double ex = exp_neg(x, tab);
         const double ir2 = rcp_nr(r2);
-        const int set = x >= 16.0 ? 0 : (x > 1.0 ? 1 : 2);
+        const int set = e1_set(x);
         const double *c = e1s + 22 * set;
         const double y = set == 2 ? x : ir2 * a.inv_xi2;
         double pa = 0.0, pb = 0.0;                        // (as in real_pair)
