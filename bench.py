@@ -92,7 +92,7 @@ def spread_reductions():
 
 FILTER_FLOP_PER_MODE = 60
 DRAM_BYTES = {"spread": 1.080e9, "gather": 0.755e9, "real": 0.171e9}
-REAL_WARP_INST_PER_PAIR = 31.1     # ncu smsp__inst_executed / SLP+DLP pair evaluations
+REAL_WARP_INST_PER_PAIR = 30.5     # ncu smsp__inst_executed / SLP+DLP pair evaluations
 REAL_FP32_INST_PER_EVAL = 420.0    # ncu FADD 265 + FFMA 110 + FMUL 45 thread instructions per evaluation
 GATHER_WARP_INST_PER_TARGET = 476.0    # ncu smsp__inst_executed / targets (k_gather_tc<4>)
 # Algorithmic HBM bytes of one launch, each array read or written once:
