@@ -24,7 +24,7 @@ from dataclasses import dataclass
 import numpy as np
 
 from . import _lib
-from .mex import _Arg, _Out, _bind_stream, _plan, _same_n
+from .mex import _Arg, _Out, _bind_stream, _interleaved, _plan, _same_n
 
 
 @dataclass
@@ -356,7 +356,7 @@ class Geometry:
             x = x[None]
         if x.ndim != 3 or x.shape[1] != 2 or x.shape[2] != self.ns:
             raise ValueError(f"{name} must be nrhs x 2 x nsrc")
-        buf = np.ascontiguousarray(np.transpose(x, (0, 2, 1)))
+        buf = _interleaved(x)
         return buf.ctypes.data, x.shape[0], buf
 
     def apply(self, f_slp=None, f_dlp=None):
