@@ -286,16 +286,16 @@ __global__ void k_sorted_pair(int64_t n, const int *__restrict__ perm,
 //
 // One warp walks a sequence of targets.  For each target the candidate
 // sources of its own box (every pair, no cutoff) and its 8 periodic
-// neighbour boxes (pairs with r2 < Lx*Ly/nside_x/nside_y) form one list,
-// scanned 32 at a time.  The cutoff test runs in FP32 with a rigorous
+// neighbour boxes (pairs with r2 < Lx*Ly/nside_x/nside_y), three rows of
+// consecutive boxes mostly, are scanned 32 at a time.  The cutoff test runs in FP32 with a rigorous
 // rounding-error band; only candidates inside the band take the reference's
 // exact FP64 test, separately for the SLP offset s-(t-z) and the DLP offset
 // (s-t)+z.  Accepted pairs go into a per-warp FIFO that carries over from one
 // target to the next, so the FP64 pair evaluation always runs on 32 lanes.
 // Each lane keeps register sums tagged with the target they belong to; when
-// its next pair is for a later target, the lanes flush with a segmented
-// warp reduction into a small ring of per-target accumulators, and a target
-// is written out once every lane has moved past it.
+// its next pair is for a later target, the lanes flush with a warp reduction
+// per target into a small ring of per-target accumulators, and targets that
+// every lane has moved past are written out several at a time.
 //
 // Per pair the SLP and DLP share one exp(-xi^2 r^2) (table-driven, Tang's
 // method) and one reciprocal 1/r2 (rcp.approx + Newton).  E1 uses the
