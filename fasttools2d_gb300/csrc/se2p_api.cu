@@ -2163,7 +2163,7 @@ static int geom_build(se2p_geom g, const double *psrc, const double *ptar, const
     CKS(ensure_t(pl, S_GTGT, nz, &tgt));
     CKS(ensure_t(pl, S_GMETA, nz, &meta));
     CK(cudaMemsetAsync(tgt, 0xff, sizeof(int) * nz, st));   // padding slots: tgt = -1
-    CK(launch_geom_rows(ra, g->slp, g->dlp, true, nullptr, g->slice, g->src, tgt, meta, st,
+    CK(launch_geom_rows(ra, g->slp, g->dlp, true, g->rowptr, g->slice, g->src, tgt, meta, st,
                         pl->launches));
     CK(launch_geom_coef(ra, g->slp, g->dlp, nslot, g->src, tgt, meta, g->cf, st, pl->launches));
     CK(cudaStreamSynchronize(st));
