@@ -684,9 +684,10 @@ static int tc_counts(se2p_plan pl, const SpreadArgs *sa, const GatherArgs *ga, c
 // (with sa, after tc_counts)
 // The sources' set for the spread and / or the points' of the gather, in the same
 // launches (a set of its own took 15 us more at small sizes: 1000 sources on themselves
-// 164 us with both at once, 182 without).
+// 164 us with both at once, 182 without).  The sources' set serves nbound right-hand
+// sides, whose bound slots are bstride words apart from sa->bound on.
 static int tc_prepare(se2p_plan pl, const SpreadArgs *sa, TcSet *ts, const GatherArgs *ga, TcSet *tt,
-                      cudaStream_t ks)
+                      cudaStream_t ks, int nbound = 1, int bstride = 0)
 {
     TcPrepArgs b{};
     int nset = 0;
@@ -699,7 +700,7 @@ static int tc_prepare(se2p_plan pl, const SpreadArgs *sa, TcSet *ts, const Gathe
         b.s[k].a.count = count;
         count += b.s[k].ntile;
     }
-    CK(launch_tc_points(b, nset, sa ? sa->bound : nullptr, ks, pl->launches));
+    CK(launch_tc_points(b, nset, sa ? sa->bound : nullptr, nbound, bstride, ks, pl->launches));
     return SE2P_OK;
 }
 
@@ -2282,7 +2283,7 @@ static int geom_kspace_multi(se2p_geom g, int nr, const double *coef, int64_t cs
         sa.bound = reinterpret_cast<const unsigned long long *>(ws + bslot);
         if (tc) {
             TcSet t;
-            CKS(tc_prepare(pl, &sa, &t, tg ? &ga : nullptr, &tset, ks));
+            CKS(tc_prepare(pl, &sa, &t, tg ? &ga : nullptr, &tset, ks, nr, (int)bstride));
             for (int r = 0; r < nr; r++) CKS(tc_spread(pl, rhs_spread(r), t, nc, ks));
         } else {
             CK(launch_spread_fix_multi(sa, nc, kY, nr, cstride, (int64_t)(nc * G), (int)bstride, ks,

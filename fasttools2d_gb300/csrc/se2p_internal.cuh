@@ -719,7 +719,7 @@ __device__ __forceinline__ int fix_shift(unsigned long long bits)
 // (list_tmp then holds 2 n ints).
 // (a.count of the sets zeroed before)
 cudaError_t launch_tc_points(const TcPrepArgs &b, int nset, const unsigned long long *bound,
-                             cudaStream_t st, int64_t &launches);
+                             int nbound, int bstride, cudaStream_t st, int64_t &launches);
 cudaError_t launch_gather_tc(const TcGatherArgs &a, int nc, cudaStream_t st, int64_t &launches);
 cudaError_t launch_gather_adj_tc(const TcGatherAdjArgs &a, cudaStream_t st, int64_t &launches);
 cudaError_t launch_spread_tc(const TcSpreadArgs &a, int nc, cudaStream_t st, int64_t &launches);

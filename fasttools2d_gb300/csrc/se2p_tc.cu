@@ -303,15 +303,20 @@ __global__ void __launch_bounds__(256) k_tc_list(TcPrepArgs b)
 // sums are exact, but each item's patch is rounded to the grid's unit once).
 // The other tiles keep the order the atomics gave them.  A block ranks 256
 // slots by counting smaller keys, the keys read through shared memory.
+// With nbound right-hand sides on the same sources the list serves them all, so it is
+// left unwritten only where none of their spreads will read it.
 __global__ void __launch_bounds__(256) k_tc_order(int64_t n, const int2 *__restrict__ tile,
                                                   const int *__restrict__ start, int kmax,
                                                   const int *__restrict__ key,
                                                   const int *__restrict__ list,
                                                   int *__restrict__ out,
-                                                  const unsigned long long *__restrict__ bound)
+                                                  const unsigned long long *__restrict__ bound,
+                                                  int nbound, int bstride)
 {
     chain_enter();
-    if (*bound == kFixedOff) return;                 // crowded: the FP64 spread runs instead
+    bool off = true;                                 // crowded: the FP64 spread runs instead
+    for (int r = 0; r < nbound; r++) off = off && bound[(int64_t)r * bstride] == kFixedOff;
+    if (off) return;
     __shared__ __align__(16) int ks[256];
     __shared__ int range[2];
     const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1492,7 +1497,7 @@ __global__ void __launch_bounds__(kGaThreads, 1) k_gather_adj_tc(TcGatherAdjArgs
 // Launchers
 // ---------------------------------------------------------------------------
 cudaError_t launch_tc_points(const TcPrepArgs &b, int nset, const unsigned long long *bound,
-                             cudaStream_t st, int64_t &launches)
+                             int nbound, int bstride, cudaStream_t st, int64_t &launches)
 {
     int64_t n = 0;
     int ntile = 0;
@@ -1509,7 +1514,7 @@ cudaError_t launch_tc_points(const TcPrepArgs &b, int nset, const unsigned long 
         const TcSetArgs &t = b.s[k];
         if (t.perm && t.a.n > 0) {
             launch_chained(k_tc_order, (unsigned)((t.a.n + 255) / 256), 256, 0, st, t.a.n, t.a.tile, t.start, t.kmax, t.key,
-                                                                       t.list, t.ordered, bound);
+                                                                       t.list, t.ordered, bound, nbound, bstride);
             launches++;
         }
     }
