@@ -608,9 +608,18 @@ struct TcSet {
     bool ready = false;
 };
 
+// Whether the points' records (tc_seed) can hold Gaussians of exponent alpha per node
+// spacing squared: alpha log2(e) in units of 2^-59 and its double in 64 bits, and
+// exp(-2 alpha) below 1 as a fraction of 2^62.  (The drivers' eta gives alpha = 5.67 / P;
+// eta is a free argument of the gateways.)
+static bool tc_alpha_ok(double alpha)
+{
+    return alpha * 1.4426950408889634074 < 15.99 && std::exp(-2.0 * alpha) < 1.0 - 0x1p-50;
+}
+
 // Whether the tensor-core spread runs.  It can for w = h P/2, where both axes'
-// factors are at most 1 (its weights are formed for that), grids of at least a
-// patch and stencils that leave a tile.  It costs about 24 ns per item and pair of
+// factors are at most 1 (its weights are formed for that), exponents that the points'
+// records hold, grids of at least a patch and stencils that leave a tile.  It costs about 24 ns per item and pair of
 // grids, an item holding at most a tile's sources; k_spread_fix about 0.1 ms and
 // 1.1 ns per source and grid: with few sources per tile the latter wins (2^16
 // sources, SLP: 0.59 against 0.25 ms on 2688^2 nodes, 0.20 against 0.23 ms on
@@ -618,7 +627,7 @@ struct TcSet {
 static bool tc_ok(const SpreadArgs &sa, int nc)
 {
     if (sa.P < 4 || sa.P > kTcMaxP || sa.Mx < kTcX || sa.My < kTcY ||
-        !(std::fabs(sa.w - sa.h * sa.P / 2) <= 1e-14 * sa.w))
+        !(std::fabs(sa.w - sa.h * sa.P / 2) <= 1e-14 * sa.w) || !tc_alpha_ok(-sa.a * sa.h * sa.h))
         return false;
     const double ntile = std::ceil((double)sa.Mx / (kTcX - sa.P)) * std::ceil((double)sa.My / (kTcY - sa.P));
     return 24.0 * ((nc + 1) / 2) * std::min(ntile, (double)sa.ns) <= 1e5 + 1.1 * nc * (double)sa.ns;
@@ -735,7 +744,7 @@ static int tc_spread(se2p_plan pl, const SpreadArgs &sa, const TcSet &t, int nc,
 static bool tg_ok(const GatherArgs &ga, int nout)
 {
     if (ga.P < 4 || ga.P > kTcMaxP || ga.Mx < kTgX || ga.My < kTgY ||
-        !(std::fabs(ga.w - ga.h * ga.P / 2) <= 1e-14 * ga.w))
+        !(std::fabs(ga.w - ga.h * ga.P / 2) <= 1e-14 * ga.w) || !tc_alpha_ok(-ga.a * ga.h * ga.h))
         return false;
     const double ntile = std::ceil((double)ga.Mx / (kTgX - ga.P)) * std::ceil((double)ga.My / (kTgY - ga.P));
     return (14.0 + 13.0 * nout) * std::min(ntile, (double)ga.nt) <= 2.5e5 + 0.35 * nout * nout * (double)ga.nt;
