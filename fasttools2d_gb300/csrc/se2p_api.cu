@@ -735,8 +735,29 @@ static int tc_spread(se2p_plan pl, const SpreadArgs &sa, const TcSet &t, int nc,
     return SE2P_OK;
 }
 
+// The scale of the tensor-core gathers' int64 grids: |g| below 2^61 (tg_sums_ok).
+constexpr int kTgBits = 61;
+
+// Whether the tensor-core gathers' 64-bit sums hold Gaussians of exponent alpha.  With
+// |g| below 2^kTgBits and S the largest sum of a stencil row's factors, the inner sums
+// V = sum_j Y_j g stay below 2^60 S and a target's sum of V X / 4 below 2^58 S^2: S^2
+// below 32 keeps both in 63 bits.  The adjoint's row of j Y holds |j Y| below 2; its
+// sums, below 2^58 sum |j Y| and for the x moment 2^55 S sum |i X|, are then far from
+// the end too (S is about sqrt(pi / alpha), sum |j Y| about 1 / alpha < 11).  The
+// drivers' alpha of 5.67 / P gives S = 3.65 at P = 24; the line lies at about 2.4 times
+// their eta there, 2.2 at P = 26 and 5 at P = 12, and the integer or float-float gathers
+// take what is flatter.
+static bool tg_sums_ok(double alpha, int P, bool adjoint)
+{
+    // (over all offsets of a point from its nodes the sum is largest on a node)
+    double S = 1.0, most = 0.0;
+    for (int k = 1; k <= P / 2 + 1; k++) S += 2.0 * std::exp(-alpha * k * k);
+    for (int k = 1; k <= P / 2; k++) most = std::max(most, k * std::exp(-alpha * (k - 1) * (k - 1)));
+    return S * S < 31.9 && (!adjoint || most < 1.99);
+}
+
 // Whether the tensor-core gather runs: for the same stencils as the spread, grids of
-// at least a patch, and enough targets per tile.  It costs about 40 ns (two
+// at least a patch, sums that fit, and enough targets per tile.  It costs about 40 ns (two
 // grids) or 66 ns (four) per item, k_gather_fix 1.4 or 5.6 ns per target beside
 // a fixed 0.25 ms or so (2^16 targets, two grids: 0.97 against 0.41 ms on 2688^2
 // nodes, 0.12 against 0.21 ms on 512^2; 300,000 targets, four grids: 1.73
@@ -744,16 +765,14 @@ static int tc_spread(se2p_plan pl, const SpreadArgs &sa, const TcSet &t, int nc,
 static bool tg_ok(const GatherArgs &ga, int nout)
 {
     if (ga.P < 4 || ga.P > kTcMaxP || ga.Mx < kTgX || ga.My < kTgY ||
-        !(std::fabs(ga.w - ga.h * ga.P / 2) <= 1e-14 * ga.w) || !tc_alpha_ok(-ga.a * ga.h * ga.h))
+        !(std::fabs(ga.w - ga.h * ga.P / 2) <= 1e-14 * ga.w) || !tc_alpha_ok(-ga.a * ga.h * ga.h) ||
+        !tg_sums_ok(-ga.a * ga.h * ga.h, ga.P, nout == 5))
         return false;
     const double ntile = std::ceil((double)ga.Mx / (kTgX - ga.P)) * std::ceil((double)ga.My / (kTgY - ga.P));
     return (14.0 + 13.0 * nout) * std::min(ntile, (double)ga.nt) <= 2.5e5 + 0.35 * nout * nout * (double)ga.nt;
 }
 
-// The gather of nout grids (int64 at scale kTgBits): the patch sums stay below
-// 2^63 with |g| below 2^61 and the factors' sum along y below 4.
-constexpr int kTgBits = 61;
-
+// The gather of nout grids.
 static int tg_gather(se2p_plan pl, const GatherArgs &ga, const TcSet &t, int nout, cudaStream_t ks)
 {
     TcGatherArgs ta{};

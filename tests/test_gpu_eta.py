@@ -68,3 +68,17 @@ def test_narrow_gaussians(ft, plans, P, alpha):
     eta = 2 * xi * xi / (M * M) / alpha
     _kspace(ft, plans, M, P, xi, eta)
     _gradients(ft, plans, M, P, xi, eta)
+
+
+FLAT = [0.3, 1.0, 1.2, 1.5, 2.0, 2.4, 2.6, 3.0, 4.0, 6.0, 8.0]
+
+
+@pytest.mark.parametrize("P", [4, 12, 24, 26])
+@pytest.mark.parametrize("ratio", FLAT)
+def test_flat_gaussians(ft, plans, P, ratio):
+    """eta at multiples of the drivers' choice (which is 0.05 here, so that the filter
+    does not amplify the rounding of either side)."""
+    M = 256
+    xi = 0.95 * np.sqrt(np.pi * P) * np.sqrt(0.05) / (P / M)
+    _kspace(ft, plans, M, P, xi, 0.05 * ratio)
+    _gradients(ft, plans, M, P, xi, 0.05 * ratio)
