@@ -100,6 +100,7 @@ struct se2p_plan_st {
     std::vector<float4> tw_host[2];
     // set by a tensor-core kernel whose wait ran out (mapped host memory)
     int *tc_err = nullptr, *tc_err_dev = nullptr;
+    int tc_polls = kTcPolls;
     // pending (start, end) event pairs per stage, resolved by se2p_plan_stage_times
     std::vector<std::pair<cudaEvent_t, cudaEvent_t>> pending[T_NUM_STAGES];
     double stage_ms[T_NUM_STAGES] = {0};
@@ -730,7 +731,7 @@ static int tc_spread(se2p_plan pl, const SpreadArgs &sa, const TcSet &t, int nc,
     ta.nty = t.pa.nty;
     ta.s = t.s;
     ta.bound = sa.bound;
-    ta.err = pl->tc_err_dev;
+    ta.wait = TcWait{pl->tc_polls, pl->tc_err_dev};
     CK(launch_spread_tc(ta, nc, ks, pl->launches));
     return SE2P_OK;
 }
@@ -793,7 +794,7 @@ static int tg_gather(se2p_plan pl, const GatherArgs &ga, const TcSet &t, int nou
     ta.nt = ga.nt;
     ta.scale = ga.scale;
     ta.out = ga.out;
-    ta.err = pl->tc_err_dev;
+    ta.wait = TcWait{pl->tc_polls, pl->tc_err_dev};
     CK(launch_gather_tc(ta, nout, ks, pl->launches));
     return SE2P_OK;
 }
@@ -1655,7 +1656,7 @@ int run_adjoint(se2p_plan pl, const Job &J, const AdjIo &io)
             ta.scale = ga.scale;
             ta.dscale = 2.0 * ga.a * h;
             ta.out = gk;
-            ta.err = pl->tc_err_dev;
+            ta.wait = TcWait{pl->tc_polls, pl->tc_err_dev};
             CK(launch_gather_adj_tc(ta, ks, pl->launches));
             ga.tc = true;
         }
@@ -1801,6 +1802,15 @@ int se2p_plan_set_overlap(se2p_plan pl, int on)
 {
     if (!pl) return SE2P_ERR_ARG;
     pl->overlap = on != 0;
+    return SE2P_OK;
+}
+
+int se2p_plan_set_wait_limit(se2p_plan pl, int polls)
+{
+    if (!pl) return SE2P_ERR_ARG;
+    if (polls < 0 || polls > kTcPolls)
+        return fail(pl, SE2P_ERR_ARG, "the wait limit must be between 0 and %d polls", kTcPolls);
+    pl->tc_polls = polls;
     return SE2P_OK;
 }
 

@@ -399,6 +399,14 @@ struct TcPrepArgs {
     TcSetArgs s[2];
 };
 
+// The bounded waits of the tensor-core kernels: polls (of up to 20 us) before one gives
+// up, and the word that is set then (mapped host memory).
+constexpr int kTcPolls = 1 << 16;
+struct TcWait {
+    int polls;
+    int *err;
+};
+
 struct TcSpreadArgs {
     const void *fac;
     const int *list;            // tile by tile, the points' numbers
@@ -409,7 +417,7 @@ struct TcSpreadArgs {
     int Mx, My, P, Tx, nty, Ty;
     unsigned long long s;       // exp(-2 alpha) 2^64
     const unsigned long long *bound;   // S, as in k_spread_fix
-    int *err;                   // set when a wait ran out
+    TcWait wait;
 };
 
 // Tensor-core gather: patches of kTgX x kTgY nodes, stencil origins in tiles of
@@ -428,7 +436,7 @@ struct TcGatherArgs {
     int64_t nt;
     double scale;
     double2 *out;               // NC/2 outputs per target, [k * nt + t]
-    int *err;
+    TcWait wait;
 };
 
 // Tensor-core adjoint gather: the gather's tiles and items, the points being the
@@ -446,7 +454,7 @@ struct TcGatherAdjArgs {
     const double *coef;         // 5 per source
     double Lhx, Lhy, h, scale, dscale;   // dscale = 2 a h: the derivative's factor
     double *out;                // 7 per source: 5 values, gradient x, y
-    int *err;
+    TcWait wait;
 };
 
 struct FilterArgs {

@@ -379,25 +379,65 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar)
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
-// Waits for the phase of the given parity; gives up after kTcSpin polls of up to
-// 20 us (or when another thread has), sets the shared abort flag and the error word.
-constexpr int kTcSpin = 1 << 16;
-__device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity, volatile int *abort_sh,
-                                          int *err)
+// One poll, of up to 20 us, of the phase of the given parity.
+__device__ __forceinline__ bool mbar_poll(uint32_t bar, uint32_t parity)
 {
-    for (int i = 0; i < kTcSpin; i++) {
-        uint32_t ok;
-        asm volatile("{\n\t.reg .pred p;\n\t"
-                     "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, 20000;\n\t"
-                     "selp.u32 %0, 1, 0, p;\n\t}"
-                     : "=r"(ok)
-                     : "r"(bar), "r"(parity)
-                     : "memory");
-        if (ok) return;
-        if (*abort_sh) return;
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p;\n\t"
+                 "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, 20000;\n\t"
+                 "selp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(ok)
+                 : "r"(bar), "r"(parity)
+                 : "memory");
+    return ok;
+}
+
+// Waits for the phase of the given parity; gives up after w.polls polls (or when another
+// thread has), sets the shared abort flag and the error word, and returns false.  What the
+// phase guards is then not there: the thread must touch none of it and go to the next of
+// its group's barriers, which end with tc_stop for all threads of the group together.
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int *abort_sh,
+                                          const TcWait &w)
+{
+    for (int i = 0; i < w.polls; i++) {
+        if (mbar_poll(bar, parity)) return true;
+        if (*abort_sh) return false;
     }
     *abort_sh = 1;
-    *err = 1;
+    *w.err = 1;
+    __threadfence_system();
+    return false;
+}
+
+// Barrier of THREADS threads that says whether any of them has seen the abort flag: the
+// same answer for all, so that they leave their loops together.
+template <int ID, int THREADS>
+__device__ __forceinline__ bool tc_stop(volatile int *abort_sh)
+{
+    uint32_t stop;
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %1, 0;\n\t"
+                 "bar.red.or.pred q, %2, %3, p;\n\t"
+                 "selp.u32 %0, 1, 0, q;\n\t}"
+                 : "=r"(stop)
+                 : "r"(*abort_sh), "n"(ID), "n"(THREADS)
+                 : "memory");
+    return stop;
+}
+
+__device__ __forceinline__ void tc_commit(uint32_t bar)
+{
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
+                 : "memory");
+}
+
+// The end of the issuing thread: everything it issued must have completed before shared
+// memory and TMEM are given back, also where its waits have given up.
+__device__ __forceinline__ void tc_drain(uint32_t bar, const TcWait &w)
+{
+    tc_commit(bar);
+    for (int i = 0; i < kTcPolls; i++)
+        if (mbar_poll(bar, 0)) return;
+    *w.err = 1;
     __threadfence_system();
 }
 
@@ -414,12 +454,6 @@ __device__ __forceinline__ void bulk_add_u64(void *dst, uint32_t src, int bytes)
 {
     asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.u64 [%0], [%1], %2;" ::"l"(dst),
                  "r"(src), "r"(bytes)
-                 : "memory");
-}
-
-__device__ __forceinline__ void tc_commit(uint32_t bar)
-{
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
                  : "memory");
 }
 
@@ -646,18 +680,18 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_spread_tc(TcSpreadArgs a)
     if (warp == kTcBuild / 32) {
         if (lane == 0) {
             int nfull[2] = {0, 0}, ng = 0;
-            for (int v = v0; v < v1; v++) {
+            bool ok = true;
+            for (int v = v0; v < v1 && ok; v++) {
                 const int4 item = a.items[split ? v / NG : v];
                 const int nk = (item.z + 15) >> 4;
                 const int g0 = split ? v % NG : 0, g1 = split ? g0 + 1 : NG;
-                for (int g = g0; g < g1; g++, ng++) {
+                for (int g = g0; g < g1 && ok; g++, ng++) {
                     for (int k = 0; k < nk; k++) {
                         const int b = k & 1;
-                        mbar_wait(smem_u32(&sh.full[b]), nfull[b]++ & 1, ab, a.err);
-                        if (k == 0 && ng > 0)
-                            mbar_wait(smem_u32(&sh.tfree), (ng - 1) & 1, ab, a.err);
+                        ok = mbar_wait(smem_u32(&sh.full[b]), nfull[b]++ & 1, ab, a.wait) &&
+                             !(k == 0 && ng > 0 && !mbar_wait(smem_u32(&sh.tfree), (ng - 1) & 1, ab, a.wait));
+                        if (!ok) break;
                         tc_fence_after();
-                        if (*ab) continue;
                         const uint32_t Aa = smem_u32(Ash) + b * tc_a_bytes(NS);
                         const uint32_t Ba = smem_u32(Bsh) + k * 2 * kBK;
 #pragma unroll
@@ -668,12 +702,10 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_spread_tc(TcSpreadArgs a)
                         }
                         tc_commit(smem_u32(&sh.free[b]));
                     }
-                    tc_commit(smem_u32(&sh.done));
+                    if (ok) tc_commit(smem_u32(&sh.done));
                 }
             }
-            // everything issued has completed before TMEM is given back
-            tc_commit(smem_u32(&sh.fin));
-            mbar_wait(smem_u32(&sh.fin), 0, ab, a.err);
+            tc_drain(smem_u32(&sh.fin), a.wait);
         }
         __syncwarp();
     } else if (warp == kTcBuild / 32 + 1) {
@@ -703,7 +735,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_spread_tc(TcSpreadArgs a)
                     for (int c = 0; c < NC; c++) cf[u][c] = 0.0;
                 }
             }
-            if (n > 1) mbar_wait(smem_u32(&sh.sfree[b]), (n / 2 - 1) & 1, ab, a.err);
+            if (n > 1 && !__all_sync(~0u, mbar_wait(smem_u32(&sh.sfree[b]), (n / 2 - 1) & 1, ab, a.wait))) break;
 #pragma unroll
             for (int u = 0; u < kTcK / 32; u++) q.meta[lane + 32 * u] = meta[u];
 #pragma unroll
@@ -726,7 +758,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_spread_tc(TcSpreadArgs a)
                     q.neg[c][lane + 32 * u] = (unsigned char)(w >> 63);
                 }
             }
-            if (n > 0) mbar_wait(smem_u32(&sh.seedfree), (n - 1) & 1, ab, a.err);
+            if (n > 0 && !__all_sync(~0u, mbar_wait(smem_u32(&sh.seedfree), (n - 1) & 1, ab, a.wait))) break;
 #pragma unroll
             for (int u = 0; u < kTcK / 32; u++) {
                 if (!f[u]) continue;
@@ -745,16 +777,17 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_spread_tc(TcSpreadArgs a)
         const int wg = tid / (kTcBuild / 2), wt = tid & (kTcBuild / 2 - 1);   // operand buffer, thread in it
         int nfill = 0, ng = 0, n = 0;
         const __half2 one = __float2half2_rn(1.0f), mone = __float2half2_rn(-1.0f);
-        auto bsync = [] { asm volatile("bar.sync 1, %0;" ::"n"(kTcBuild) : "memory"); };
-        for (int v = v0; v < v1; v++, n++) {
+        auto bstop = [&] { return tc_stop<1, kTcBuild>(ab); };
+        bool stop = false;
+        for (int v = v0; v < v1 && !stop; v++, n++) {
             const int4 item = a.items[split ? v / NG : v];
             const int g0 = split ? v % NG : 0, g1 = split ? g0 + 1 : NG;
             const int cnt = item.z, nk = (cnt + 15) >> 4, KP = nk * 16;
             const TcSources &src = sh.src[n & 1];
-            mbar_wait(smem_u32(&sh.ready), n & 1, ab, a.err);
+            const bool have = mbar_wait(smem_u32(&sh.ready), n & 1, ab, a.wait);
             // the factors along x and y, outward from the nearest node on both
             // sides, in the chunk-aligned windows of the stencils
-            for (int t = tid; t < 4 * kTcK; t += kTcBuild) {
+            for (int t = have ? tid : 4 * kTcK; t < 4 * kTcK; t += kTcBuild) {
                 const int q = t / kTcK, ax = q & 1, s = t % kTcK;
                 if (s >= cnt) continue;
                 const int meta = src.meta[s], ic = P / 2 + ((meta >> (16 + ax)) & 1);
@@ -769,7 +802,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_spread_tc(TcSpreadArgs a)
                 }
             }
             mbar_arrive(smem_u32(&sh.seedfree));
-            bsync();
+            if (bstop()) break;
             // B: the digits of Y, four nodes of one source per step (the
             // window's chunks first, so that a warp's lanes agree)
             for (int t = tid; t < kTcK * (kTcY / 4); t += kTcBuild) {
@@ -788,10 +821,12 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_spread_tc(TcSpreadArgs a)
                 }
             }
             fence_async_shared();
-            bsync();
+            if (bstop()) break;
             for (int g = g0; g < g1; g++, ng++) {
+                bool ok = true;
                 for (int k = wg; k < nk; k += 2) {
-                    if (nfill > 0) mbar_wait(smem_u32(&sh.free[wg]), (nfill - 1) & 1, ab, a.err);
+                    ok = nfill == 0 || mbar_wait(smem_u32(&sh.free[wg]), (nfill - 1) & 1, ab, a.wait);
+                    if (!ok) break;
                     nfill++;
                     // A: 16 sources x two grids x 16 half chunks of 4 nodes,
                     // the window's in the loop's first pass
@@ -820,10 +855,10 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_spread_tc(TcSpreadArgs a)
                     mbar_arrive(smem_u32(&sh.full[wg]));
                 }
                 // the levels -> int64 at the grid's scale -> staging -> grid
-                mbar_wait(smem_u32(&sh.done), ng & 1, ab, a.err);
+                ok = __all_sync(~0u, ok && mbar_wait(smem_u32(&sh.done), ng & 1, ab, a.wait));
                 tc_fence_after();
                 const int quad = warp & 3, row = quad * 32 + lane, c = 2 * g + (quad >> 1);
-                if (c < NC) {
+                if (ok && c < NC) {
                     // c X Y 2^S = (H 2^32 + L) 2^-sh_n, sh_n > 0: H levels 0 .. 2, L levels 3 .. 6
                     const int sh_n = 62 - S - src.ec[c], sh_m = min(sh_n - 32, 60);
                     const long long round = 1ll << ((sh_n <= 32 ? sh_n : sh_m) - 1);
@@ -858,9 +893,10 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_spread_tc(TcSpreadArgs a)
                 mbar_arrive(smem_u32(&sh.tfree));
                 if (g == g1 - 1) mbar_arrive(smem_u32(&sh.sfree[n & 1]));
                 fence_async_shared();
-                bsync();
+                stop = bstop();
+                if (stop) break;
                 // one bulk reduction per row of nodes (two where it wraps)
-                if (tid < 128 && 2 * g + (tid >> 6) < NC && !*ab) {
+                if (tid < 128 && 2 * g + (tid >> 6) < NC) {
                     int x = item.x / a.nty * a.Tx + (tid & 63);
                     if (x >= a.Mx) x -= a.Mx;
                     const int y = item.x % a.nty * a.Ty, m = min(kTcY, a.My - y);
@@ -871,7 +907,8 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_spread_tc(TcSpreadArgs a)
                     asm volatile("cp.async.bulk.commit_group;" ::: "memory");
                     asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
                 }
-                bsync();
+                stop = bstop();
+                if (stop) break;
             }
         }
         if (tid < 128) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
@@ -1015,12 +1052,13 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_gather_tc(TcGatherArgs a)
     if (warp == kTcBuild / 32) {
         if (lane == 0) {
             int n = 0;
-            for (int v = v0; v < v1; v++) {
+            bool ok = true;
+            for (int v = v0; v < v1 && ok; v++) {
                 for (int c = 0; c < NC; c++, n++) {
-                    mbar_wait(smem_u32(&sh.bfull), n & 1, ab, a.err);
-                    if (n > 0) mbar_wait(smem_u32(&sh.tfree), (n - 1) & 1, ab, a.err);
+                    ok = mbar_wait(smem_u32(&sh.bfull), n & 1, ab, a.wait) &&
+                         (n == 0 || mbar_wait(smem_u32(&sh.tfree), (n - 1) & 1, ab, a.wait));
+                    if (!ok) break;
                     tc_fence_after();
-                    if (*ab) continue;
 #pragma unroll 1
                     for (int k = 0; k < kTgY / 16; k++)
 #pragma unroll
@@ -1032,9 +1070,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_gather_tc(TcGatherArgs a)
                     tc_commit(smem_u32(&sh.done));
                 }
             }
-            // everything issued has completed before TMEM is given back
-            tc_commit(smem_u32(&sh.fin));
-            mbar_wait(smem_u32(&sh.fin), 0, ab, a.err);
+            tc_drain(smem_u32(&sh.fin), a.wait);
         }
         __syncwarp();
     } else if (warp == kTcBuild / 32 + 1) {
@@ -1056,13 +1092,13 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_gather_tc(TcGatherArgs a)
                     meta[u] = f[u]->meta;
                 }
             }
-            if (n > 1) mbar_wait(smem_u32(&sh.sfree[b]), (n / 2 - 1) & 1, ab, a.err);
+            if (n > 1 && !__all_sync(~0u, mbar_wait(smem_u32(&sh.sfree[b]), (n / 2 - 1) & 1, ab, a.wait))) break;
 #pragma unroll
             for (int u = 0; u < kTgT / 32; u++) {
                 sh.meta[b][lane + 32 * u] = meta[u];
                 sh.idx[b][lane + 32 * u] = idx[u];
             }
-            if (n > 0) mbar_wait(smem_u32(&sh.seedfree), (n - 1) & 1, ab, a.err);
+            if (n > 0 && !__all_sync(~0u, mbar_wait(smem_u32(&sh.seedfree), (n - 1) & 1, ab, a.wait))) break;
 #pragma unroll
             for (int u = 0; u < kTgT / 32; u++) {
                 if (!f[u]) continue;
@@ -1083,14 +1119,14 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_gather_tc(TcGatherArgs a)
         const bool epi = (warp & 2) == 0;            // TMEM lanes 0 .. 63: targets
         const int et = (warp & 1) * 32 + lane, eh = warp >> 2;            // target, half of the columns
         const int bt = ((warp >> 2) * 2 + (warp & 1)) * 32 + lane;        // builder thread
-        auto bsync = [] { asm volatile("bar.sync 1, %0;" ::"n"(kTcBuild) : "memory"); };
+        auto bstop = [&] { return tc_stop<1, kTcBuild>(ab); };
         for (int v = v0; v < v1; v++, n++) {
             const int4 item = a.items[v];
             const int cnt = item.z, b = n & 1;
-            mbar_wait(smem_u32(&sh.ready), n & 1, ab, a.err);
+            const bool have = mbar_wait(smem_u32(&sh.ready), n & 1, ab, a.wait);
             // the factors: x in the patch's coordinates (as fractions of 2^62), y in
             // the chunk-aligned window (B's region holds them until A is built)
-            for (int t = tid; t < 4 * kTgT; t += kTcBuild) {
+            for (int t = have ? tid : 4 * kTgT; t < 4 * kTgT; t += kTcBuild) {
                 const int q = t / kTgT, ax = q & 1, s = t % kTgT;
                 if (s >= cnt) continue;
                 const int meta = sh.meta[b][s], ic = P / 2 + ((meta >> (16 + ax)) & 1);
@@ -1105,7 +1141,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_gather_tc(TcGatherArgs a)
                 }
             }
             mbar_arrive(smem_u32(&sh.seedfree));
-            bsync();
+            if (bstop()) break;
             for (int t = tid; t < kTgT * (kTgY / 4); t += kTcBuild) {
                 const int slot = t / (2 * kTgT), s = (t >> 1) % kTgT, half = t & 1;
                 const int ch = (((sh.meta[b][s] >> 11) & 31) + slot) & (kTgY / 8 - 1);
@@ -1120,13 +1156,13 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_gather_tc(TcGatherArgs a)
                 }
             }
             fence_async_shared();
-            bsync();
+            if (bstop()) break;
             const int x0 = item.x / a.nty * a.Tx, y0 = item.x % a.nty * a.Ty;
             long long first = 0;                     // the first of a pair's two sums
             for (int c = 0; c < NC; c++, nc++) {
                 if (!epi) {
                     // B: 32 columns x 8 chunks of 8 nodes
-                    if (c > 0) mbar_wait(smem_u32(&sh.done), (nc - 1) & 1, ab, a.err);
+                    if (c > 0 && !mbar_wait(smem_u32(&sh.done), (nc - 1) & 1, ab, a.wait)) break;
                     const long long *grid = a.grid + (int64_t)c * a.Mx * a.My;
 #pragma unroll 1
                     for (int t = bt; t < kTgX * (kTgY / 8); t += 128) {
@@ -1152,11 +1188,11 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_gather_tc(TcGatherArgs a)
                     fence_async_shared();
                     mbar_arrive(smem_u32(&sh.bfull));
                 } else {
-                    mbar_wait(smem_u32(&sh.done), nc & 1, ab, a.err);
+                    const bool ok = __all_sync(~0u, mbar_wait(smem_u32(&sh.done), nc & 1, ab, a.wait));
                     tc_fence_after();
                     long long acc = 0;
 #pragma unroll 1
-                    for (int h = 0; h < kTgX / 16; h++) {
+                    for (int h = ok ? 0 : kTgX / 16; h < kTgX / 16; h++) {
                         const int i0 = eh * (kTgX / 2) + 8 * h;
                         uint32_t r[kTcDigits][8];
 #pragma unroll
@@ -1178,14 +1214,14 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_gather_tc(TcGatherArgs a)
                     mbar_arrive(smem_u32(&sh.tfree));
                     // the two halves of the columns
                     if (eh) sh.part[et] = acc;
-                    asm volatile("bar.sync 2, 128;" ::: "memory");
+                    if (tc_stop<2, 128>(ab)) break;
                     if (!eh) {
                         acc += sh.part[et];
                         if (c & 1) {
                             const int j = sh.idx[b][et];
                             const unsigned long long gb = a.gmax[c / 2];
                             const double s = gb == 0 ? 0.0 : ldexp(a.scale, 3 - grid_shift(gb, a.Bg));
-                            if (j >= 0 && !*ab)
+                            if (j >= 0)
                                 a.out[(int64_t)(c / 2) * a.nt + j] = make_double2((double)first * s, (double)acc * s);
                         } else {
                             first = acc;
@@ -1196,7 +1232,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_gather_tc(TcGatherArgs a)
             }
             mbar_arrive(smem_u32(&sh.sfree[b]));
             // the item's last product has read A and B (the epilogue waited for it)
-            bsync();
+            if (bstop()) break;
         }
     }
     tc_fence_before();
@@ -1282,13 +1318,14 @@ __global__ void __launch_bounds__(kGaThreads, 1) k_gather_adj_tc(TcGatherAdjArgs
     if (warp == 16) {
         if (lane == 0) {
             int n = 0;
-            for (int v = v0; v < v1; v++) {
+            bool ok = true;
+            for (int v = v0; v < v1 && ok; v++) {
                 for (int c = 0; c < 5; c++, n++) {
                     const int b = n & 1;
-                    mbar_wait(smem_u32(&sh.bfull[b]), (n >> 1) & 1, ab, a.err);
-                    if (n > 1) mbar_wait(smem_u32(&sh.tfree[b]), ((n >> 1) - 1) & 1, ab, a.err);
+                    ok = mbar_wait(smem_u32(&sh.bfull[b]), (n >> 1) & 1, ab, a.wait) &&
+                         (n <= 1 || mbar_wait(smem_u32(&sh.tfree[b]), ((n >> 1) - 1) & 1, ab, a.wait));
+                    if (!ok) break;
                     tc_fence_after();
-                    if (*ab) continue;
 #pragma unroll 1
                     for (int k = 0; k < kTgY / 16; k++)
 #pragma unroll
@@ -1300,9 +1337,7 @@ __global__ void __launch_bounds__(kGaThreads, 1) k_gather_adj_tc(TcGatherAdjArgs
                     tc_commit(smem_u32(&sh.done[b]));
                 }
             }
-            // everything issued has completed before TMEM is given back
-            tc_commit(smem_u32(&sh.fin));
-            mbar_wait(smem_u32(&sh.fin), 0, ab, a.err);
+            tc_drain(smem_u32(&sh.fin), a.wait);
         }
         __syncwarp();
     } else if (warp == 17) {
@@ -1310,7 +1345,7 @@ __global__ void __launch_bounds__(kGaThreads, 1) k_gather_adj_tc(TcGatherAdjArgs
         for (int v = v0; v < v1; v++, n++) {
             const int4 item = a.items[v];
             const int b = n & 1;
-            if (n > 1) mbar_wait(smem_u32(&sh.sfree[b]), (n / 2 - 1) & 1, ab, a.err);
+            if (n > 1 && !__all_sync(~0u, mbar_wait(smem_u32(&sh.sfree[b]), (n / 2 - 1) & 1, ab, a.wait))) break;
             const TcPoint *f[kTgT / 32];
 #pragma unroll
             for (int u = 0; u < kTgT / 32; u++) {
@@ -1333,7 +1368,7 @@ __global__ void __launch_bounds__(kGaThreads, 1) k_gather_adj_tc(TcGatherAdjArgs
                 sh.meta[b][s] = meta;
                 sh.idx[b][s] = j;
             }
-            if (n > 0) mbar_wait(smem_u32(&sh.seedfree), (n - 1) & 1, ab, a.err);
+            if (n > 0 && !__all_sync(~0u, mbar_wait(smem_u32(&sh.seedfree), (n - 1) & 1, ab, a.wait))) break;
 #pragma unroll
             for (int u = 0; u < kTgT / 32; u++) {
                 if (!f[u]) continue;
@@ -1351,14 +1386,14 @@ __global__ void __launch_bounds__(kGaThreads, 1) k_gather_adj_tc(TcGatherAdjArgs
     } else {
         int n = 0, nc = 0;                           // items, grids so far
         const __half2 one = __float2half2_rn(1.0f);
-        auto bsync = [] { asm volatile("bar.sync 1, 512;" ::: "memory"); };
+        auto bstop = [&] { return tc_stop<1, 512>(ab); };
         for (int v = v0; v < v1; v++, n++) {
             const int4 item = a.items[v];
             const int cnt = item.z, b = n & 1;
-            mbar_wait(smem_u32(&sh.ready), n & 1, ab, a.err);
+            const bool have = mbar_wait(smem_u32(&sh.ready), n & 1, ab, a.wait);
             if (tid < 4 * kTgT) {
                 const int q = tid / kTgT, ax = q & 1, s = tid % kTgT;
-                if (s < cnt) {
+                if (have && s < cnt) {
                     const int meta = sh.meta[b][s], ic = P / 2 + ((meta >> (16 + ax)) & 1);
                     const int r = ax ? (meta >> 8) & 7 : meta & 0xff, w = ax ? win : kTgX;
                     const unsigned long long e = ax ? sh.seed[1][s] : sh.seed[0][s] >> 2;
@@ -1372,7 +1407,7 @@ __global__ void __launch_bounds__(kGaThreads, 1) k_gather_adj_tc(TcGatherAdjArgs
                 }
                 mbar_arrive(smem_u32(&sh.seedfree));
             }
-            bsync();
+            if (bstop()) break;
             for (int t = tid; t < 2 * kTgT * (kTgY / 4); t += 512) {
                 const int der = t / (kTgT * (kTgY / 4)), t1 = t % (kTgT * (kTgY / 4));
                 const int slot = t1 / (2 * kTgT), s = (t1 >> 1) % kTgT, half = t1 & 1, row = 64 * der + s;
@@ -1399,13 +1434,13 @@ __global__ void __launch_bounds__(kGaThreads, 1) k_gather_adj_tc(TcGatherAdjArgs
                 }
             }
             fence_async_shared();
-            bsync();
+            if (bstop()) break;
             const int x0 = item.x / a.nty * a.Tx, y0 = item.x % a.nty * a.Ty;
             for (int c = 0; c < 5; c++, nc++) {
                 const int tb = nc & 1;
                 if (warp >= 8) {
                     // B: 32 columns x 8 chunks of 8 nodes, one each
-                    if (nc > 1) mbar_wait(smem_u32(&sh.done[tb]), ((nc >> 1) - 1) & 1, ab, a.err);
+                    if (nc > 1 && !mbar_wait(smem_u32(&sh.done[tb]), ((nc >> 1) - 1) & 1, ab, a.wait)) break;
                     const int bt = tid - 256, i = bt % kTgX, ch = bt / kTgX;
                     int x = x0 + i, y = y0 + 8 * ch;
                     if (x >= a.Mx) x -= a.Mx;
@@ -1430,7 +1465,7 @@ __global__ void __launch_bounds__(kGaThreads, 1) k_gather_adj_tc(TcGatherAdjArgs
                 } else {
                     const int quad = warp & 3, eh = warp >> 2, t = (quad & 1) * 32 + lane;
                     const int mid = (sh.meta[b][t] & 0xff) + P / 2;
-                    mbar_wait(smem_u32(&sh.done[tb]), (nc >> 1) & 1, ab, a.err);
+                    if (!__all_sync(~0u, mbar_wait(smem_u32(&sh.done[tb]), (nc >> 1) & 1, ab, a.wait))) break;
                     tc_fence_after();
                     long long acc = 0, accx = 0;
 #pragma unroll 1
@@ -1461,8 +1496,8 @@ __global__ void __launch_bounds__(kGaThreads, 1) k_gather_adj_tc(TcGatherAdjArgs
                 }
             }
             // (the item's last products have read A: the epilogue waited for them)
-            bsync();
-            if (tid < cnt && !*ab) {
+            if (bstop()) break;
+            if (tid < cnt) {
                 const int j = sh.idx[b][tid];
                 const double ux = sh.ux[b][tid], uy = sh.uy[b][tid];
                 double gx = 0.0, gy = 0.0;
@@ -1483,7 +1518,7 @@ __global__ void __launch_bounds__(kGaThreads, 1) k_gather_adj_tc(TcGatherAdjArgs
                 o[6] = gy * a.dscale;
             }
             mbar_arrive(smem_u32(&sh.sfree[b]));
-            bsync();
+            if (bstop()) break;
         }
     }
     tc_fence_before();

@@ -65,6 +65,12 @@ const char *se2p_plan_last_error(se2p_plan plan);
  * chain, unless overlap is switched off (on = 0): then every stage runs in
  * order on the plan's stream, e.g. to time kernels in isolation. */
 int se2p_plan_set_overlap(se2p_plan plan, int on);
+/* Every wait inside the tensor-core kernels ends after a number of polls of up to 20 us
+ * each (65536, the default and the most); a kernel whose wait ran out leaves the rest of
+ * its work, and the call, or where its arguments are all in device memory the plan's
+ * next call, returns SE2P_ERR_CUDA.  Small numbers are for tests: with 0 every wait
+ * runs out at once. */
+int se2p_plan_set_wait_limit(se2p_plan plan, int polls);
 /* Bytes of device workspace the plan currently holds. */
 int64_t se2p_plan_workspace_bytes(se2p_plan plan);
 /* Number of kernels this plan has launched so far (its own, not cuFFT's). */
