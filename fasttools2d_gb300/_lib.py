@@ -27,7 +27,8 @@ EXPORTS = (
     "se2p_plan_enable_timing", "se2p_num_stages", "se2p_stage_name", "se2p_plan_stage_times",
     "se2p_plan_probe_atomics",
     "se2p_plan_count_pairs", "se2p_slp_real_noalloc", "se2p_plan_set_precision",
-    "se2p_plan_set_overlap", "se2p_plan_set_wait_limit", "se2p_stokes_ewald_adjoint",
+    "se2p_plan_set_overlap", "se2p_plan_set_wait_limit",
+    "se2p_plan_synchronize", "se2p_stokes_ewald_adjoint",
     "se2p_geom_create", "se2p_geom_apply", "se2p_geom_bytes", "se2p_geom_pairs",
     "se2p_geom_destroy",
 )
@@ -91,6 +92,7 @@ def load(path: str = LIB_PATH):
         L.se2p_plan_set_precision.argtypes = [P, i32]
         L.se2p_plan_set_overlap.argtypes = [P, i32]
         L.se2p_plan_set_wait_limit.argtypes = [P, i32]
+        L.se2p_plan_synchronize.argtypes = [P]
         L.se2p_slp_real_noalloc.argtypes = [_dp, i64, _dp, i64, _dp, d, i32, i32, d, d, _dp, P]
         PP = ctypes.POINTER(Params)
         L.se2p_slp_ewald.argtypes = [P, PP, _dp, i64, _dp, i64, _dp, _dp, _dp, _dp]
@@ -148,6 +150,10 @@ class Plan:
 
     def set_overlap(self, on: bool = True):
         self.check(self.lib.se2p_plan_set_overlap(self.handle, 1 if on else 0))
+
+    def synchronize(self):
+        """Wait for the work queued by calls on CUDA tensors, and raise what went wrong in it."""
+        self.check(self.lib.se2p_plan_synchronize(self.handle))
 
     def set_wait_limit(self, polls: int = 1 << 16):
         """Polls (of up to 20 us) after which a wait inside a tensor-core kernel gives up."""

@@ -98,8 +98,9 @@ struct se2p_plan_st {
     int tw_len[2] = {0, 0};
     const void *tw_dev[2] = {nullptr, nullptr};
     std::vector<float4> tw_host[2];
-    // set by a tensor-core kernel whose wait ran out (mapped host memory)
-    int *tc_err = nullptr, *tc_err_dev = nullptr;
+    // set by a tensor-core kernel whose wait ran out: mapped host memory, and a device word
+    // that makes the call's outputs NaN
+    int *tc_err = nullptr, *tc_err_dev = nullptr, *tc_bad = nullptr;
     int tc_polls = kTcPolls;
     // pending (start, end) event pairs per stage, resolved by se2p_plan_stage_times
     std::vector<std::pair<cudaEvent_t, cudaEvent_t>> pending[T_NUM_STAGES];
@@ -591,12 +592,13 @@ static int gather_fixed_bits(const SpreadArgs &sa)
     return std::min(62, 64 - e);
 }
 
-// A tensor-core kernel of an earlier call gave up waiting: its results are void.
+// A tensor-core kernel of a call gave up waiting: that call's results are NaN.
 static int tc_check(se2p_plan pl)
 {
     volatile int *e = pl->tc_err;
     if (!*e) return SE2P_OK;
     *e = 0;
+    CK(cudaMemsetAsync(pl->tc_bad, 0, sizeof(int), pl->stream));   // (behind that call's outputs)
     return fail(pl, SE2P_ERR_CUDA, "a tensor-core kernel ran out of time waiting for its operands");
 }
 
@@ -731,7 +733,7 @@ static int tc_spread(se2p_plan pl, const SpreadArgs &sa, const TcSet &t, int nc,
     ta.nty = t.pa.nty;
     ta.s = t.s;
     ta.bound = sa.bound;
-    ta.wait = TcWait{pl->tc_polls, pl->tc_err_dev};
+    ta.wait = TcWait{pl->tc_polls, pl->tc_err_dev, pl->tc_bad};
     CK(launch_spread_tc(ta, nc, ks, pl->launches));
     return SE2P_OK;
 }
@@ -794,7 +796,7 @@ static int tg_gather(se2p_plan pl, const GatherArgs &ga, const TcSet &t, int nou
     ta.nt = ga.nt;
     ta.scale = ga.scale;
     ta.out = ga.out;
-    ta.wait = TcWait{pl->tc_polls, pl->tc_err_dev};
+    ta.wait = TcWait{pl->tc_polls, pl->tc_err_dev, pl->tc_bad};
     CK(launch_gather_tc(ta, nout, ks, pl->launches));
     return SE2P_OK;
 }
@@ -1349,6 +1351,7 @@ int run(se2p_plan pl, const Job &J, const Io &io)
     const double2 *uk_slp = (J.kspace && J.slp) ? uk : nullptr;
     const double2 *uk_dlp = (J.kspace && J.dlp) ? uk + (J.slp ? nt : 0) : nullptr;
     AssembleArgs as;
+    as.bad = pl->tc_bad;
     if (J.slp && o_us.dev)
         as.add(io.mode_slp, J.real ? ur_slp : nullptr, uk_slp, nullptr, o_us.dev, o_urs.dev, o_uks.dev);
     if (J.dlp && o_ud.dev)
@@ -1656,7 +1659,7 @@ int run_adjoint(se2p_plan pl, const Job &J, const AdjIo &io)
             ta.scale = ga.scale;
             ta.dscale = 2.0 * ga.a * h;
             ta.out = gk;
-            ta.wait = TcWait{pl->tc_polls, pl->tc_err_dev};
+            ta.wait = TcWait{pl->tc_polls, pl->tc_err_dev, pl->tc_bad};
             CK(launch_gather_adj_tc(ta, ks, pl->launches));
             ga.tc = true;
         }
@@ -1674,7 +1677,7 @@ int run_adjoint(se2p_plan pl, const Job &J, const AdjIo &io)
         StageTimer tm(pl, T_ASSEMBLE);
         CK(launch_adj_assemble(ns, sperm, gr, gk, wcoef, nt, part, ps, dlp ? fd : zeros,
                                dlp ? nr : zeros, 1.0 / (J.Lx * J.Ly), slp, dlp, o_p.dev,
-                               o_fs.dev, o_fd.dev, o_n.dev, st, pl->launches));
+                               o_fs.dev, o_fd.dev, o_n.dev, pl->tc_bad, st, pl->launches));
     }
     CKS(finish_out(pl, o_p));
     CKS(finish_out(pl, o_fs));
@@ -1726,7 +1729,10 @@ int se2p_plan_create(se2p_plan *plan, int device)
         cudaEventCreateWithFlags(&pl->cin0, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&pl->cin1, cudaEventDisableTiming) != cudaSuccess ||
         cudaHostAlloc(&pl->tc_err, sizeof(int), cudaHostAllocMapped) != cudaSuccess ||
-        cudaHostGetDevicePointer(&pl->tc_err_dev, pl->tc_err, 0) != cudaSuccess) {
+        cudaHostGetDevicePointer(&pl->tc_err_dev, pl->tc_err, 0) != cudaSuccess ||
+        cudaMalloc(&pl->tc_bad, sizeof(int)) != cudaSuccess ||
+        cudaMemsetAsync(pl->tc_bad, 0, sizeof(int), pl->own) != cudaSuccess ||
+        cudaStreamSynchronize(pl->own) != cudaSuccess) {
         cudaGetLastError();
         se2p_plan_destroy(pl);
         return SE2P_ERR_CUDA;
@@ -1766,6 +1772,7 @@ int se2p_plan_destroy(se2p_plan pl)
     if (pl->cin1) cudaEventDestroy(pl->cin1);
     if (pl->own) cudaStreamDestroy(pl->own);
     if (pl->tc_err) cudaFreeHost(pl->tc_err);
+    if (pl->tc_bad) cudaFree(pl->tc_bad);
     delete pl;
     return SE2P_OK;
 }
@@ -1803,6 +1810,14 @@ int se2p_plan_set_overlap(se2p_plan pl, int on)
     if (!pl) return SE2P_ERR_ARG;
     pl->overlap = on != 0;
     return SE2P_OK;
+}
+
+int se2p_plan_synchronize(se2p_plan pl)
+{
+    if (!pl) return SE2P_ERR_ARG;
+    DeviceGuard guard(pl->device);
+    CK(cudaStreamSynchronize(pl->stream));           // (each call joins its other streams into it)
+    return tc_check(pl);
 }
 
 int se2p_plan_set_wait_limit(se2p_plan pl, int polls)
@@ -2512,6 +2527,7 @@ int se2p_geom_apply(se2p_geom g, int nrhs, const double *f_slp, const double *f_
         CK(cudaStreamWaitEvent(st, pl->join, 0));
         StageTimer tm(pl, T_ASSEMBLE);
         AssembleArgs as;
+        as.bad = pl->tc_bad;
         for (int r = 0; r < nb; r++) {
             const int rr = r0 + r;
             const double2 *ukr = uk + (size_t)r * nk2 * nt;

@@ -282,6 +282,7 @@ struct AssembleOut {
 struct AssembleArgs {
     AssembleOut o[8];
     int nout = 0;
+    const int *bad = nullptr;   // set: a kernel gave up, the k-space part (and u) becomes NaN
     void add(int mode, const double2 *ur, const double2 *uk, const double2 *zm, double2 *u,
              double2 *ur_out = nullptr, double2 *uk_out = nullptr)
     {
@@ -400,11 +401,12 @@ struct TcPrepArgs {
 };
 
 // The bounded waits of the tensor-core kernels: polls (of up to 20 us) before one gives
-// up, and the word that is set then (mapped host memory).
+// up, and the words that are set then, one for the host (mapped memory) and one for the
+// kernel that writes the call's outputs.
 constexpr int kTcPolls = 1 << 16;
 struct TcWait {
     int polls;
-    int *err;
+    int *err, *bad;
 };
 
 struct TcSpreadArgs {
@@ -670,8 +672,8 @@ cudaError_t launch_adj_assemble(int64_t n, const int *perm, const double *gr, co
                                 const double *w, int64_t nt, double2 *part,
                                 const double2 *praw, const double2 *fd, const double2 *nrm,
                                 double inv_area, int slp, int dlp, double2 *g_pos,
-                                double2 *g_fs, double2 *g_fd, double2 *g_n, cudaStream_t st,
-                                int64_t &launches);
+                                double2 *g_fs, double2 *g_fd, double2 *g_n, const int *bad,
+                                cudaStream_t st, int64_t &launches);
 cudaError_t launch_spread_f32(const SpreadArgsF &a, int nc, int sms, cudaStream_t st,
                               int64_t &launches);
 cudaError_t launch_filter_f32(const FilterArgsF &a, cudaStream_t st, int64_t &launches);

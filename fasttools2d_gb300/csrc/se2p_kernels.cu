@@ -14,6 +14,7 @@
 // (accepted pairs compacted before the Pade/exp work, a flattened (P+1)^2
 // stencil per spread source, one gather target per lane).
 #include "se2p_internal.cuh"
+#include <math_constants.h>
 
 #include <algorithm>
 
@@ -3199,13 +3200,17 @@ __global__ void k_adj_assemble(int64_t n, const int *__restrict__ perm,
                                const double2 *__restrict__ praw, const double2 *__restrict__ fd,
                                const double2 *__restrict__ nrm, double inv_area, int slp, int dlp,
                                double2 *__restrict__ g_pos, double2 *__restrict__ g_fs,
-                               double2 *__restrict__ g_fd, double2 *__restrict__ g_n)
+                               double2 *__restrict__ g_fd, double2 *__restrict__ g_n,
+                               const int *__restrict__ bad)
 {
     chain_enter();
     const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= n) return;
     const int i = perm[j];
-    const double *r = gr + 7 * j, *k = gk + 7 * j;
+    const double *r = gr + 7 * j, *kp = gk + 7 * j;
+    double k[7];
+#pragma unroll
+    for (int c = 0; c < 7; c++) k[c] = *bad ? CUDART_NAN : kp[c];   // (a kernel gave up)
     const double q = 1.0 / (4.0 * kPi);
     double gp1 = r[5] * q + k[5], gp2 = r[6] * q + k[6];
     if (slp && g_fs) g_fs[i] = make_double2(r[0] * q + k[0], r[1] * q + k[1]);
@@ -3288,6 +3293,7 @@ __global__ void __launch_bounds__(256) k_assemble(int64_t n, const int *__restri
     const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= n) return;
     const int i = perm[j];
+    const bool bad = a.bad && *a.bad;
 #pragma unroll 1
     for (int o = 0; o < a.nout; o++) {
         const AssembleOut &q = a.o[o];
@@ -3309,6 +3315,7 @@ __global__ void __launch_bounds__(256) k_assemble(int64_t n, const int *__restri
                 k.x -= z.x;
                 k.y -= z.y;
             }
+            if (bad) k = make_double2(CUDART_NAN, CUDART_NAN);
         }
         double2 v;
         switch (q.mode) {
@@ -3605,8 +3612,8 @@ cudaError_t launch_adj_assemble(int64_t n, const int *perm, const double *gr, co
                                 const double *w, int64_t nt, double2 *part,
                                 const double2 *praw, const double2 *fd, const double2 *nrm,
                                 double inv_area, int slp, int dlp, double2 *g_pos,
-                                double2 *g_fs, double2 *g_fd, double2 *g_n, cudaStream_t st,
-                                int64_t &launches)
+                                double2 *g_fs, double2 *g_fd, double2 *g_n, const int *bad,
+                                cudaStream_t st, int64_t &launches)
 {
     if (dlp) {
         k_wsum_part<<<kZeroModeParts, 256, 0, st>>>(nt, w, 4, 2, part);
@@ -3616,7 +3623,7 @@ cudaError_t launch_adj_assemble(int64_t n, const int *perm, const double *gr, co
     if (n > 0) {
         launch_chained(k_adj_assemble, grid_for(n, 256), 256, 0, st, n, perm, gr, gk, part + kZeroModeParts,
                                                          praw, fd, nrm, inv_area, slp, dlp,
-                                                         g_pos, g_fs, g_fd, g_n);
+                                                         g_pos, g_fs, g_fd, g_n, bad);
         launches++;
     }
     return cudaGetLastError();

@@ -392,8 +392,15 @@ __device__ __forceinline__ bool mbar_poll(uint32_t bar, uint32_t parity)
     return ok;
 }
 
+__device__ __forceinline__ void tc_give_up(const TcWait &w)
+{
+    *w.bad = 1;
+    *w.err = 1;
+    __threadfence_system();
+}
+
 // Waits for the phase of the given parity; gives up after w.polls polls (or when another
-// thread has), sets the shared abort flag and the error word, and returns false.  What the
+// thread has), sets the shared abort flag and the error words, and returns false.  What the
 // phase guards is then not there: the thread must touch none of it and go to the next of
 // its group's barriers, which end with tc_stop for all threads of the group together.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int *abort_sh,
@@ -404,8 +411,7 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
         if (*abort_sh) return false;
     }
     *abort_sh = 1;
-    *w.err = 1;
-    __threadfence_system();
+    tc_give_up(w);
     return false;
 }
 
@@ -437,8 +443,7 @@ __device__ __forceinline__ void tc_drain(uint32_t bar, const TcWait &w)
     tc_commit(bar);
     for (int i = 0; i < kTcPolls; i++)
         if (mbar_poll(bar, 0)) return;
-    *w.err = 1;
-    __threadfence_system();
+    tc_give_up(w);
 }
 
 __device__ __forceinline__ void fence_async_shared()

@@ -14,7 +14,7 @@
  * memory of the plan's device; the library stages host data itself.  With
  * any host argument the call returns after the results are in host memory;
  * with device-only arguments the work is queued on the plan's stream and the
- * call returns without synchronising.
+ * call returns without synchronising; se2p_plan_synchronize waits for it.
  *
  * Calls on one plan must not overlap; distinct plans are independent.
  * Every function returns an se2p_status; se2p_plan_last_error() gives the
@@ -65,11 +65,16 @@ const char *se2p_plan_last_error(se2p_plan plan);
  * chain, unless overlap is switched off (on = 0): then every stage runs in
  * order on the plan's stream, e.g. to time kernels in isolation. */
 int se2p_plan_set_overlap(se2p_plan plan, int on);
+/* Waits until the work queued on the plan's stream is done, and returns what went wrong
+ * in it. */
+int se2p_plan_synchronize(se2p_plan plan);
 /* Every wait inside the tensor-core kernels ends after a number of polls of up to 20 us
- * each (65536, the default and the most); a kernel whose wait ran out leaves the rest of
- * its work, and the call, or where its arguments are all in device memory the plan's
- * next call, returns SE2P_ERR_CUDA.  Small numbers are for tests: with 0 every wait
- * runs out at once. */
+ * each (65536, the default and the most).  A kernel whose wait ran out leaves the rest of
+ * its work, and every output of the call that holds a k-space part is NaN.  A call that
+ * returns its results in host memory returns SE2P_ERR_CUDA then; for one that only
+ * queued its work, se2p_plan_synchronize does or, where that is not asked, the next call
+ * on the plan, which does nothing else (calls queued before it was found are NaN as
+ * well).  Small numbers are for tests: with 0 every wait runs out at once. */
 int se2p_plan_set_wait_limit(se2p_plan plan, int polls);
 /* Bytes of device workspace the plan currently holds. */
 int64_t se2p_plan_workspace_bytes(se2p_plan plan);

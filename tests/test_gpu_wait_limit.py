@@ -23,33 +23,73 @@ def _cloud(N, seed):
     return p, q, rng.standard_normal((2, N)), np.vstack([np.cos(th), np.sin(th)])
 
 
-def _calls(ft, plan, N):
+def _call(ft, plan, op, N):
     p, q, f, n = _cloud(N, 3)
     prm = ft.EwaldParams.derived(60.0, 12, 12, 192, 192, 24, 1.0, 1.0)
+    if op == "slp":
+        return (ft.slp_ewald(p, q, f, prm, plan=plan),)
+    if op == "stokes":
+        return ft.stokes_ewald(p, q, f, f, n, prm, plan=plan)
+    if op == "adjoint":
+        return ft.stokes_ewald_adjoint(p, q, f, f, n, f, f, prm, plan=plan)
     geo = ft.Geometry(p, q, prm, n=n, plan=plan)
-    return {"slp": lambda: (ft.slp_ewald(p, q, f, prm, plan=plan),),
-            "stokes": lambda: ft.stokes_ewald(p, q, f, f, n, prm, plan=plan),
-            "adjoint": lambda: ft.stokes_ewald_adjoint(p, q, f, f, n, f, f, prm, plan=plan),
-            "geometry": lambda: geo.apply(np.stack([f, 2 * f]), np.stack([f, 2 * f]))}
+    try:
+        return geo.apply(np.stack([f, 2 * f]), np.stack([f, 2 * f]))
+    finally:
+        geo.close()
 
 
 @pytest.mark.parametrize("N", [500, 40000])
 @pytest.mark.parametrize("op", ["slp", "stokes", "adjoint", "geometry"])
 def test_a_wait_that_runs_out(ft, op, N):
     plan = ft.Plan(0)
-    call = _calls(ft, plan, N)[op]
-    want = call()
+    want = _call(ft, plan, op, N)
     for polls in (0, 1, 0):
         plan.set_wait_limit(polls)
         try:
-            got = call()
+            got = _call(ft, plan, op, N)
             assert polls > 0                         # (it may have been fast enough)
             assert all(relerr(x, y) < 1e-11 for x, y in zip(got, want))
         except ft.Se2pError as e:
             assert e.code == 2 and "tensor-core" in str(e)
         plan.set_wait_limit()
-        got = call()
+        got = _call(ft, plan, op, N)
         assert all(relerr(x, y) < 1e-11 for x, y in zip(got, want))
+    plan.close()
+
+
+@pytest.mark.parametrize("op", ["slp", "adjoint"])
+def test_queued_calls(ft, op):
+    """On CUDA tensors the call has returned before its kernels run: its results are NaN,
+    and the plan's synchronize or its next call reports it, once."""
+    import torch
+    p, q, f, n = (torch.tensor(np.ascontiguousarray(x.T), device="cuda") for x in _cloud(5000, 8))
+    prm = ft.EwaldParams.derived(60.0, 12, 12, 192, 192, 24, 1.0, 1.0)
+    plan = ft.Plan(0)
+
+    def call():
+        if op == "slp":
+            return ft.slp_ewald(p, q, f, prm, parts=True, plan=plan)
+        return ft.stokes_ewald_adjoint(p, q, f, f, n, f, f, prm, plan=plan)
+
+    want = call()
+    plan.synchronize()
+    for ask in (plan.synchronize, call):
+        plan.set_wait_limit(0)
+        got = call()
+        torch.cuda.synchronize()
+        if op == "slp":
+            assert torch.isnan(got[0]).all() and torch.isnan(got[2]).all()
+            assert (got[1] - want[1]).abs().max() <= 1e-12 * want[1].abs().max()
+        else:
+            assert all(torch.isnan(g).all() for g in got)
+        plan.set_wait_limit()
+        with pytest.raises(ft.Se2pError, match="tensor-core"):
+            ask()
+        got = call()
+        plan.synchronize()
+        for x, y in zip(got, want):
+            assert relerr(x.cpu().numpy(), y.cpu().numpy()) < 1e-11
     plan.close()
 
 
