@@ -665,9 +665,12 @@ cudaError_t launch_fft_rows_ff(double2 *data, int64_t rows, const FftRowsFF &p, 
                                cudaStream_t st, int64_t &launches)
 {
     if (rows <= 0) return cudaSuccess;
-    const size_t smem = sizeof(f2) * 2 * ((size_t)(2 * sh_len(p.L) + 1) & ~(size_t)1);
+    auto bytes = [](int L) { return sizeof(f2) * 2 * ((size_t)(2 * sh_len(L) + 1) & ~(size_t)1); };
+    const size_t smem = bytes(p.L);
+    // (the limit is the process's, not the launch's: that of the longest row, so that
+    // another thread's call cannot lower it in between)
     cudaError_t e = cudaFuncSetAttribute(k_fft_rows_ff, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
+                                         (int)bytes(kFftFFMaxLen));
     if (e != cudaSuccess) return e;
     const int per_sm = (int)std::max<size_t>(1, (size_t)(200 * 1024) / (smem + 1024));
     const int64_t cap = (int64_t)sm_count() * per_sm;

@@ -1564,11 +1564,12 @@ cudaError_t launch_tc_points(const TcPrepArgs &b, int nset, const unsigned long 
 template <int NC, int NS>
 static cudaError_t spread_tc(const TcSpreadArgs &a, cudaStream_t st)
 {
-    const int bytes = tc_spread_smem(NS, a.P);
-    const cudaError_t e =
-        cudaFuncSetAttribute(k_spread_tc<NC, NS>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    // (the limit is the process's, not the launch's: that of the widest stencil, so that
+    // another thread's call cannot lower it in between)
+    const cudaError_t e = cudaFuncSetAttribute(k_spread_tc<NC, NS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               tc_spread_smem(NS, kTcMaxP));
     if (e != cudaSuccess) return e;
-    launch_chained(k_spread_tc<NC, NS>, 2 * sm_count(), kTcThreads, bytes, st, a);
+    launch_chained(k_spread_tc<NC, NS>, 2 * sm_count(), kTcThreads, tc_spread_smem(NS, a.P), st, a);
     return cudaGetLastError();
 }
 
