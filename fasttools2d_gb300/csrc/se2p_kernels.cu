@@ -413,14 +413,14 @@ __device__ __forceinline__ void nbhd_build(Nbhd &N, const RealArgs &a, int lane,
 // r2f within e (3 R + 2 e) + 3 u r2f; for the rest (r2f > 1.5 cut2) the same bound
 // relative to d leaves r2 > cut2 as long as e < R / 20.  Where that does not hold
 // (coordinates far outside the cell, or cut2 near the end of the FP32 range) every
-// candidate takes the exact test.
+// candidate takes the exact test, also one whose r2f is infinite: no r2f is at least NaN.
 __device__ __forceinline__ float2 cut_band(const Nbhd &N, float2 P, float cut2f)
 {
     const float R = 1.25f * sqrtf(cut2f);
     const float e = 0x1p-22f * (R + fmaxf(fabsf(P.x) + N.zmax.x, fabsf(P.y) + N.zmax.y));
     const float band = 1.1f * (e * (3.0f * R + 2.0f * e) + 0x1p-21f * R * R);
     const bool ok = e < 0.05f * R && cut2f > 1e-30f && cut2f < 1e30f;
-    return ok ? make_float2(cut2f - band, cut2f + band) : make_float2(-1.f, INFINITY);
+    return ok ? make_float2(cut2f - band, cut2f + band) : make_float2(-1.f, CUDART_NAN_F);
 }
 
 // A piece as the test of its candidates needs it (the same in every lane).
