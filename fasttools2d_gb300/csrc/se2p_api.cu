@@ -669,14 +669,14 @@ static int tc_set(se2p_plan pl, int which, const double2 *p, int64_t n, const Ar
     CKS(ensure_t(pl, which ? S_TGTILE : S_TCTILE, nz, &pa.tile));
     CKS(ensure_t(pl, which ? S_TGSTART : S_TCSTART, 2 * (size_t)ntile + 2, &start));
     CKS(ensure_t(pl, which ? S_TGLIST : S_TCLIST, nz, &t.list));
-    if (perm) CKS(ensure_t(pl, S_TCLTMP, 2 * nz, &ltmp));
+    if (perm) CKS(ensure_t(pl, S_TCLTMP, 4 * nz, &ltmp));   // (two for k_tc_order_long)
     CKS(ensure_t(pl, which ? S_TGITEMS : S_TCITEMS, std::min(nz, (size_t)ntile) + nz / kmax + 1, &t.items));
     pa.fac = fac;
     int *istart = start + ntile + 1;
     t.nitems = istart + ntile;
     t.ready = true;
-    o = TcSetArgs{pa, kmax, ntile, perm, start, istart, perm ? ltmp : t.list, perm ? ltmp + n : nullptr,
-                  t.list, t.items, t.nitems};
+    o = TcSetArgs{pa, kmax, ntile, perm, start, istart, perm ? ltmp + 2 * n : t.list, perm ? ltmp + 3 * n : nullptr,
+                  t.list, ltmp, t.items, t.nitems};
     return SE2P_OK;
 }
 

@@ -393,6 +393,7 @@ struct TcSetArgs {
     int *start, *istart;        // per tile: first slot, first item
     int *list, *key;            // slot -> point; with perm, slot -> caller's number
     int *ordered;               // with perm: list with the slots of long tiles in the caller's order
+    int *tmp;                   // with perm: room for ordering (2 n, 16-byte aligned)
     int4 *items;
     int *nitems;
 };

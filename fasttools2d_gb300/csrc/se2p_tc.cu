@@ -19,6 +19,7 @@
 #include <cuda_fp16.h>
 
 #include <algorithm>
+#include <climits>
 
 namespace se2p {
 
@@ -305,8 +306,20 @@ __global__ void __launch_bounds__(256) k_tc_list(TcPrepArgs b)
 // slots by counting smaller keys, the keys read through shared memory.
 // With nbound right-hand sides on the same sources the list serves them all, so it is
 // left unwritten only where none of their spreads will read it.
+// The ranking grows with the square of a tile's slots: beyond kOrderFrom sources
+// k_tc_order_long takes the tiles of more than kOrderLong.
+constexpr int kOrderLong = 4096, kOrderFrom = 1 << 16;
+
+__device__ __forceinline__ bool all_off(const unsigned long long *__restrict__ bound, int nbound, int bstride)
+{
+    if (bound[0] != kFixedOff) return false;
+    for (int r = 1; r < nbound; r++)
+        if (bound[(int64_t)r * bstride] != kFixedOff) return false;
+    return true;
+}
+
 __global__ void __launch_bounds__(256) k_tc_order(int64_t n, const int2 *__restrict__ tile,
-                                                  const int *__restrict__ start, int kmax,
+                                                  const int *__restrict__ start, int kmax, int longest,
                                                   const int *__restrict__ key,
                                                   const int *__restrict__ list,
                                                   int *__restrict__ out,
@@ -314,9 +327,7 @@ __global__ void __launch_bounds__(256) k_tc_order(int64_t n, const int2 *__restr
                                                   int nbound, int bstride)
 {
     chain_enter();
-    bool off = true;                                 // crowded: the FP64 spread runs instead
-    for (int r = 0; r < nbound; r++) off = off && bound[(int64_t)r * bstride] == kFixedOff;
-    if (off) return;
+    if (all_off(bound, nbound, bstride)) return;     // crowded: the FP64 spread runs instead
     __shared__ __align__(16) int ks[256];
     __shared__ int range[2];
     const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -331,7 +342,9 @@ __global__ void __launch_bounds__(256) k_tc_order(int64_t n, const int2 *__restr
         const int t = tile[j].x;
         a = start[t];
         b = start[t + 1];
-        if (b - a > kmax) {
+        if (b - a > longest) {
+            b = a;
+        } else if (b - a > kmax) {
             mine = key[k];
             atomicMin(&range[0], a);
             atomicMax(&range[1], b);
@@ -359,6 +372,105 @@ __global__ void __launch_bounds__(256) k_tc_order(int64_t n, const int2 *__restr
         __syncthreads();
     }
     if (b > a) out[a + r] = j;
+}
+
+// Tiles of more than kOrderLong slots (coarse grids, and sources without a density, which
+// the bound does not count as crowded), a block each: the keys, which are distinct, fall
+// into up to kOrderBins equal intervals between their least and their largest, and
+// are ranked within their interval.  tmp: room for the n slots' keys, then for their points.
+// Bound: latency of one block's passes over its tile.  Whole k-space calls, ranking by
+// squares alone against this: 2^17 sources of one tile, 50 of them with a density, 2.44
+// against 0.65 ms, 2^19 27.8 against 2.26; 2^20 uniform sources on 128^2 nodes, P = 4, 11.6
+// against 2.33 ms, on 256^2, P = 12, 3.46 against 2.07.  At the line both take the same (one
+// tile of 4096: 0.24 ms; of 8192: 0.27 against 0.25).  Its launch is 3 us of every call
+// (32,768 boundary points 484 against 487 us), so that up to kOrderFrom sources, 0.44
+// against 0.32 ms at most for 2^15, there is none.
+constexpr int kOrderThreads = 1024, kOrderLogBins = 13, kOrderBins = 1 << kOrderLogBins;
+
+__global__ void __launch_bounds__(kOrderThreads) k_tc_order_long(int64_t n, int ntile, const int *__restrict__ start,
+                                                                 const int *__restrict__ key,
+                                                                 const int *__restrict__ list,
+                                                                 int *__restrict__ out, int *tmp,
+                                                                 const unsigned long long *__restrict__ bound,
+                                                                 int nbound, int bstride)
+{
+    chain_enter();
+    if (all_off(bound, nbound, bstride)) return;
+    __shared__ int bins[kOrderBins], found[kOrderThreads], warp_tot[kOrderThreads / 32], nfound, klo, khi;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    for (int64_t t0 = blockIdx.x; t0 < ntile; t0 += (int64_t)gridDim.x * kOrderThreads) {
+        const int64_t t = t0 + (int64_t)tid * gridDim.x;
+        const bool mine = t < ntile && start[t + 1] - start[t] > kOrderLong;
+        if (!__syncthreads_or(mine)) continue;
+        if (tid == 0) nfound = 0;
+        __syncthreads();
+        if (mine) found[atomicAdd(&nfound, 1)] = (int)t;
+        __syncthreads();
+        for (int f = 0; f < nfound; f++) {
+            const int first = start[found[f]], end = start[found[f] + 1];
+            if (tid == 0) {
+                klo = 0x7fffffff;
+                khi = 0;
+            }
+            for (int q = tid; q < kOrderBins; q += kOrderThreads) bins[q] = 0;
+            __syncthreads();
+            int lo = 0x7fffffff, hi = 0;
+            for (int k = first + tid; k < end; k += kOrderThreads) {
+                lo = min(lo, key[k]);
+                hi = max(hi, key[k]);
+            }
+            lo = __reduce_min_sync(~0u, lo);
+            hi = __reduce_max_sync(~0u, hi);
+            if (lane == 0) {
+                atomicMin(&klo, lo);
+                atomicMax(&khi, hi);
+            }
+            __syncthreads();
+            const int base = klo, sh = max(0, 32 - kOrderLogBins - __clz(khi - klo));   // (hi - lo) >> sh < kOrderBins
+            for (int k = first + tid; k < end; k += kOrderThreads) atomicAdd(&bins[(key[k] - base) >> sh], 1);
+            __syncthreads();
+            // the bins' first places: an exclusive scan, kPer consecutive bins per thread
+            constexpr int kPer = kOrderBins / kOrderThreads;
+            int c[kPer], sum = 0;
+#pragma unroll
+            for (int q = 0; q < kPer; q++) sum += c[q] = bins[tid * kPer + q];
+            int inc = sum;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const int x = __shfl_up_sync(~0u, inc, d);
+                if (lane >= d) inc += x;
+            }
+            if (lane == 31) warp_tot[wid] = inc;
+            __syncthreads();
+            int run = first + inc - sum;
+            for (int w = 0; w < wid; w++) run += warp_tot[w];
+#pragma unroll
+            for (int q = 0; q < kPer; q++) {
+                bins[tid * kPer + q] = run;
+                run += c[q];
+            }
+            __syncthreads();
+            for (int k = first + tid; k < end; k += kOrderThreads) {
+                const int v = key[k], m = atomicAdd(&bins[(v - base) >> sh], 1);
+                tmp[m] = v;
+                tmp[n + m] = list[k];
+            }
+            __syncthreads();
+            // (a bin's word is now the end of its interval)
+            for (int k = first + tid; k < end; k += kOrderThreads) {
+                const int v = tmp[k], q = (v - base) >> sh, a = q ? bins[q - 1] : first, b = bins[q];
+                int r = a, m = a;
+                for (; m < b && (m & 3); m++) r += tmp[m] < v;
+                for (; m + 4 <= b; m += 4) {
+                    const int4 w = *reinterpret_cast<const int4 *>(tmp + m);
+                    r += (w.x < v) + (w.y < v) + (w.z < v) + (w.w < v);
+                }
+                for (; m < b; m++) r += tmp[m] < v;
+                out[r] = tmp[n + k];
+            }
+            __syncthreads();
+        }
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -1553,9 +1665,15 @@ cudaError_t launch_tc_points(const TcPrepArgs &b, int nset, const unsigned long 
     for (int k = 0; k < nset; k++) {
         const TcSetArgs &t = b.s[k];
         if (t.perm && t.a.n > 0) {
-            launch_chained(k_tc_order, (unsigned)((t.a.n + 255) / 256), 256, 0, st, t.a.n, t.a.tile, t.start, t.kmax, t.key,
-                                                                       t.list, t.ordered, bound, nbound, bstride);
+            const bool lg = t.a.n > kOrderFrom;
+            launch_chained(k_tc_order, (unsigned)((t.a.n + 255) / 256), 256, 0, st, t.a.n, t.a.tile, t.start, t.kmax,
+                           lg ? kOrderLong : INT_MAX, t.key, t.list, t.ordered, bound, nbound, bstride);
             launches++;
+            if (lg) {
+                launch_chained(k_tc_order_long, std::min(t.ntile, 2 * sm_count()), kOrderThreads, 0, st, t.a.n, t.ntile,
+                               t.start, t.key, t.list, t.ordered, t.tmp, bound, nbound, bstride);
+                launches++;
+            }
         }
     }
     return cudaGetLastError();
