@@ -649,6 +649,7 @@ static int tc_set(se2p_plan pl, int which, const double2 *p, int64_t n, const Ar
     pa.Lhy = g.Lhy;
     pa.h = g.h;
     pa.inv_h = 1.0 / g.h;
+    pa.near = std::max(0x1p-20, 1.1e-13 * pa.inv_h);   // (closest_node's snap: 1e-13)
     const double alpha = -g.a * g.h * g.h;
     pa.al2 = (unsigned long long)std::llround(std::ldexp(alpha * 1.4426950408889634074, 59));
     t.s = (unsigned long long)std::llround(std::ldexp(std::exp(-2.0 * alpha), 62)) << 2;

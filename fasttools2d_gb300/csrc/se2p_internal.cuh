@@ -376,6 +376,7 @@ struct TcPointArgs {
     const double2 *p;           // points
     int64_t n;
     double Lhx, Lhy, h, inv_h;
+    double near;                // nodes within which closest_node decides
     unsigned long long al2;     // alpha log2(e) in units of 2^-59, alpha = 2 xi^2 h^2 / eta
     int Mx, My, P;
     int Tx, Ty, ntx, nty;       // tile size in stencil origins, tiles per axis

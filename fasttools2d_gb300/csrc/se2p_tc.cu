@@ -143,9 +143,10 @@ __device__ __forceinline__ int tc_wrap(int i, int M)
 }
 
 // Stencil origin along one axis, and the offset from it in nodes as a fraction
-// of 2^64: closest_node's arithmetic wherever x lies within 2^-20 of a node,
-// elsewhere products with 1/h in place of its divisions (no decision is near).
-__device__ __forceinline__ bool tc_axis(double x, double Lh, double h, double inv_h, int half,
+// of 2^64: closest_node's arithmetic wherever x lies within `near` nodes of one (2^-20,
+// and more where h is so small that its snap at 1e-13 reaches farther), elsewhere
+// products with 1/h in place of its divisions (no decision is near).
+__device__ __forceinline__ bool tc_axis(double x, double Lh, double h, double inv_h, double near, int half,
                                         int &m, unsigned long long &u)
 {
     const double q = x * inv_h, fl = floor(q);
@@ -153,11 +154,11 @@ __device__ __forceinline__ bool tc_axis(double x, double Lh, double h, double in
     const double fr = q - fl, gr = t - ft;
     m = (int)ft - half;
     const double o = xsub(x, xmul(h, fl)) * inv_h;
-    // o 2^64 from the bit pattern (2^-20 < o < 1)
+    // o 2^64 from the bit pattern (2^-20 < o < 1 where it counts)
     const unsigned long long b = (unsigned long long)__double_as_longlong(o);
     u = ((b << 11) | (1ull << 63)) >> (1022 - (int)(b >> 52));
-    const double lo = 0x1p-20, hi = 1.0 - 0x1p-20;
-    return fr > lo && fr < hi && gr > lo && gr < hi && fabs(x) < 1e9 * h;
+    const double hi = 1.0 - near;
+    return fr > near && fr < hi && gr > near && gr < hi && fabs(x) < 1e9 * h;
 }
 
 // The factors X[i] = exp(-alpha (u - (i - P/2))^2), u in [0, 1) the offset in
@@ -192,8 +193,8 @@ __global__ void __launch_bounds__(256) k_tc_points(TcPrepArgs b)
     const double2 S = a.p[j];
     int mx, my;
     unsigned long long ux, uy;
-    const bool okx = tc_axis(S.x, a.Lhx, a.h, a.inv_h, a.P / 2, mx, ux);
-    const bool oky = tc_axis(S.y, a.Lhy, a.h, a.inv_h, a.P / 2, my, uy);
+    const bool okx = tc_axis(S.x, a.Lhx, a.h, a.inv_h, a.near, a.P / 2, mx, ux);
+    const bool oky = tc_axis(S.y, a.Lhy, a.h, a.inv_h, a.near, a.P / 2, my, uy);
     if (!(okx && oky)) {
         double px, py;
         closest_node(S.x, S.y, a.Lhx, a.Lhy, a.h, a.P, mx, my, px, py);
