@@ -2253,12 +2253,14 @@ static bool geom_multi_ok(se2p_geom g, int *kY_out, double *kfac_out, int *mult_
 // FP64 form (geom_multi_ok): coef holds nr blocks of nc coefficients per
 // sorted source (stride cstride doubles); uk receives per right-hand side r
 // the gathered sums at uk + r (nout / 2) nt, kind after kind, sorted target
-// order.  One spread launch covers all nr right-hand sides (each source's
-// stencil origin and Gaussian factors formed once), then each one's forward
-// transforms, filter and inverse transforms run into its own grids, and one
-// gather launch covers them all (each target's factors formed once).  A
-// right-hand side whose sources crowd too much for the integer sums, or whose
-// values are not finite, takes the FP64 spread or gather as in run().
+// order.  On the tensor cores (tc_ok, tg_ok) the points' records, tiles and
+// items are made once, and one spread and one gather launch per right-hand side
+// read them.  Otherwise one launch of k_spread_fix_multi and one of
+// k_gather_fix_multi cover all nr of them, each point's stencil origin and
+// Gaussian factors formed once.  In between, each one's forward transforms, filter
+// and inverse transforms run in its own grids.  A right-hand side whose sources
+// crowd too much for the integer sums, or whose values are not finite, takes
+// the FP64 spread or gather as in run(), whatever the others do.
 static int geom_kspace_multi(se2p_geom g, int nr, const double *coef, int64_t cstride,
                              cudaStream_t ks, double2 *uk)
 {

@@ -726,15 +726,6 @@ __device__ __forceinline__ int fix_shift(unsigned long long bits)
 // and kfac = mult 2^(2 kY).  When the bound slot ends up all ones the FP64
 // spread runs (launch it behind launch_spread_fix with a.bound set) and the
 // grids hold doubles.
-// Factor records, tiles and items of n points (kmax per item); with perm, tiles
-// of several items are put in the order of the caller's point numbers
-// (list_tmp then holds 2 n ints).
-// (a.count of the sets zeroed before)
-cudaError_t launch_tc_points(const TcPrepArgs &b, int nset, const unsigned long long *bound,
-                             int nbound, int bstride, cudaStream_t st, int64_t &launches);
-cudaError_t launch_gather_tc(const TcGatherArgs &a, int nc, cudaStream_t st, int64_t &launches);
-cudaError_t launch_gather_adj_tc(const TcGatherAdjArgs &a, cudaStream_t st, int64_t &launches);
-cudaError_t launch_spread_tc(const TcSpreadArgs &a, int nc, cudaStream_t st, int64_t &launches);
 int64_t spread_bound_words(int Mx, int My, int P);
 int64_t spread_bound_slot(int Mx, int My, int P);
 cudaError_t launch_spread_bound(const SpreadArgs &a, int nc, double kfac, int mult, double *ws,
@@ -752,6 +743,15 @@ cudaError_t launch_gather_fix_multi(const GatherArgs &a, int nc, int nr, int64_t
                                     int64_t ostride, cudaStream_t st, int64_t &launches);
 cudaError_t launch_gather_fp64_fallback(const GatherArgs &a, int nc, cudaStream_t st,
                                         int64_t &launches);
+// Tensor-core kernels (se2p_tc.cu).  launch_tc_points: records, tiles and items of
+// nset point sets (the sets' counts zeroed before); with perm, tiles of several items are
+// put in the order of the caller's point numbers, unless all nbound bound slots (bstride
+// words apart) leave the spreads of the set to the FP64 kernel.
+cudaError_t launch_tc_points(const TcPrepArgs &b, int nset, const unsigned long long *bound,
+                             int nbound, int bstride, cudaStream_t st, int64_t &launches);
+cudaError_t launch_spread_tc(const TcSpreadArgs &a, int nc, cudaStream_t st, int64_t &launches);
+cudaError_t launch_gather_tc(const TcGatherArgs &a, int nc, cudaStream_t st, int64_t &launches);
+cudaError_t launch_gather_adj_tc(const TcGatherAdjArgs &a, cudaStream_t st, int64_t &launches);
 cudaError_t launch_pack_fixed_pairs(const long long *grid, int nc, int64_t G,
                                     const unsigned long long *bound, double2 *z, cudaStream_t st,
                                     int64_t &launches);

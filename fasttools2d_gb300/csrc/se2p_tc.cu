@@ -743,6 +743,7 @@ template <int NC, int NS>
 __global__ void __launch_bounds__(kTcThreads, 2) k_spread_tc(TcSpreadArgs a)
 {
     chain_enter();
+    static_assert(NS == kTcDigits && NS == 7, "the epilogue combines levels 0 .. 6");
     constexpr int NG = (NC + 1) / 2;
     constexpr int kBK = NS * (kTcY / 8) * 128;       // B: bytes per 8 sources
     extern __shared__ __align__(128) char tc_smem[];

@@ -90,11 +90,14 @@ const char *se2p_version(void);
  *   - real space: the far pairs (1 < xi^2 r^2 < 64) in float-float arithmetic
  *     (pairs of FP32 values carrying about 48 bits); near pairs, the SLP self
  *     term and the exact cutoff decisions in FP64;
- *   - spread and gather: exact integer arithmetic -- every Gaussian factor
- *     rounded once to 62 bits, products as the high words of 64 x 64-bit
- *     integer products rounded to nearest, sums as exact int64 additions (the
- *     spread grid is bitwise reproducible); crowded grids or non-finite
- *     values fall back to the FP64 spread and gather;
+ *   - spread and gather: integer arithmetic.  On the tensor cores the 64-bit
+ *     fixed-point factors, strengths and grid values are cut into base-256 digits
+ *     and the leading seven digits' products summed exactly (off by 2^-56 of the
+ *     largest strength, 2^-53 of the largest grid value); for few points per grid
+ *     tile, and for Gaussians far narrower or flatter than the drivers' eta makes
+ *     them, products are the high words of 64 x 64-bit integers.  Sums are
+ *     exact int64 additions (the spread grid is bitwise reproducible); crowded
+ *     grids or non-finite values fall back to the FP64 spread and gather;
  *   - FFT: float-float mixed-radix row transforms (cuFFT Z2Z for lengths with
  *     prime factors above 7);
  *   - filter, DLP k=0 term and the final sums: FP64.
@@ -118,7 +121,8 @@ int se2p_plan_set_precision(se2p_plan plan, int precision);
  * Replaces the drivers' `verbose` tic/toc prints (StokesSLP_ewald_2p.m:106-131):
  * with timing on, every stage of every call (h2d, wrap, sort, coef, real,
  * spread, fft_fwd, filter, fft_inv, gather, zero_mode, assemble, d2h) is
- * bracketed by CUDA events on the plan's stream.  se2p_plan_stage_times
+ * bracketed by CUDA events on the plan's stream (the wrap is part of sort; its own
+ * stage counts no calls).  se2p_plan_stage_times
  * waits for the pending events and returns, per stage, the accumulated
  * milliseconds and call counts (arrays of se2p_num_stages() entries). */
 int se2p_plan_enable_timing(se2p_plan plan, int on);
